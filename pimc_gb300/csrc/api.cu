@@ -272,6 +272,8 @@ int pgb_create(const pgb_params* p, pgb_ctx** out) {
         if ((e = cudaMalloc(&c.d_prev, nb * sizeof(int2))) != cudaSuccess) break;
         if ((e = cudaMalloc(&c.d_on, nb)) != cudaSuccess) break;
         if ((e = cudaMalloc(&c.d_nbs, c.M * sizeof(int))) != cudaSuccess) break;
+        if (p->precision == PGB_FP64 && (p->gradvfactor[0] > kEPS || p->gradvfactor[1] > kEPS))
+            if ((e = cudaMalloc(&c.d_force64, nb * 3 * sizeof(double))) != cudaSuccess) break;
     } while (0);
     if (e != cudaSuccess) { rc = c.cuda_fail(e, "cudaMalloc(context)"); g_last_error = c.err; pgb_destroy(h); return rc; }
     // The table abscissae accumulate r += dr sequentially (potential.h:176-183);
@@ -305,6 +307,7 @@ int pgb_destroy(pgb_ctx* h) {
     if (c.d_scratch) cudaFree(c.d_scratch);
     if (c.d_tc_tables) cudaFree(c.d_tc_tables);
     if (c.d_force32) cudaFree(c.d_force32);
+    if (c.d_force64) cudaFree(c.d_force64);
     if (c.h_pinned) cudaFreeHost(c.h_pinned);
     if (c.stream) cudaStreamDestroy(c.stream);
     delete h;
@@ -556,8 +559,8 @@ int pgb_bead_actions(pgb_ctx* h, const int32_t* beads, int k, int shift, int mod
     const float4* fall = slice_forces(c, &rc);
     if (rc) return rc;
     cudaError_t e = (c.p.precision != PGB_MIXED)
-        ? launch_bead_actions64(v, d_b, k, shift, mode, c.p.tau, c.p.lambda,
-                                c.p.vfactor, c.p.gradvfactor, nullptr, d_o, c.stream)
+        ? launch_bead_actions64(v, d_b, k, shift, mode, c.p.tau, c.p.lambda, c.p.vfactor,
+                                c.p.gradvfactor, nullptr, c.d_force64, full_list(c), d_o, c.stream)
         : full_list(c)
         ? launch_bead_actions32_full(v, c.az, d_b, k, shift, mode, c.p.tau, c.p.lambda,
                                      c.p.vfactor, c.p.gradvfactor, nullptr, fall, 0, d_o, c.stream)
@@ -1079,11 +1082,15 @@ int trial_launch(Ctx& c, const int2* d_b, const double* d_pos, int k, int shift,
             e = launch_bead_actions32(v, c.az, d_b, k, shift, mode, c.p.tau, c.p.lambda, c.p.vfactor,
                                       c.p.gradvfactor, nullptr, d_old, c.stream);
     } else {
+        const bool whole = full_list(c);
+        if (whole && launch_trial_actions64(v, d_b, k, shift, mode, c.p.tau, c.p.lambda, c.p.vfactor,
+                                            c.p.gradvfactor, d_pos, c.d_force64, d_delta, c.stream, &e))
+            return e == cudaSuccess ? PGB_OK : c.cuda_fail(e, "trial actions launch");
         e = launch_bead_actions64(v, d_b, k, shift, mode, c.p.tau, c.p.lambda, c.p.vfactor,
-                                  c.p.gradvfactor, d_pos, d_new, c.stream);
+                                  c.p.gradvfactor, d_pos, c.d_force64, whole, d_new, c.stream);
         if (e == cudaSuccess)
             e = launch_bead_actions64(v, d_b, k, shift, mode, c.p.tau, c.p.lambda, c.p.vfactor,
-                                      c.p.gradvfactor, nullptr, d_old, c.stream);
+                                      c.p.gradvfactor, nullptr, c.d_force64, whole, d_old, c.stream);
     }
     if (e == cudaSuccess) {
         pgb::k_delta<<<(k + 255) / 256, 256, 0, c.stream>>>(d_new, d_old, d_delta, k);

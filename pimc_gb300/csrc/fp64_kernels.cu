@@ -3,7 +3,11 @@
 // Compiled with -fmad=false: every multiply and add rounds once, in the order
 // the reference writes it, so each pair term equals the oracle's bit for bit
 // and totals differ only through summation order (parallel reductions).
-#include "pgb_device.cuh"
+#include <cooperative_groups.h>
+
+#include "pair64.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace pgb {
 
@@ -116,16 +120,389 @@ cudaError_t launch_potential_batch64(const PathView& v, const double* d_sep,
     return cudaGetLastError();
 }
 
+// Sums of Q per-thread values over the CTA: all to shared memory, then one
+// warp a quantity, so that the twelve FP64 adds of a quantity run once and on
+// all four sub-partitions instead of in every warp.
+constexpr int kPairBlock = 256;
+
+template <int Q>
+__device__ __forceinline__ void block_sums(const double (&val)[Q], double (*buf)[kPairBlock], double* out) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __syncthreads();
+    #pragma unroll
+    for (int q = 0; q < Q; ++q) buf[q][tid] = val[q];
+    __syncthreads();
+    for (int q = warp; q < Q; q += kPairBlock / 32) {
+        double s = buf[q][lane];
+        #pragma unroll
+        for (int i = 1; i < kPairBlock / 32; ++i) s += buf[q][lane + 32 * i];
+        s = warp_sum(s);
+        if (lane == 0) out[q] = s;
+    }
+    __syncthreads();
+}
+
+// what a bead's action is made of, and its assembly (action.cpp:487-740)
+struct BeadSpec {
+    int shift, mode;
+    double tau, lambda, vf[2], gf[2];
+    __device__ __forceinline__ bool need_v() const { return mode != PGB_ACTION_CORR; }
+    __device__ __forceinline__ bool need_c(int s) const {
+        return gf[s % 2] > kEPS && (mode == PGB_ACTION_CORR || (mode == PGB_ACTION_FULL && shift == 1));
+    }
+    __device__ __forceinline__ double action(int s, double V, double T, double fx, double fy, double fz) const {
+        const double t = (double)shift * tau;
+        const double bareU = vf[s % 2] * t * V;
+        const double corU = need_c(s) ? gf[s % 2] * t * t * t * lambda * (T + (fx * fx + fy * fy + fz * fz)) : 0.0;
+        return mode == PGB_ACTION_BARE ? bareU : mode == PGB_ACTION_CORR ? corU : bareU + corU;
+    }
+};
+
+// True when a worm end lies on slice s, so that pair factors differ from 1
+__device__ __forceinline__ bool worm_on_slice(const PathView& v, int s) {
+    return s == v.worm[0] || s == v.worm[2] || s == v.worm[4] || s == v.worm[6];
+}
+
 // ---------------------------------------------------------------------------
-// Per-bead potential action, one CTA per bead.
+// Per-bead potential action, a cluster of CTAs per bead.
 //
 // Phase 1 builds the LookupTable interaction list of the bead (every active
 // bead of the same slice, other than itself, with |r2 - r1|^2 < rc^2;
-// lookuptable.cpp:464-516) in particle order, and sums Vnn
-// (action.cpp:1044-1060).  Phase 2 evaluates gradVnnSquared
-// (action.cpp:1282-1337): one thread per list member b2 accumulates
-// F3 = sum_{b3 in list, b3 != b2} gradV(r2 - r3) from shared memory.
+// lookuptable.cpp:464-516), sums Vnn (action.cpp:1044-1060) and keeps each
+// member's F2 = gradV(r2 - r1).  Phase 2 is gradVnnSquared
+// (action.cpp:1282-1337), T = sum_n |F2_n|^2 + 2 F2_n . F3_n with
+// F3_n = sum over the other members m of gradV(r_n - r_m).  gradV is odd, so
+//     sum_n F2_n . F3_n = sum_{n<m} gradV(r_n - r_m) . (F2_n - F2_m):
+// each pair of members once.  Pairs go to threads by offset around the list,
+// (n, n + o mod size), o <= size / 2, so neighbouring lanes read neighbouring
+// members; the cluster's CTAs take turns at them and the first one adds the
+// shares through distributed shared memory.
+//
+// Bound: the FP64 pipe, about 27 instructions a pair, 16 clocks of an SM a
+// warp instruction.  31 beads of a 64-particle GSF path (a bisection's range):
+// 173 us with one thread a member and every ordered pair in the direct form,
+// 15.6 us here; as trials 2 x 173 and 21.6 us.  kBoth evaluates the trial and the current position of the
+// bead over one pass of the members' pairs, and writes the difference.
 // ---------------------------------------------------------------------------
+constexpr int kMaxCluster = 8;
+
+// shared memory a list member takes
+constexpr int bead_pairs_bytes(bool both) { return (both ? 9 : 6) * (int)sizeof(double) + 3 * (int)sizeof(float); }
+
+template <bool kBoth>
+__global__ void __launch_bounds__(kPairBlock)
+k_bead_pairs64(PathView v, double invdr, const int2* __restrict__ beads, BeadSpec a, int csize,
+               const double* __restrict__ over, double* __restrict__ out) {
+    constexpr int Q = kBoth ? 10 : 5;
+    extern __shared__ double smem[];
+    const int Ne = v.Ne;
+    double *lx = smem, *ly = lx + Ne, *lz = ly + Ne;                     // members' positions
+    double *fx = lz + Ne, *fy = fx + Ne, *fz = fy + Ne;                  // F2 at the trial (or current) position
+    double *gx = fz + Ne, *gy = gx + Ne, *gz = gy + Ne;                  // F2 at the current position (kBoth)
+    float* ux = reinterpret_cast<float*>(kBoth ? gz + Ne : gx);          // box fractions
+    float *uy = ux + Ne, *uz = uy + Ne;
+    __shared__ double buf[Q][kPairBlock];
+    __shared__ double sums[Q], cross[2], share[kMaxCluster][2];
+    __shared__ int wcount[kPairBlock / 32];
+    __shared__ int s_total;
+
+    const int b = blockIdx.x / csize, rank = blockIdx.x - b * csize;
+    const int s = beads[b].x, p = beads[b].y;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    if (s < 0 || s >= v.M || p < 0 || p >= Ne || !v.on[(size_t)s * Ne + p]) {
+        if (tid == 0 && rank == 0) out[b] = 0.0;
+        return;                                  // the whole cluster
+    }
+    const bool need_v = a.need_v(), need_c = a.need_c(s);
+    if (!need_c && rank > 0) return;             // no shares: no cluster barrier below
+
+    const double* X = v.pos + (size_t)s * 3 * Ne;
+    const float4* P = v.pos32 + (size_t)s * Ne;
+    const float Ix = (float)v.sideInv[0], Iy = (float)v.sideInv[1], Iz = (float)v.sideInv[2];
+    // `over` (trial positions) replaces the bead's stored position
+    const double x1 = over ? over[3 * b] : X[p];
+    const double y1 = over ? over[3 * b + 1] : X[Ne + p];
+    const double z1 = over ? over[3 * b + 2] : X[2 * Ne + p];
+    const float u1 = box_fraction((float)x1, Ix), u2 = box_fraction((float)y1, Iy), u3 = box_fraction((float)z1, Iz);
+    double xo = 0.0, yo = 0.0, zo = 0.0;
+    float o1 = 0.f, o2 = 0.f, o3 = 0.f;
+    if (kBoth) {
+        xo = X[p]; yo = X[Ne + p]; zo = X[2 * Ne + p];
+        o1 = box_fraction((float)xo, Ix); o2 = box_fraction((float)yo, Iy); o3 = box_fraction((float)zo, Iz);
+    }
+    const bool worm = worm_on_slice(v, s);
+    const int st1 = worm ? bead_state(v, s, p) : 2;
+    if (tid == 0) s_total = 0;
+    __syncthreads();
+
+    // Vn Sn Fn(3) [Vo So Fo(3)]
+    double val[Q] = {};
+    for (int base = 0; base < Ne; base += kPairBlock) {
+        const int j = base + tid;
+        bool in = false;
+        double xj = 0.0, yj = 0.0, zj = 0.0, ax = 0.0, ay = 0.0, az = 0.0, bx = 0.0, by = 0.0, bz = 0.0;
+        float vx = 0.f, vy = 0.f, vz = 0.f;
+        if (j < Ne && j != p && v.on[(size_t)s * Ne + j]) {
+            xj = X[j]; yj = X[Ne + j]; zj = X[2 * Ne + j];
+            const float4 f = P[j];
+            vx = box_fraction(f.x, Ix); vy = box_fraction(f.y, Iy); vz = box_fraction(f.z, Iz);
+            // LookupTable stores sep = getSeparation(bead2, bead1) = r2 - r1
+            const Pair64 d = pair64(v, invdr, xj - x1, yj - y1, zj - z1, vx - u1, vy - u2, vz - u3);
+            in = d.r2 < v.rc2;
+            const double fac = worm ? pair_factor(st1, bead_state(v, s, j)) : 1.0;
+            if (in) {
+                if (need_v) val[0] += fac * table64(v.tV, d.k);
+                if (need_c) {
+                    const double g = table64(v.tdV, d.k) * d.y;
+                    ax = g * d.dx; ay = g * d.dy; az = g * d.dz;
+                    val[1] = __fma_rn(ax, ax, __fma_rn(ay, ay, __fma_rn(az, az, val[1])));
+                    val[2] -= ax; val[3] -= ay; val[4] -= az;
+                }
+            }
+            if (kBoth) {                         // whole lists: the same members, unless a position is not finite
+                const Pair64 e = pair64(v, invdr, xj - xo, yj - yo, zj - zo, vx - o1, vy - o2, vz - o3);
+                if (e.r2 < v.rc2) {
+                    in = true;
+                    if (need_v) val[Q - 5] += fac * table64(v.tV, e.k);
+                    if (need_c) {
+                        const double g = table64(v.tdV, e.k) * e.y;
+                        bx = g * e.dx; by = g * e.dy; bz = g * e.dz;
+                        val[Q - 4] = __fma_rn(bx, bx, __fma_rn(by, by, __fma_rn(bz, bz, val[Q - 4])));
+                        val[Q - 3] -= bx; val[Q - 2] -= by; val[Q - 1] -= bz;
+                    }
+                }
+            }
+        }
+        if (!need_c) continue;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (lane == 0) wcount[w] = __popc(m);
+        __syncthreads();
+        int off = s_total;
+        for (int i = 0; i < w; ++i) off += wcount[i];
+        if (in) {
+            const int q = off + __popc(m & ((1u << lane) - 1u));
+            lx[q] = xj; ly[q] = yj; lz[q] = zj;
+            fx[q] = ax; fy[q] = ay; fz[q] = az;
+            if (kBoth) { gx[q] = bx; gy[q] = by; gz[q] = bz; }
+            ux[q] = vx; uy[q] = vy; uz[q] = vz;
+        }
+        __syncthreads();
+        if (tid == 0) { int tot = 0; for (int i = 0; i < kPairBlock / 32; ++i) tot += wcount[i]; s_total += tot; }
+        __syncthreads();
+    }
+    double tn = 0.0, to = 0.0;
+    if (need_c) {
+        // the first CTA's shared memory is written below: it has started by then
+        if (csize > 1) cg::this_cluster().sync();
+        const int n = s_total;
+        double c[2] = {0.0, 0.0};
+        if (n > 1) {
+            const int half = (n - 1) / 2, total = n * half + (n % 2 ? 0 : n / 2);
+            const int stride = csize * kPairBlock, so = stride / n, si = stride - so * n;
+            int idx = rank * kPairBlock + tid;
+            int o = idx / n, i = idx - o * n;
+            ++o;
+            for (; idx < total; idx += stride) {
+                int j = i + o;
+                if (j >= n) j -= n;
+                const Pair64 d = pair64(v, invdr, lx[i] - lx[j], ly[i] - ly[j], lz[i] - lz[j], ux[i] - ux[j],
+                                        uy[i] - uy[j], uz[i] - uz[j]);
+                const double g = table64(v.tdV, d.k) * d.y;
+                c[0] = __fma_rn(g, __fma_rn(d.dx, fx[i] - fx[j], __fma_rn(d.dy, fy[i] - fy[j], d.dz * (fz[i] - fz[j]))), c[0]);
+                if (kBoth)
+                    c[1] = __fma_rn(g, __fma_rn(d.dx, gx[i] - gx[j], __fma_rn(d.dy, gy[i] - gy[j], d.dz * (gz[i] - gz[j]))), c[1]);
+                i += si; o += so;
+                if (i >= n) { i -= n; ++o; }
+            }
+        }
+        if (kBoth) block_sums<2>(c, buf, cross);
+        else { const double c1[1] = {c[0]}; block_sums<1>(c1, buf, cross); }
+        if (csize > 1) {
+            cg::cluster_group cl = cg::this_cluster();
+            if (tid < (kBoth ? 2 : 1)) cl.map_shared_rank(&share[0][0], 0)[2 * rank + tid] = cross[tid];
+            cl.sync();
+            if (rank > 0) return;
+            for (int r = 0; r < csize; ++r) { tn += share[r][0]; if (kBoth) to += share[r][1]; }
+        } else { tn = cross[0]; if (kBoth) to = cross[1]; }
+    }
+    block_sums<Q>(val, buf, sums);
+    if (tid == 0) {
+        double U = a.action(s, sums[0], sums[1] + 2.0 * tn, sums[2], sums[3], sums[4]);
+        if (kBoth) U -= a.action(s, sums[Q - 5], sums[Q - 4] + 2.0 * to, sums[Q - 3], sums[Q - 2], sums[Q - 1]);
+        out[b] = U;
+    }
+}
+
+// Same-slice forces F_b = sum over active b3 != b of gradV(r_b - r_b3) of the
+// slices whose action has a gradient term, [M][3][Ne].  One CTA per slice and
+// block of kForceRows beads, four (eight) threads a bead over the partners.
+constexpr int kForceRows = 64;
+
+__global__ void __launch_bounds__(kPairBlock)
+k_slice_forces64(PathView v, double invdr, int even, int odd, double* __restrict__ force) {
+    extern __shared__ double smem[];
+    const int s = blockIdx.y, Ne = v.Ne;
+    if (!(s % 2 ? odd : even)) return;
+    double *lx = smem, *ly = lx + Ne, *lz = ly + Ne;
+    float *ux = reinterpret_cast<float*>(lz + Ne), *uy = ux + Ne, *uz = uy + Ne;
+    __shared__ double acc[3][kPairBlock];
+    const float Ix = (float)v.sideInv[0], Iy = (float)v.sideInv[1], Iz = (float)v.sideInv[2];
+    for (int j = threadIdx.x; j < Ne; j += kPairBlock) {
+        const double* X = v.pos + (size_t)s * 3 * Ne;
+        const float4 f = v.pos32[(size_t)s * Ne + j];
+        lx[j] = X[j]; ly[j] = X[Ne + j]; lz[j] = X[2 * Ne + j];
+        ux[j] = box_fraction(f.x, Ix); uy[j] = box_fraction(f.y, Iy); uz[j] = box_fraction(f.z, Iz);
+    }
+    __syncthreads();
+    const int b0 = blockIdx.x * kForceRows, nb = min(kForceRows, Ne - b0);
+    const int rows = nb > 32 ? 64 : 32, parts = kPairBlock / rows;
+    const int r = threadIdx.x & (rows - 1), part = threadIdx.x / rows, i = b0 + r;
+    double Fx = 0.0, Fy = 0.0, Fz = 0.0;
+    if (r < nb && v.on[(size_t)s * Ne + i]) {
+        for (int j = part; j < Ne; j += parts) {
+            if (j == i || !v.on[(size_t)s * Ne + j]) continue;
+            const Pair64 d = pair64(v, invdr, lx[i] - lx[j], ly[i] - ly[j], lz[i] - lz[j], ux[i] - ux[j], uy[i] - uy[j],
+                                    uz[i] - uz[j]);
+            if (!(d.r2 < v.rc2)) continue;       // not finite: in no list
+            const double g = table64(v.tdV, d.k) * d.y;
+            Fx = __fma_rn(g, d.dx, Fx); Fy = __fma_rn(g, d.dy, Fy); Fz = __fma_rn(g, d.dz, Fz);
+        }
+    }
+    acc[0][threadIdx.x] = Fx; acc[1][threadIdx.x] = Fy; acc[2][threadIdx.x] = Fz;
+    __syncthreads();
+    if (part < 3 && r < nb) {                    // one part a component
+        double t = acc[part][r];
+        for (int q = 1; q < parts; ++q) t += acc[part][r + q * rows];
+        force[((size_t)s * 3 + part) * Ne + i] = t;
+    }
+}
+
+// 16 values a lane summed over the warp by recursive halving (16 adds instead
+// of 80): lane l returns the sum of value l / 2
+__device__ __forceinline__ double warp_sum16(double (&x)[16], int lane) {
+    #pragma unroll
+    for (int h = 8, o = 16; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = lane & o;
+        #pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const double give = up ? x[i] : x[i + h];
+            x[i] = (up ? x[i + h] : x[i]) + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    return x[0] + __shfl_xor_sync(0xffffffffu, x[0], 1);
+}
+
+// Many beads: one warp a bead, O(n) a bead, the inner sums of the gradient
+// term from the slice forces, F3_n = F_n - gradV(r_n - r_p) with r_p the
+// bead's stored position.  Needs lists that take in the whole slice.  Each
+// warp takes kWarpBeads beads in turn; the assembly runs one bead a lane.
+constexpr int kWarpBeads = 4;
+constexpr int kBlockBeads = kWarpBeads * kPairBlock / 32;
+
+template <bool kBoth>
+__global__ void __launch_bounds__(kPairBlock)
+k_bead_warp64(PathView v, double invdr, const int2* __restrict__ beads, int k, BeadSpec a,
+              const double* __restrict__ over, const double* __restrict__ force, double* __restrict__ out) {
+    __shared__ double part[kBlockBeads][11];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, Ne = v.Ne;
+    const float Ix = (float)v.sideInv[0], Iy = (float)v.sideInv[1], Iz = (float)v.sideInv[2];
+    auto active = [&](int2 b) {
+        return b.x >= 0 && b.x < v.M && b.y >= 0 && b.y < Ne && v.on[(size_t)b.x * Ne + b.y];
+    };
+    for (int r = 0; r < kWarpBeads; ++r) {
+        const int lb = warp * kWarpBeads + r;
+        const long long b = (long long)blockIdx.x * kBlockBeads + lb;
+        if (b >= k) break;
+        const int s = beads[b].x, p = beads[b].y;
+        if (!active(beads[b])) continue;
+        const bool need_v = a.need_v(), need_c = a.need_c(s);
+        const double* X = v.pos + (size_t)s * 3 * Ne;
+        const double* F = force + (size_t)s * 3 * Ne;
+        const float4* P = v.pos32 + (size_t)s * Ne;
+        const double xo = X[p], yo = X[Ne + p], zo = X[2 * Ne + p];
+        const float o1 = box_fraction((float)xo, Ix), o2 = box_fraction((float)yo, Iy), o3 = box_fraction((float)zo, Iz);
+        const double x1 = kBoth ? over[3 * b] : xo, y1 = kBoth ? over[3 * b + 1] : yo, z1 = kBoth ? over[3 * b + 2] : zo;
+        const float u1 = box_fraction((float)x1, Ix), u2 = box_fraction((float)y1, Iy), u3 = box_fraction((float)z1, Iz);
+        const bool worm = worm_on_slice(v, s);
+        const int st1 = worm ? bead_state(v, s, p) : 2;
+        double x[16] = {};                       // V T F(3) at the stored position, then at the trial one
+        for (int j = lane; j < Ne; j += 32) {
+            if (j == p || !v.on[(size_t)s * Ne + j]) continue;
+            const double xj = X[j], yj = X[Ne + j], zj = X[2 * Ne + j];
+            const float4 f = P[j];
+            const float vx = box_fraction(f.x, Ix), vy = box_fraction(f.y, Iy), vz = box_fraction(f.z, Iz);
+            const double fac = worm ? pair_factor(st1, bead_state(v, s, j)) : 1.0;
+            const Pair64 e = pair64(v, invdr, xj - xo, yj - yo, zj - zo, vx - o1, vy - o2, vz - o3);
+            Pair64 d = e;
+            if (kBoth) d = pair64(v, invdr, xj - x1, yj - y1, zj - z1, vx - u1, vy - u2, vz - u3);
+            const bool ine = e.r2 < v.rc2, ind = d.r2 < v.rc2;       // true unless a position is not finite
+            if (need_v) {
+                if (ine) x[0] += fac * table64(v.tV, e.k);
+                if (kBoth && ind) x[5] += fac * table64(v.tV, d.k);
+            }
+            if (need_c) {
+                double ex = 0.0, ey = 0.0, ez = 0.0;
+                if (ine) {
+                    const double g = table64(v.tdV, e.k) * e.y;
+                    ex = g * e.dx; ey = g * e.dy; ez = g * e.dz;
+                }
+                // |F2|^2 + 2 F2.F3 = F2 . (F2 + 2 F3), F3 without the bead's own term
+                const double hx = 2.0 * (F[j] - ex), hy = 2.0 * (F[Ne + j] - ey), hz = 2.0 * (F[2 * Ne + j] - ez);
+                x[1] = __fma_rn(ex, ex + hx, __fma_rn(ey, ey + hy, __fma_rn(ez, ez + hz, x[1])));
+                x[2] -= ex; x[3] -= ey; x[4] -= ez;
+                if (kBoth && ind) {
+                    const double g = table64(v.tdV, d.k) * d.y;
+                    const double tx = g * d.dx, ty = g * d.dy, tz = g * d.dz;
+                    x[6] = __fma_rn(tx, tx + hx, __fma_rn(ty, ty + hy, __fma_rn(tz, tz + hz, x[6])));
+                    x[7] -= tx; x[8] -= ty; x[9] -= tz;
+                }
+            }
+        }
+        const double t = warp_sum16(x, lane);
+        if (!(lane & 1) && lane < 20) part[lb][lane >> 1] = t;
+    }
+    __syncthreads();
+    const long long b = (long long)blockIdx.x * kBlockBeads + lane;
+    if (warp == 0 && b < k) {
+        double U = 0.0;
+        if (active(beads[b])) {
+            const int s = beads[b].x;
+            const double* q = part[lane];
+            U = a.action(s, q[0], q[1], q[2], q[3], q[4]);
+            if (kBoth) U = a.action(s, q[5], q[6], q[7], q[8], q[9]) - U;
+        }
+        out[b] = U;
+    }
+}
+
+// From kManyBeads on the warp form is the faster: below, it leaves warps idle
+// (a GSF call also needs the forces of all slices first).
+constexpr int kManyBeads = 1216;                 // two beads a sub-partition of 152 SMs
+
+template <bool kBoth>
+static cudaError_t bead_pairs64(const PathView& v, const int2* d_beads, int k, const BeadSpec& a, bool corr,
+                                const double* d_over, double* d_out, cudaStream_t s) {
+    const size_t smem = (size_t)v.Ne * bead_pairs_bytes(kBoth);
+    const cudaError_t ae = set_smem_limit(k_bead_pairs64<kBoth>, 200 * 1024);
+    if (ae != cudaSuccess) return ae;
+    int c = 1;
+    if (corr)
+        while (c < kMaxCluster && 2 * c * k <= 2 * 152) c *= 2;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)k * c);
+    cfg.blockDim = dim3(kPairBlock);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = c; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = c > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_bead_pairs64<kBoth>, v, 1.0 / v.dr, d_beads, a, c, d_over, d_out);
+}
+
+// The same with the list alone in shared memory, every ordered pair of members
+// in the direct form: for slices whose list and forces do not fit above.
 constexpr int kBeadBlock = 256;
 
 __global__ void __launch_bounds__(kBeadBlock)
@@ -239,19 +616,57 @@ k_bead_actions64(PathView v, const int2* __restrict__ beads, int k, int shift, i
     }
 }
 
+static bool has_corr(int shift, int mode, const double gf[2]) {
+    return (gf[0] > kEPS || gf[1] > kEPS) && (mode == PGB_ACTION_CORR || (mode == PGB_ACTION_FULL && shift == 1));
+}
+
+// The warp form: whole lists, many beads, and for a gradient term the forces
+// of one slice in shared memory.  Returns false when the call is not for it.
+static bool bead_warp64(const PathView& v, const int2* d_beads, int k, const BeadSpec& a, bool corr,
+                        const double* d_over, double* d_force, double* d_out, cudaStream_t s, cudaError_t* e) {
+    const size_t fsmem = (size_t)v.Ne * (3 * sizeof(double) + 3 * sizeof(float));
+    if (k < kManyBeads || (corr && (!d_force || fsmem > 200 * 1024))) return false;
+    if (corr) {
+        if ((*e = set_smem_limit(k_slice_forces64, 200 * 1024)) != cudaSuccess) return true;
+        k_slice_forces64<<<dim3((v.Ne + kForceRows - 1) / kForceRows, v.M), kPairBlock, fsmem, s>>>(
+            v, 1.0 / v.dr, a.gf[0] > kEPS, a.gf[1] > kEPS, d_force);
+    }
+    const int grid = (k + kBlockBeads - 1) / kBlockBeads;
+    if (d_over) k_bead_warp64<true><<<grid, kPairBlock, 0, s>>>(v, 1.0 / v.dr, d_beads, k, a, d_over, d_force, d_out);
+    else k_bead_warp64<false><<<grid, kPairBlock, 0, s>>>(v, 1.0 / v.dr, d_beads, k, a, nullptr, d_force, d_out);
+    *e = cudaGetLastError();
+    return true;
+}
+
 cudaError_t launch_bead_actions64(const PathView& v, const int2* d_beads, int k, int shift,
                                   int mode, double tau, double lambda, const double vf[2],
-                                  const double gf[2], const double* d_over, double* d_out,
-                                  cudaStream_t s) {
+                                  const double gf[2], const double* d_over, double* d_force, bool whole,
+                                  double* d_out, cudaStream_t s) {
     if (k <= 0) return cudaSuccess;
-    size_t smem = (size_t)v.Ne * (3 * sizeof(double) + sizeof(int));
-    {
-        const cudaError_t ae = set_smem_limit(k_bead_actions64, 200 * 1024);
-        if (ae != cudaSuccess) return ae;
-    }
+    const BeadSpec a{shift, mode, tau, lambda, {vf[0], vf[1]}, {gf[0], gf[1]}};
+    const bool corr = has_corr(shift, mode, gf);
+    cudaError_t e = cudaSuccess;
+    if (whole && !d_over && bead_warp64(v, d_beads, k, a, corr, nullptr, d_force, d_out, s, &e)) return e;
+    if ((size_t)v.Ne * bead_pairs_bytes(false) <= 200 * 1024)
+        return bead_pairs64<false>(v, d_beads, k, a, corr, d_over, d_out, s);
+    const size_t smem = (size_t)v.Ne * (3 * sizeof(double) + sizeof(int));
+    if ((e = set_smem_limit(k_bead_actions64, 200 * 1024)) != cudaSuccess) return e;
     k_bead_actions64<<<k, kBeadBlock, smem, s>>>(v, d_beads, k, shift, mode, tau, lambda,
                                                  vf[0], vf[1], gf[0], gf[1], d_over, d_out);
     return cudaGetLastError();
+}
+
+bool launch_trial_actions64(const PathView& v, const int2* d_beads, int k, int shift, int mode, double tau,
+                            double lambda, const double vf[2], const double gf[2], const double* d_over,
+                            double* d_force, double* d_out, cudaStream_t s, cudaError_t* e) {
+    *e = cudaSuccess;
+    if (k <= 0) return true;
+    const BeadSpec a{shift, mode, tau, lambda, {vf[0], vf[1]}, {gf[0], gf[1]}};
+    const bool corr = has_corr(shift, mode, gf);
+    if (bead_warp64(v, d_beads, k, a, corr, d_over, d_force, d_out, s, e)) return true;
+    if ((size_t)v.Ne * bead_pairs_bytes(true) > 200 * 1024) return false;
+    *e = bead_pairs64<true>(v, d_beads, k, a, corr, d_over, d_out, s);
+    return true;
 }
 
 // ---------------------------------------------------------------------------

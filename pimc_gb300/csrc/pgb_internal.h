@@ -83,6 +83,7 @@ struct Ctx {
     void* d_tc_tables = nullptr;   // split-BF16 DFT and cosine matrices of this M (built once)
     float4* d_force32 = nullptr;   // per-bead same-slice forces of the current configuration
     bool force_valid = false;      // cleared by every position change
+    double* d_force64 = nullptr;   // scratch of the FP64 many-bead form: slice forces [M][3][Ne]
     void* h_pinned = nullptr; size_t pinned_bytes = 0;
     // plain-form worm state: the LookupTable's per-slice lists of a single
     // grid box (their order decides swap pivots) and the Worm scalars
@@ -123,10 +124,20 @@ cudaError_t launch_build_tables(const double* d_r, int n, AzizParams az,
 cudaError_t launch_potential_batch64(const PathView& v, const double* d_sep,
                                      double* d_out, int n, int what,
                                      cudaStream_t s);
+// `whole`: the cutoff takes in every separation, so a bead's list is its whole
+// slice; d_force: room for the FP64 slice forces [M][3][Ne], needed from
+// kManyBeads beads on with a gradient term
 cudaError_t launch_bead_actions64(const PathView& v, const int2* d_beads, int k,
                                   int shift, int mode, double tau, double lambda,
                                   const double vf[2], const double gf[2],
-                                  const double* d_over, double* d_out, cudaStream_t s);
+                                  const double* d_over, double* d_force, bool whole,
+                                  double* d_out, cudaStream_t s);
+// U(d_over) - U(current) of every bead in one launch, for whole lists; false
+// when a slice is too large for it
+bool launch_trial_actions64(const PathView& v, const int2* d_beads, int k, int shift, int mode,
+                            double tau, double lambda, const double vf[2], const double gf[2],
+                            const double* d_over, double* d_force, double* d_out, cudaStream_t s,
+                            cudaError_t* e);
 cudaError_t launch_slice_terms64(const PathView& v, int window, int want_tmat,
                                  double* d_terms /* [8][M] */, cudaStream_t s);
 // maxR2 > 0: only beads with x^2 + y^2 < maxR2 (cylinder estimators)
