@@ -149,17 +149,31 @@ const float4* slice_forces(Ctx& c, int* rc) {
     return c.d_force32;
 }
 
-// per-slice terms, internal layout [9][M]: vint g2 r1 r2 d1 d2 kin xch kinprev
-int compute_terms(Ctx& c, std::vector<double>& h, bool want_tmat) {
+// The per-slice sums that an estimator reads, by the parity of the slice.
+struct TermsWanted {
+    int even, odd;               // kSliceNone .. kSliceT
+    bool window;                 // r1, r2, d1, d2, xch
+};
+// potential and, where the action has one, the gradient term
+TermsWanted want_action(const Ctx& c) {
+    return {c.p.gradvfactor[0] > kEPS ? kSliceF : kSliceV, c.p.gradvfactor[1] > kEPS ? kSliceF : kSliceV, false};
+}
+// the virial's: forces everywhere, the T matrix where the action has a gradient term
+TermsWanted want_virial(const Ctx& c) {
+    return {c.p.gradvfactor[0] > kEPS ? kSliceT : kSliceF, c.p.gradvfactor[1] > kEPS ? kSliceT : kSliceF, true};
+}
+
+// per-slice terms, internal layout [8][M]: vint g2 r1 r2 d1 d2 kin xch
+int compute_terms(Ctx& c, std::vector<double>& h, TermsWanted want) {
     int rc = need_path(c); if (rc) return rc;
-    size_t bytes = (size_t)8 * c.M * sizeof(double);
-    rc = c.ensure_scratch(bytes); if (rc) return rc;
-    double* d = static_cast<double*>(c.d_scratch);
     PathView v = c.view();
+    size_t bytes = (size_t)8 * c.M * sizeof(double);
+    rc = c.ensure_scratch(c.p.precision == PGB_MIXED ? bytes : slice_terms64_work(v)); if (rc) return rc;
+    double* d = static_cast<double*>(c.d_scratch);
     int window = c.p.virial_window > 0 ? c.p.virial_window : 5;
     cudaError_t e = (c.p.precision == PGB_MIXED)
         ? launch_slice_terms32(v, c.az, window, d, c.stream)
-        : launch_slice_terms64(v, window, want_tmat ? 1 : 0, d, c.stream);
+        : launch_slice_terms64(v, want.window ? window : 0, want.even, want.odd, c.d_arrived, d, c.stream);
     if (e != cudaSuccess) return c.cuda_fail(e, "slice terms launch");
     h.assign((size_t)8 * c.M, 0.0);
     PGB_CUDA(&c, cudaMemcpyAsync(h.data(), d, bytes, cudaMemcpyDeviceToHost, c.stream));
@@ -272,6 +286,8 @@ int pgb_create(const pgb_params* p, pgb_ctx** out) {
         if ((e = cudaMalloc(&c.d_prev, nb * sizeof(int2))) != cudaSuccess) break;
         if ((e = cudaMalloc(&c.d_on, nb)) != cudaSuccess) break;
         if ((e = cudaMalloc(&c.d_nbs, c.M * sizeof(int))) != cudaSuccess) break;
+        if ((e = cudaMalloc(&c.d_arrived, c.M * sizeof(unsigned))) != cudaSuccess) break;
+        if ((e = cudaMemsetAsync(c.d_arrived, 0, c.M * sizeof(unsigned), c.stream)) != cudaSuccess) break;
         if (p->precision == PGB_FP64 && (p->gradvfactor[0] > kEPS || p->gradvfactor[1] > kEPS))
             if ((e = cudaMalloc(&c.d_force64, nb * 3 * sizeof(double))) != cudaSuccess) break;
     } while (0);
@@ -308,6 +324,7 @@ int pgb_destroy(pgb_ctx* h) {
     if (c.d_tc_tables) cudaFree(c.d_tc_tables);
     if (c.d_force32) cudaFree(c.d_force32);
     if (c.d_force64) cudaFree(c.d_force64);
+    if (c.d_arrived) cudaFree(c.d_arrived);
     if (c.h_pinned) cudaFreeHost(c.h_pinned);
     if (c.stream) cudaStreamDestroy(c.stream);
     delete h;
@@ -603,7 +620,7 @@ int pgb_full_action(pgb_ctx* h, double* out) {
     if (check_ctx(h) || !out) return PGB_EINVAL;
     Ctx& c = h->c;
     std::vector<double> t;
-    int rc = compute_terms(c, t, false); if (rc) return rc;
+    int rc = compute_terms(c, t, want_action(c)); if (rc) return rc;
     double totU = 0.0, tt = c.p.tau;
     for (int s = 0; s < c.M; ++s) {
         int eo = s % 2;
@@ -619,7 +636,7 @@ int pgb_kinetic_action(pgb_ctx* h, double* out) {
     if (check_ctx(h) || !out) return PGB_EINVAL;
     Ctx& c = h->c;
     std::vector<double> t;
-    int rc = compute_terms(c, t, false); if (rc) return rc;
+    int rc = compute_terms(c, t, {kSliceNone, kSliceNone, false}); if (rc) return rc;
     // each link is counted from both of its beads (action.cpp:306-323)
     double totK = 0.0;
     for (int s = 0; s < c.M; ++s) totK += 2.0 * t[(size_t)6 * c.M + s];
@@ -631,8 +648,10 @@ int pgb_slice_terms_compute(pgb_ctx* h, pgb_slice_terms* o) {
     if (check_ctx(h) || !o) return PGB_EINVAL;
     Ctx& c = h->c;
     std::vector<double> t;
-    bool tm = (o->r2 || o->d2);
-    int rc = compute_terms(c, t, tm); if (rc) return rc;
+    const int level = (o->r2 || o->d2) ? kSliceT : (o->g2 || o->r1 || o->d1) ? kSliceF : o->vint ? kSliceV : kSliceNone;
+    // the window's chains go with the forces (xch)
+    const int least = o->xch ? std::max<int>(level, kSliceF) : level;
+    int rc = compute_terms(c, t, {least, least, o->r1 || o->r2 || o->d1 || o->d2 || o->xch}); if (rc) return rc;
     double* dst[8] = {o->vint, o->g2, o->r1, o->r2, o->d1, o->d2, o->kin, o->xch};
     for (int q = 0; q < 8; ++q)
         if (dst[q]) std::memcpy(dst[q], t.data() + (size_t)q * c.M, c.M * sizeof(double));
@@ -644,7 +663,7 @@ int pgb_energy(pgb_ctx* h, double out[9]) {
     if (check_ctx(h) || !out) return PGB_EINVAL;
     Ctx& c = h->c;
     std::vector<double> t;
-    int rc = compute_terms(c, t, false); if (rc) return rc;
+    int rc = compute_terms(c, t, want_action(c)); if (rc) return rc;
     const int M = c.M;
     const double tau = c.p.tau, lambda = c.p.lambda;
     const double* vint = t.data();
@@ -690,7 +709,7 @@ int pgb_virial(pgb_ctx* h, int quirk, double est[19]) {
     if (check_ctx(h) || !est) return PGB_EINVAL;
     Ctx& c = h->c;
     std::vector<double> t;
-    int rc = compute_terms(c, t, true); if (rc) return rc;
+    int rc = compute_terms(c, t, want_virial(c)); if (rc) return rc;
     const int M = c.M;
     const double* vint = t.data();
     const double* g2 = t.data() + M;

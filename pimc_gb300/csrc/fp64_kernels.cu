@@ -670,153 +670,226 @@ bool launch_trial_actions64(const PathView& v, const int2* d_beads, int k, int s
 }
 
 // ---------------------------------------------------------------------------
-// Per-slice terms of the estimators, one CTA per slice, one thread per bead
-// b1 < numBeadsAtSlice (looping when there are more beads than threads).
+// Per-slice terms of the estimators:
 //   vint: LocalAction::V(slice)            action.cpp:902-947 (i<j, sep r2-r1)
 //   g2:   gradVSquared(slice)              action.cpp:1188-1223
 //   r1,d1: rDOTgradUterm1/deltadotgradUterm1 sums (action.cpp:1446,1588)
 //   r2,d2: T-matrix terms of rDOTgradUterm2/deltadotgradUterm2 (1503,1700)
 //   kin:  sum |getVelocity|^2                path.h:189-203
 //   xch:  sum (r_{t+W}-r_t).(r_{t+1}-r_t)     estimator.cpp:1138-1152
-// Output layout: terms[q * M + t] for q = 0..7 in the order above.
+// Output layout: terms[q * M + t] for q = 0..7 in the order above; terms above
+// a slice's level (kSliceNone .. kSliceT) are 0.
+//
+// Bound: the FP64 pipe, 16 clocks of an SM a warp instruction.  A potential
+// alone takes each pair once (about 20 instructions); forces take each ordered
+// pair, because the sums belong to one bead: 64 beads a CTA, four (eight)
+// threads a bead over its partners, 24 instructions a pair, 39 with the T
+// matrix (one coefficient c1 = (V'' - |V'|/r)/r^2 on r r^T and |V'|/r on the
+// diagonal, where the direct form divides eighteen times).  The centroid
+// window's two chains of links run on two of those threads.  An energy and a
+// virial sample of 64 particles, 124 slices, primitive action: 2 x 586 us with
+// one thread a bead, everything computed in the direct form; 73 us together
+// here (the potential alone, then forces).
 // ---------------------------------------------------------------------------
-constexpr int kSliceBlock = 128;
+constexpr int kSliceRows = 64;
 
-__device__ __forceinline__ double3 pos64(const PathView& v, int s, int p) {
-    const double* X = v.pos + (size_t)s * 3 * v.Ne;
-    return make_double3(X[p], X[v.Ne + p], X[2 * v.Ne + p]);
+__device__ __forceinline__ double3 pos64(const PathView& v, int2 b) {
+    const double* X = v.pos + (size_t)b.x * 3 * v.Ne;
+    return make_double3(X[b.y], X[v.Ne + b.y], X[2 * v.Ne + b.y]);
 }
-__device__ __forceinline__ double3 sepb(const PathView& v, int2 a, int2 b) {
-    double3 ra = pos64(v, a.x, a.y), rb = pos64(v, b.x, b.y);
-    return make_double3(min_image(ra.x - rb.x, v.side[0], v.sideInv[0]),
-                        min_image(ra.y - rb.y, v.side[1], v.sideInv[1]),
-                        min_image(ra.z - rb.z, v.side[2], v.sideInv[2]));
+__device__ __forceinline__ float3 fraction64(const PathView& v, int2 b) {
+    const float4 f = v.pos32[(size_t)b.x * v.Ne + b.y];
+    return make_float3(box_fraction(f.x, (float)v.sideInv[0]), box_fraction(f.y, (float)v.sideInv[1]),
+                       box_fraction(f.z, (float)v.sideInv[2]));
 }
-__device__ __forceinline__ double3 velocity64(const PathView& v, int s, int p) {
-    int2 n = v.next[(size_t)s * v.Ne + p];
-    if (n.x == kXXX && n.y == kXXX) return make_double3(0.0, 0.0, 0.0);
-    return sepb(v, n, make_int2(s, p));
+// getSeparation(a, b) = r_a - r_b in the box (path.h:179-184)
+__device__ __forceinline__ double3 link64(const PathView& v, double3 a, float3 ua, double3 b, float3 ub) {
+    bool ok = true;
+    const double x = a.x - b.x, y = a.y - b.y, z = a.z - b.z;
+    double3 d = make_double3(image64(x, ua.x - ub.x, v.side[0], ok), image64(y, ua.y - ub.y, v.side[1], ok),
+                             image64(z, ua.z - ub.z, v.side[2], ok));
+    if (!ok)
+        d = make_double3(min_image(x, v.side[0], v.sideInv[0]), min_image(y, v.side[1], v.sideInv[1]),
+                         min_image(z, v.side[2], v.sideInv[2]));
+    return d;
 }
 
-__global__ void __launch_bounds__(kSliceBlock)
-k_slice_terms64(PathView v, int window, int want_tmat, double* __restrict__ terms) {
-    extern __shared__ double sm[];
-    const int s = blockIdx.x;
-    const int Ne = v.Ne;
-    const int n = v.nbs[s];
-    double* sx = sm;
-    double* sy = sx + Ne;
-    double* sz = sy + Ne;
-    __shared__ double red[kSliceBlock / 32];
-    const double* X = v.pos + (size_t)s * 3 * Ne;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        sx[j] = X[j]; sy[j] = X[Ne + j]; sz[j] = X[2 * Ne + j];
+// The sum over g < window of the displacement from a bead to its g-th
+// neighbour along `link`, the displacement to the window-th one and the first
+// step; an open end stops the walk.
+struct ChainSums { double3 sum, reach, step; };
+__device__ __forceinline__ ChainSums chain64(const PathView& v, const int2* __restrict__ link, int s, int p, int window) {
+    ChainSums c{};
+    int2 at = make_int2(s, p);
+    double3 r = pos64(v, at);
+    float3 u = fraction64(v, at);
+    for (int g = 0; g < window; ++g) {
+        c.sum.x += c.reach.x; c.sum.y += c.reach.y; c.sum.z += c.reach.z;
+        at = link[(size_t)at.x * v.Ne + at.y];
+        if (at.x < 0) break;
+        const double3 q = pos64(v, at);
+        const float3 w = fraction64(v, at);
+        const double3 d = link64(v, q, w, r, u);
+        c.reach.x += d.x; c.reach.y += d.y; c.reach.z += d.z;
+        if (g == 0) c.step = d;
+        r = q; u = w;
+    }
+    return c;
+}
+
+// one slice's row block with forces (and the T matrix): adds to the thread's
+// vint g2 r1 r2 d1 d2 kin xch
+template <bool kT>
+__device__ __forceinline__ void slice_rows64(const PathView& v, double invdr, int s, int n, int b0, int window,
+                                             const double* lx, const double* ly, const double* lz,
+                                             double (*buf)[kPairBlock], double (&val)[8]) {
+    constexpr int Q = kT ? 10 : 3;
+    const int nb = min(kSliceRows, n - b0);
+    if (nb <= 0) return;                                        // uniform over the CTA
+    const int rows = nb > 32 ? 64 : 32, parts = kPairBlock / rows, tid = threadIdx.x;
+    const int r = tid & (rows - 1), part = tid / rows, i = b0 + r;
+    const float4* P = v.pos32 + (size_t)s * v.Ne;
+    const float Ix = (float)v.sideInv[0], Iy = (float)v.sideInv[1], Iz = (float)v.sideInv[2];
+    const bool worm = worm_on_slice(v, s);
+    // F(3), T: xx yy zz xy xz yz and the diagonal's sum
+    double acc[10] = {};
+    if (r < nb) {
+        const double x1 = lx[i], y1 = ly[i], z1 = lz[i];
+        const float4 f = P[i];
+        const float u1 = box_fraction(f.x, Ix), u2 = box_fraction(f.y, Iy), u3 = box_fraction(f.z, Iz);
+        const int st1 = worm ? bead_state(v, s, i) : 2;
+        for (int j = part; j < n; j += parts) {
+            if (j == i) continue;
+            const float4 q = P[j];
+            const Pair64 d = pair64(v, invdr, x1 - lx[j], y1 - ly[j], z1 - lz[j], u1 - box_fraction(q.x, Ix),
+                                    u2 - box_fraction(q.y, Iy), u3 - box_fraction(q.z, Iz));
+            const double dV = table64(v.tdV, d.k), g = dV * d.y;
+            acc[0] = __fma_rn(g, d.dx, acc[0]); acc[1] = __fma_rn(g, d.dy, acc[1]); acc[2] = __fma_rn(g, d.dz, acc[2]);
+            if (j > i) val[0] += (worm ? pair_factor(st1, bead_state(v, s, j)) : 1.0) * table64(v.tV, d.k);
+            if (kT) {
+                const double c0 = fabs(g), c1 = (table64(v.td2V, d.k) - c0) * (d.y * d.y);
+                const double tx = c1 * d.dx, ty = c1 * d.dy, tz = c1 * d.dz;
+                acc[3] = __fma_rn(tx, d.dx, acc[3] + c0); acc[4] = __fma_rn(ty, d.dy, acc[4] + c0);
+                acc[5] = __fma_rn(tz, d.dz, acc[5] + c0);
+                acc[6] = __fma_rn(tx, d.dy, acc[6]); acc[7] = __fma_rn(tx, d.dz, acc[7]); acc[8] = __fma_rn(ty, d.dz, acc[8]);
+            }
+        }
+    }
+    // the bead's neighbours along its worldline: forward on its first thread,
+    // backward on its second
+    ChainSums c{};
+    if (r < nb && part < 2 && window > 0) c = chain64(v, part ? v.prev : v.next, s, i, window);
+    __syncthreads();
+    #pragma unroll
+    for (int q = 0; q < Q; ++q) buf[q][tid] = acc[q];
+    if (part == 1) { buf[Q][r] = c.sum.x; buf[Q][64 + r] = c.sum.y; buf[Q][128 + r] = c.sum.z; }
+    __syncthreads();
+    for (int q = part; q < Q; q += parts) {                     // every part adds some of the quantities
+        double t = buf[q][r];
+        for (int k = 1; k < parts; ++k) t += buf[q][r + k * rows];
+        buf[q][r] = t;
     }
     __syncthreads();
-
-    double a_vint = 0, a_g2 = 0, a_r1 = 0, a_r2 = 0, a_d1 = 0, a_d2 = 0, a_kin = 0, a_xch = 0;
-    for (int b1 = threadIdx.x; b1 < n; b1 += blockDim.x) {
-        const double x1 = sx[b1], y1 = sy[b1], z1 = sz[b1];
-        const int st1 = bead_state(v, s, b1);
-        double3 F = make_double3(0.0, 0.0, 0.0);
-        double T[3][3] = {{0,0,0},{0,0,0},{0,0,0}};
-        for (int b2 = 0; b2 < n; ++b2) {
-            if (b2 == b1) continue;
-            double3 rD = make_double3(min_image(x1 - sx[b2], v.side[0], v.sideInv[0]),
-                                      min_image(y1 - sy[b2], v.side[1], v.sideInv[1]),
-                                      min_image(z1 - sz[b2], v.side[2], v.sideInv[2]));
-            double3 g = gradV64(v, rD);
-            F.x += g.x; F.y += g.y; F.z += g.z;
-            if (want_tmat) {
-                double rmag = sqrt(dot3(rD, rD));
-                double dVi = sqrt(dot3(g, g));
-                double g2Vi = grad2V64(v, rD);
-                double dV = dVi + 0.0;
-                double d2V = g2Vi + 0.0;
-                double r3 = pow(rmag, 3);
-                double rr[3] = {rD.x, rD.y, rD.z};
-                #pragma unroll
-                for (int a = 0; a < 3; ++a)
-                    #pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        T[a][c] += rr[a]*rr[c]*d2V/(rmag*rmag) - rr[a]*rr[c]*dV/r3;
-                        if (a == c) T[a][c] += dV/rmag;
-                    }
-            }
-            if (b2 > b1) {
-                // V(slice) uses sep = getSeparation(bead2, bead1) = r2 - r1
-                double3 d21 = make_double3(min_image(sx[b2] - x1, v.side[0], v.sideInv[0]),
-                                           min_image(sy[b2] - y1, v.side[1], v.sideInv[1]),
-                                           min_image(sz[b2] - z1, v.side[2], v.sideInv[2]));
-                a_vint += pair_factor(st1, bead_state(v, s, b2)) * V64(v, d21);
-            }
-        }
-        double3 r1v = make_double3(x1, y1, z1);
-        a_g2 += dot3(F, F);
-        a_r1 += dot3(F, r1v);
-        double3 TF = make_double3(0.0, 0.0, 0.0);
-        if (want_tmat) {
-            double ip0 = 0.0; ip0 += T[0][0]*F.x; ip0 += T[0][1]*F.y; ip0 += T[0][2]*F.z;
-            double ip1 = 0.0; ip1 += T[1][0]*F.x; ip1 += T[1][1]*F.y; ip1 += T[1][2]*F.z;
-            double ip2 = 0.0; ip2 += T[2][0]*F.x; ip2 += T[2][1]*F.y; ip2 += T[2][2]*F.z;
-            TF = make_double3(0.0 + ip0, 0.0 + ip1, 0.0 + ip2);
-            a_r2 += dot3(TF, r1v);
-        }
-        // centroid deviation delta (action.cpp:1625-1645)
-        if (window > 0) {
-            double3 rm_ = make_double3(0,0,0), rl_ = make_double3(0,0,0), com = make_double3(0,0,0);
-            int2 bn = make_int2(s, b1), bp = make_int2(s, b1);
-            int2 nOld = bn, pOld = bp;
-            for (int gm = 0; gm < window; ++gm) {
-                // next(bead1, gamma) / prev(bead1, gamma)
-                int2 cn = make_int2(s, b1), cp = make_int2(s, b1);
-                for (int q = 0; q < gm; ++q) cn = v.next[(size_t)cn.x * Ne + cn.y];
-                for (int q = 0; q < gm; ++q) cp = v.prev[(size_t)cp.x * Ne + cp.y];
-                double3 a = sepb(v, cn, nOld), c = sepb(v, cp, pOld);
-                rm_.x += a.x; rm_.y += a.y; rm_.z += a.z;
-                rl_.x += c.x; rl_.y += c.y; rl_.z += c.z;
-                com.x += (x1 + rm_.x) + (x1 + rl_.x);
-                com.y += (y1 + rm_.y) + (y1 + rl_.y);
-                com.z += (z1 + rm_.z) + (z1 + rl_.z);
-                nOld = cn; pOld = cp;
-            }
-            double den = 2.0 * window;
-            double3 dl = make_double3(min_image(x1 - com.x / den, v.side[0], v.sideInv[0]),
-                                      min_image(y1 - com.y / den, v.side[1], v.sideInv[1]),
-                                      min_image(z1 - com.z / den, v.side[2], v.sideInv[2]));
-            a_d1 += dot3(F, dl);
-            if (want_tmat) a_d2 += dot3(TF, dl);
-            // virial exchange term: vel1 = sum_{g=1..W} sep(next^g, next^{g-1})
-            double3 vel1 = make_double3(0,0,0);
-            int2 o = make_int2(s, b1), c2 = o;
-            for (int gm = 1; gm <= window; ++gm) {
-                c2 = v.next[(size_t)c2.x * Ne + c2.y];
-                double3 a = sepb(v, c2, o);
-                vel1.x += a.x; vel1.y += a.y; vel1.z += a.z;
-                o = c2;
-            }
-            double3 vel2 = velocity64(v, s, b1);
-            a_xch += dot3(vel1, vel2);
-        }
-        double3 vel = velocity64(v, s, b1);
-        a_kin += dot3(vel, vel);
-    }
-    double vals[8] = {a_vint, a_g2, a_r1, a_r2, a_d1, a_d2, a_kin, a_xch};
-    #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        double t = block_sum(vals[q], red);
-        if (threadIdx.x == 0) terms[(size_t)q * v.M + s] = t;
+    if (r >= nb || part) return;
+    const double Fx = buf[0][r], Fy = buf[1][r], Fz = buf[2][r];
+    const double x1 = lx[i], y1 = ly[i], z1 = lz[i];
+    val[1] = __fma_rn(Fx, Fx, __fma_rn(Fy, Fy, Fz * Fz));
+    if (window <= 0) return;
+    val[2] = __fma_rn(Fx, x1, __fma_rn(Fy, y1, Fz * z1));
+    // centroid deviation delta = r - com, com the mean of the window's two
+    // walks (action.cpp:1625-1645)
+    const double den = -1.0 / (2.0 * window);
+    const double ex = min_image((c.sum.x + buf[Q][r]) * den, v.side[0], v.sideInv[0]);
+    const double ey = min_image((c.sum.y + buf[Q][64 + r]) * den, v.side[1], v.sideInv[1]);
+    const double ez = min_image((c.sum.z + buf[Q][128 + r]) * den, v.side[2], v.sideInv[2]);
+    val[4] = __fma_rn(Fx, ex, __fma_rn(Fy, ey, Fz * ez));
+    val[7] = __fma_rn(c.reach.x, c.step.x, __fma_rn(c.reach.y, c.step.y, c.reach.z * c.step.z));
+    if (kT) {
+        const double a = buf[6][r], b = buf[7][r], e = buf[8][r];
+        const double TFx = __fma_rn(buf[3][r], Fx, __fma_rn(a, Fy, b * Fz));
+        const double TFy = __fma_rn(a, Fx, __fma_rn(buf[4][r], Fy, e * Fz));
+        const double TFz = __fma_rn(b, Fx, __fma_rn(e, Fy, buf[5][r] * Fz));
+        val[3] = __fma_rn(TFx, x1, __fma_rn(TFy, y1, TFz * z1));
+        val[5] = __fma_rn(TFx, ex, __fma_rn(TFy, ey, TFz * ez));
     }
 }
 
-cudaError_t launch_slice_terms64(const PathView& v, int window, int want_tmat,
-                                 double* d_terms, cudaStream_t s) {
-    size_t smem = (size_t)v.Ne * 3 * sizeof(double);
-    {
-        const cudaError_t ae = set_smem_limit(k_slice_terms64, 200 * 1024);
-        if (ae != cudaSuccess) return ae;
+// blocks of a slice: row blocks of kSliceRows beads; with several, each leaves
+// its eight sums in `part` and the last to arrive adds them in block order
+__global__ void __launch_bounds__(kPairBlock)
+k_slice_terms64(PathView v, double invdr, int window, int even, int odd, unsigned* __restrict__ arrived,
+                double* __restrict__ part, double* __restrict__ terms) {
+    extern __shared__ double sm[];
+    __shared__ double buf[11][kPairBlock];
+    __shared__ double sums[8];
+    __shared__ bool last;
+    const int s = blockIdx.y, Ne = v.Ne, n = v.nbs[s], tid = threadIdx.x, nblk = gridDim.x;
+    const int level = s % 2 ? odd : even, b0 = blockIdx.x * kSliceRows;
+    double *lx = sm, *ly = lx + Ne, *lz = ly + Ne;
+    if (level > kSliceNone) {
+        const double* X = v.pos + (size_t)s * 3 * Ne;
+        for (int j = tid; j < n; j += kPairBlock) { lx[j] = X[j]; ly[j] = X[Ne + j]; lz[j] = X[2 * Ne + j]; }
+        __syncthreads();
     }
-    k_slice_terms64<<<v.M, kSliceBlock, smem, s>>>(v, window, want_tmat, d_terms);
+    double val[8] = {};
+    if (level == kSliceT) slice_rows64<true>(v, invdr, s, n, b0, window, lx, ly, lz, buf, val);
+    else if (level == kSliceF) slice_rows64<false>(v, invdr, s, n, b0, window, lx, ly, lz, buf, val);
+    else if (level == kSliceV && n > 1) {
+        // each pair once, by offset around the slice (as in k_bead_pairs64)
+        const float4* P = v.pos32 + (size_t)s * Ne;
+        const float Ix = (float)v.sideInv[0], Iy = (float)v.sideInv[1], Iz = (float)v.sideInv[2];
+        const bool worm = worm_on_slice(v, s);
+        const int half = (n - 1) / 2, total = n * half + (n % 2 ? 0 : n / 2);
+        const int stride = nblk * kPairBlock, so = stride / n, si = stride - so * n;
+        int idx = blockIdx.x * kPairBlock + tid;
+        int o = idx / n, i = idx - o * n;
+        ++o;
+        for (; idx < total; idx += stride) {
+            int j = i + o;
+            if (j >= n) j -= n;
+            const float4 a = P[i], b = P[j];
+            const Pair64 d = pair64(v, invdr, lx[i] - lx[j], ly[i] - ly[j], lz[i] - lz[j],
+                                    box_fraction(a.x, Ix) - box_fraction(b.x, Ix), box_fraction(a.y, Iy) - box_fraction(b.y, Iy),
+                                    box_fraction(a.z, Iz) - box_fraction(b.z, Iz));
+            val[0] += (worm ? pair_factor(bead_state(v, s, i), bead_state(v, s, j)) : 1.0) * table64(v.tV, d.k);
+            i += si; o += so;
+            if (i >= n) { i -= n; ++o; }
+        }
+    }
+    if (tid < kSliceRows && b0 + tid < n) {
+        const int2 at = make_int2(s, b0 + tid), nx = v.next[(size_t)s * Ne + at.y];
+        if (nx.x >= 0) {
+            const double3 d = link64(v, pos64(v, nx), fraction64(v, nx), pos64(v, at), fraction64(v, at));
+            val[6] = __fma_rn(d.x, d.x, __fma_rn(d.y, d.y, d.z * d.z));
+        }
+    }
+    block_sums<8>(val, buf, sums);
+    if (nblk == 1) {
+        if (tid < 8) terms[(size_t)tid * v.M + s] = sums[tid];
+        return;
+    }
+    if (tid < 8) { part[((size_t)s * nblk + blockIdx.x) * 8 + tid] = sums[tid]; __threadfence(); }
+    __syncthreads();
+    if (tid == 0) last = atomicInc(arrived + s, nblk - 1) == nblk - 1;      // back to 0 for the next call
+    __syncthreads();
+    if (!last || tid >= 8) return;
+    __threadfence();
+    double t = 0.0;
+    for (int k = 0; k < nblk; ++k) t += __ldcg(part + ((size_t)s * nblk + k) * 8 + tid);
+    terms[(size_t)tid * v.M + s] = t;
+}
+
+static int slice_blocks(int Ne) { return (Ne + kSliceRows - 1) / kSliceRows; }
+
+size_t slice_terms64_work(const PathView& v) { return (size_t)8 * v.M * (1 + slice_blocks(v.Ne)) * sizeof(double); }
+
+cudaError_t launch_slice_terms64(const PathView& v, int window, int even, int odd, unsigned* d_arrived,
+                                 double* d_terms, cudaStream_t s) {
+    const size_t smem = (size_t)v.Ne * 3 * sizeof(double);
+    const cudaError_t ae = set_smem_limit(k_slice_terms64, 200 * 1024);
+    if (ae != cudaSuccess) return ae;
+    k_slice_terms64<<<dim3(slice_blocks(v.Ne), v.M), kPairBlock, smem, s>>>(
+        v, 1.0 / v.dr, window, even, odd, d_arrived, d_terms + (size_t)8 * v.M, d_terms);
     return cudaGetLastError();
 }
 

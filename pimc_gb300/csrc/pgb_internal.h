@@ -83,6 +83,7 @@ struct Ctx {
     void* d_tc_tables = nullptr;   // split-BF16 DFT and cosine matrices of this M (built once)
     float4* d_force32 = nullptr;   // per-bead same-slice forces of the current configuration
     bool force_valid = false;      // cleared by every position change
+    unsigned* d_arrived = nullptr; // per-slice counters of the FP64 slice terms (zero between calls)
     double* d_force64 = nullptr;   // scratch of the FP64 many-bead form: slice forces [M][3][Ne]
     void* h_pinned = nullptr; size_t pinned_bytes = 0;
     // plain-form worm state: the LookupTable's per-slice lists of a single
@@ -138,8 +139,14 @@ bool launch_trial_actions64(const PathView& v, const int2* d_beads, int k, int s
                             double tau, double lambda, const double vf[2], const double gf[2],
                             const double* d_over, double* d_force, double* d_out, cudaStream_t s,
                             cudaError_t* e);
-cudaError_t launch_slice_terms64(const PathView& v, int window, int want_tmat,
-                                 double* d_terms /* [8][M] */, cudaStream_t s);
+// What a slice's terms are asked for: nothing of its pairs, their potential,
+// with forces (g2, r1, d1), with the T matrix (r2, d2)
+enum { kSliceNone = -1, kSliceV = 0, kSliceF = 1, kSliceT = 2 };
+// d_terms: slice_terms64_work(v) bytes, the first [8][M] the result; d_arrived:
+// M counters, zero between calls; window <= 0: no r1, r2, d1, d2, xch
+size_t slice_terms64_work(const PathView& v);
+cudaError_t launch_slice_terms64(const PathView& v, int window, int even, int odd, unsigned* d_arrived,
+                                 double* d_terms, cudaStream_t s);
 // maxR2 > 0: only beads with x^2 + y^2 < maxR2 (cylinder estimators)
 cudaError_t launch_rhoq64(const PathView& v, const double* d_q, int nq,
                           double* d_rho /* [q][M][2] */, cudaStream_t s, double maxR2 = 0.0);

@@ -56,3 +56,25 @@ def test_beads_outside_the_box_take_the_direct_form(pgb, oracle_lib, shift_box):
     beads = np.array([[0, 0], [0, 1], [0, 19], [1, 0]], np.int32)
     got, _ = a.bead_actions(beads)
     assert rel_err(got, [o.bead_action(int(s), int(p)) for s, p in beads]) <= 1e-12
+
+
+@pytest.mark.parametrize("n,m", [(2, 4), (32, 6), (33, 6), (64, 6), (65, 8), (129, 6)])
+@pytest.mark.parametrize("action", ["primitive", "gsf", "li_broughton"])
+def test_slice_terms_row_blocks(pgb, oracle_lib, n, m, action):
+    """Row blocks of 32 and 64 beads, several blocks a slice, the levels that
+    the energy, the full action and the virial ask for (1e-11 for the virial's
+    products of sums, as elsewhere), twice: the arrival counters return to 0."""
+    L = 2.9 * n ** (1.0 / 3.0)
+    cfg = pgb.worldlines.seeded_worldlines(n, m, L, 6.0596, 0.004, 7 + n)
+    if n > 8:
+        cfg = pgb.worldlines.permute(cfg, [(1, 4), (2, 5, 7)])
+    a, o = make_pair(pgb, oracle_lib, cfg, L, m, n, 0.004, 6.0596, action=action, mu=-3.0)
+    for _ in range(2):
+        assert rel_err(a.energy(), o.energy()) <= 1e-12
+        assert rel_err(a.virial(), o.virial()) <= 1e-11
+        assert abs(a.full_action() - o.full_action()) <= 1e-12 * max(1.0, abs(o.full_action()))
+        assert abs(a.kinetic_action() - o.kinetic_action()) <= 1e-12 * max(1.0, abs(o.kinetic_action()))
+    t = a.slice_terms()
+    for s in range(m):
+        assert abs(t["vint"][s] - o.V_slice(s)[1]) <= 1e-12 * max(1, abs(t["vint"][s]))
+        assert abs(t["g2"][s] - o.slice_fn("gradVSquared_slice", s)) <= 1e-12 * max(1, t["g2"][s])
