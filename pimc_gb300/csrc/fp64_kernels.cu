@@ -341,7 +341,7 @@ constexpr int kForceRows = 64;
 __global__ void __launch_bounds__(kPairBlock)
 k_slice_forces64(PathView v, double invdr, int even, int odd, double* __restrict__ force) {
     extern __shared__ double smem[];
-    const int s = blockIdx.y, Ne = v.Ne;
+    const int s = blockIdx.x, Ne = v.Ne;
     if (!(s % 2 ? odd : even)) return;
     double *lx = smem, *ly = lx + Ne, *lz = ly + Ne;
     float *ux = reinterpret_cast<float*>(lz + Ne), *uy = ux + Ne, *uz = uy + Ne;
@@ -354,7 +354,7 @@ k_slice_forces64(PathView v, double invdr, int even, int odd, double* __restrict
         ux[j] = box_fraction(f.x, Ix); uy[j] = box_fraction(f.y, Iy); uz[j] = box_fraction(f.z, Iz);
     }
     __syncthreads();
-    const int b0 = blockIdx.x * kForceRows, nb = min(kForceRows, Ne - b0);
+    const int b0 = blockIdx.y * kForceRows, nb = min(kForceRows, Ne - b0);
     const int rows = nb > 32 ? 64 : 32, parts = kPairBlock / rows;
     const int r = threadIdx.x & (rows - 1), part = threadIdx.x / rows, i = b0 + r;
     double Fx = 0.0, Fy = 0.0, Fz = 0.0;
@@ -628,7 +628,7 @@ static bool bead_warp64(const PathView& v, const int2* d_beads, int k, const Bea
     if (k < kManyBeads || (corr && (!d_force || fsmem > 200 * 1024))) return false;
     if (corr) {
         if ((*e = set_smem_limit(k_slice_forces64, 200 * 1024)) != cudaSuccess) return true;
-        k_slice_forces64<<<dim3((v.Ne + kForceRows - 1) / kForceRows, v.M), kPairBlock, fsmem, s>>>(
+        k_slice_forces64<<<dim3(v.M, (v.Ne + kForceRows - 1) / kForceRows), kPairBlock, fsmem, s>>>(
             v, 1.0 / v.dr, a.gf[0] > kEPS, a.gf[1] > kEPS, d_force);
     }
     const int grid = (k + kBlockBeads - 1) / kBlockBeads;
@@ -823,8 +823,8 @@ k_slice_terms64(PathView v, double invdr, int window, int even, int odd, unsigne
     __shared__ double buf[11][kPairBlock];
     __shared__ double sums[8];
     __shared__ bool last;
-    const int s = blockIdx.y, Ne = v.Ne, n = v.nbs[s], tid = threadIdx.x, nblk = gridDim.x;
-    const int level = s % 2 ? odd : even, b0 = blockIdx.x * kSliceRows;
+    const int s = blockIdx.x, Ne = v.Ne, n = v.nbs[s], tid = threadIdx.x, nblk = gridDim.y;
+    const int level = s % 2 ? odd : even, b0 = blockIdx.y * kSliceRows;
     double *lx = sm, *ly = lx + Ne, *lz = ly + Ne;
     if (level > kSliceNone) {
         const double* X = v.pos + (size_t)s * 3 * Ne;
@@ -841,7 +841,7 @@ k_slice_terms64(PathView v, double invdr, int window, int even, int odd, unsigne
         const bool worm = worm_on_slice(v, s);
         const int half = (n - 1) / 2, total = n * half + (n % 2 ? 0 : n / 2);
         const int stride = nblk * kPairBlock, so = stride / n, si = stride - so * n;
-        int idx = blockIdx.x * kPairBlock + tid;
+        int idx = blockIdx.y * kPairBlock + tid;
         int o = idx / n, i = idx - o * n;
         ++o;
         for (; idx < total; idx += stride) {
@@ -868,7 +868,7 @@ k_slice_terms64(PathView v, double invdr, int window, int even, int odd, unsigne
         if (tid < 8) terms[(size_t)tid * v.M + s] = sums[tid];
         return;
     }
-    if (tid < 8) { part[((size_t)s * nblk + blockIdx.x) * 8 + tid] = sums[tid]; __threadfence(); }
+    if (tid < 8) { part[((size_t)s * nblk + blockIdx.y) * 8 + tid] = sums[tid]; __threadfence(); }
     __syncthreads();
     if (tid == 0) last = atomicInc(arrived + s, nblk - 1) == nblk - 1;      // back to 0 for the next call
     __syncthreads();
@@ -888,51 +888,207 @@ cudaError_t launch_slice_terms64(const PathView& v, int window, int even, int od
     const size_t smem = (size_t)v.Ne * 3 * sizeof(double);
     const cudaError_t ae = set_smem_limit(k_slice_terms64, 200 * 1024);
     if (ae != cudaSuccess) return ae;
-    k_slice_terms64<<<dim3(slice_blocks(v.Ne), v.M), kPairBlock, smem, s>>>(
+    k_slice_terms64<<<dim3(v.M, slice_blocks(v.Ne)), kPairBlock, smem, s>>>(
         v, 1.0 / v.dr, window, even, odd, d_arrived, d_terms + (size_t)8 * v.M, d_terms);
     return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
 // rho_q(t) = sum_j exp(i q . r_j(t)) in FP64 (raw positions, as gpu_isf uses
-// raw bead coordinates).  One warp per (q, t).
+// raw bead coordinates).
+//
+// A lattice vector q = 2 pi n / L (every vector of the reference's lattice
+// lists) needs no sine per bead: exp(i q . r) is the product of
+// exp(2 pi i n_d r_d / L_d) over the dimensions, and a CTA keeps those powers
+// of its slice's beads in shared memory, n_d = 0 .. the largest |n_d| of its
+// vectors, each power the product of the two half powers (log2 n roundings).
+// One thread sums one vector over the beads: eight FP64 multiply-adds a bead
+// where sincos and the phase take about seventy, and the FP64 pipe (16 clocks
+// of an SM a warp instruction) is the bound.  A list that enumerates a grid
+// symmetric about 0 has -q at the mirrored place; its density is the complex
+// conjugate and is written, not summed.  Thread i takes vectors i and
+// nq - 1 - i.  Other vectors (shells) take the sine and cosine of q . r.
+// 64 beads, 124 slices, 389 vectors with |q| < 2 in mirrored order: 219 -> 52 us;
+// 128 beads, 250 slices, 300 lattice vectors in no order: 623 -> 230 us (ncu,
+// cold).  Relative error against 113-bit phases, before and now: 4e-16 and
+// 7e-16, 6e-16 and 5e-16, at 500 beads 2.4e-15 and 2.0e-15; of F(q,tau) 2e-16
+// both.
 // ---------------------------------------------------------------------------
-__global__ void k_rhoq64(PathView v, const double* __restrict__ q, int nq, double maxR2,
-                         double* __restrict__ rho) {
-    int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    int total = nq * v.M;
-    if (gw >= total) return;
-    int iq = gw / v.M, t = gw % v.M;
-    double qx = q[3*iq], qy = q[3*iq+1], qz = q[3*iq+2];
+constexpr int kRhoThreads = 128;                 // one warp a sub-partition
+constexpr int kRhoPowers = 64;                   // largest |n_d| of the table form
+constexpr int kRhoSmem = 96 * 1024;              // two CTAs an SM
+
+// n_d when q_d is 2 pi n_d / L_d to rounding, else kRhoPowers + 1
+__device__ __forceinline__ int lattice_index(double q, double L) {
+    const double kTwoPi = 6.283185307179586476925;
+    const double n = rint(q * L / kTwoPi);
+    const bool ok = fabs(n) <= (double)kRhoPowers && fabs(q - n * (kTwoPi / L)) <= 1.0e-15 * fabs(q);
+    return ok ? (int)n : kRhoPowers + 1;
+}
+
+// exp(2 pi i n u) from the table of powers, the conjugate for n < 0
+__device__ __forceinline__ double2 power_of(const double2* E, int n) {
+    double2 e = E[n < 0 ? -n : n];
+    e.y = __hiloint2double(__double2hiint(e.y) ^ (n & 0x80000000), __double2loint(e.y));
+    return e;
+}
+
+__global__ void __launch_bounds__(kRhoThreads)
+k_rhoq64(PathView v, const double* __restrict__ q, int nq, double maxR2, double* __restrict__ rho) {
+    extern __shared__ double2 E[];               // [bead][dimension][power]
+    __shared__ int s_max;
+    __shared__ double2 half[2][kRhoThreads];
+    const int t = blockIdx.x, tid = threadIdx.x, n = v.nbs[t];
+    // few vectors: several parts of the beads a vector
+    const int slots = (nq + 1) / 2, first = blockIdx.y * kRhoThreads, mine = min(kRhoThreads, slots - first);
+    const int wide = mine > 64 ? 128 : mine > 32 ? 64 : 32, parts = kRhoThreads / wide;
+    const int sl = tid & (wide - 1), part = tid / wide;
+    const int iq = first + sl, jq = nq - 1 - iq;
+    const bool live = sl < mine;
     const double* X = v.pos + (size_t)t * 3 * v.Ne;
-    int n = v.nbs[t];
-    double re = 0.0, im = 0.0;
-    for (int j = lane; j < n; j += 32) {
-        // cylinder restriction: only beads with x^2 + y^2 < maxR^2
-        if (maxR2 > 0.0 && !(X[j] * X[j] + X[v.Ne + j] * X[v.Ne + j] < maxR2)) continue;
-        double ph = 0.0;
-        ph += qx * X[j]; ph += qy * X[v.Ne + j]; ph += qz * X[2 * v.Ne + j];
-        double sn, cs;
-        sincos(ph, &sn, &cs);
-        re += cs; im += sn;
+    int ka[3] = {0, 0, 0}, kb[3] = {0, 0, 0};
+    bool mirrored = true, second = false;
+    if (tid == 0) s_max = 0;
+    __syncthreads();
+    if (live) {
+        second = jq != iq;
+        for (int d = 0; d < 3; ++d) {
+            const double a = q[3 * iq + d], b = q[3 * jq + d];
+            mirrored = mirrored && a == -b;
+            ka[d] = lattice_index(a, v.side[d]);
+            kb[d] = lattice_index(b, v.side[d]);
+        }
     }
-    re = warp_sum(re); im = warp_sum(im);
-    if (lane == 0) { rho[2 * (size_t)gw] = re; rho[2 * (size_t)gw + 1] = im; }
+    auto top = [](const int* k) { return max(abs(k[0]), max(abs(k[1]), abs(k[2]))); };
+    const bool latA = live && top(ka) <= kRhoPowers;
+    const bool sumB = live && second && !mirrored, latB = sumB && top(kb) <= kRhoPowers;
+    const int most = max(latA ? top(ka) : -1, latB ? top(kb) : -1);
+    if (most >= 0) atomicMax(&s_max, most + 1);
+    __syncthreads();
+    double2 A = make_double2(0.0, 0.0), B = A;
+    const int np = s_max;                        // powers 0 .. np - 1; 0: no lattice vector here
+    if (np > 0) {
+        const int chunk = max(parts, kRhoSmem / (3 * np * (int)sizeof(double2)));
+        const bool any = __any_sync(0xffffffffu, latA), two = __any_sync(0xffffffffu, latB);
+        for (int j0 = 0; j0 < n; j0 += chunk) {
+            const int nj = min(chunk, n - j0);
+            __syncthreads();
+            for (int x = tid; x < 3 * nj; x += kRhoThreads) {
+                const int d = x / nj, j = x - d * nj;
+                const double r = X[d * v.Ne + j0 + j];
+                double2* e = E + (size_t)(3 * j + d) * np;
+                double sn, cs;
+                sincospi(2.0 * (r * v.sideInv[d]), &sn, &cs);
+                // cylinder restriction: beads outside x^2 + y^2 < maxR^2 count 0
+                const double rx = X[j0 + j], ry = X[v.Ne + j0 + j];
+                const double one = (d == 0 && maxR2 > 0.0 && !(rx * rx + ry * ry < maxR2)) ? 0.0 : 1.0;
+                e[0] = make_double2(one, 0.0);
+                if (np > 1) e[1] = make_double2(one * cs, one * sn);
+                for (int k = 2; k < np; ++k) {
+                    const double2 a = e[k >> 1], b = e[k - (k >> 1)];
+                    e[k] = make_double2(__fma_rn(a.x, b.x, -(a.y * b.y)), __fma_rn(a.x, b.y, a.y * b.x));
+                }
+            }
+            __syncthreads();
+            if (any && two) {
+                for (int j = part; j < nj; j += parts) {
+                    const double2* e = E + (size_t)3 * j * np;
+                    if (latA) {
+                        const double2 x = power_of(e, ka[0]), y = power_of(e + np, ka[1]), z = power_of(e + 2 * np, ka[2]);
+                        const double cr = __fma_rn(y.x, z.x, -(y.y * z.y)), ci = __fma_rn(y.x, z.y, y.y * z.x);
+                        A.x = __fma_rn(x.x, cr, __fma_rn(-x.y, ci, A.x));
+                        A.y = __fma_rn(x.x, ci, __fma_rn(x.y, cr, A.y));
+                    }
+                    if (latB) {
+                        const double2 x = power_of(e, kb[0]), y = power_of(e + np, kb[1]), z = power_of(e + 2 * np, kb[2]);
+                        const double cr = __fma_rn(y.x, z.x, -(y.y * z.y)), ci = __fma_rn(y.x, z.y, y.y * z.x);
+                        B.x = __fma_rn(x.x, cr, __fma_rn(-x.y, ci, B.x));
+                        B.y = __fma_rn(x.x, ci, __fma_rn(x.y, cr, B.y));
+                    }
+                }
+            } else if (any || two) {
+                const bool lat = any ? latA : latB;
+                const int k0 = any ? ka[0] : kb[0], k1 = any ? ka[1] : kb[1], k2 = any ? ka[2] : kb[2];
+                double2 S = make_double2(0.0, 0.0);
+                if (lat)
+                    for (int j = part; j < nj; j += parts) {
+                        const double2* e = E + (size_t)3 * j * np;
+                        const double2 x = power_of(e, k0), y = power_of(e + np, k1), z = power_of(e + 2 * np, k2);
+                        const double cr = __fma_rn(y.x, z.x, -(y.y * z.y)), ci = __fma_rn(y.x, z.y, y.y * z.x);
+                        S.x = __fma_rn(x.x, cr, __fma_rn(-x.y, ci, S.x));
+                        S.y = __fma_rn(x.x, ci, __fma_rn(x.y, cr, S.y));
+                    }
+                if (any) { A.x += S.x; A.y += S.y; } else { B.x += S.x; B.y += S.y; }
+            }
+        }
+    }
+    auto direct = [&](int i, double2& S) {
+        const double qx = q[3 * i], qy = q[3 * i + 1], qz = q[3 * i + 2];
+        for (int j = part; j < n; j += parts) {
+            if (maxR2 > 0.0 && !(X[j] * X[j] + X[v.Ne + j] * X[v.Ne + j] < maxR2)) continue;
+            double ph = 0.0;
+            ph += qx * X[j]; ph += qy * X[v.Ne + j]; ph += qz * X[2 * v.Ne + j];
+            double sn, cs;
+            sincos(ph, &sn, &cs);
+            S.x += cs; S.y += sn;
+        }
+    };
+    if (live && !latA) direct(iq, A);
+    if (sumB && !latB) direct(jq, B);
+    if (parts > 1) {                             // uniform over the CTA
+        half[0][tid] = A; half[1][tid] = B;
+        __syncthreads();
+        if (part) return;
+        for (int k = 1; k < parts; ++k) {
+            const double2 a = half[0][tid + k * wide], b = half[1][tid + k * wide];
+            A.x += a.x; A.y += a.y; B.x += b.x; B.y += b.y;
+        }
+    }
+    if (!live) return;
+    double2* R = reinterpret_cast<double2*>(rho);
+    R[(size_t)iq * v.M + t] = A;
+    if (second) R[(size_t)jq * v.M + t] = mirrored ? make_double2(A.x, -A.y) : B;
 }
 
 cudaError_t launch_rhoq64(const PathView& v, const double* d_q, int nq, double* d_rho,
                           cudaStream_t s, double maxR2) {
-    long long warps = (long long)nq * v.M;
-    int blocks = (int)((warps * 32 + 255) / 256);
-    if (blocks < 1) return cudaSuccess;
-    k_rhoq64<<<blocks, 256, 0, s>>>(v, d_q, nq, maxR2, d_rho);
+    if (nq < 1) return cudaSuccess;
+    const cudaError_t ae = set_smem_limit(k_rhoq64, kRhoSmem);
+    if (ae != cudaSuccess) return ae;
+    const int slots = (nq + 1) / 2;
+    k_rhoq64<<<dim3(v.M, (slots + kRhoThreads - 1) / kRhoThreads), kRhoThreads, kRhoSmem, s>>>(v, d_q, nq, maxR2, d_rho);
     return cudaGetLastError();
 }
 
-// F(q,tau) = norm * sum_t Re(rho_t conj(rho_{t+tau})), tau in [0, M/2]
-__global__ void k_isf_direct64(const double* __restrict__ rho, int nq, int M, double norm,
-                               double* __restrict__ out) {
+// F(q,tau) = norm * sum_t Re(rho_t conj(rho_{t+tau})), tau in [0, M/2].  One
+// CTA a wave vector, its densities in shared memory with the first half
+// repeated behind them (no wrap in the loop), one thread a tau: two FP64
+// multiply-adds a term, the FP64 pipe the bound.  300 vectors, M = 250:
+// 79 us with one thread an output from L1, 35 us here.
+constexpr int kIsfThreads = 128;
+
+__global__ void __launch_bounds__(kIsfThreads)
+k_isf_direct64(const double* __restrict__ rho, int M, double norm, double* __restrict__ out) {
+    extern __shared__ double2 E[];
+    const int nt = M / 2 + 1;
+    const double2* r = reinterpret_cast<const double2*>(rho) + (size_t)blockIdx.x * M;
+    for (int t = threadIdx.x; t < M + nt; t += kIsfThreads) E[t] = r[t < M ? t : t - M];
+    __syncthreads();
+    for (int tau = threadIdx.x; tau < nt; tau += kIsfThreads) {
+        double re = 0.0, im = 0.0;
+        #pragma unroll 4
+        for (int t = 0; t < M; ++t) {
+            const double2 a = E[t], b = E[t + tau];
+            re = __fma_rn(a.x, b.x, re);
+            im = __fma_rn(a.y, b.y, im);
+        }
+        out[(size_t)blockIdx.x * nt + tau] = (re + im) * norm;
+    }
+}
+
+// the same straight from memory, for slices whose densities do not fit
+__global__ void k_isf_long64(const double* __restrict__ rho, int nq, int M, double norm,
+                             double* __restrict__ out) {
     int nt = M / 2 + 1;
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= (long long)nq * nt) return;
@@ -948,10 +1104,16 @@ __global__ void k_isf_direct64(const double* __restrict__ rho, int nq, int M, do
 
 cudaError_t launch_isf_direct64(const double* d_rho, int nq, int M, double norm,
                                 double* d_out, cudaStream_t s) {
+    if (nq < 1) return cudaSuccess;
+    const size_t smem = (size_t)(M + M / 2 + 1) * sizeof(double2);
+    if (smem <= 200 * 1024) {
+        const cudaError_t ae = set_smem_limit(k_isf_direct64, 200 * 1024);
+        if (ae != cudaSuccess) return ae;
+        k_isf_direct64<<<nq, kIsfThreads, smem, s>>>(d_rho, M, norm, d_out);
+        return cudaGetLastError();
+    }
     long long n = (long long)nq * (M / 2 + 1);
-    int blocks = (int)((n + 255) / 256);
-    if (blocks < 1) return cudaSuccess;
-    k_isf_direct64<<<blocks, 256, 0, s>>>(d_rho, nq, M, norm, d_out);
+    k_isf_long64<<<(int)((n + 255) / 256), 256, 0, s>>>(d_rho, nq, M, norm, d_out);
     return cudaGetLastError();
 }
 
