@@ -1202,7 +1202,7 @@ int pgb_superfluid(pgb_ctx* h, double* out26) {
     rc = c.ensure_scratch(winding_work_bytes()); if (rc) return rc;
     double* d_work = static_cast<double*>(c.d_scratch);
     double* d_out = d_work + (winding_work_bytes() / sizeof(double) - 5);
-    PGB_CUDA(&c, launch_winding(c.view(), d_work, d_out, c.stream));
+    PGB_CUDA(&c, launch_winding(c.view(), c.d_arrived, d_work, d_out, c.stream));
     double s5[5];
     PGB_CUDA(&c, cudaMemcpyAsync(s5, d_out, sizeof(s5), cudaMemcpyDeviceToHost, c.stream));
     PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
@@ -1232,9 +1232,9 @@ int pgb_permutation_cycles(pgb_ctx* h, double* out40) {
     const int nw = c.h_nbs.empty() ? 0 : c.h_nbs[0];
     for (int i = 0; i < 40; ++i) out40[i] = 0.0;
     if (nw == 0) return PGB_OK;
-    rc = c.ensure_scratch((size_t)nw * sizeof(int)); if (rc) return rc;
+    rc = c.ensure_scratch(cycles_work_ints(c.view(), nw) * sizeof(int)); if (rc) return rc;
     int* d_len = static_cast<int*>(c.d_scratch);
-    PGB_CUDA(&c, launch_cycles(c.view(), nw, d_len, c.stream));
+    PGB_CUDA(&c, launch_cycles(c.view(), nw, c.d_arrived, d_len, c.stream));
     std::vector<int> len(nw);
     PGB_CUDA(&c, cudaMemcpyAsync(len.data(), d_len, nw * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
     PGB_CUDA(&c, cudaStreamSynchronize(c.stream));

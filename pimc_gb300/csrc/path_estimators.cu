@@ -3,6 +3,8 @@
 // cycles (estimator.cpp:2000-2074, 2735-2781, 3181-3246).  FP64, compiled
 // with -fmad=false so that every separation, and therefore every histogram
 // bin, is the one the reference computes.
+#include <algorithm>
+
 #include "pgb_device.cuh"
 
 namespace pgb {
@@ -14,62 +16,89 @@ constexpr int kEstBlock = 256;
 // ActionBase::updateSepHist's binning (action.cpp:216-224):
 // nR = int(|r_b2 - r_b1| / dSep).  One CTA per slice.  The slice is staged
 // in shared memory as FP32; each pair's bin is first found in FP32 and, only
-// when the FP32 quotient lies within kEdge of a bin edge, recomputed from the
+// when the FP32 quotient lies within an edge's width of a bin's end, recomputed from the
 // FP64 positions exactly as the reference does, so every count is the
-// reference's.  Error of the FP32 quotient x = |r| / dSep: a position
-// (|r_d| <= L/2) rounds by at most 2^-24 L, the difference, the minimum image
-// and the sum of squares add a few such roundings, so |r| is off by at most
-// about 2^-20 L; with dSep = sqrt(3) L / 100 that is 100 / (sqrt(3) 2^20)
-// = 5.5e-5 of a bin for any box, plus 3e-6 from 1/dSep: below 6e-5, a third
-// of kEdge.  The FP64 recomputation then runs for about 4e-4 of the pairs:
-// one FP64 warp instruction costs the issue of sixteen FP32 ones on this
-// GPU, so the edge is kept narrow.  Counts go to per-warp shared
-// histograms, so the result is order-free.
-constexpr float kEdge = 2.0e-4f;
-constexpr int kSepWarps = kEstBlock / 32;
+// reference's.  Error of the FP32 quotient x = |r| / dSep, dSep = sqrt(3) L / 100:
+// a position (|r_d| <= L/2) rounds by at most 2^-25 L, the difference of two
+// and its image by twice that each, so |r| is off by at most sqrt(3) 3 2^-24 L,
+// 1.8e-5 of a bin; the sum of squares, the reciprocal root and 1/dSep add
+// 2e-5 at 50 bins, the step of the quotient 8e-6: together less than half of
+// the edge, kSepEdge steps.  The FP64 recomputation
+// runs for 2e-4 of the pairs; its sixty dependent FP64 instructions take a
+// warp about 5 us (the FP64 pipe takes 64 clocks of a sub-partition for a warp
+// instruction), so these pairs are listed and done together at the end, one a
+// thread.  A shared-memory atomic takes about a clock a lane even without
+// conflicts (30 us a call), so every lane of every warp counts in its own
+// column with plain loads and stores.  What is left is the issue rate, about
+// 45 instructions a pair, and sixteen warps a CTA against their latency.
+// 256 beads, 250 slices: 43 us with eight warps, an atomic histogram each and
+// floor, compare and IEEE root in floating point (64 instructions), 27 us
+// here.
+constexpr int kSepBits = 16;                 // 127 bins of 2^16 steps fill the mantissa
+constexpr int kSepEdge = 7;                  // 1.07e-4 of a bin
+constexpr int kSepBlock = 512;               // 256 where a slice leaves no room for sixteen histograms
+constexpr int kSepNear = 512;
 
-__global__ void __launch_bounds__(kEstBlock)
-k_sep_hist(PathView v, int t0, double dSep, unsigned long long* __restrict__ hist) {
+// FP32 constants made on the host: a division or conversion in FP64 by every
+// warp of every CTA takes longer than the pairs of a small slice
+struct SepF { float side[3], inv[3], step, far; };
+
+__device__ __forceinline__ int sep_bin64(const PathView& v, int t, int b1, int b2, double dSep) {
+    const double3 d = sep64(v, t, b2, b1);
+    return (int)(sqrt(d.x * d.x + d.y * d.y + d.z * d.z) / dSep);
+}
+
+__global__ void __launch_bounds__(kSepBlock)
+k_sep_hist(PathView v, SepF f, int t0, double dSep, unsigned long long* __restrict__ hist) {
     extern __shared__ float4 sp[];                       // [n] slice positions, FP32
-    __shared__ unsigned int sh[kSepWarps][kPcfBins];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int b = threadIdx.x; b < kSepWarps * kPcfBins; b += blockDim.x) (&sh[0][0])[b] = 0u;
+    __shared__ int2 near_pair[kSepNear];
+    __shared__ int s_near;
+    if (threadIdx.x == 0) s_near = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, threads = blockDim.x, warps = threads >> 5;
+    unsigned* counts = reinterpret_cast<unsigned*>(sp + v.Ne);      // [warp][bin][lane]
+    unsigned* own = counts + warp * (32 * kPcfBins) + lane;
+    for (int b = threadIdx.x; b < warps * 32 * kPcfBins; b += threads) counts[b] = 0u;
     const int t = t0 + blockIdx.x;
     const int n = v.nbs[t];
-    const double* X = v.pos + (size_t)t * 3 * v.Ne;
-    for (int j = threadIdx.x; j < n; j += blockDim.x)
-        sp[j] = make_float4((float)X[j], (float)X[v.Ne + j], (float)X[2 * v.Ne + j], 0.f);
+    for (int j = threadIdx.x; j < n; j += threads) sp[j] = v.pos32[(size_t)t * v.Ne + j];
     __syncthreads();
-    const float Lx = (float)v.side[0], Ly = (float)v.side[1], Lz = (float)v.side[2];
-    const float Lix = (float)v.sideInv[0], Liy = (float)v.sideInv[1], Liz = (float)v.sideInv[2];
-    const float invSep = (float)(1.0 / dSep);
-    const float edge = kEdge;
-    for (int b1 = warp; b1 < n - 1; b1 += kSepWarps) {
+    const float Lx = f.side[0], Ly = f.side[1], Lz = f.side[2], Lix = f.inv[0], Liy = f.inv[1], Liz = f.inv[2];
+    const float step = f.step, far = f.far;
+    for (int b1 = warp; b1 < n - 1; b1 += warps) {
         const float4 r1 = sp[b1];
         for (int b2 = b1 + 1 + lane; b2 < n; b2 += 32) {
             const float4 r2 = sp[b2];
             float dx = r2.x - r1.x, dy = r2.y - r1.y, dz = r2.z - r1.z;
-            dx -= Lx * rint_add(dx * Lix);
-            dy -= Ly * rint_add(dy * Liy);
-            dz -= Lz * rint_add(dz * Liz);
-            const float x = sqrtf(dx * dx + dy * dy + dz * dz) * invSep;
-            // floor(x) without float/int conversions: adding 2^23 rounded
-            // down leaves floor(x) in the mantissa bits, for 0 <= x < 2^22
-            const float xf = __fadd_rd(x, 8388608.0f);
-            int nR = __float_as_int(xf) - 0x4B000000;
-            const float f = x - __fsub_rn(xf, 8388608.0f);
-            if (f < edge || f > 1.0f - edge) {
-                const double3 d = sep64(v, t, b2, b1);
-                nR = (int)(sqrt(d.x * d.x + d.y * d.y + d.z * d.z) / dSep);
+            dx = fmaf(-Lx, rint_add(dx * Lix), dx);
+            dy = fmaf(-Ly, rint_add(dy * Liy), dy);
+            dz = fmaf(-Lz, rint_add(dz * Liz), dz);
+            const float rr = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+            float ri;
+            asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ri) : "f"(fmaxf(rr, 1.0e-30f)));
+            // x with kSepBits fraction bits in the mantissa of 2^23 + x 2^kSepBits
+            const int i = __float_as_int(fmaf(fminf(rr * ri, far), step, 8388608.0f));
+            if (((i + kSepEdge) & ((1 << kSepBits) - 1)) < 2 * kSepEdge) {
+                const int at = atomicAdd(&s_near, 1);
+                if (at < kSepNear) { near_pair[at] = make_int2(b1, b2); continue; }
+                const int nR = sep_bin64(v, t, b1, b2, dSep);
+                if (nR >= 0 && nR < kPcfBins) ++own[32 * nR];
+                continue;
             }
-            if (nR >= 0 && nR < kPcfBins) atomicAdd(&sh[warp][nR], 1u);
+            const int nR = (i >> kSepBits) & 127;
+            if (nR < kPcfBins) ++own[32 * nR];
         }
     }
     __syncthreads();
-    for (int b = threadIdx.x; b < kPcfBins; b += blockDim.x) {
-        unsigned long long c = 0;
-        for (int w = 0; w < kSepWarps; ++w) c += sh[w][b];
-        if (c) atomicAdd(&hist[b], c);
+    for (int k = threadIdx.x; k < min(s_near, kSepNear); k += threads) {
+        const int nR = sep_bin64(v, t, near_pair[k].x, near_pair[k].y, dSep);
+        if (nR >= 0 && nR < kPcfBins) ++own[32 * nR];
+    }
+    __syncthreads();
+    for (int b = warp; b < kPcfBins; b += warps) {
+        unsigned int c = 0;
+        for (int w = 0; w < warps; ++w) c += counts[(w * kPcfBins + b) * 32 + lane];
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0 && c) atomicAdd(&hist[b], (unsigned long long)c);
     }
 }
 
@@ -78,100 +107,173 @@ cudaError_t launch_sep_hist(const PathView& v, int slice, unsigned long long* d_
     if (e != cudaSuccess) return e;
     const double dSep = 0.5 * sqrt(3.0) * v.side[2] / (1.0 * kPcfBins);   // action.cpp:192
     const int t0 = slice >= 0 ? slice : 0, nt = slice >= 0 ? 1 : v.M;
-    const size_t smem = (size_t)v.Ne * sizeof(float4);
+    const size_t pos = (size_t)v.Ne * sizeof(float4), column = kPcfBins * sizeof(unsigned);
+    const int threads = pos + kSepBlock * column <= 200 * 1024 ? kSepBlock : 256;
+    const size_t smem = pos + threads * column;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;   // one slice in shared memory
     {
         const cudaError_t ae = set_smem_limit(k_sep_hist, 200 * 1024);
         if (ae != cudaSuccess) return ae;
     }
-    k_sep_hist<<<nt, kEstBlock, smem, s>>>(v, t0, dSep, d_hist);
+    SepF f;
+    for (int d = 0; d < 3; ++d) { f.side[d] = (float)v.side[d]; f.inv[d] = (float)v.sideInv[d]; }
+    f.step = (float)((1 << kSepBits) / dSep);
+    f.far = (float)(127.0 * dSep);
+    k_sep_hist<<<nt, threads, smem, s>>>(v, f, t0, dSep, d_hist);
     return cudaGetLastError();
+}
+
+// The last CTA of a grid to arrive; the others' global writes are visible to
+// it.  The counter returns to 0 for the next call.
+__device__ __forceinline__ bool last_to_arrive(unsigned* counter, unsigned blocks) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(counter, blocks - 1) == blocks - 1;
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
 }
 
 // Winding and area sums of SuperfluidFractionEstimator::accumulate
 // (estimator.cpp:2008-2036): W = sum of getVelocity over the active beads
 // (path.h:189-203), Az and I from each bead and its next one.  Partial sums
-// per CTA in a fixed order, then one CTA adds the partials in order, so the
-// result does not depend on scheduling.
+// per CTA in a fixed order; the last CTA adds the partials, a warp a sum, in
+// a fixed order, so the result does not depend on scheduling.  A launch of its
+// own for that, one thread a sum, took as long as the partials (12 us of 21).
 __global__ void __launch_bounds__(kEstBlock)
-k_winding_partials(PathView v, double* __restrict__ part) {
-    __shared__ double red[5][kEstBlock];
-    double w0 = 0.0, w1 = 0.0, w2 = 0.0, az = 0.0, in = 0.0;
-    const long long nb = (long long)v.M * v.Ne;
-    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < nb;
-         idx += (long long)gridDim.x * blockDim.x) {
-        const int t = (int)(idx / v.Ne), p = (int)(idx - (long long)t * v.Ne);
-        if (p >= v.nbs[t]) continue;
-        const int2 nx = v.next[(size_t)t * v.Ne + p];
+k_winding(PathView v, unsigned* __restrict__ arrived, double* __restrict__ part, double* __restrict__ out5) {
+    __shared__ double red[5][kEstBlock / 32];
+    double w[5] = {};
+    const size_t nb = (size_t)v.M * v.Ne;
+    const unsigned Ne = v.Ne;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (size_t idx = blockIdx.x * kEstBlock + threadIdx.x; idx < nb; idx += gridDim.x * kEstBlock) {
+        const unsigned t = (idx >> 32) ? (unsigned)(idx / Ne) : (unsigned)idx / Ne;
+        const unsigned p = (unsigned)(idx - (size_t)t * Ne);
+        if (p >= (unsigned)v.nbs[t]) continue;
+        const int2 nx = v.next[idx];
         if (nx.x < 0) continue;                              // getVelocity = 0, no area term
-        const double* X = v.pos + (size_t)t * 3 * v.Ne;
-        const double* Y = v.pos + (size_t)nx.x * 3 * v.Ne;
-        const double p1x = X[p], p1y = X[v.Ne + p], p1z = X[2 * v.Ne + p];
-        const double p2x = Y[nx.y], p2y = Y[v.Ne + nx.y], p2z = Y[2 * v.Ne + nx.y];
-        w0 += min_image(p2x - p1x, v.side[0], v.sideInv[0]);
-        w1 += min_image(p2y - p1y, v.side[1], v.sideInv[1]);
-        w2 += min_image(p2z - p1z, v.side[2], v.sideInv[2]);
-        az += p1x * p2y - p2x * p1y;
-        in += p1x * p2x + p1y * p2y;
+        const double* X = v.pos + (size_t)t * 3 * Ne;
+        const double* Y = v.pos + (size_t)nx.x * 3 * Ne;
+        const double p1x = X[p], p1y = X[Ne + p], p1z = X[2 * Ne + p];
+        const double p2x = Y[nx.y], p2y = Y[Ne + nx.y], p2z = Y[2 * Ne + nx.y];
+        w[0] += min_image(p2x - p1x, v.side[0], v.sideInv[0]);
+        w[1] += min_image(p2y - p1y, v.side[1], v.sideInv[1]);
+        w[2] += min_image(p2z - p1z, v.side[2], v.sideInv[2]);
+        w[3] += p1x * p2y - p2x * p1y;
+        w[4] += p1x * p2x + p1y * p2y;
     }
-    red[0][threadIdx.x] = w0; red[1][threadIdx.x] = w1; red[2][threadIdx.x] = w2;
-    red[3][threadIdx.x] = az; red[4][threadIdx.x] = in;
+    #pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        const double x = warp_sum(w[k]);
+        if (lane == 0) red[k][warp] = x;
+    }
     __syncthreads();
-    for (int o = kEstBlock / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o)
-            for (int k = 0; k < 5; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x < 5) part[(size_t)blockIdx.x * 5 + threadIdx.x] = red[threadIdx.x][0];
-}
-
-__global__ void k_winding_total(const double* __restrict__ part, int nblocks, double* __restrict__ out5) {
     if (threadIdx.x < 5) {
-        double s = 0.0;
-        for (int b = 0; b < nblocks; ++b) s += part[(size_t)b * 5 + threadIdx.x];
-        out5[threadIdx.x] = s;
+        double x = 0.0;
+        for (int k = 0; k < kEstBlock / 32; ++k) x += red[threadIdx.x][k];
+        part[(size_t)blockIdx.x * 5 + threadIdx.x] = x;
     }
+    if (!last_to_arrive(arrived, gridDim.x) || warp >= 5) return;
+    double x = 0.0;
+    for (unsigned b = lane; b < gridDim.x; b += 32) x += __ldcg(part + (size_t)b * 5 + warp);
+    x = warp_sum(x);
+    if (lane == 0) out5[warp] = x;
 }
 
 constexpr int kWindBlocks = 152;
 
 size_t winding_work_bytes() { return (size_t)kWindBlocks * 5 * sizeof(double) + 5 * sizeof(double); }
 
-cudaError_t launch_winding(const PathView& v, double* d_work, double* d_out5, cudaStream_t s) {
-    k_winding_partials<<<kWindBlocks, kEstBlock, 0, s>>>(v, d_work);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_winding_total<<<1, 32, 0, s>>>(d_work, kWindBlocks, d_out5);
+cudaError_t launch_winding(const PathView& v, unsigned* d_arrived, double* d_work, double* d_out5, cudaStream_t s) {
+    const size_t nb = (size_t)v.M * v.Ne;
+    const int blocks = (int)std::min<size_t>(kWindBlocks, (nb + kEstBlock - 1) / kEstBlock);
+    k_winding<<<blocks, kEstBlock, 0, s>>>(v, d_arrived, d_work, d_out5);
     return cudaGetLastError();
 }
 
 // Cycle lengths of PermutationCycleEstimator::accumulate
-// (estimator.cpp:2735-2781): one thread per active bead of slice 0 walks
-// its worldline through the next links.  The reference counts a cycle at
-// its first slice-0 bead in index order, i.e. at the smallest one, so each
-// thread counts its cycle only if it met no smaller slice-0 bead.  A walk
-// is bounded by M * Ne steps (a longer one is not a cycle: -1).
-__global__ void k_cycles(PathView v, int* __restrict__ len_out) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+// (estimator.cpp:2735-2781): a slice-0 bead's worldline through the next links
+// back to slice 0.  The reference counts a cycle at its first slice-0 bead in
+// index order, i.e. at the smallest one; 0 is written for the others and -1
+// where the worldline does not close.
+//
+// A walk is a chain of dependent loads, M a particle of the cycle (74 us at
+// 124 slices, 154 us at 250, cycles of three).  Links go to the next slice, so
+// a segment of kSegment slices is a map from its first slice's beads to those
+// of the segment behind it: every segment and bead walks at once, the last
+// CTA composes the maps into slice 0's permutation in shared memory and
+// follows its cycles there: 14 and 18 us.  A link to any other slice raises `odd`
+// and the last CTA walks every bead link by link.
+constexpr int kSegment = 16;
+
+__global__ void __launch_bounds__(kEstBlock)
+k_cycles(PathView v, int nseg, unsigned* __restrict__ arrived, int* __restrict__ odd, int* __restrict__ map,
+         int* __restrict__ len_out) {
+    extern __shared__ int perm[];
+    const int Ne = v.Ne, tid = threadIdx.x;
+    const int seg = blockIdx.x % nseg, p0 = (blockIdx.x / nseg) * kEstBlock + tid;
+    if (p0 < Ne) {
+        int p = p0, t = seg * kSegment;
+        const int end = min(v.M, t + kSegment);
+        for (; t < end && p >= 0; ++t) {
+            const int2 b = v.next[(size_t)t * Ne + p];
+            if (b.x >= 0 && b.x != (t + 1 == v.M ? 0 : t + 1)) { *odd = 1; p = -1; }
+            else p = b.x < 0 ? -1 : b.y;
+        }
+        map[(size_t)seg * Ne + p0] = p;
+    }
+    if (!last_to_arrive(arrived, gridDim.x)) return;
     const int nw = v.nbs[0];
-    if (n >= nw) return;
-    const long long limit = (long long)v.M * v.Ne;
-    int2 b = make_int2(0, n);
-    long long wl = 0;
-    bool smallest = true, closed = false;
-    do {
-        ++wl;
-        if (b.x == 0 && b.y < n) smallest = false;
-        b = v.next[(size_t)b.x * v.Ne + b.y];
-        if (b.x < 0) break;                                  // open worldline
-        if (b.x == 0 && b.y == n) { closed = true; break; }
-    } while (wl <= limit);
-    len_out[n] = (closed && smallest) ? (int)wl : (closed ? 0 : -1);
+    if (__ldcg(odd)) {
+        for (int n = tid; n < nw; n += kEstBlock) {
+            const long long limit = (long long)v.M * Ne;
+            int2 b = make_int2(0, n);
+            long long wl = 0;
+            bool smallest = true, closed = false;
+            do {
+                ++wl;
+                if (b.x == 0 && b.y < n) smallest = false;
+                b = v.next[(size_t)b.x * Ne + b.y];
+                if (b.x < 0) break;                          // open worldline
+                if (b.x == 0 && b.y == n) { closed = true; break; }
+            } while (wl <= limit);
+            len_out[n] = (closed && smallest) ? (int)wl : (closed ? 0 : -1);
+        }
+        return;
+    }
+    for (int n = tid; n < nw; n += kEstBlock) {
+        int p = n;
+        for (int k = 0; k < nseg && p >= 0; ++k) p = __ldcg(map + (size_t)k * Ne + p);
+        perm[n] = p < nw ? p : -1;
+    }
+    __syncthreads();
+    for (int n = tid; n < nw; n += kEstBlock) {
+        int p = n, steps = 0;
+        bool smallest = true;
+        do {
+            ++steps;
+            if (p < n) smallest = false;
+            p = perm[p];
+        } while (p >= 0 && p != n && steps <= nw);
+        len_out[n] = p != n ? -1 : smallest ? steps * v.M : 0;
+    }
 }
 
-cudaError_t launch_cycles(const PathView& v, int nw, int* d_len, cudaStream_t s) {
+static int cycle_segments(const PathView& v) { return (v.M + kSegment - 1) / kSegment; }
+
+size_t cycles_work_ints(const PathView& v, int nw) { return 1 + (size_t)nw + (size_t)cycle_segments(v) * v.Ne; }
+
+// d_work: cycles_work_ints ints, the first nw the lengths
+cudaError_t launch_cycles(const PathView& v, int nw, unsigned* d_arrived, int* d_work, cudaStream_t s) {
     if (nw <= 0) return cudaSuccess;
-    k_cycles<<<(nw + 127) / 128, 128, 0, s>>>(v, d_len);
+    int* odd = d_work + nw;
+    cudaError_t e = cudaMemsetAsync(odd, 0, sizeof(int), s);
+    if (e != cudaSuccess) return e;
+    const int nseg = cycle_segments(v);
+    k_cycles<<<nseg * ((v.Ne + kEstBlock - 1) / kEstBlock), kEstBlock, nw * sizeof(int), s>>>(v, nseg, d_arrived, odd,
+                                                                                            odd + 1, d_work);
     return cudaGetLastError();
 }
 

@@ -83,7 +83,7 @@ struct Ctx {
     void* d_tc_tables = nullptr;   // split-BF16 DFT and cosine matrices of this M (built once)
     float4* d_force32 = nullptr;   // per-bead same-slice forces of the current configuration
     bool force_valid = false;      // cleared by every position change
-    unsigned* d_arrived = nullptr; // per-slice counters of the FP64 slice terms (zero between calls)
+    unsigned* d_arrived = nullptr; // M arrival counters of kernels whose last CTA adds up (zero between calls)
     double* d_force64 = nullptr;   // scratch of the FP64 many-bead form: slice forces [M][3][Ne]
     void* h_pinned = nullptr; size_t pinned_bytes = 0;
     // plain-form worm state: the LookupTable's per-slice lists of a single
@@ -187,8 +187,11 @@ cudaError_t launch_isf_direct32(const float2* d_rho, int nq, int M, double norm,
 // path_estimators.cu (g(r), winding, permutation cycles; FP64, -fmad=false)
 cudaError_t launch_sep_hist(const PathView& v, int slice, unsigned long long* d_hist, cudaStream_t s);
 size_t winding_work_bytes();
-cudaError_t launch_winding(const PathView& v, double* d_work, double* d_out5, cudaStream_t s);
-cudaError_t launch_cycles(const PathView& v, int nw, int* d_len, cudaStream_t s);
+// d_arrived: one counter, zero between calls
+cudaError_t launch_winding(const PathView& v, unsigned* d_arrived, double* d_work, double* d_out5, cudaStream_t s);
+// d_work: cycles_work_ints ints, the first nw the cycle lengths
+size_t cycles_work_ints(const PathView& v, int nw);
+cudaError_t launch_cycles(const PathView& v, int nw, unsigned* d_arrived, int* d_work, cudaStream_t s);
 // slice-0 beads with x^2 + y^2 < maxR2 (one int)
 cudaError_t launch_count_inside(const PathView& v, double maxR2, int* d_out, cudaStream_t s);
 // isf_tc.cu (tcgen05 split-BF16 DFT correlation)
