@@ -286,6 +286,8 @@ int pgb_create(const pgb_params* p, pgb_ctx** out) {
         if ((e = cudaMalloc(&c.d_prev, nb * sizeof(int2))) != cudaSuccess) break;
         if ((e = cudaMalloc(&c.d_on, nb)) != cudaSuccess) break;
         if ((e = cudaMalloc(&c.d_nbs, c.M * sizeof(int))) != cudaSuccess) break;
+        if (p->precision == PGB_MIXED)
+            if ((e = cudaMalloc(&c.d_trial_count, (2 * nb + 1) * sizeof(int))) != cudaSuccess) break;
         if ((e = cudaMalloc(&c.d_arrived, c.M * sizeof(unsigned))) != cudaSuccess) break;
         if ((e = cudaMemsetAsync(c.d_arrived, 0, c.M * sizeof(unsigned), c.stream)) != cudaSuccess) break;
         if (p->precision == PGB_FP64 && (p->gradvfactor[0] > kEPS || p->gradvfactor[1] > kEPS))
@@ -325,6 +327,7 @@ int pgb_destroy(pgb_ctx* h) {
     if (c.d_force32) cudaFree(c.d_force32);
     if (c.d_force64) cudaFree(c.d_force64);
     if (c.d_arrived) cudaFree(c.d_arrived);
+    if (c.d_trial_count) cudaFree(c.d_trial_count);
     if (c.h_pinned) cudaFreeHost(c.h_pinned);
     if (c.stream) cudaStreamDestroy(c.stream);
     delete h;
@@ -1089,8 +1092,19 @@ int trial_launch(Ctx& c, const int2* d_b, const double* d_pos, int k, int shift,
         int rc = PGB_OK;
         const float4* fall = slice_forces(c, &rc);
         if (rc) return rc;
-        e = launch_bead_actions32_full(v, c.az, d_b, k, shift, mode, c.p.tau, c.p.lambda,
-                                       c.p.vfactor, c.p.gradvfactor, d_pos, fall, 1, d_delta, c.stream);
+        // the sorted records take the place of d_new and d_old
+        const char *w0 = reinterpret_cast<const char*>(d_new), *w1 = w0 + (size_t)k * sizeof(float4);
+        auto apart = [&](const void* q, size_t bytes) {
+            return static_cast<const char*>(q) + bytes <= w0 || w1 <= static_cast<const char*>(q);
+        };
+        const bool room = d_old == d_new + k && reinterpret_cast<uintptr_t>(d_new) % sizeof(float4) == 0 &&
+                          apart(d_delta, (size_t)k * sizeof(double)) && apart(d_pos, (size_t)k * 3 * sizeof(double)) &&
+                          apart(d_b, (size_t)k * sizeof(int2));
+        e = room && trials32_sorted(v, k)
+            ? launch_trials32(v, c.az, d_b, k, shift, mode, c.p.tau, c.p.lambda, c.p.vfactor, c.p.gradvfactor, d_pos,
+                              fall, c.d_trial_count, reinterpret_cast<float4*>(d_new), d_delta, c.stream)
+            : launch_bead_actions32_full(v, c.az, d_b, k, shift, mode, c.p.tau, c.p.lambda,
+                                         c.p.vfactor, c.p.gradvfactor, d_pos, fall, 1, d_delta, c.stream);
         if (e != cudaSuccess) return c.cuda_fail(e, "trial actions launch");
         return PGB_OK;
     }
@@ -1134,14 +1148,14 @@ int pgb_trial_actions(pgb_ctx* h, const int32_t* beads, const double* pos, int k
             return c.fail(PGB_EINVAL, "trial_actions: bead out of range");
     size_t bb = ((size_t)k * sizeof(int2) + 255) & ~(size_t)255;
     size_t pb = ((size_t)k * 3 * sizeof(double) + 255) & ~(size_t)255;
-    size_t ob = ((size_t)k * sizeof(double) + 255) & ~(size_t)255;
-    rc = c.ensure_scratch(bb + pb + 3 * ob); if (rc) return rc;
+    size_t ob = ((size_t)k * 2 * sizeof(double) + 255) & ~(size_t)255;
+    rc = c.ensure_scratch(bb + pb + ob + (size_t)k * sizeof(double)); if (rc) return rc;
     char* d = static_cast<char*>(c.d_scratch);
     PGB_CUDA(&c, cudaMemcpyAsync(d, beads, (size_t)k * sizeof(int2), cudaMemcpyHostToDevice, c.stream));
     PGB_CUDA(&c, cudaMemcpyAsync(d + bb, pos, (size_t)k * 3 * sizeof(double), cudaMemcpyHostToDevice, c.stream));
     double* d_new = reinterpret_cast<double*>(d + bb + pb);
-    double* d_old = reinterpret_cast<double*>(d + bb + pb + ob);
-    double* d_del = reinterpret_cast<double*>(d + bb + pb + 2 * ob);
+    double* d_old = d_new + k;
+    double* d_del = reinterpret_cast<double*>(d + bb + pb + ob);
     rc = trial_launch(c, reinterpret_cast<int2*>(d), reinterpret_cast<double*>(d + bb), k, shift, mode,
                       d_new, d_old, d_del);
     if (rc) return rc;

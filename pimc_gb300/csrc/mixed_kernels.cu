@@ -3,6 +3,8 @@
 // Pair potentials and gradients are the analytic Aziz form in FP32 (no
 // table), read from the float4 position mirror; each thread accumulates its
 // pairs with Kahan compensation and the block folds the partial sums in FP64.
+#include <algorithm>
+
 #include "pgb_device.cuh"
 
 namespace pgb {
@@ -224,6 +226,19 @@ __device__ __forceinline__ float pair_factor32(int st1, int st2) {
     return 0.5f;
 }
 
+// A bead's action from its FP64 sums; the roundings are spelt out so that the
+// two kernels that assemble actions give the same bits.
+__device__ __forceinline__ double assemble32(int mode, bool need_c, double vf, double gf, double t, double lambda,
+                                             double V, double T, double fx, double fy, double fz) {
+    const double bareU = __dmul_rn(__dmul_rn(vf, t), V);
+    double corU = 0.0;
+    if (need_c) {
+        const double f2 = __fma_rn(fx, fx, __fma_rn(fy, fy, __dmul_rn(fz, fz)));
+        corU = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(gf, t), t), t), lambda), __dadd_rn(T, f2));
+    }
+    return (mode == PGB_ACTION_BARE) ? bareU : (mode == PGB_ACTION_CORR) ? corU : __dadd_rn(bareU, corU);
+}
+
 __global__ void __launch_bounds__(kWarpBeadBlock)
 k_bead_actions32_full(PathView v, AzizF az, const int2* __restrict__ beads, int k, int shift,
                       int mode, double tau, double lambda, double vf0, double vf1, double gf0,
@@ -299,9 +314,18 @@ k_bead_actions32_full(PathView v, AzizF az, const int2* __restrict__ beads, int 
                 }
             }
         }
-        const float2 parts[10] = {warp_ff(vn), warp_ff(vo), warp_ff(tn), warp_ff(to),
-                                  ff_butterfly(fnx, 0.f), ff_butterfly(fny, 0.f), ff_butterfly(fnz, 0.f),
-                                  ff_butterfly(fox, 0.f), ff_butterfly(foy, 0.f), ff_butterfly(foz, 0.f)};
+        // only the sums the action has: a butterfly is 45 instructions
+        float2 parts[10] = {};
+        parts[0] = warp_ff(vn);
+        if (both) parts[1] = warp_ff(vo);
+        if (need_c) {
+            parts[2] = warp_ff(tn);
+            parts[4] = ff_butterfly(fnx, 0.f); parts[5] = ff_butterfly(fny, 0.f); parts[6] = ff_butterfly(fnz, 0.f);
+            if (both) {
+                parts[3] = warp_ff(to);
+                parts[7] = ff_butterfly(fox, 0.f); parts[8] = ff_butterfly(foy, 0.f); parts[9] = ff_butterfly(foz, 0.f);
+            }
+        }
         if (lane == 0) {
             #pragma unroll
             for (int q = 0; q < 10; ++q) s_part[lb][q] = parts[q];
@@ -325,13 +349,11 @@ k_bead_actions32_full(PathView v, AzizF az, const int2* __restrict__ beads, int 
                 const float2* q = s_part[lane];
                 auto dd = [](float2 x) { return (double)x.x + (double)x.y; };
                 auto action = [&](double V, double T, double fx, double fy, double fz) {
-                    const double bareU = vf * t * V;
-                    const double corU = need_c ? gf * t * t * t * lambda * (T + (fx * fx + fy * fy + fz * fz)) : 0.0;
-                    return (mode == PGB_ACTION_BARE) ? bareU : (mode == PGB_ACTION_CORR) ? corU : bareU + corU;
+                    return assemble32(mode, need_c, vf, gf, t, lambda, V, T, fx, fy, fz);
                 };
                 res = action(need_v ? dd(q[0]) : 0.0, dd(q[2]), dd(q[4]), dd(q[5]), dd(q[6]));
                 if (both)
-                    res -= action(need_v ? dd(q[1]) : 0.0, dd(q[3]), dd(q[7]), dd(q[8]), dd(q[9]));
+                    res = __dsub_rn(res, action(need_v ? dd(q[1]) : 0.0, dd(q[3]), dd(q[7]), dd(q[8]), dd(q[9])));
             }
             out[b] = res;
         }
@@ -347,6 +369,326 @@ cudaError_t launch_bead_actions32_full(const PathView& v, AzizParams a, const in
     k_bead_actions32_full<<<(k + kBeadsPerBlock - 1) / kBeadsPerBlock, kWarpBeadBlock, 0, s>>>(
         v, make_aziz_f(a), d_beads, k, shift, mode, tau, lambda, vf[0], vf[1], gf[0], gf[1],
         d_over, d_force, delta, d_out);
+    return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
+// Many trials of few beads.  A trial's difference needs the bead's current
+// action and, for the gradient term, every partner's force less the bead's
+// own term: the same for all trials of the bead.  The trials are sorted by
+// bead on the device (count, offsets, scatter: the sorted record is the FP32
+// position and the trial's index), a warp takes a bead, evaluates its current
+// position once, keeps the partners (and those forces) in shared memory and
+// then makes the trials four at a time, so four independent chains of pair
+// arithmetic are in flight.  The sums of a group are reduced together by
+// recursive halving, in the butterfly's own tree, so every sum has the bits
+// k_bead_actions32_full gives it; the FP64 assembly runs one trial a lane.
+//
+// Bound: the issue rate, 47 instructions a pair (79 with the gradient), and
+// instruction fetch: the loops of both parities and the reductions together
+// are larger than the instruction caches, so the even slices' beads go first
+// and the reductions are not inlined (1.01 -> 0.87 ms).  10^6 trials, N = 256,
+// M = 250, GSF: 2.75 ms with both positions evaluated for every trial, 0.87 ms
+// here.
+// ---------------------------------------------------------------------------
+constexpr int kTrialWarps = 4;
+// Sorting pays from about three trials a bead on (N = 256, gradient: 2 a bead
+// 306 against 374 us, 4 a bead 398 against 719; N = 400: 2 a bead 227 against
+// 220, 4 a bead 282 against 395) once its three small launches, 12 us, are
+// less than the pairs saved (N = 64: 4 a bead, 32 k trials 58 against 54 us, 16
+// a bead 92 against 168; N = 16: 8 k trials 34 against 19).
+constexpr double kTrialsPerBead = 3.0;
+constexpr double kTrialPairs = 2.5e6;            // trials times partners
+
+__device__ __forceinline__ bool bead_active(const PathView& v, int2 b) {
+    return b.x >= 0 && b.x < v.M && b.y >= 0 && b.y < v.Ne && v.on[(size_t)b.x * v.Ne + b.y];
+}
+
+// each trial's rank among its bead's trials (kept in the first word of its
+// output until the scatter)
+__global__ void k_trial_count(PathView v, const int2* __restrict__ beads, int k, int* __restrict__ count,
+                              double* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= k) return;
+    const int2 b = beads[i];
+    if (bead_active(v, b)) *reinterpret_cast<int*>(out + i) = atomicAdd(count + (size_t)b.x * v.Ne + b.y, 1);
+}
+
+// a slice's beads get consecutive places; the slices any order
+__global__ void __launch_bounds__(256)
+k_trial_offsets(PathView v, const int* __restrict__ count, int* __restrict__ cursor, int* __restrict__ offset) {
+    __shared__ int wsum[8], s_base;
+    const int s = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int b0 = 0; b0 < v.Ne; b0 += 256) {
+        const int b = b0 + threadIdx.x;
+        const int c = b < v.Ne ? count[(size_t)s * v.Ne + b] : 0;
+        int x = c;
+        #pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) wsum[warp] = x;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int t = 0;
+            for (int w = 0; w < 8; ++w) { const int y = wsum[w]; wsum[w] = t; t += y; }
+            s_base = t ? atomicAdd(cursor, t) : 0;
+        }
+        __syncthreads();
+        if (b < v.Ne) offset[(size_t)s * v.Ne + b] = s_base + wsum[warp] + x - c;
+        __syncthreads();
+    }
+}
+
+__global__ void k_trial_scatter(PathView v, const int2* __restrict__ beads, const double* __restrict__ pos, int k,
+                                const int* __restrict__ offset, float4* __restrict__ sorted, double* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= k) return;
+    const int2 b = beads[i];
+    if (!bead_active(v, b)) { out[i] = 0.0; return; }
+    const int at = offset[(size_t)b.x * v.Ne + b.y] + *reinterpret_cast<const int*>(out + i);
+    sorted[at] = make_float4((float)pos[3 * (size_t)i], (float)pos[3 * (size_t)i + 1], (float)pos[3 * (size_t)i + 2],
+                             __int_as_float(i));
+}
+
+// one step of ff_butterfly's tree
+__device__ __forceinline__ float2 ff_add(float2 a, float2 b) {
+    const float sum = a.x + b.x;
+    const float bp = sum - a.x;
+    const float err = (a.x - (sum - bp)) + (b.x - bp);
+    return make_float2(sum, (a.y + b.y) + err);
+}
+__device__ __forceinline__ float2 ff_xor(float2 a, int o) {
+    return make_float2(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o));
+}
+// R sums over the warp; lane l returns sum l / (32 / R)
+template <int R>
+__device__ __forceinline__ float2 ff_halve(float2 (&x)[R], int lane) {
+    int o = 16;
+    #pragma unroll
+    for (int h = R / 2; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = lane & o;
+        #pragma unroll
+        for (int i = 0; i < h; ++i) x[i] = ff_add(up ? x[i + h] : x[i], ff_xor(up ? x[i] : x[i + h], o));
+    }
+    for (; o > 0; o >>= 1) x[0] = ff_add(x[0], ff_xor(x[0], o));
+    return x[0];
+}
+
+static __device__ __noinline__ float2 ff_sums4(float2 a, float2 b, float2 c, float2 d, int lane) {
+    float2 x[4] = {a, b, c, d};
+    return ff_halve<4>(x, lane);
+}
+static __device__ __noinline__ float2 ff_sums2(float2 a, float2 b, int lane) {
+    float2 x[2] = {a, b};
+    return ff_halve<2>(x, lane);
+}
+template <int R>
+__device__ __forceinline__ float2 ff_sums(float2 (&x)[R], int lane) {
+    if constexpr (R == 4) return ff_sums4(x[0], x[1], x[2], x[3], lane);
+    else return ff_sums2(x[0], x[1], lane);
+}
+
+struct BoxF { float L0, L1, L2, I0, I1, I2; };
+
+// what a warp keeps of up to 32 finished trials: V T F(3) at the trial
+// position, then at the current one, as (hi, lo)
+struct TrialBuffer {
+    float2 part[10][32];
+    int id[32], slice[32];
+};
+
+// R trials of one bead over the staged partners (P: position and pair factor,
+// negative for none; F: the partner's force less the bead's own term)
+template <int R, bool kC>
+__device__ __forceinline__ void trial_group(const float4* __restrict__ trial, int count, const float4* P, const float4* F,
+                                            int Ne, const BoxF& B, const AzizF& az, bool need_v, int lane, int slice,
+                                            const float2 (&old)[5], TrialBuffer& buf, int used) {
+    float4 r[R];
+    #pragma unroll
+    for (int i = 0; i < R; ++i) r[i] = trial[min(i, count - 1)];
+    KahanF vn[R], tn[R];
+    float fx[R], fy[R], fz[R];
+    #pragma unroll
+    for (int i = 0; i < R; ++i) fx[i] = fy[i] = fz[i] = 0.f;
+    for (int j = lane; j < Ne; j += 32) {
+        const float4 rj = P[j];
+        if (rj.w < 0.f) continue;
+        float4 f3 = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (kC) f3 = F[j];
+        #pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const float dx = min_image32(rj.x - r[i].x, B.L0, B.I0);
+            const float dy = min_image32(rj.y - r[i].y, B.L1, B.I1);
+            const float dz = min_image32(rj.z - r[i].z, B.L2, B.I2);
+            const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+            if (need_v) vn[i].add(rj.w * aziz_v32(r2, az));
+            if (kC) {
+                const float g = aziz_g32(r2, az);
+                const float F2x = g * dx, F2y = g * dy, F2z = g * dz;
+                fx[i] -= F2x; fy[i] -= F2y; fz[i] -= F2z;
+                tn[i].add(fmaf(2.0f, fmaf(F2x, f3.x, fmaf(F2y, f3.y, F2z * f3.z)),
+                               fmaf(F2x, F2x, fmaf(F2y, F2y, F2z * F2z))));
+            }
+        }
+    }
+    const int mine = lane / (32 / R), slot = used + mine;
+    const bool write = (lane & (32 / R - 1)) == 0 && mine < count;
+    float2 x[R], sum[5] = {};
+    #pragma unroll
+    for (int i = 0; i < R; ++i) x[i] = make_float2(vn[i].s, -vn[i].c);
+    sum[0] = ff_sums<R>(x, lane);
+    if (kC) {
+        #pragma unroll
+        for (int i = 0; i < R; ++i) x[i] = make_float2(tn[i].s, -tn[i].c);
+        sum[1] = ff_sums<R>(x, lane);
+        #pragma unroll
+        for (int i = 0; i < R; ++i) x[i] = make_float2(fx[i], 0.f);
+        sum[2] = ff_sums<R>(x, lane);
+        #pragma unroll
+        for (int i = 0; i < R; ++i) x[i] = make_float2(fy[i], 0.f);
+        sum[3] = ff_sums<R>(x, lane);
+        #pragma unroll
+        for (int i = 0; i < R; ++i) x[i] = make_float2(fz[i], 0.f);
+        sum[4] = ff_sums<R>(x, lane);
+    }
+    if (write) {
+        #pragma unroll
+        for (int q = 0; q < 5; ++q) { buf.part[q][slot] = sum[q]; buf.part[5 + q][slot] = old[q]; }
+        buf.id[slot] = __float_as_int(trial[mine].w);
+        buf.slice[slot] = slice;
+    }
+    __syncwarp();
+}
+
+__global__ void __launch_bounds__(kTrialWarps * 32, 5)
+k_trials32(PathView v, AzizF az, BoxF B, const int* __restrict__ count, const int* __restrict__ offset,
+           const float4* __restrict__ sorted, const float4* __restrict__ fall, int shift, int mode, double tau,
+           double lambda, double vf0, double vf1, double gf0, double gf1, double* __restrict__ out) {
+    extern __shared__ float4 sp[];
+    __shared__ TrialBuffer buffers[kTrialWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, Ne = v.Ne;
+    float4 *P = sp + (size_t)warp * 2 * Ne, *F = P + Ne;
+    TrialBuffer& buf = buffers[warp];
+    const bool need_v = (mode != PGB_ACTION_CORR);
+    auto corr = [&](int s) {
+        const double gf = s % 2 ? gf1 : gf0;
+        return (mode == PGB_ACTION_CORR) ? (gf > kEPS) : (mode == PGB_ACTION_FULL) ? (shift == 1 && gf > kEPS) : false;
+    };
+    const bool even_c = corr(0), odd_c = corr(1);
+    int used = 0;
+    auto flush = [&]() {
+        if (lane < used) {
+            const int s = buf.slice[lane];
+            const double vf = s % 2 ? vf1 : vf0, gf = s % 2 ? gf1 : gf0;
+            const double t = (double)shift * tau;
+            const bool need_c = s % 2 ? odd_c : even_c;
+            auto dd = [&](int q) { const float2 x = buf.part[q][lane]; return (double)x.x + (double)x.y; };
+            auto action = [&](double V, double T, double fx, double fy, double fz) {
+                return assemble32(mode, need_c, vf, gf, t, lambda, V, T, fx, fy, fz);
+            };
+            double res;
+            if (need_c) {
+                res = action(need_v ? dd(0) : 0.0, dd(1), dd(2), dd(3), dd(4));
+                res = __dsub_rn(res, action(need_v ? dd(5) : 0.0, dd(6), dd(7), dd(8), dd(9)));
+            } else {
+                res = action(need_v ? dd(0) : 0.0, 0.0, 0.0, 0.0, 0.0);
+                res = __dsub_rn(res, action(need_v ? dd(5) : 0.0, 0.0, 0.0, 0.0, 0.0));
+            }
+            out[buf.id[lane]] = res;
+        }
+        used = 0;
+        __syncwarp();
+    };
+    const size_t beads = (size_t)v.M * Ne;
+    for (size_t b = (size_t)blockIdx.x * kTrialWarps + warp; b < beads; b += (size_t)gridDim.x * kTrialWarps) {
+        // the even slices' beads, then the odd ones': an SM's warps run the
+        // same loops, whose code does not fit the instruction cache together
+        const int line = (int)(b / Ne), p = (int)(b - (size_t)line * Ne), evens = (v.M + 1) / 2;
+        const int s = line < evens ? 2 * line : 2 * (line - evens) + 1;
+        const size_t at = (size_t)s * Ne + p;
+        const int n = count[at];
+        if (n == 0) continue;
+        const bool need_c = s % 2 ? odd_c : even_c;
+        const float4* trial = sorted + offset[at];
+        // the current position, and the partners for the trials
+        const float4* R = v.pos32 + (size_t)s * Ne;
+        const float4* Fs = fall + (size_t)s * Ne;
+        const float4 rpo = R[p];
+        const int st1 = bead_state(v, s, p);
+        KahanF vo, to;
+        float fox = 0.f, foy = 0.f, foz = 0.f;
+        for (int j = lane; j < Ne; j += 32) {
+            if (j == p || !v.on[(size_t)s * Ne + j]) { P[j] = make_float4(0.f, 0.f, 0.f, -1.f); continue; }
+            const float4 rj = R[j];
+            const float fac = pair_factor32(st1, bead_state(v, s, j));
+            const float ox = min_image32(rj.x - rpo.x, B.L0, B.I0);
+            const float oy = min_image32(rj.y - rpo.y, B.L1, B.I1);
+            const float oz = min_image32(rj.z - rpo.z, B.L2, B.I2);
+            const float ro2 = fmaf(ox, ox, fmaf(oy, oy, oz * oz));
+            if (need_v) vo.add(fac * aziz_v32(ro2, az));
+            P[j] = make_float4(rj.x, rj.y, rj.z, fac);
+            if (need_c) {
+                const float go = aziz_g32(ro2, az);
+                const float Fox = go * ox, Foy = go * oy, Foz = go * oz;
+                const float4 fa = Fs[j];
+                // F3: the slice force on j less the term of p at its current position
+                const float F3x = fa.x - Fox, F3y = fa.y - Foy, F3z = fa.z - Foz;
+                fox -= Fox; foy -= Foy; foz -= Foz;
+                to.add(fmaf(2.0f, fmaf(Fox, F3x, fmaf(Foy, F3y, Foz * F3z)),
+                            fmaf(Fox, Fox, fmaf(Foy, Foy, Foz * Foz))));
+                F[j] = make_float4(F3x, F3y, F3z, 0.f);
+            }
+        }
+        float2 old[5] = {};
+        old[0] = warp_ff(vo);
+        if (need_c) {
+            old[1] = warp_ff(to);
+            old[2] = ff_butterfly(fox, 0.f); old[3] = ff_butterfly(foy, 0.f); old[4] = ff_butterfly(foz, 0.f);
+        }
+        __syncwarp();
+        for (int i = 0; i < n;) {
+            const int left = n - i, take = left >= 3 ? min(left, 4) : left;
+            if (used + take > 32) flush();
+            if (take >= 3) {
+                if (need_c) trial_group<4, true>(trial + i, take, P, F, Ne, B, az, need_v, lane, s, old, buf, used);
+                else trial_group<4, false>(trial + i, take, P, F, Ne, B, az, need_v, lane, s, old, buf, used);
+            } else {
+                if (need_c) trial_group<2, true>(trial + i, take, P, F, Ne, B, az, need_v, lane, s, old, buf, used);
+                else trial_group<2, false>(trial + i, take, P, F, Ne, B, az, need_v, lane, s, old, buf, used);
+            }
+            used += take;
+            i += take;
+        }
+    }
+    flush();
+}
+
+bool trials32_sorted(const PathView& v, int k) {
+    return (double)k >= kTrialsPerBead * v.M * v.Ne && (double)k * v.Ne >= kTrialPairs &&
+           (size_t)v.Ne * 2 * kTrialWarps * sizeof(float4) <= 160 * 1024;
+}
+
+cudaError_t launch_trials32(const PathView& v, AzizParams a, const int2* d_beads, int k, int shift, int mode, double tau,
+                            double lambda, const double vf[2], const double gf[2], const double* d_pos,
+                            const float4* d_force, int* d_count, float4* d_sorted, double* d_out, cudaStream_t s) {
+    const size_t nb = (size_t)v.M * v.Ne, smem = (size_t)v.Ne * 2 * kTrialWarps * sizeof(float4);
+    int *offset = d_count + nb + 1, *cursor = d_count + nb;
+    cudaError_t e = set_smem_limit(k_trials32, 160 * 1024);
+    if (e != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(d_count, 0, (nb + 1) * sizeof(int), s)) != cudaSuccess) return e;
+    const int blocks = (k + 255) / 256;
+    k_trial_count<<<blocks, 256, 0, s>>>(v, d_beads, k, d_count, d_out);
+    k_trial_offsets<<<v.M, 256, 0, s>>>(v, d_count, cursor, offset);
+    k_trial_scatter<<<blocks, 256, 0, s>>>(v, d_beads, d_pos, k, offset, d_sorted, d_out);
+    const BoxF B{(float)v.side[0], (float)v.side[1], (float)v.side[2], (float)v.sideInv[0], (float)v.sideInv[1], (float)v.sideInv[2]};
+    // two beads a warp: the assembly's lanes half full, the CTAs short enough
+    // to even out (eight beads a warp 1.05 ms, two 1.01)
+    const size_t each = std::max<size_t>(1, std::min<size_t>(2, nb / (152 * 16)));
+    const int grid = (int)((nb + kTrialWarps * each - 1) / (kTrialWarps * each));
+    k_trials32<<<grid, kTrialWarps * 32, smem, s>>>(v, make_aziz_f(a), B, d_count, offset, d_sorted, d_force, shift, mode,
+                                                    tau, lambda, vf[0], vf[1], gf[0], gf[1], d_out);
     return cudaGetLastError();
 }
 

@@ -83,6 +83,7 @@ struct Ctx {
     void* d_tc_tables = nullptr;   // split-BF16 DFT and cosine matrices of this M (built once)
     float4* d_force32 = nullptr;   // per-bead same-slice forces of the current configuration
     bool force_valid = false;      // cleared by every position change
+    int* d_trial_count = nullptr;  // counters and places of trials sorted by bead (mixed form)
     unsigned* d_arrived = nullptr; // M arrival counters of kernels whose last CTA adds up (zero between calls)
     double* d_force64 = nullptr;   // scratch of the FP64 many-bead form: slice forces [M][3][Ne]
     void* h_pinned = nullptr; size_t pinned_bytes = 0;
@@ -165,6 +166,12 @@ cudaError_t launch_bead_actions32_full(const PathView& v, AzizParams az, const i
                                        const double vf[2], const double gf[2], const double* d_over,
                                        const float4* d_force, int delta, double* d_out,
                                        cudaStream_t s);
+// trials sorted by bead, for whole lists and enough trials a bead
+// (trials32_sorted): d_count 2 M Ne + 1 ints, d_sorted k records
+bool trials32_sorted(const PathView& v, int k);
+cudaError_t launch_trials32(const PathView& v, AzizParams a, const int2* d_beads, int k, int shift, int mode, double tau,
+                            double lambda, const double vf[2], const double gf[2], const double* d_pos,
+                            const float4* d_force, int* d_count, float4* d_sorted, double* d_out, cudaStream_t s);
 // F[t][b] = sum over active b3 != b of gradV(r_b - r_b3) on slice t, FP32 [M][Ne]
 cudaError_t launch_slice_forces32(const PathView& v, AzizParams az, float4* d_force, cudaStream_t s);
 cudaError_t launch_slice_terms32(const PathView& v, AzizParams az, int window,
