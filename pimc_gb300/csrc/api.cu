@@ -168,11 +168,11 @@ int compute_terms(Ctx& c, std::vector<double>& h, TermsWanted want) {
     int rc = need_path(c); if (rc) return rc;
     PathView v = c.view();
     size_t bytes = (size_t)8 * c.M * sizeof(double);
-    rc = c.ensure_scratch(c.p.precision == PGB_MIXED ? bytes : slice_terms64_work(v)); if (rc) return rc;
+    rc = c.ensure_scratch(c.p.precision == PGB_MIXED ? slice_terms32_work(v) : slice_terms64_work(v)); if (rc) return rc;
     double* d = static_cast<double*>(c.d_scratch);
     int window = c.p.virial_window > 0 ? c.p.virial_window : 5;
     cudaError_t e = (c.p.precision == PGB_MIXED)
-        ? launch_slice_terms32(v, c.az, window, d, c.stream)
+        ? launch_slice_terms32(v, c.az, want.window ? window : 0, want.even, want.odd, c.d_arrived, d, c.stream)
         : launch_slice_terms64(v, want.window ? window : 0, want.even, want.odd, c.d_arrived, d, c.stream);
     if (e != cudaSuccess) return c.cuda_fail(e, "slice terms launch");
     h.assign((size_t)8 * c.M, 0.0);

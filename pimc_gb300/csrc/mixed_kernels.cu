@@ -28,6 +28,14 @@ cudaError_t launch_pos32_from64(const PathView& v, float4* d_pos32, cudaStream_t
     return cudaGetLastError();
 }
 
+// The box in FP32, made on the host: in a kernel the six conversions take the
+// FP64 pipe 16 clocks each, for every warp.
+struct BoxF { float L0, L1, L2, I0, I1, I2; };
+static BoxF box_f(const PathView& v) {
+    return {(float)v.side[0], (float)v.side[1], (float)v.side[2],
+            (float)v.sideInv[0], (float)v.sideInv[1], (float)v.sideInv[2]};
+}
+
 // d^2V/dr^2 in FP32 (potential.cpp:1877-1907 with d2F of potential.h:976-983)
 __device__ __forceinline__ float aziz_d2v32(float r2, const AzizF& a) {
     float rinv = rsqrtf(r2);
@@ -490,8 +498,6 @@ __device__ __forceinline__ float2 ff_sums(float2 (&x)[R], int lane) {
     else return ff_sums2(x[0], x[1], lane);
 }
 
-struct BoxF { float L0, L1, L2, I0, I1, I2; };
-
 // what a warp keeps of up to 32 finished trials: V T F(3) at the trial
 // position, then at the current one, as (hi, lo)
 struct TrialBuffer {
@@ -682,7 +688,7 @@ cudaError_t launch_trials32(const PathView& v, AzizParams a, const int2* d_beads
     k_trial_count<<<blocks, 256, 0, s>>>(v, d_beads, k, d_count, d_out);
     k_trial_offsets<<<v.M, 256, 0, s>>>(v, d_count, cursor, offset);
     k_trial_scatter<<<blocks, 256, 0, s>>>(v, d_beads, d_pos, k, offset, d_sorted, d_out);
-    const BoxF B{(float)v.side[0], (float)v.side[1], (float)v.side[2], (float)v.sideInv[0], (float)v.sideInv[1], (float)v.sideInv[2]};
+    const BoxF B = box_f(v);
     // two beads a warp: the assembly's lanes half full, the CTAs short enough
     // to even out (eight beads a warp 1.05 ms, two 1.01)
     const size_t each = std::max<size_t>(1, std::min<size_t>(2, nb / (152 * 16)));
@@ -738,120 +744,236 @@ cudaError_t launch_slice_forces32(const PathView& v, AzizParams a, float4* d_for
     return cudaGetLastError();
 }
 
-// Mixed-precision per-slice estimator terms; same outputs and layout as
-// k_slice_terms64 (vint, g2, r1, r2, d1, d2, kin, xch).
-constexpr int kSliceBlock32 = 128;
+// Mixed-precision per-slice estimator terms; same outputs, layout and levels
+// as k_slice_terms64 (vint, g2, r1, r2, d1, d2, kin, xch).
+//
+// A bead's force and T matrix are FP32 sums over its partners in index order,
+// one thread a bead.  Column c < 128 of a slice collects the beads c, c + 128,
+// ... in Kahan sums, the potential of the pairs b2 > b1 and the beads' other
+// terms; a Kahan sum depends on its order, so this one is kept whatever the
+// launch.  64 beads a CTA, so that 250 slices of 256 beads give every
+// sub-partition three warps instead of one and a half, with four pairs in
+// flight; a column's potential stays with its first bead's thread, the beads'
+// other terms go through memory to the last CTA of the slice.
+//
+// Bound: latency at this occupancy, then the issue rate (about 55 instructions
+// a pair, 100 with the T matrix).  Energy and virial of 256 beads, 250 slices,
+// GSF: 2 x 138 us with everything computed by 128 threads a slice, 162 us both
+// here.
+constexpr int kSliceRows32 = 64, kSliceColumns32 = 128;
 
-__global__ void __launch_bounds__(kSliceBlock32)
-k_slice_terms32(PathView v, AzizF az, int window, double* __restrict__ terms) {
-    extern __shared__ float4 sp[];
-    __shared__ double red[kSliceBlock32 / 32];
-    const int s = blockIdx.x, Ne = v.Ne, n = v.nbs[s];
-    const float L0 = (float)v.side[0], L1 = (float)v.side[1], L2 = (float)v.side[2];
-    const float I0 = (float)v.sideInv[0], I1 = (float)v.sideInv[1], I2 = (float)v.sideInv[2];
-    for (int j = threadIdx.x; j < n; j += blockDim.x) sp[j] = v.pos32[(size_t)s * Ne + j];
-    __syncthreads();
-    KahanF a_vint, a_g2, a_r1, a_r2, a_d1, a_d2, a_kin, a_xch;
-    for (int b1 = threadIdx.x; b1 < n; b1 += blockDim.x) {
-        float4 r1 = sp[b1];
-        int st1 = bead_state(v, s, b1);
+// adds x to a Kahan sum where `take`, without a branch
+__device__ __forceinline__ void kahan_add_if(KahanF& k, float x, bool take) {
+    const float y = x - k.c, t = k.s + y, c = (t - k.s) - y;
+    k.s = take ? t : k.s;
+    k.c = take ? c : k.c;
+}
+// keeps the rounding of x: it is not merged into the addition it goes to
+__device__ __forceinline__ float rounded(float x) { asm("" : "+f"(x)); return x; }
+
+struct SliceRow32 {
+    const PathView& v;
+    const AzizF& az;
+    const BoxF& B;
+    const float4* sp;
+    int s, n;
+    bool worm;
+    __device__ __forceinline__ float factor(int st1, int b2) const {
+        return worm ? (float)pair_factor(st1, bead_state(v, s, b2)) : 1.0f;
+    }
+    __device__ __forceinline__ int state(int b1) const { return worm ? bead_state(v, s, b1) : 2; }
+    // the potential of bead b1's pairs with the beads behind it
+    __device__ __forceinline__ void potential(int b1, KahanF& vint) const {
+        const float4 r1 = sp[b1];
+        const int st1 = state(b1);
+        #pragma unroll 4
+        for (int b2 = b1 + 1; b2 < n; ++b2) {
+            const float4 r2 = sp[b2];
+            const float dx = min_image32(r1.x - r2.x, B.L0, B.I0);
+            const float dy = min_image32(r1.y - r2.y, B.L1, B.I1);
+            const float dz = min_image32(r1.z - r2.z, B.L2, B.I2);
+            const float V = rounded(aziz_v32(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), az));
+            vint.add(factor(st1, b2) * V);
+        }
+    }
+    // bead b1's force and T matrix (xx xy xz yy yz zz) over all partners, and
+    // for kV the potential of the pairs behind it
+    template <bool kT, bool kV>
+    __device__ __forceinline__ void forces(int b1, float (&F)[3], float (&T)[6], KahanF& vint) const {
+        const float4 r1 = sp[b1];
+        const int st1 = state(b1);
         float Fx = 0.f, Fy = 0.f, Fz = 0.f;
         float T00 = 0.f, T01 = 0.f, T02 = 0.f, T11 = 0.f, T12 = 0.f, T22 = 0.f;
+        #pragma unroll 4
         for (int b2 = 0; b2 < n; ++b2) {
-            if (b2 == b1) continue;
-            float4 r2 = sp[b2];
-            float dx = min_image32(r1.x - r2.x, L0, I0);
-            float dy = min_image32(r1.y - r2.y, L1, I1);
-            float dz = min_image32(r1.z - r2.z, L2, I2);
-            float rr = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+            // the bead itself: separation 0, force coefficient 0
+            const bool self = b2 == b1;
+            const float4 r2 = sp[b2];
+            const float dx = min_image32(r1.x - r2.x, B.L0, B.I0);
+            const float dy = min_image32(r1.y - r2.y, B.L1, B.I1);
+            const float dz = min_image32(r1.z - r2.z, B.L2, B.I2);
+            const float rr = self ? 1.0f : fmaf(dx, dx, fmaf(dy, dy, dz * dz));
             float V, g;
             aziz_vg32(rr, az, V, g);
+            g = self ? 0.0f : g;
             Fx = fmaf(g, dx, Fx); Fy = fmaf(g, dy, Fy); Fz = fmaf(g, dz, Fz);
-            if (b2 > b1) a_vint.add((float)pair_factor(st1, bead_state(v, s, b2)) * V);
-            // T-matrix: (d2V/r^2 - |dV|/r^3) r r^T + |dV|/r I
-            float rinv = rsqrtf(rr);
-            float dV = fabsf(g) * rr * rinv;
-            float d2V = aziz_d2v32(rr, az);
-            float c1 = (d2V - dV * rinv) * rinv * rinv;
-            float c0 = dV * rinv;
-            T00 = fmaf(c1, dx * dx, T00 + c0); T11 = fmaf(c1, dy * dy, T11 + c0);
-            T22 = fmaf(c1, dz * dz, T22 + c0);
-            T01 = fmaf(c1, dx * dy, T01); T02 = fmaf(c1, dx * dz, T02); T12 = fmaf(c1, dy * dz, T12);
+            if (kV) kahan_add_if(vint, factor(st1, b2) * rounded(V), b2 > b1);
+            if (kT) {
+                // T-matrix: (d2V/r^2 - |dV|/r^3) r r^T + |dV|/r I
+                const float rinv = rsqrtf(rr);
+                const float dV = fabsf(g) * rr * rinv;
+                const float d2V = aziz_d2v32(rr, az);
+                const float c1 = (d2V - dV * rinv) * rinv * rinv;
+                const float c0 = dV * rinv;
+                T00 = fmaf(c1, dx * dx, T00 + c0); T11 = fmaf(c1, dy * dy, T11 + c0);
+                T22 = fmaf(c1, dz * dz, T22 + c0);
+                T01 = fmaf(c1, dx * dy, T01); T02 = fmaf(c1, dx * dz, T02); T12 = fmaf(c1, dy * dz, T12);
+            }
         }
-        a_g2.add(fmaf(Fx, Fx, fmaf(Fy, Fy, Fz * Fz)));
-        a_r1.add(fmaf(Fx, r1.x, fmaf(Fy, r1.y, Fz * r1.z)));
-        float TFx = fmaf(T00, Fx, fmaf(T01, Fy, T02 * Fz));
-        float TFy = fmaf(T01, Fx, fmaf(T11, Fy, T12 * Fz));
-        float TFz = fmaf(T02, Fx, fmaf(T12, Fy, T22 * Fz));
-        a_r2.add(fmaf(TFx, r1.x, fmaf(TFy, r1.y, TFz * r1.z)));
-        if (window > 0) {
-            float mx = 0, my = 0, mz = 0, lx = 0, ly = 0, lz = 0, cx = 0, cy = 0, cz = 0;
-            int2 cn = make_int2(s, b1), cp = cn;
-            float4 pn = r1, pp = r1;
-            for (int gm = 0; gm < window; ++gm) {
-                if (gm > 0) {
-                    cn = v.next[(size_t)cn.x * Ne + cn.y];
-                    cp = v.prev[(size_t)cp.x * Ne + cp.y];
+        F[0] = Fx; F[1] = Fy; F[2] = Fz;
+        T[0] = T00; T[1] = T01; T[2] = T02; T[3] = T11; T[4] = T12; T[5] = T22;
+    }
+};
+
+// work: [M][9][Ne] floats, the beads' terms 1..7 and the columns' potential as
+// Kahan pairs in 0 and 8
+__global__ void __launch_bounds__(kSliceRows32)
+k_slice_terms32(PathView v, AzizF az, BoxF B, int window, int even, int odd, unsigned* __restrict__ arrived,
+                float* __restrict__ work, double* __restrict__ terms) {
+    extern __shared__ float4 sp[];
+    __shared__ double sums[8][kSliceRows32 / 32];
+    __shared__ bool last;
+    const int s = blockIdx.x, Ne = v.Ne, n = v.nbs[s], nblk = gridDim.y, tid = threadIdx.x;
+    const int level = s % 2 ? odd : even, b1 = blockIdx.y * kSliceRows32 + tid;
+    if (level > kSliceNone) {
+        for (int j = tid; j < n; j += kSliceRows32) sp[j] = v.pos32[(size_t)s * Ne + j];
+        __syncthreads();
+    }
+    const SliceRow32 row{v, az, B, sp, s, n,
+                         s == v.worm[0] || s == v.worm[2] || s == v.worm[4] || s == v.worm[6]};
+    float* W = work + (size_t)s * 9 * Ne;
+    if (b1 < n) {
+        const float4 r1 = v.pos32[(size_t)s * Ne + b1];
+        const bool column = b1 < kSliceColumns32;
+        float val[8] = {};
+        KahanF vint;
+        if (level == kSliceV && column) row.potential(b1, vint);
+        else if (level >= kSliceF) {
+            float F[3], T[6];
+            if (level == kSliceT) {
+                if (blockIdx.y < 2) row.forces<true, true>(b1, F, T, vint);
+                else row.forces<true, false>(b1, F, T, vint);
+            } else {
+                if (blockIdx.y < 2) row.forces<false, true>(b1, F, T, vint);
+                else row.forces<false, false>(b1, F, T, vint);
+            }
+            const float Fx = F[0], Fy = F[1], Fz = F[2];
+            val[1] = fmaf(Fx, Fx, fmaf(Fy, Fy, Fz * Fz));
+            if (window > 0) {
+                val[2] = fmaf(Fx, r1.x, fmaf(Fy, r1.y, Fz * r1.z));
+                const float TFx = fmaf(T[0], Fx, fmaf(T[1], Fy, T[2] * Fz));
+                const float TFy = fmaf(T[1], Fx, fmaf(T[3], Fy, T[4] * Fz));
+                const float TFz = fmaf(T[2], Fx, fmaf(T[4], Fy, T[5] * Fz));
+                val[3] = fmaf(TFx, r1.x, fmaf(TFy, r1.y, TFz * r1.z));
+                float mx = 0, my = 0, mz = 0, lx = 0, ly = 0, lz = 0, cx = 0, cy = 0, cz = 0;
+                int2 cn = make_int2(s, b1), cp = cn;
+                float4 pn = r1, pp = r1;
+                for (int gm = 0; gm < window; ++gm) {
+                    if (gm > 0) {
+                        if (cn.x >= 0) cn = v.next[(size_t)cn.x * Ne + cn.y];
+                        if (cp.x >= 0) cp = v.prev[(size_t)cp.x * Ne + cp.y];
+                    }
+                    // an open end stops the walk
+                    const float4 qn = cn.x >= 0 ? v.pos32[(size_t)cn.x * Ne + cn.y] : pn;
+                    const float4 qp = cp.x >= 0 ? v.pos32[(size_t)cp.x * Ne + cp.y] : pp;
+                    mx += min_image32(qn.x - pn.x, B.L0, B.I0); my += min_image32(qn.y - pn.y, B.L1, B.I1);
+                    mz += min_image32(qn.z - pn.z, B.L2, B.I2);
+                    lx += min_image32(qp.x - pp.x, B.L0, B.I0); ly += min_image32(qp.y - pp.y, B.L1, B.I1);
+                    lz += min_image32(qp.z - pp.z, B.L2, B.I2);
+                    cx += (r1.x + mx) + (r1.x + lx); cy += (r1.y + my) + (r1.y + ly);
+                    cz += (r1.z + mz) + (r1.z + lz);
+                    pn = qn; pp = qp;
                 }
-                float4 qn = v.pos32[(size_t)cn.x * Ne + cn.y], qp = v.pos32[(size_t)cp.x * Ne + cp.y];
-                mx += min_image32(qn.x - pn.x, L0, I0); my += min_image32(qn.y - pn.y, L1, I1);
-                mz += min_image32(qn.z - pn.z, L2, I2);
-                lx += min_image32(qp.x - pp.x, L0, I0); ly += min_image32(qp.y - pp.y, L1, I1);
-                lz += min_image32(qp.z - pp.z, L2, I2);
-                cx += (r1.x + mx) + (r1.x + lx); cy += (r1.y + my) + (r1.y + ly);
-                cz += (r1.z + mz) + (r1.z + lz);
-                pn = qn; pp = qp;
+                float den = 1.0f / (2.0f * window);
+                float dlx = min_image32(r1.x - cx * den, B.L0, B.I0);
+                float dly = min_image32(r1.y - cy * den, B.L1, B.I1);
+                float dlz = min_image32(r1.z - cz * den, B.L2, B.I2);
+                val[4] = fmaf(Fx, dlx, fmaf(Fy, dly, Fz * dlz));
+                val[5] = fmaf(TFx, dlx, fmaf(TFy, dly, TFz * dlz));
+                float v1x = 0, v1y = 0, v1z = 0;
+                int2 c2 = make_int2(s, b1);
+                float4 po = r1;
+                float v2x = 0, v2y = 0, v2z = 0;
+                for (int gm = 1; gm <= window; ++gm) {
+                    c2 = v.next[(size_t)c2.x * Ne + c2.y];
+                    if (c2.x < 0) break;
+                    float4 q = v.pos32[(size_t)c2.x * Ne + c2.y];
+                    const float ex = min_image32(q.x - po.x, B.L0, B.I0), ey = min_image32(q.y - po.y, B.L1, B.I1);
+                    const float ez = min_image32(q.z - po.z, B.L2, B.I2);
+                    v1x += ex; v1y += ey; v1z += ez;
+                    if (gm == 1) { v2x = ex; v2y = ey; v2z = ez; }
+                    po = q;
+                }
+                val[7] = fmaf(v1x, v2x, fmaf(v1y, v2y, v1z * v2z));
             }
-            float den = 1.0f / (2.0f * window);
-            float dlx = min_image32(r1.x - cx * den, L0, I0);
-            float dly = min_image32(r1.y - cy * den, L1, I1);
-            float dlz = min_image32(r1.z - cz * den, L2, I2);
-            a_d1.add(fmaf(Fx, dlx, fmaf(Fy, dly, Fz * dlz)));
-            a_d2.add(fmaf(TFx, dlx, fmaf(TFy, dly, TFz * dlz)));
-            float v1x = 0, v1y = 0, v1z = 0;
-            int2 c2 = make_int2(s, b1);
-            float4 po = r1;
-            for (int gm = 1; gm <= window; ++gm) {
-                c2 = v.next[(size_t)c2.x * Ne + c2.y];
-                float4 q = v.pos32[(size_t)c2.x * Ne + c2.y];
-                v1x += min_image32(q.x - po.x, L0, I0); v1y += min_image32(q.y - po.y, L1, I1);
-                v1z += min_image32(q.z - po.z, L2, I2);
-                po = q;
-            }
-            int2 nx = v.next[(size_t)s * Ne + b1];
-            float v2x = 0, v2y = 0, v2z = 0;
-            if (!(nx.x == kXXX && nx.y == kXXX)) {
-                float4 q = v.pos32[(size_t)nx.x * Ne + nx.y];
-                v2x = min_image32(q.x - r1.x, L0, I0); v2y = min_image32(q.y - r1.y, L1, I1);
-                v2z = min_image32(q.z - r1.z, L2, I2);
-            }
-            a_xch.add(fmaf(v1x, v2x, fmaf(v1y, v2y, v1z * v2z)));
         }
         int2 nx = v.next[(size_t)s * Ne + b1];
         if (!(nx.x == kXXX && nx.y == kXXX)) {
             float4 q = v.pos32[(size_t)nx.x * Ne + nx.y];
-            float ax = min_image32(q.x - r1.x, L0, I0), ay = min_image32(q.y - r1.y, L1, I1);
-            float az_ = min_image32(q.z - r1.z, L2, I2);
-            a_kin.add(fmaf(ax, ax, fmaf(ay, ay, az_ * az_)));
+            float ax = min_image32(q.x - r1.x, B.L0, B.I0), ay = min_image32(q.y - r1.y, B.L1, B.I1);
+            float az_ = min_image32(q.z - r1.z, B.L2, B.I2);
+            val[6] = fmaf(ax, ax, fmaf(ay, ay, az_ * az_));
         }
+        if (column && level > kSliceNone)
+            for (int b = b1 + kSliceColumns32; b < n; b += kSliceColumns32) row.potential(b, vint);
+        #pragma unroll
+        for (int q = 1; q < 8; ++q) W[(size_t)q * Ne + b1] = val[q];
+        if (column) { W[b1] = vint.s; W[(size_t)8 * Ne + b1] = vint.c; }
+        __threadfence();
     }
-    double vals[8] = {a_vint.value(), a_g2.value(), a_r1.value(), a_r2.value(),
-                      a_d1.value(), a_d2.value(), a_kin.value(), a_xch.value()};
-    #pragma unroll
+    __syncthreads();
+    if (nblk > 1) {
+        if (tid == 0) last = atomicInc(arrived + s, nblk - 1) == nblk - 1;      // back to 0 for the next call
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+    }
+    // the columns' sums, in double-float over the warp, FP64 from there on
+    #pragma unroll 1
     for (int q = 0; q < 8; ++q) {
-        double t = block_sum(vals[q], red);
-        if (threadIdx.x == 0) terms[(size_t)q * v.M + s] = t;
+        float2 t = make_float2(0.f, 0.f);
+        for (int c = tid; c < kSliceColumns32; c += kSliceRows32) {
+            KahanF k;
+            if (q == 0) {
+                if (c < n) { k.s = __ldcg(W + c); k.c = __ldcg(W + (size_t)8 * Ne + c); }
+            } else
+                for (int b = c; b < n; b += kSliceColumns32) k.add(__ldcg(W + (size_t)q * Ne + b));
+            const float2 u = warp_ff(k);
+            const float sum = t.x + u.x, bp = sum - t.x;
+            t = make_float2(sum, (t.y + u.y) + ((t.x - (sum - bp)) + (u.x - bp)));
+        }
+        if ((tid & 31) == 0) sums[q][tid >> 5] = (double)t.x + (double)t.y;
     }
+    __syncthreads();
+    if (tid < 8) terms[(size_t)tid * v.M + s] = sums[tid][0] + sums[tid][1];
 }
 
-cudaError_t launch_slice_terms32(const PathView& v, AzizParams a, int window, double* d_terms,
-                                 cudaStream_t s) {
+static int slice_blocks32(int Ne) { return (Ne + kSliceRows32 - 1) / kSliceRows32; }
+
+size_t slice_terms32_work(const PathView& v) {
+    return (size_t)8 * v.M * sizeof(double) + (size_t)9 * v.M * v.Ne * sizeof(float);
+}
+
+cudaError_t launch_slice_terms32(const PathView& v, AzizParams a, int window, int even, int odd, unsigned* d_arrived,
+                                 double* d_terms, cudaStream_t s) {
     size_t smem = (size_t)v.Ne * sizeof(float4);
     {
         const cudaError_t ae = set_smem_limit(k_slice_terms32, 200 * 1024);
         if (ae != cudaSuccess) return ae;
     }
-    k_slice_terms32<<<v.M, kSliceBlock32, smem, s>>>(v, make_aziz_f(a), window, d_terms);
+    k_slice_terms32<<<dim3(v.M, slice_blocks32(v.Ne)), kSliceRows32, smem, s>>>(
+        v, make_aziz_f(a), box_f(v), window, even, odd, d_arrived,
+        reinterpret_cast<float*>(d_terms + (size_t)8 * v.M), d_terms);
     return cudaGetLastError();
 }
 

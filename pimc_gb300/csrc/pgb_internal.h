@@ -174,7 +174,9 @@ cudaError_t launch_trials32(const PathView& v, AzizParams a, const int2* d_beads
                             const float4* d_force, int* d_count, float4* d_sorted, double* d_out, cudaStream_t s);
 // F[t][b] = sum over active b3 != b of gradV(r_b - r_b3) on slice t, FP32 [M][Ne]
 cudaError_t launch_slice_forces32(const PathView& v, AzizParams az, float4* d_force, cudaStream_t s);
-cudaError_t launch_slice_terms32(const PathView& v, AzizParams az, int window,
+// as launch_slice_terms64, with slice_terms32_work(v) bytes
+size_t slice_terms32_work(const PathView& v);
+cudaError_t launch_slice_terms32(const PathView& v, AzizParams az, int window, int even, int odd, unsigned* d_arrived,
                                  double* d_terms, cudaStream_t s);
 cudaError_t launch_pos32_from64(const PathView& v, float4* d_pos32,
                                 cudaStream_t s);

@@ -7,6 +7,8 @@
 //     S(q)     = 1/(N M) sum_t |rho_q(t)|^2
 //     F(q,tau) = 1/(N M) sum_t Re[rho_q(t) conj(rho_q(t+tau))]
 // which turns O(Q M N^2) (S) and O(Q M^2 N^2) (F) into O(Q M N) + O(Q M^2).
+#include <algorithm>
+
 #include "pgb_device.cuh"
 
 namespace pgb {
@@ -159,85 +161,147 @@ cudaError_t launch_rhoq32(const PathView& v, const double* d_q, int nq, float2* 
     return cudaGetLastError();
 }
 
-__global__ void k_ssf_from_rho32(const float2* __restrict__ rho, int nq, int M, double norm,
-                                 double* __restrict__ out) {
-    __shared__ double red[8];
-    int iq = blockIdx.x;
-    double acc = 0.0;
-    for (int t = threadIdx.x; t < M; t += blockDim.x) {
-        float2 r = rho[(size_t)iq * M + t];
-        acc += (double)r.x * r.x + (double)r.y * r.y;
+// S(q) = norm sum_t |rho_q(t)|^2, one warp a wave vector: four FP64
+// instructions a density, the FP64 pipe the bound, and one reduction a vector
+// instead of eight.  2048 vectors, M = 512: 26 -> 13 us.
+constexpr int kSsfBlock = 128;
+
+__global__ void __launch_bounds__(kSsfBlock)
+k_ssf_from_rho32(const float2* __restrict__ rho, int nq, int M, double norm, double* __restrict__ out) {
+    const int iq = blockIdx.x * (kSsfBlock / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (iq >= nq) return;
+    double re = 0.0, im = 0.0;
+    #pragma unroll 4
+    for (int t = lane; t < M; t += 32) {
+        const float2 r = rho[(size_t)iq * M + t];
+        const double x = r.x, y = r.y;
+        re = __fma_rn(x, x, re);
+        im = __fma_rn(y, y, im);
     }
-    double s = block_sum(acc, red);
-    if (threadIdx.x == 0) out[iq] = s * norm;
+    const double s = warp_sum(re + im);
+    if (lane == 0) out[iq] = s * norm;
 }
 
 cudaError_t launch_ssf_from_rho32(const float2* d_rho, int nq, int M, double norm,
                                   double* d_out, cudaStream_t s) {
     if (nq <= 0) return cudaSuccess;
-    k_ssf_from_rho32<<<nq, 256, 0, s>>>(d_rho, nq, M, norm, d_out);
+    constexpr int each = kSsfBlock / 32;
+    k_ssf_from_rho32<<<(nq + each - 1) / each, kSsfBlock, 0, s>>>(d_rho, nq, M, norm, d_out);
     return cudaGetLastError();
 }
 
-// CUDA-core circular correlation: one CTA per q, rho_q staged in shared
-// memory, each thread owns kTauPerThread consecutive tau and slides a
-// register window along t (one new shared load per kTauPerThread FMAs pairs).
+// CUDA-core circular correlation: each thread owns kTauPerThread consecutive
+// tau of one wave vector and slides a register window along t, one new shared
+// load and one broadcast for kTauPerThread complex multiply-adds; sums of 64
+// terms in FP32, those in FP64.  Several vectors share a CTA, so that its
+// lanes are full (a vector needs (M/2 + 1)/8 threads); their densities are
+// repeated beyond M for the window, with one entry of padding in eight, so
+// that the threads' windows, eight entries apart, fall into different banks.
+// 1579 vectors, M = 250: 36 us with one vector a CTA, a modulo a step and the
+// windows in four banks, 25 us here.
 constexpr int kTauPerThread = 8;
+constexpr int kIsfBlock = 128;
 
-__global__ void k_isf_direct32(const float2* __restrict__ rho, int nq, int M, double norm,
-                               double* __restrict__ out) {
+__host__ __device__ __forceinline__ int isf_pad(int i) { return i + (i >> 3); }
+// float2 entries a vector takes: M + the last window's end, padded
+__host__ __device__ __forceinline__ int isf_row(int M) { return isf_pad(M + M / 2 + 1 + 2 * kTauPerThread) + 1; }
+
+__global__ void __launch_bounds__(kIsfBlock)
+k_isf_direct32(const float2* __restrict__ rho, int nq, int M, int each, int per, double norm,
+               double* __restrict__ out) {
     extern __shared__ float2 sr[];
-    const int iq = blockIdx.x;
-    const int nt = M / 2 + 1;
-    for (int t = threadIdx.x; t < M; t += blockDim.x) sr[t] = rho[(size_t)iq * M + t];
+    const int nt = M / 2 + 1, row = isf_row(M), ext = M + nt + 2 * kTauPerThread;
+    const int q0 = blockIdx.x * each, qn = min(each, nq - q0);
+    for (int q = 0; q < qn; ++q)
+        for (int t = threadIdx.x; t < ext; t += kIsfBlock)
+            sr[q * row + isf_pad(t)] = rho[(size_t)(q0 + q) * M + t % M];
     __syncthreads();
-    for (int tau0 = threadIdx.x * kTauPerThread; tau0 < nt; tau0 += blockDim.x * kTauPerThread) {
+    for (int w = threadIdx.x; w < qn * per; w += kIsfBlock) {
+        const int q = w / per, tau0 = (w - q * per) * kTauPerThread;
+        const float2* S = sr + q * row;
         double acc[kTauPerThread];
-        float win_r[kTauPerThread], win_i[kTauPerThread];
+        float2 win[kTauPerThread];
         #pragma unroll
-        for (int k = 0; k < kTauPerThread; ++k) {
-            acc[k] = 0.0;
-            int t2 = (tau0 + k) % M;
-            win_r[k] = sr[t2].x; win_i[k] = sr[t2].y;
-        }
-        int t = 0;
-        while (t < M) {
+        for (int k = 0; k < kTauPerThread; ++k) { acc[k] = 0.0; win[k] = S[isf_pad(tau0 + k)]; }
+        for (int t0 = 0; t0 < M; t0 += 64) {
             float c[kTauPerThread];
             #pragma unroll
             for (int k = 0; k < kTauPerThread; ++k) c[k] = 0.f;
-            int tend = min(M, t + 64);
-            for (; t < tend; ++t) {
-                float2 a = sr[t];
+            const int tend = min(M, t0 + 64);
+            int t = t0;
+            for (; t + kTauPerThread <= tend; t += kTauPerThread) {
+                // at step u the window's entry of tau0 + k is win[(u + k) % 8]
+                const float2* A = S + isf_pad(t);
+                const float2* N = S + isf_pad(t + tau0 + kTauPerThread);
                 #pragma unroll
-                for (int k = 0; k < kTauPerThread; ++k) c[k] = fmaf(a.x, win_r[k], fmaf(a.y, win_i[k], c[k]));
+                for (int u = 0; u < kTauPerThread; ++u) {
+                    const float2 a = A[u];
+                    #pragma unroll
+                    for (int k = 0; k < kTauPerThread; ++k) {
+                        const float2 b = win[(u + k) % kTauPerThread];
+                        c[k] = fmaf(a.x, b.x, fmaf(a.y, b.y, c[k]));
+                    }
+                    win[u] = N[u];
+                }
+            }
+            for (; t < tend; ++t) {                                  // the last M % 8
+                const float2 a = S[isf_pad(t)];
                 #pragma unroll
-                for (int k = 0; k < kTauPerThread - 1; ++k) { win_r[k] = win_r[k+1]; win_i[k] = win_i[k+1]; }
-                int tn = (t + 1 + tau0 + kTauPerThread - 1) % M;
-                win_r[kTauPerThread - 1] = sr[tn].x; win_i[kTauPerThread - 1] = sr[tn].y;
+                for (int k = 0; k < kTauPerThread; ++k) c[k] = fmaf(a.x, win[k].x, fmaf(a.y, win[k].y, c[k]));
+                #pragma unroll
+                for (int k = 0; k < kTauPerThread - 1; ++k) win[k] = win[k + 1];
+                win[kTauPerThread - 1] = S[isf_pad(t + tau0 + kTauPerThread)];
             }
             #pragma unroll
             for (int k = 0; k < kTauPerThread; ++k) acc[k] += c[k];
         }
         #pragma unroll
         for (int k = 0; k < kTauPerThread; ++k)
-            if (tau0 + k < nt) out[(size_t)iq * nt + tau0 + k] = acc[k] * norm;
+            if (tau0 + k < nt) out[(size_t)(q0 + q) * nt + tau0 + k] = acc[k] * norm;
+    }
+}
+
+// the same from memory, for M whose densities do not fit in shared memory with
+// their repetition
+__global__ void __launch_bounds__(256)
+k_isf_long32(const float2* __restrict__ rho, int M, double norm, double* __restrict__ out) {
+    extern __shared__ float2 sr[];
+    const int iq = blockIdx.x;
+    const int nt = M / 2 + 1;
+    for (int t = threadIdx.x; t < M; t += blockDim.x) sr[t] = rho[(size_t)iq * M + t];
+    __syncthreads();
+    for (int tau = threadIdx.x; tau < nt; tau += blockDim.x) {
+        double acc = 0.0;
+        for (int t0 = 0; t0 < M; t0 += 64) {
+            float c = 0.f;
+            const int tend = min(M, t0 + 64);
+            for (int t = t0; t < tend; ++t) {
+                const float2 a = sr[t], b = sr[t + tau < M ? t + tau : t + tau - M];
+                c = fmaf(a.x, b.x, fmaf(a.y, b.y, c));
+            }
+            acc += c;
+        }
+        out[(size_t)iq * nt + tau] = acc * norm;
     }
 }
 
 cudaError_t launch_isf_direct32(const float2* d_rho, int nq, int M, double norm, double* d_out,
                                 cudaStream_t s) {
     if (nq <= 0) return cudaSuccess;
-    int nt = M / 2 + 1;
-    int threads = (nt + kTauPerThread - 1) / kTauPerThread;
-    threads = ((threads + 31) / 32) * 32;
-    if (threads > 256) threads = 256;
-    const size_t smem = (size_t)M * sizeof(float2);
-    if (smem > 200 * 1024) return cudaErrorInvalidValue;    // one q's densities in shared memory
-    if (smem > 48 * 1024) {
+    const int per = (M / 2 + 1 + kTauPerThread - 1) / kTauPerThread;
+    const size_t row = (size_t)isf_row(M) * sizeof(float2);
+    if (row <= 200 * 1024) {
+        const int each = std::max<int>(1, std::min<size_t>(std::max(1, kIsfBlock / per), 200 * 1024 / row));
         const cudaError_t ae = set_smem_limit(k_isf_direct32, 200 * 1024);
         if (ae != cudaSuccess) return ae;
+        k_isf_direct32<<<(nq + each - 1) / each, kIsfBlock, each * row, s>>>(d_rho, nq, M, each, per, norm, d_out);
+        return cudaGetLastError();
     }
-    k_isf_direct32<<<nq, threads, smem, s>>>(d_rho, nq, M, norm, d_out);
+    const size_t smem = (size_t)M * sizeof(float2);
+    if (smem > 200 * 1024) return cudaErrorInvalidValue;    // one q's densities in shared memory
+    const cudaError_t ae = set_smem_limit(k_isf_long32, 200 * 1024);
+    if (ae != cudaSuccess) return ae;
+    k_isf_long32<<<nq, 256, smem, s>>>(d_rho, M, norm, d_out);
     return cudaGetLastError();
 }
 
