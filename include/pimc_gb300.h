@@ -586,7 +586,7 @@ typedef struct {
     double sigma2;
     double side[3];
     int    periodic[3];
-    int    precision;          /* PGB_FP64: the CPU form bit for bit up to exp();
+    int    precision;          /* PGB_FP64: the CPU form up to an ulp of sqrt and exp;
                                   PGB_MIXED: FP32 kernel values, compensated sum */
 } pgb_gp_params;
 int pgb_gp_create(const pgb_gp_params* p, const double* training /* [n][4] */, int n,

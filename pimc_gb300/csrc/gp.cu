@@ -14,8 +14,8 @@
 // and chunk of training points, streamed through shared memory in index
 // order; the chunk sums are added in chunk order.  Chunks exist only to fill
 // the GPU when a call has few points: from about 155 k points on there is one
-// chunk and every sum has the CPU form's order and rounding (up to exp(),
-// which may differ by an ulp from the host's); with several chunks the sum is
+// chunk and every sum has the CPU form's order; the exponential
+// and the root may differ by an ulp from the host's.  With several chunks the sum is
 // regrouped, a relative change of order 1e-16 of sum_k |K w_k|.
 // Mixed kernel: the separations and kernel values in FP32 and the sum in a
 // double-float pair (TwoSum), about 1e-7 of sum_k |K w_k| off the FP64 value.
@@ -35,75 +35,172 @@ namespace pgb {
 struct GpDev {
     double off[3], scale[3], invell[3], pside[3], sideInv[3];
     double standard_mean, standard_std, mu, sigma2;
+    double reach[3];  // largest |training coordinate| / side, 0 where not periodic
+    double perInv[3]; // 1 / side, 0 where not periodic
     int nu2;          // 2 nu: 1, 3 or 5
     int n;            // training points
 };
 
-constexpr int kGpBlock = 256;
-constexpr int kGpTile = 512;            // training points per shared-memory tile
-
-__device__ __forceinline__ double matern64(int nu2, double r) {
-    const double kSqrt3 = 1.7320508075688772935, kSqrt5 = 2.2360679774997896964;
-    if (nu2 == 1) return exp(-r);
-    if (nu2 == 3) { const double x = kSqrt3 * r; return (1.0 + x) * exp(-x); }
-    const double x = kSqrt5 * r;
-    return (1.0 + x + x * x / 3.0) * exp(-x);
+// No separation from a point can reach half a box, so the periodic images
+// change nothing: inputs are normalised to order one and the box is not.
+__device__ __forceinline__ bool gp_inside(const GpDev& g, double r0, double r1, double r2) {
+    return g.reach[0] + fabs(r0) * g.perInv[0] < 0.4999 && g.reach[1] + fabs(r1) * g.perInv[1] < 0.4999 &&
+           g.reach[2] + fabs(r2) * g.perInv[2] < 0.4999;
 }
 
-__device__ __forceinline__ float matern32(int nu2, float r) {
+constexpr int kGpBlock = 256;           // inference points a CTA
+constexpr int kGpTile = 256;            // training points per shared-memory tile
+
+// x / 3, correctly rounded (Markstein's division by a constant)
+__device__ __forceinline__ double third(double x) {
+    const double k = 1.0 / 3.0, q = x * k;
+    return __fma_rn(__fma_rn(-3.0, q, x), k, q);
+}
+
+// sqrt(d) for 2^-960 <= d < 2^960 from the hardware's 20-bit reciprocal root,
+// Householder's third-order step and one residual correction: within an ulp
+// of the correctly rounded root, 9 FP64 instructions
+__device__ __forceinline__ double root64(double d) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = __fma_rn(-(d * y), y, 1.0);
+    y = __fma_rn(y * e, __fma_rn(0.375, e, 0.5), y);
+    const double r = d * y;
+    return __fma_rn(__fma_rn(-r, r, d), 0.5 * y, r);
+}
+
+// exp(-x), x >= 0, by Tang's table method (ACM TOMS 15, 1989): with
+// n = round(-64 x / ln 2), exp(-x) = 2^(n/64) exp(-x - n ln 2 / 64), the first
+// factor from the 64 tabulated 2^(j/64), the second, whose argument is below
+// ln 2 / 128, from five Taylor terms (relative remainder 4e-17).  Ten FP64
+// instructions where exp() takes about forty; below one ulp in all.
+constexpr int kExpTable = 64;
+__device__ __forceinline__ double exp_neg64(double x, const double* T) {
+    if ((unsigned)__double2hiint(x) >= 0x4085E000u) return exp(-x);     // 700 and up, NaN
+    const double magic = 6755399441055744.0;                         // 1.5 2^52
+    const double t = __fma_rn(x, -92.332482616893657, magic);         // 64 / ln 2
+    const int n = __double2loint(t);
+    const double f = t - magic;
+    // ln 2 / 64 in two parts; f times the first is exact
+    double r = __fma_rn(f, -6.93147180369123816490e-01 / 64.0, -x);
+    r = __fma_rn(f, -1.90821492927058770002e-10 / 64.0, r);
+    const double q = __fma_rn(r, __fma_rn(r, __fma_rn(r, 1.0 / 120.0, 1.0 / 24.0), 1.0 / 6.0), 0.5);
+    const double p = __fma_rn(r * r, q, r);
+    const double s = T[n & (kExpTable - 1)];
+    const double y = __fma_rn(s, p, s);
+    return __hiloint2double(__double2hiint(y) + ((n >> 6) << 20), __double2loint(y));
+}
+
+template <int NU2>
+__device__ __forceinline__ double matern64(double r, const double* T) {
+    const double kSqrt3 = 1.7320508075688772935, kSqrt5 = 2.2360679774997896964;
+    if (NU2 == 1) return exp_neg64(r, T);
+    if (NU2 == 3) { const double x = kSqrt3 * r; return (1.0 + x) * exp_neg64(x, T); }
+    const double x = kSqrt5 * r;
+    return (1.0 + x + third(x * x)) * exp_neg64(x, T);
+}
+
+template <int NU2>
+__device__ __forceinline__ float matern32(float r) {
     const float kSqrt3 = 1.7320508f, kSqrt5 = 2.2360680f;
-    if (nu2 == 1) return expf(-r);
-    if (nu2 == 3) { const float x = kSqrt3 * r; return (1.0f + x) * expf(-x); }
+    if (NU2 == 1) return expf(-r);
+    if (NU2 == 3) { const float x = kSqrt3 * r; return (1.0f + x) * expf(-x); }
     const float x = kSqrt5 * r;
     return (1.0f + x + x * x * (1.0f / 3.0f)) * expf(-x);
 }
 
-// Grid: x over blocks of kGpBlock inference points, y over chunks of
-// `chunk` training points; each thread sums its chunk in index order and
-// writes the partial sum; k_gp*_combine adds the chunks in chunk order.  With
-// one chunk the FP64 sum is the CPU form's sequential sum.
-__global__ void __launch_bounds__(kGpBlock)
-k_gp64(GpDev g, const double4* __restrict__ train, const double* __restrict__ pos, int count,
-       int chunk, double* __restrict__ part) {
-    __shared__ double4 tile[kGpTile];
+// The normalised points, once a call: every chunk's CTA dividing for itself
+// would take the FP64 pipe longer than its share of the kernel values.  w is 1
+// where no image is needed (gp_inside).
+template <typename T4>
+__global__ void k_gp_points(GpDev g, const double* __restrict__ pos, int count, T4* __restrict__ r) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int kb = blockIdx.y * chunk, ke = min(g.n, kb + chunk);
-    double r0 = 0.0, r1 = 0.0, r2 = 0.0;
-    if (i < count) {
-        r0 = (pos[3 * (size_t)i] - g.off[0]) / g.scale[0];
-        r1 = (pos[3 * (size_t)i + 1] - g.off[1]) / g.scale[1];
-        r2 = (pos[3 * (size_t)i + 2] - g.off[2]) / g.scale[2];
+    if (i >= count) return;
+    const double x = (pos[3 * (size_t)i] - g.off[0]) / g.scale[0];
+    const double y = (pos[3 * (size_t)i + 1] - g.off[1]) / g.scale[1];
+    const double z = (pos[3 * (size_t)i + 2] - g.off[2]) / g.scale[2];
+    T4 o;
+    o.x = x; o.y = y; o.z = z; o.w = gp_inside(g, x, y, z) ? 1 : 0;
+    r[i] = o;
+}
+
+__device__ __forceinline__ double gp_value(const GpDev& g, double acc) {
+    return g.standard_mean + g.standard_std * (g.mu + g.sigma2 * acc);
+}
+
+// The last CTA of a block of points to arrive (its counter returns to 0)
+__device__ __forceinline__ bool gp_last(unsigned* arrived) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(arrived + blockIdx.x, gridDim.y - 1) == gridDim.y - 1;
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// Grid: x over blocks of kGpBlock inference points, y over chunks of `chunk`
+// training points.  Each thread sums its chunk in index order; with several
+// chunks the last CTA of a block of points adds the partial sums in chunk
+// order.  With one chunk the FP64 sum is the CPU form's sequential sum.
+//
+// FP64 bound: the FP64 pipe (16 clocks of an SM a warp instruction), about 40
+// instructions a kernel value.  2048 training points, 1500 points, nu = 5/2:
+// 2424 us with images always, IEEE root, division by three, exp() and chunks
+// of 512; 311 us here.  200 and 200: 836 and 33 us.
+template <int NU2, bool kWrap>
+__device__ __forceinline__ double gp_sum64(const GpDev& g, const double4* __restrict__ tile, const double* T, int nt,
+                                           double r0, double r1, double r2, double acc) {
+    for (int k = 0; k < nt; ++k) {
+        const double4 t = tile[k];
+        double s0 = t.x - r0, s1 = t.y - r1, s2 = t.z - r2;
+        if (kWrap) {
+            s0 -= g.pside[0] * floor(s0 * g.sideInv[0] + 0.5);
+            s1 -= g.pside[1] * floor(s1 * g.sideInv[1] + 0.5);
+            s2 -= g.pside[2] * floor(s2 * g.sideInv[2] + 0.5);
+        }
+        s0 = s0 * g.invell[0]; s1 = s1 * g.invell[1]; s2 = s2 * g.invell[2];
+        double d2 = 0.0;
+        d2 += s0 * s0; d2 += s1 * s1; d2 += s2 * s2;
+        // 2^-960 .. 2^959 by the exponent bits: a comparison in FP64 costs as much as a product
+        const bool normal = (unsigned)__double2hiint(d2) - 0x03F00000u < 0x77F00000u;
+        const double r = normal ? root64(d2) : sqrt(d2);
+        acc += matern64<NU2>(r, T) * t.w;
     }
+    return acc;
+}
+
+template <int NU2>
+__global__ void __launch_bounds__(kGpBlock)
+k_gp64(GpDev g, const double4* __restrict__ train, const double4* __restrict__ points, int count,
+       int chunk, unsigned* __restrict__ arrived, double* __restrict__ part, double* __restrict__ out) {
+    __shared__ double4 tile[kGpTile];
+    __shared__ double T[kExpTable];
+    const int i = blockIdx.x * kGpBlock + threadIdx.x;
+    const int kb = blockIdx.y * chunk, ke = min(g.n, kb + chunk);
+    double4 r = make_double4(0.0, 0.0, 0.0, 1.0);
+    if (i < count) r = points[i];
+    if (threadIdx.x < kExpTable) T[threadIdx.x] = reinterpret_cast<const double*>(train + g.n)[threadIdx.x];
+    const bool inside = __all_sync(0xffffffffu, r.w != 0.0);
     double acc = 0.0;
     for (int k0 = kb; k0 < ke; k0 += kGpTile) {
         const int nt = min(kGpTile, ke - k0);
         __syncthreads();
-        for (int k = threadIdx.x; k < nt; k += blockDim.x) tile[k] = train[k0 + k];
+        for (int k = threadIdx.x; k < nt; k += kGpBlock) tile[k] = train[k0 + k];
         __syncthreads();
-        if (i < count) {
-            for (int k = 0; k < nt; ++k) {
-                const double4 t = tile[k];
-                double s0 = t.x - r0, s1 = t.y - r1, s2 = t.z - r2;
-                s0 -= g.pside[0] * floor(s0 * g.sideInv[0] + 0.5);
-                s1 -= g.pside[1] * floor(s1 * g.sideInv[1] + 0.5);
-                s2 -= g.pside[2] * floor(s2 * g.sideInv[2] + 0.5);
-                s0 = s0 * g.invell[0]; s1 = s1 * g.invell[1]; s2 = s2 * g.invell[2];
-                double d2 = 0.0;
-                d2 += s0 * s0; d2 += s1 * s1; d2 += s2 * s2;
-                acc += matern64(g.nu2, sqrt(d2)) * t.w;
-            }
-        }
+        if (i < count) acc = inside ? gp_sum64<NU2, false>(g, tile, T, nt, r.x, r.y, r.z, acc)
+                                    : gp_sum64<NU2, true>(g, tile, T, nt, r.x, r.y, r.z, acc);
+    }
+    if (gridDim.y == 1) {
+        if (i < count) out[i] = gp_value(g, acc);
+        return;
     }
     if (i < count) part[(size_t)blockIdx.y * count + i] = acc;
-}
-
-__global__ void k_gp64_combine(GpDev g, const double* __restrict__ part, int nsplit, int count,
-                               double* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    double acc = part[i];
-    for (int s = 1; s < nsplit; ++s) acc += part[(size_t)s * count + i];
-    out[i] = g.standard_mean + g.standard_std * (g.mu + g.sigma2 * acc);
+    if (!gp_last(arrived) || i >= count) return;
+    acc = __ldcg(part + i);
+    #pragma unroll 4
+    for (int s = 1; s < gridDim.y; ++s) acc += __ldcg(part + (size_t)s * count + i);
+    out[i] = gp_value(g, acc);
 }
 
 __device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float x) {
@@ -114,52 +211,97 @@ __device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float x) {
     lo = __fadd_rn(lo, e);
 }
 
-__global__ void __launch_bounds__(kGpBlock)
-k_gp32(GpDev g, const float4* __restrict__ train, const double* __restrict__ pos, int count,
-       int chunk, float2* __restrict__ part) {
-    __shared__ float4 tile[kGpTile];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int kb = blockIdx.y * chunk, ke = min(g.n, kb + chunk);
-    float r0 = 0.f, r1 = 0.f, r2 = 0.f;
-    if (i < count) {
-        r0 = (float)((pos[3 * (size_t)i] - g.off[0]) / g.scale[0]);
-        r1 = (float)((pos[3 * (size_t)i + 1] - g.off[1]) / g.scale[1]);
-        r2 = (float)((pos[3 * (size_t)i + 2] - g.off[2]) / g.scale[2]);
+// Mixed form: two points a thread, so that two chains of kernel values are in
+// flight over one load of the training point.  Bound: the issue rate, about 40
+// instructions a kernel value, twelve less where no image is needed (floor
+// takes the special-function pipe, which the root and the exponential need).
+// 4096 points, 16384 training points: 151 us and 13 us for the chunks' sums
+// with one point a thread, images always and nu chosen in the loop; 110 us
+// here with the sums.
+constexpr int kGpThreads32 = kGpBlock / 2;
+
+template <int NU2, bool kWrap>
+__device__ __forceinline__ float gp_kernel32(const float4 t, const float (&r)[3], const float (&ps)[3], const float (&si)[3],
+                                             const float (&il)[3]) {
+    float s0 = t.x - r[0], s1 = t.y - r[1], s2 = t.z - r[2];
+    if (kWrap) {
+        s0 = fmaf(-ps[0], floorf(fmaf(s0, si[0], 0.5f)), s0);
+        s1 = fmaf(-ps[1], floorf(fmaf(s1, si[1], 0.5f)), s1);
+        s2 = fmaf(-ps[2], floorf(fmaf(s2, si[2], 0.5f)), s2);
     }
-    const float ps0 = (float)g.pside[0], ps1 = (float)g.pside[1], ps2 = (float)g.pside[2];
-    const float si0 = (float)g.sideInv[0], si1 = (float)g.sideInv[1], si2 = (float)g.sideInv[2];
-    const float il0 = (float)g.invell[0], il1 = (float)g.invell[1], il2 = (float)g.invell[2];
-    float hi = 0.f, lo = 0.f;
+    s0 *= il[0]; s1 *= il[1]; s2 *= il[2];
+    return matern32<NU2>(sqrtf(fmaf(s0, s0, fmaf(s1, s1, s2 * s2)))) * t.w;
+}
+
+// the FP32 constants, made on the host
+struct GpF { float ps[3], si[3], il[3]; };
+
+template <int NU2>
+__global__ void __launch_bounds__(kGpThreads32)
+k_gp32(GpDev g, GpF f, const float4* __restrict__ train, const float4* __restrict__ points, int count,
+       int chunk, unsigned* __restrict__ arrived, float2* __restrict__ part, double* __restrict__ out) {
+    __shared__ float4 tile[kGpTile];
+    const int kb = blockIdx.y * chunk, ke = min(g.n, kb + chunk);
+    int i[2];
+    float r[2][3] = {}, hi[2] = {}, lo[2] = {};
+    bool inside = true;
+    #pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        i[p] = blockIdx.x * kGpBlock + p * kGpThreads32 + threadIdx.x;
+        if (i[p] < count) {
+            const float4 x = points[i[p]];
+            r[p][0] = x.x; r[p][1] = x.y; r[p][2] = x.z;
+            inside = inside && x.w != 0.f;
+        }
+    }
+    inside = __all_sync(0xffffffffu, inside);
+    const bool live = i[0] < count, both = __any_sync(0xffffffffu, i[1] < count);
     for (int k0 = kb; k0 < ke; k0 += kGpTile) {
         const int nt = min(kGpTile, ke - k0);
         __syncthreads();
-        for (int k = threadIdx.x; k < nt; k += blockDim.x) tile[k] = train[k0 + k];
+        for (int k = threadIdx.x; k < nt; k += kGpThreads32) tile[k] = train[k0 + k];
         __syncthreads();
-        if (i < count) {
+        if (!live) continue;
+        if (inside && both) {
+            #pragma unroll 4
             for (int k = 0; k < nt; ++k) {
                 const float4 t = tile[k];
-                float s0 = t.x - r0, s1 = t.y - r1, s2 = t.z - r2;
-                s0 = fmaf(-ps0, floorf(fmaf(s0, si0, 0.5f)), s0) * il0;
-                s1 = fmaf(-ps1, floorf(fmaf(s1, si1, 0.5f)), s1) * il1;
-                s2 = fmaf(-ps2, floorf(fmaf(s2, si2, 0.5f)), s2) * il2;
-                const float d = sqrtf(fmaf(s0, s0, fmaf(s1, s1, s2 * s2)));
-                two_sum_acc(hi, lo, matern32(g.nu2, d) * t.w);
+                two_sum_acc(hi[0], lo[0], gp_kernel32<NU2, false>(t, r[0], f.ps, f.si, f.il));
+                two_sum_acc(hi[1], lo[1], gp_kernel32<NU2, false>(t, r[1], f.ps, f.si, f.il));
+            }
+        } else if (inside) {
+            #pragma unroll 4
+            for (int k = 0; k < nt; ++k)
+                two_sum_acc(hi[0], lo[0], gp_kernel32<NU2, false>(tile[k], r[0], f.ps, f.si, f.il));
+        } else {
+            for (int k = 0; k < nt; ++k) {
+                const float4 t = tile[k];
+                two_sum_acc(hi[0], lo[0], gp_kernel32<NU2, true>(t, r[0], f.ps, f.si, f.il));
+                if (both) two_sum_acc(hi[1], lo[1], gp_kernel32<NU2, true>(t, r[1], f.ps, f.si, f.il));
             }
         }
     }
-    if (i < count) part[(size_t)blockIdx.y * count + i] = make_float2(hi, lo);
-}
-
-__global__ void k_gp32_combine(GpDev g, const float2* __restrict__ part, int nsplit, int count,
-                               double* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    double acc = 0.0;
-    for (int s = 0; s < nsplit; ++s) {
-        const float2 p = part[(size_t)s * count + i];
-        acc += (double)p.x + (double)p.y;
+    const bool split = gridDim.y > 1;
+    #pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        if (i[p] >= count) continue;
+        if (split) part[(size_t)blockIdx.y * count + i[p]] = make_float2(hi[p], lo[p]);
+        else out[i[p]] = gp_value(g, (double)hi[p] + (double)lo[p]);
     }
-    out[i] = g.standard_mean + g.standard_std * (g.mu + g.sigma2 * acc);
+    if (!split || !gp_last(arrived)) return;
+    #pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        if (i[p] >= count) continue;
+        // leading parts by TwoSum, the trailing parts with their errors
+        float h = 0.f, l = 0.f;
+        #pragma unroll 8
+        for (int s = 0; s < gridDim.y; ++s) {
+            const float2 x = __ldcg(part + (size_t)s * count + i[p]);
+            two_sum_acc(h, l, x.x);
+            l += x.y;
+        }
+        out[i[p]] = gp_value(g, (double)h + (double)l);
+    }
 }
 
 // --------------------------------------------------------------------------
@@ -261,8 +403,10 @@ struct pgb_gp {
     // per-call scratch: positions, values, fold, cut flags (grown on demand)
     void* d_buf = nullptr;
     size_t buf_bytes = 0;
-    void* d_part = nullptr;              // per-chunk partial sums
+    void* d_part = nullptr;              // the normalised points, the per-chunk partial sums
     size_t part_bytes = 0;
+    unsigned* d_arrived = nullptr;       // a counter a block of points, zero between calls
+    int arrived_blocks = 0;
     std::string err;
     int fail(int code, const std::string& m) { err = m; return code; }
     int cfail(cudaError_t e, const char* where) {
@@ -283,42 +427,58 @@ int ensure_buf(pgb_gp* h, size_t bytes) {
     return PGB_OK;
 }
 
-// Chunks of training points so that the grid covers the GPU: about four
-// CTAs per SM, chunks no shorter than one shared-memory tile.
-int gp_splits(const pgb_gp* h, int count) {
-    const int bx = (count + kGpBlock - 1) / kGpBlock;
-    const int want = (4 * 152 + bx - 1) / bx;
-    const int maxs = (h->g.n + kGpTile - 1) / kGpTile;
-    return std::max(1, std::min(want, maxs));
-}
+// Chunks of training points so that the grid covers the GPU: about eight CTAs
+// an SM (they even out to the last one), chunks of at least 32 points (FP64:
+// 8), below which staging a chunk and adding its sum cost what it saves.  From
+// 608 blocks of points on there is one chunk.
+constexpr int kGpLeast32 = 32, kGpLeast64 = 8;
 
 cudaError_t launch_gp(pgb_gp* h, const double* d_pos, int count, double* d_out) {
     if (count <= 0) return cudaSuccess;
     const int bx = (count + kGpBlock - 1) / kGpBlock;
-    const int ns = gp_splits(h, count);
-    // chunk: a whole number of tiles, so only the last chunk is short
-    const int tiles = (h->g.n + kGpTile - 1) / kGpTile;
-    const int chunk = ((tiles + ns - 1) / ns) * kGpTile;
+    const int want = bx >= 4 * 152 ? 1 : (8 * 152 + bx - 1) / bx;
+    const int least = h->p.precision == PGB_MIXED ? kGpLeast32 : kGpLeast64;
+    const int ns = std::max(1, std::min(want, (h->g.n + least - 1) / least));
+    const int chunk = (((h->g.n + ns - 1) / ns + 7) / 8) * 8;
     const int nsplit = (h->g.n + chunk - 1) / chunk;
-    const size_t need = (size_t)nsplit * count * sizeof(double2);
+    // the points, then the chunks' sums
+    const size_t points = (size_t)count * (h->p.precision == PGB_MIXED ? sizeof(float4) : sizeof(double4));
+    const size_t need = points + (nsplit > 1 ? (size_t)nsplit * count * sizeof(double) : 0);
     if (need > h->part_bytes) {
         if (h->d_part) { cudaStreamSynchronize(h->stream); cudaFree(h->d_part); h->d_part = nullptr; h->part_bytes = 0; }
         cudaError_t e = cudaMalloc(&h->d_part, need);
         if (e != cudaSuccess) { h->d_part = nullptr; return e; }
         h->part_bytes = need;
     }
-    dim3 grid(bx, nsplit);
-    if (h->p.precision == PGB_MIXED) {
-        k_gp32<<<grid, kGpBlock, 0, h->stream>>>(h->g, h->d_train32, d_pos, count, chunk,
-                                                static_cast<float2*>(h->d_part));
-        k_gp32_combine<<<bx, kGpBlock, 0, h->stream>>>(h->g, static_cast<const float2*>(h->d_part),
-                                                      nsplit, count, d_out);
-    } else {
-        k_gp64<<<grid, kGpBlock, 0, h->stream>>>(h->g, h->d_train64, d_pos, count, chunk,
-                                                static_cast<double*>(h->d_part));
-        k_gp64_combine<<<bx, kGpBlock, 0, h->stream>>>(h->g, static_cast<const double*>(h->d_part),
-                                                      nsplit, count, d_out);
+    if (nsplit > 1 && bx > h->arrived_blocks) {
+        if (h->d_arrived) { cudaStreamSynchronize(h->stream); cudaFree(h->d_arrived); h->d_arrived = nullptr; h->arrived_blocks = 0; }
+        const int blocks = std::max(bx, 4 * 152);        // more blocks than that take one chunk
+        cudaError_t e = cudaMalloc(&h->d_arrived, blocks * sizeof(unsigned));
+        if (e != cudaSuccess) { h->d_arrived = nullptr; return e; }
+        if ((e = cudaMemsetAsync(h->d_arrived, 0, blocks * sizeof(unsigned), h->stream)) != cudaSuccess) return e;
+        h->arrived_blocks = blocks;
     }
+    dim3 grid(bx, nsplit);
+    const GpDev& g = h->g;
+    char* base = static_cast<char*>(h->d_part);
+    auto run = [&](auto k32, auto k64) {
+        if (h->p.precision == PGB_MIXED) {
+            GpF f;
+            for (int d = 0; d < 3; ++d) { f.ps[d] = (float)g.pside[d]; f.si[d] = (float)g.sideInv[d]; f.il[d] = (float)g.invell[d]; }
+            float4* r = reinterpret_cast<float4*>(base);
+            k_gp_points<float4><<<(count + 127) / 128, 128, 0, h->stream>>>(g, d_pos, count, r);
+            k32<<<grid, kGpThreads32, 0, h->stream>>>(g, f, h->d_train32, r, count, chunk, h->d_arrived,
+                                                      reinterpret_cast<float2*>(base + points), d_out);
+        } else {
+            double4* r = reinterpret_cast<double4*>(base);
+            k_gp_points<double4><<<(count + 127) / 128, 128, 0, h->stream>>>(g, d_pos, count, r);
+            k64<<<grid, kGpBlock, 0, h->stream>>>(g, h->d_train64, r, count, chunk, h->d_arrived,
+                                                  reinterpret_cast<double*>(base + points), d_out);
+        }
+    };
+    if (g.nu2 == 1) run(k_gp32<1>, k_gp64<1>);
+    else if (g.nu2 == 3) run(k_gp32<3>, k_gp64<3>);
+    else run(k_gp32<5>, k_gp64<5>);
     return cudaGetLastError();
 }
 
@@ -361,12 +521,23 @@ int pgb_gp_create(const pgb_gp_params* p, const double* training, int n, pgb_gp*
     }
     g.standard_mean = p->standard_mean; g.standard_std = p->standard_std;
     g.mu = p->mean; g.sigma2 = p->sigma2; g.nu2 = nu2; g.n = n;
-    std::vector<double4> t64((size_t)n);
+    double most[3] = {0.0, 0.0, 0.0};                    // a NaN stays: no point is inside then
+    // the training rows and, behind them, the 64 powers 2^(j/64) of exp_neg64
+    std::vector<double4> t64((size_t)n + kExpTable / 4);
     std::vector<float4> t32((size_t)n);
     for (int k = 0; k < n; ++k) {
         const double* r = training + 4 * (size_t)k;
         t64[k] = make_double4(r[0], r[1], r[2], r[3]);
         t32[k] = make_float4((float)r[0], (float)r[1], (float)r[2], (float)r[3]);
+        for (int d = 0; d < 3; ++d) {
+            const double x = std::fabs(r[d]);
+            most[d] = x > most[d] || x != x ? x : most[d];
+        }
+    }
+    for (int j = 0; j < kExpTable; ++j) reinterpret_cast<double*>(t64.data() + n)[j] = std::exp2(j / 64.0);
+    for (int d = 0; d < 3; ++d) {
+        g.perInv[d] = p->periodic[d] ? g.sideInv[d] : 0.0;
+        g.reach[d] = most[d] * g.perInv[d];
     }
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&h->d_train64, t64.size() * sizeof(double4));
@@ -386,6 +557,7 @@ int pgb_gp_destroy(pgb_gp* h) {
     if (!h) return PGB_OK;
     if (h->stream) cudaStreamSynchronize(h->stream);
     cudaFree(h->d_train64); cudaFree(h->d_train32); cudaFree(h->d_buf); cudaFree(h->d_part);
+    cudaFree(h->d_arrived);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return PGB_OK;
