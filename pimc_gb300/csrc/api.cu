@@ -893,8 +893,8 @@ namespace {
 size_t rho_region(const Ctx& c, int nq) {
     return ((size_t)nq * c.M * 2 * sizeof(double) + 255) & ~(size_t)255;
 }
-size_t posbuf_region(const Ctx& c) {
-    return (c.p.precision == PGB_MIXED) ? ((rhoq32_work_bytes(c.view()) + 255) & ~(size_t)255) : 0;
+size_t posbuf_region(const Ctx& c, int nq) {
+    return (c.p.precision == PGB_MIXED) ? ((rhoq32_work_bytes(c.view(), nq) + 255) & ~(size_t)255) : 0;
 }
 int scatter_common(Ctx& c, const double* d_q, int nq, int what, int mode, double* d_out,
                    void* d_work, double maxR2 = 0.0) {
@@ -918,21 +918,24 @@ int scatter_common(Ctx& c, const double* d_q, int nq, int what, int mode, double
     } else {
         float2* d_rho = static_cast<float2*>(d_work);
         void* posbuf = static_cast<char*>(d_work) + rho_region(c, nq);
-        e = launch_rhoq32(v, d_q, nq, d_rho, posbuf, c.stream, maxR2);
-        if (e == cudaSuccess) {
-            if (what == 0) e = launch_ssf_from_rho32(d_rho, nq, c.M, norm, d_out, c.stream);
-            else if (mode == 1) {
-                if (!isf_tc_supported(c.M))
-                    return c.fail(PGB_EINVAL, "tensor-core F(q,tau) needs M a multiple of 128 and <= 2048");
-                if (!c.d_tc_tables) {
-                    e = cudaMalloc(&c.d_tc_tables, isf_tc_table_bytes(c.M));
-                    if (e != cudaSuccess) { c.d_tc_tables = nullptr; return c.cuda_fail(e, "cudaMalloc(F(q,tau) tables)"); }
-                    e = isf_tc_build_tables(c.M, c.d_tc_tables, c.stream);
-                    if (e != cudaSuccess) return c.cuda_fail(e, "F(q,tau) tables");
-                }
-                void* tc = static_cast<char*>(d_work) + rho_region(c, nq) + posbuf_region(c);
-                e = launch_isf_tc(d_rho, nq, c.M, norm, d_out, tc, c.d_tc_tables, c.stream);
-            } else e = launch_isf_direct32(d_rho, nq, c.M, norm, d_out, c.stream);
+        if (what == 1 && mode == 1) {
+            if (!isf_tc_supported(c.M))
+                return c.fail(PGB_EINVAL, "tensor-core F(q,tau) needs M a multiple of 128 and <= 2048");
+            if (!c.d_tc_tables) {
+                e = cudaMalloc(&c.d_tc_tables, isf_tc_table_bytes(c.M));
+                if (e != cudaSuccess) { c.d_tc_tables = nullptr; return c.cuda_fail(e, "cudaMalloc(F(q,tau) tables)"); }
+                e = isf_tc_build_tables(c.M, c.d_tc_tables, c.stream);
+                if (e != cudaSuccess) return c.cuda_fail(e, "F(q,tau) tables");
+            }
+            void* tc = static_cast<char*>(d_work) + rho_region(c, nq) + posbuf_region(c, nq);
+            const IsfOperand split = isf_tc_operand(nq, c.M, tc);
+            e = launch_rhoq32(v, d_q, nq, nullptr, posbuf, c.stream, 0.0, &split);
+            if (e == cudaSuccess) e = launch_isf_tc(nq, c.M, norm, d_out, tc, c.d_tc_tables, c.stream);
+        } else {
+            e = launch_rhoq32(v, d_q, nq, d_rho, posbuf, c.stream, maxR2);
+            if (e == cudaSuccess)
+                e = what == 0 ? launch_ssf_from_rho32(d_rho, nq, c.M, norm, d_out, c.stream)
+                              : launch_isf_direct32(d_rho, nq, c.M, norm, d_out, c.stream);
         }
     }
     if (e != cudaSuccess) return c.cuda_fail(e, "structure factor launch");
@@ -942,7 +945,7 @@ int scatter_common(Ctx& c, const double* d_q, int nq, int what, int mode, double
 size_t scatter_work_bytes(const Ctx& c, int nq, int what, int mode) {
     size_t extra = (c.p.precision == PGB_MIXED && what == 1 && mode == 1)
                        ? isf_tc_scratch_bytes(nq, c.M) : 0;
-    return rho_region(c, nq) + posbuf_region(c) + extra;
+    return rho_region(c, nq) + posbuf_region(c, nq) + extra;
 }
 
 int scatter_host(pgb_ctx* h, const double* q, int nq, int what, int mode, double* out) {
@@ -969,7 +972,7 @@ int scatter_host(pgb_ctx* h, const double* q, int nq, int what, int mode, double
     int tc_err = 0;
     if (tc) {
         // the tensor-core pipeline's error word: a bounded wait ran out
-        const char* w = base + off_w + rho_region(c, nq) + posbuf_region(c);
+        const char* w = base + off_w + rho_region(c, nq) + posbuf_region(c, nq);
         PGB_CUDA(&c, cudaMemcpyAsync(&tc_err, w + isf_tc_error_offset(nq, c.M), sizeof(int),
                                      cudaMemcpyDeviceToHost, c.stream));
     }

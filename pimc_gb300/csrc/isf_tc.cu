@@ -11,48 +11,45 @@
 // Both run as split-BF16 products, A = Ah + Al, B = Bh + Bl,
 // A B ~ Ah Bh + Ah Bl + Al Bh, accumulated in FP32 in tensor memory.
 //
-// Kernel: one CTA of 128 threads per 128 x 256 output tile.  The prep
-// kernels write every operand in tile order: the 64-wide K chunk of a tile is
+// Kernel: one CTA of 128 threads per 128 x 128 output tile (the last column tile
+// of GEMM 2, whose M/2 + 1 columns leave one over, as narrow as the columns it
+// has).  The operands' makers (the density kernel, GEMM 1's own epilogue, the
+// table kernels) write them in tile order: the 64-wide K chunk of a tile is
 // one contiguous block already in the canonical K-major core-matrix layout
 // without swizzle (8 x 16-byte core matrices; LBO = 128 B between core
 // matrices along K, SBO = 1024 B between 8-row groups), so one bulk copy
 // (cp.async.bulk, completion counted on an mbarrier) moves it into shared
-// memory.  Warp 0 lane 0 produces chunks into a two-stage ring, warp 1 lane 0
-// issues the tcgen05.mma.kind::f16 instructions (M = 128, N = 256, K = 16)
+// memory.  Warp 0 lane 0 produces chunks into a three-stage ring, warp 1 lane 0
+// issues the tcgen05.mma.kind::f16 instructions (M = 128, N <= 128, K = 16)
 // and releases each stage with tcgen05.commit; every wait is bounded.  The
-// accumulator (128 lanes x 256 FP32 columns of TMEM) is read back with
+// accumulator (128 lanes x 128 FP32 columns of TMEM) is read back with
 // tcgen05.ld by all four warps.
+//
+// Bound: the copies of one CTA's operands (64 KB a chunk) while few CTAs run.
+// 2048 vectors, M = 512: 128 columns a tile give 128 CTAs for GEMM 1 instead of
+// the 64 of 256 columns; with the densities and P split where they are made,
+// the correlation went from 14 + 28 + 8 + 28 us in five launches to 31 us in
+// two.
 #include <cuda_bf16.h>
 #include <atomic>
 #include <cstdint>
 
-#include "pgb_device.cuh"
+#include "isf_tc.cuh"
 
 namespace pgb {
 
 namespace {
 
-constexpr int kTM = 128;          // rows per tile
-constexpr int kTN = 256;          // columns per tile (TMEM columns)
+constexpr int kTN = 128;          // columns per tile (TMEM columns)
 constexpr int kTK = 64;           // K per staged chunk
 constexpr int kThreads = 128;
 constexpr uint32_t kTileA = kTM * kTK * 2;     // bytes of one bf16 A chunk
 constexpr uint32_t kTileB = kTN * kTK * 2;     // bytes of one bf16 B chunk
-constexpr int kStages = 2;
+constexpr int kStages = 3;
 constexpr uint32_t kStageBytes = 2 * kTileA + 2 * kTileB;     // Ah, Al, Bh, Bl of one chunk
 constexpr uint32_t kSmem = kStages * kStageBytes + 1024;
 constexpr long long kMmaWaitLimit = 1LL << 24;
 constexpr unsigned long long kWaitNs = 1000000000ull;   // one second of wall clock per wait
-
-// Element index of (r, k) in a tile-ordered [rows x K] bf16 operand whose
-// tiles are TR rows x 64 K: tile (r / TR, k / 64) is one contiguous block of
-// TR * 64 elements in core-matrix order (8-row groups of 1024 B, 16-byte core
-// rows, 128 B between core matrices along K).
-__host__ __device__ __forceinline__ size_t tiled_index(int r, int k, int K, int TR) {
-    const int rt = r / TR, rr = r - rt * TR, kc = k >> 6, kk = k & 63;
-    return ((size_t)rt * (size_t)(K >> 6) + (size_t)kc) * (size_t)(TR * 64) +
-           (size_t)((rr >> 3) * 512 + (kk >> 3) * 64 + (rr & 7) * 8 + (kk & 7));
-}
 
 __device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -65,15 +62,15 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
     return d;                                          // base offset 0, no swizzle
 }
 
-// kind::f16 instruction descriptor: D = F32, A = B = BF16, both K-major,
-// N = 256, M = 128
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTN >> 3) << 17) |
-                            ((uint32_t)(kTM >> 4) << 24);
+// kind::f16 instruction descriptor: D = F32, A = B = BF16, both K-major, M = 128
+__device__ __forceinline__ uint32_t idesc(int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTM >> 4) << 24);
+}
 
-__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t acc) {
+__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t desc, uint32_t acc) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                 :: "r"(tmem), "l"(ad), "l"(bd), "r"(kIdesc), "r"(acc) : "memory");
+                 :: "r"(tmem), "l"(ad), "l"(bd), "r"(desc), "r"(acc) : "memory");
 }
 
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
@@ -140,8 +137,9 @@ __device__ __forceinline__ bool bar_wait_bounded(uint64_t* bar, uint32_t parity)
 }
 
 // Split-BF16 GEMM  C[rows x cols] = A[rows x K] B[K x cols]; A and B^T
-// [cols x K] tile-ordered (tiled_index with TR = 128 and 256), hi/lo parts.
-// mode 0: interleaved (re, im) columns -> P[row][col/2] = re^2 + im^2
+// [cols x K] tile-ordered (tiled_index with TR = 128), hi/lo parts.
+// mode 0: interleaved (re, im) columns -> P[row][col/2] = re^2 + im^2, split
+//         and tile-ordered again, the A operand of GEMM 2 with K = ldp
 // mode 1: out[row][col] = scale * C  (FP64), for row < rows_valid, col < cols_valid
 // stall_last: a test of the bounded waits.  The producer stops before the
 // last chunk (no arrival, no copy), so the MMA thread's wait for that chunk
@@ -150,7 +148,8 @@ __device__ __forceinline__ bool bar_wait_bounded(uint64_t* bar, uint32_t parity)
 __global__ void __launch_bounds__(kThreads, 1)
 k_gemm_split_bf16(const __nv_bfloat16* __restrict__ Ah, const __nv_bfloat16* __restrict__ Al,
                   const __nv_bfloat16* __restrict__ Bh, const __nv_bfloat16* __restrict__ Bl,
-                  int K, int mode, float* __restrict__ P, int ldp, double* __restrict__ out,
+                  int K, int mode, __nv_bfloat16* __restrict__ Ph, __nv_bfloat16* __restrict__ Pl, int ldp,
+                  double* __restrict__ out,
                   int ldo, int rows_valid, int cols_valid, double scale, int* __restrict__ err,
                   int stall_last) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -163,6 +162,9 @@ k_gemm_split_bf16(const __nv_bfloat16* __restrict__ Ah, const __nv_bfloat16* __r
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row0 = blockIdx.y * kTM, col0 = blockIdx.x * kTN;
     const int nk = K / kTK;
+    // columns this tile has, in whole groups of 16
+    const int tn = min(kTN, (cols_valid - col0 + 15) & ~15);
+    const uint32_t bytesB = (uint32_t)tn * kTK * 2, stage_bytes = 2 * kTileA + 2 * bytesB;
     const char* gAh = reinterpret_cast<const char*>(Ah) + (size_t)blockIdx.y * nk * kTileA;
     const char* gAl = reinterpret_cast<const char*>(Al) + (size_t)blockIdx.y * nk * kTileA;
     const char* gBh = reinterpret_cast<const char*>(Bh) + (size_t)blockIdx.x * nk * kTileB;
@@ -198,11 +200,11 @@ k_gemm_split_bf16(const __nv_bfloat16* __restrict__ Ah, const __nv_bfloat16* __r
                     break;
                 }
                 unsigned char* sA = smem + (size_t)st * kStageBytes;
-                bar_expect_tx(full + st, kStageBytes);
+                bar_expect_tx(full + st, stage_bytes);
                 bulk_g2s(sA, gAh + (size_t)c * kTileA, kTileA, full + st);
                 bulk_g2s(sA + kTileA, gAl + (size_t)c * kTileA, kTileA, full + st);
-                bulk_g2s(sA + 2 * kTileA, gBh + (size_t)c * kTileB, kTileB, full + st);
-                bulk_g2s(sA + 2 * kTileA + kTileB, gBl + (size_t)c * kTileB, kTileB, full + st);
+                bulk_g2s(sA + 2 * kTileA, gBh + (size_t)c * kTileB, bytesB, full + st);
+                bulk_g2s(sA + 2 * kTileA + kTileB, gBl + (size_t)c * kTileB, bytesB, full + st);
             }
             s_count[0] = c;
         }
@@ -210,6 +212,7 @@ k_gemm_split_bf16(const __nv_bfloat16* __restrict__ Ah, const __nv_bfloat16* __r
     } else if (warp == 1) {
         if (lane == 0) {
             int c = 0;
+            const uint32_t desc = idesc(tn);
             for (; c < nk; ++c) {
                 const int st = c % kStages;
                 if (!bar_wait_bounded(full + st, (uint32_t)((c / kStages) & 1))) {
@@ -224,9 +227,9 @@ k_gemm_split_bf16(const __nv_bfloat16* __restrict__ Ah, const __nv_bfloat16* __r
                     const uint64_t ah = smem_desc(base + ko), al = smem_desc(base + kTileA + ko);
                     const uint64_t bh = smem_desc(base + 2 * kTileA + ko);
                     const uint64_t bl = smem_desc(base + 2 * kTileA + kTileB + ko);
-                    mma_bf16(tmem, ah, bh, (c > 0 || ks > 0) ? 1u : 0u);
-                    mma_bf16(tmem, ah, bl, 1u);
-                    mma_bf16(tmem, al, bh, 1u);
+                    mma_bf16(tmem, ah, bh, desc, (c > 0 || ks > 0) ? 1u : 0u);
+                    mma_bf16(tmem, ah, bl, desc, 1u);
+                    mma_bf16(tmem, al, bh, desc, 1u);
                 }
                 mma_commit(empty + st);        // the stage is free once these MMAs are done
             }
@@ -255,14 +258,24 @@ k_gemm_split_bf16(const __nv_bfloat16* __restrict__ Ah, const __nv_bfloat16* __r
         const int r = 32 * warp + lane;
         const int row = row0 + r;
         float v[32];
-        for (int cc = 0; cc < kTN / 32; ++cc) {
+        for (int cc = 0; 32 * cc < tn; ++cc) {
             tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(32 * cc), v);
             if (mode == 0) {
                 const int w0 = (col0 + 32 * cc) >> 1;
                 if (row < rows_valid) {
+                    // eight neighbours along K are one 16-byte core row
                     #pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        P[(size_t)row * ldp + w0 + j] = fmaf(v[2 * j], v[2 * j], v[2 * j + 1] * v[2 * j + 1]);
+                    for (int j = 0; j < 16; j += 8) {
+                        __align__(16) __nv_bfloat16 h[8], l[8];
+                        #pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            const float re = v[2 * (j + u)], im = v[2 * (j + u) + 1];
+                            split_bf16(fmaf(re, re, im * im), h[u], l[u]);
+                        }
+                        const size_t o = tiled_index(row, w0 + j, ldp, kTM);
+                        *reinterpret_cast<uint4*>(Ph + o) = *reinterpret_cast<const uint4*>(h);
+                        *reinterpret_cast<uint4*>(Pl + o) = *reinterpret_cast<const uint4*>(l);
+                    }
                 }
             } else {
                 // FP32 scale, FP64 result formed on the integer pipes
@@ -283,25 +296,6 @@ k_gemm_split_bf16(const __nv_bfloat16* __restrict__ Ah, const __nv_bfloat16* __r
                      :: "r"(tmem), "r"((uint32_t)kTN) : "memory");
 }
 
-__device__ __forceinline__ void split_bf16(float x, __nv_bfloat16& h, __nv_bfloat16& l) {
-    h = __float2bfloat16_rn(x);
-    l = __float2bfloat16_rn(x - __bfloat162float(h));
-}
-
-// A1 = (Re rho | Im rho), rows >= nq are zero
-__global__ void k_prep_rho(const float2* __restrict__ rho, int nq, int M, int qpad,
-                           __nv_bfloat16* Ah, __nv_bfloat16* Al) {
-    const long long n = (long long)qpad * 2 * M;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int q = (int)(i / (2 * M)), k = (int)(i % (2 * M));
-        float x = 0.f;
-        if (q < nq) { const float2 r = rho[(size_t)q * M + (k % M)]; x = (k < M) ? r.x : r.y; }
-        const size_t o = tiled_index(q, k, 2 * M, kTM);
-        split_bf16(x, Ah[o], Al[o]);
-    }
-}
-
 // B1^T [2M cols][2M K]: col 2w -> Re X(w), col 2w+1 -> Im X(w)
 __global__ void k_prep_dft(int M, __nv_bfloat16* Bh, __nv_bfloat16* Bl) {
     const long long n = (long long)4 * M * M;
@@ -317,18 +311,6 @@ __global__ void k_prep_dft(int M, __nv_bfloat16* Bh, __nv_bfloat16* Bl) {
         else              val = (k < M) ? -sn : cs;     // Im X = sum -Re(rho) sin + Im(rho) cos
         const size_t o = tiled_index(c, k, 2 * M, kTN);
         split_bf16((float)val, Bh[o], Bl[o]);
-    }
-}
-
-// A2 = P [qpad x M] (row-major) -> tile order
-__global__ void k_prep_p(const float* __restrict__ P, int qpad, int M, __nv_bfloat16* Ah,
-                         __nv_bfloat16* Al) {
-    const long long n = (long long)qpad * M;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int q = (int)(i / M), w = (int)(i % M);
-        const size_t o = tiled_index(q, w, M, kTM);
-        split_bf16(P[i], Ah[o], Al[o]);
     }
 }
 
@@ -351,19 +333,17 @@ __global__ void k_prep_cos(int M, int colpad, __nv_bfloat16* Bh, __nv_bfloat16* 
 
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// per-call scratch: the split rho matrix, P and its split, the error flag
+// per-call scratch: the split rho matrix, the split P, the error flag
 struct Layout {
-    int qpad, colpad2;
-    size_t a1, p, a2, err, total;
+    int qpad;
+    size_t a1, a2, err, total;
 };
 
 Layout layout(int nq, int M) {
     Layout L;
     L.qpad = ((nq + kTM - 1) / kTM) * kTM;
-    L.colpad2 = ((M / 2 + 1 + kTN - 1) / kTN) * kTN;
     size_t off = 0;
     L.a1 = off; off = align256(off + (size_t)L.qpad * 2 * M * 2 * sizeof(__nv_bfloat16));
-    L.p = off;  off = align256(off + (size_t)L.qpad * M * sizeof(float));
     L.a2 = off; off = align256(off + (size_t)L.qpad * M * 2 * sizeof(__nv_bfloat16));
     L.err = off; off = align256(off + sizeof(int));
     L.total = off;
@@ -416,39 +396,40 @@ cudaError_t isf_tc_build_tables(int M, void* d_tables, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_isf_tc(const float2* d_rho, int nq, int M, double norm, double* d_out,
-                          void* d_scratch, const void* d_tables, cudaStream_t s) {
+IsfOperand isf_tc_operand(int nq, int M, void* d_scratch) {
+    const Layout L = layout(nq, M);
+    char* base = static_cast<char*>(d_scratch);
+    auto* h = reinterpret_cast<__nv_bfloat16*>(base + L.a1);
+    return {h, h + (size_t)L.qpad * 2 * M, L.qpad, reinterpret_cast<int*>(base + L.err)};
+}
+
+cudaError_t launch_isf_tc(int nq, int M, double norm, double* d_out, void* d_scratch, const void* d_tables,
+                          cudaStream_t s) {
     if (!isf_tc_supported(M) || nq <= 0 || !d_tables) return cudaErrorInvalidValue;
     const int stall = g_stall_test.load();
     const Layout L = layout(nq, M);
     const Tables T = tables(M);
+    const IsfOperand A = isf_tc_operand(nq, M, d_scratch);
     char* base = static_cast<char*>(d_scratch);
-    auto* a1h = reinterpret_cast<__nv_bfloat16*>(base + L.a1);
-    auto* a1l = a1h + (size_t)L.qpad * 2 * M;
     const char* tb = static_cast<const char*>(d_tables);
     auto* b1h = reinterpret_cast<const __nv_bfloat16*>(tb + T.b1);
     auto* b1l = b1h + (size_t)4 * M * M;
-    auto* P = reinterpret_cast<float*>(base + L.p);
     auto* a2h = reinterpret_cast<__nv_bfloat16*>(base + L.a2);
     auto* a2l = a2h + (size_t)L.qpad * M;
     auto* b2h = reinterpret_cast<const __nv_bfloat16*>(tb + T.b2);
     auto* b2l = b2h + (size_t)T.colpad2 * M;
-    int* err = reinterpret_cast<int*>(base + L.err);
     {
         const cudaError_t ae = set_smem_limit(k_gemm_split_bf16, (int)kSmem);
         if (ae != cudaSuccess) return ae;
     }
-    cudaMemsetAsync(err, 0, sizeof(int), s);
-    k_prep_rho<<<152 * 4, 256, 0, s>>>(d_rho, nq, M, L.qpad, a1h, a1l);
     // GEMM 1: [qpad x 2M] x [2M x 2M] -> P [qpad x M]
     dim3 g1(2 * M / kTN, L.qpad / kTM);
-    k_gemm_split_bf16<<<g1, kThreads, kSmem, s>>>(a1h, a1l, b1h, b1l, 2 * M, 0, P, M, nullptr, 0,
-                                                  L.qpad, 2 * M, 0.0, err, stall);
-    k_prep_p<<<152 * 4, 256, 0, s>>>(P, L.qpad, M, a2h, a2l);
+    k_gemm_split_bf16<<<g1, kThreads, kSmem, s>>>(A.hi, A.lo, b1h, b1l, 2 * M, 0, a2h, a2l, M, nullptr, 0,
+                                                  L.qpad, 2 * M, 0.0, A.err, stall);
     // GEMM 2: [qpad x M] x [M x colpad2] -> F [nq x (M/2+1)]
-    dim3 g2(L.colpad2 / kTN, L.qpad / kTM);
-    k_gemm_split_bf16<<<g2, kThreads, kSmem, s>>>(a2h, a2l, b2h, b2l, M, 1, nullptr, 0, d_out,
-                                                  M / 2 + 1, nq, M / 2 + 1, norm / (double)M, err, 0);
+    dim3 g2(T.colpad2 / kTN, L.qpad / kTM);
+    k_gemm_split_bf16<<<g2, kThreads, kSmem, s>>>(a2h, a2l, b2h, b2l, M, 1, nullptr, nullptr, 0, d_out,
+                                                  M / 2 + 1, nq, M / 2 + 1, norm / (double)M, A.err, 0);
     return cudaGetLastError();
 }
 

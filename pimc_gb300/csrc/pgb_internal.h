@@ -2,6 +2,7 @@
 // library.  Host code only sees plain pointers; kernels take a PathView.
 #pragma once
 
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstdio>
@@ -181,12 +182,13 @@ cudaError_t launch_slice_terms32(const PathView& v, AzizParams az, int window, i
 cudaError_t launch_pos32_from64(const PathView& v, float4* d_pos32,
                                 cudaStream_t s);
 // scatter.cu
-// d_work: rhoq32_work_bytes(v) of scratch for the slices as box fractions;
-// d_rho must hold nq*M*16 bytes (the second half keeps the wave-vector table)
-size_t rhoq32_work_bytes(const PathView& v);
-cudaError_t launch_rhoq32(const PathView& v, const double* d_q, int nq,
-                          float2* d_rho /* [q][M] */, void* d_work, cudaStream_t s,
-                          double maxR2 = 0.0);
+// d_work: rhoq32_work_bytes(v, nq) of scratch, 16-byte aligned, for the slices
+// as box fractions and the wave vectors in turns.  With `split` the densities
+// go there, as the tensor-core F(q,tau)'s split operand, and not to d_rho.
+struct IsfOperand;
+size_t rhoq32_work_bytes(const PathView& v, int nq);
+cudaError_t launch_rhoq32(const PathView& v, const double* d_q, int nq, float2* d_rho /* [q][M] */,
+                          void* d_work, cudaStream_t s, double maxR2 = 0.0, const IsfOperand* split = nullptr);
 cudaError_t launch_ssf_from_rho32(const float2* d_rho, int nq, int M,
                                   double norm, double* d_out, cudaStream_t s);
 cudaError_t launch_ssf_from_rho64(const double* d_rho, int nq, int M,
@@ -207,8 +209,12 @@ cudaError_t launch_count_inside(const PathView& v, double maxR2, int* d_out, cud
 size_t isf_tc_scratch_bytes(int nq, int M);
 size_t isf_tc_table_bytes(int M);
 cudaError_t isf_tc_build_tables(int M, void* d_tables, cudaStream_t s);
-cudaError_t launch_isf_tc(const float2* d_rho, int nq, int M, double norm,
-                          double* d_out, void* d_scratch, const void* d_tables, cudaStream_t s);
+// the A operand of the first GEMM: Re rho | Im rho, [qpad][2M] split and
+// tile-ordered, and the pipeline's error word, both set by launch_rhoq32
+struct IsfOperand { __nv_bfloat16 *hi, *lo; int qpad; int* err; };
+IsfOperand isf_tc_operand(int nq, int M, void* d_scratch);
+cudaError_t launch_isf_tc(int nq, int M, double norm, double* d_out, void* d_scratch, const void* d_tables,
+                          cudaStream_t s);
 bool isf_tc_supported(int M);
 // the pipeline's error word (int, 0 or 1) at this offset of the scratch
 size_t isf_tc_error_offset(int nq, int M);

@@ -9,7 +9,7 @@
 // which turns O(Q M N^2) (S) and O(Q M^2 N^2) (F) into O(Q M N) + O(Q M^2).
 #include <algorithm>
 
-#include "pgb_device.cuh"
+#include "isf_tc.cuh"
 
 namespace pgb {
 
@@ -22,13 +22,33 @@ namespace pgb {
 // only the sine and cosine.
 constexpr int kRhoBlock = 256;
 
-// The beads of every slice as fractions of the box, once per call: FP32
-// turns for general q and 32-bit fixed-point turns for lattice q.  The FP64
-// conversion runs here once per bead instead of once per (bead, q block).
-__global__ void k_rho_positions(PathView v, float4* __restrict__ uf, int4* __restrict__ ui) {
-    const size_t n = (size_t)v.M * v.Ne;
-    for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < n;
-         idx += (size_t)gridDim.x * blockDim.x) {
+// Once per call, in one launch: the beads of every slice as fractions of the
+// box, FP32 turns for general q and 32-bit fixed-point turns for lattice q (the
+// FP64 conversion runs once per bead instead of once per (bead, q block)), and
+// each wave vector in turns per box side, n_d = q_d L_d / 2 pi: FP32 turns with
+// a lattice flag in w, and the integers of lattice vectors (the reference's q
+// lists of lattice type) for the exact fixed-point phase.  The first blocks
+// take the wave vectors; `beads` is 0 where the masked form makes the bead
+// fractions.
+__global__ void k_rho_setup(PathView v, const double* __restrict__ q, int nq, int qblocks, size_t beads,
+                            float4* __restrict__ uf, int4* __restrict__ ui, float4* __restrict__ qf,
+                            int4* __restrict__ qi, int* __restrict__ err) {
+    if ((int)blockIdx.x < qblocks) {
+        const int iq = blockIdx.x * blockDim.x + threadIdx.x;
+        if (err && iq == 0) *err = 0;
+        if (iq >= nq) return;
+        const double inv2pi = 0.15915494309189533577;
+        const double dx = q[3*iq] * v.side[0] * inv2pi, dy = q[3*iq+1] * v.side[1] * inv2pi,
+                     dz = q[3*iq+2] * v.side[2] * inv2pi;
+        const double rx = rint(dx), ry = rint(dy), rz = rint(dz);
+        const bool lattice = fabs(dx - rx) < 1e-6 && fabs(dy - ry) < 1e-6 && fabs(dz - rz) < 1e-6 &&
+                             fabs(rx) < 1048576.0 && fabs(ry) < 1048576.0 && fabs(rz) < 1048576.0;
+        qf[iq] = make_float4((float)dx, (float)dy, (float)dz, lattice ? 1.f : 0.f);
+        qi[iq] = make_int4(lattice ? (int)rx : 0, lattice ? (int)ry : 0, lattice ? (int)rz : 0, 0);
+        return;
+    }
+    const size_t stride = (size_t)(gridDim.x - qblocks) * blockDim.x;
+    for (size_t idx = (size_t)(blockIdx.x - qblocks) * blockDim.x + threadIdx.x; idx < beads; idx += stride) {
         const size_t t = idx / v.Ne, j = idx - t * v.Ne;
         const double* X = v.pos + t * 3 * v.Ne;
         const double ux = X[j] * v.sideInv[0], uy = X[v.Ne + j] * v.sideInv[1],
@@ -82,28 +102,11 @@ k_rho_positions_masked(PathView v, double maxR2, float4* __restrict__ uf, int4* 
     if (threadIdx.x == 0) cnt[t] = base;
 }
 
-// Each wave vector in turns per box side, n_d = q_d L_d / 2 pi, once per call
-// (not once per slice in every CTA): FP32 turns with a lattice flag in w, and
-// the integers of lattice vectors (the reference's q lists of lattice type)
-// for the exact fixed-point phase.
-__global__ void k_rho_qsetup(PathView v, const double* __restrict__ q, int nq,
-                             float4* __restrict__ qf, int4* __restrict__ qi) {
-    const int iq = blockIdx.x * blockDim.x + threadIdx.x;
-    if (iq >= nq) return;
-    const double inv2pi = 0.15915494309189533577;
-    const double dx = q[3*iq] * v.side[0] * inv2pi, dy = q[3*iq+1] * v.side[1] * inv2pi,
-                 dz = q[3*iq+2] * v.side[2] * inv2pi;
-    const double rx = rint(dx), ry = rint(dy), rz = rint(dz);
-    const bool lattice = fabs(dx - rx) < 1e-6 && fabs(dy - ry) < 1e-6 && fabs(dz - rz) < 1e-6 &&
-                         fabs(rx) < 1048576.0 && fabs(ry) < 1048576.0 && fabs(rz) < 1048576.0;
-    qf[iq] = make_float4((float)dx, (float)dy, (float)dz, lattice ? 1.f : 0.f);
-    qi[iq] = make_int4(lattice ? (int)rx : 0, lattice ? (int)ry : 0, lattice ? (int)rz : 0, 0);
-}
-
+template <bool kSplit>
 __global__ void __launch_bounds__(kRhoBlock)
 k_rhoq32(PathView v, const float4* __restrict__ uf, const int4* __restrict__ ui,
          const int* __restrict__ cnt, const float4* __restrict__ qf, const int4* __restrict__ qi,
-         int nq, float2* __restrict__ rho) {
+         int nq, float2* __restrict__ rho, IsfOperand split) {
     extern __shared__ float4 su[];
     int4* si = reinterpret_cast<int4*>(su + v.Ne);
     const int t = blockIdx.y;
@@ -114,50 +117,75 @@ k_rhoq32(PathView v, const float4* __restrict__ uf, const int4* __restrict__ ui,
     }
     __syncthreads();
     const int iq = blockIdx.x * kRhoBlock + threadIdx.x;
-    if (iq >= nq) return;
-    // lattice wave vectors take the exact fixed-point phase, any other q the
-    // FP32 turn reduction
-    const float4 f = qf[iq];
-    if (f.w != 0.f) {
-        const int4 k = qi[iq];
-        rho[(size_t)iq * v.M + t] = rho_partial_lattice(si, n, k.x, k.y, k.z);
+    if (iq >= (kSplit ? split.qpad : nq)) return;
+    float2 r = make_float2(0.f, 0.f);
+    if (!kSplit || iq < nq) {
+        // lattice wave vectors take the exact fixed-point phase, any other q the
+        // FP32 turn reduction
+        const float4 f = qf[iq];
+        if (f.w != 0.f) {
+            const int4 k = qi[iq];
+            r = rho_partial_lattice(si, n, k.x, k.y, k.z);
+        } else {
+            r = rho_partial(su, n, f.x, f.y, f.z);
+        }
+    }
+    if (kSplit) {
+        // (Re rho | Im rho) of row iq, zero rows beyond nq; the two-byte stores
+        // hide behind the sines of the other warps
+        const size_t a = tiled_index(iq, t, 2 * v.M, kTM), b = tiled_index(iq, v.M + t, 2 * v.M, kTM);
+        split_bf16(r.x, split.hi[a], split.lo[a]);
+        split_bf16(r.y, split.hi[b], split.lo[b]);
     } else {
-        rho[(size_t)iq * v.M + t] = rho_partial(su, n, f.x, f.y, f.z);
+        rho[(size_t)iq * v.M + t] = r;
     }
 }
 
-size_t rhoq32_work_bytes(const PathView& v) {
-    return (size_t)v.M * v.Ne * (sizeof(float4) + sizeof(int4)) + (size_t)v.M * sizeof(int);
+namespace {
+struct RhoWork { size_t ui, cnt, qf, qi, total; };
+RhoWork rho_work(const PathView& v, int nq) {
+    const size_t nb = (size_t)v.M * v.Ne;
+    RhoWork w;
+    w.ui = nb * sizeof(float4);
+    w.qf = w.ui + nb * sizeof(int4);
+    w.qi = w.qf + (size_t)nq * sizeof(float4);
+    w.cnt = w.qi + (size_t)nq * sizeof(int4);
+    w.total = w.cnt + (size_t)v.M * sizeof(int);
+    return w;
 }
+}  // namespace
+
+size_t rhoq32_work_bytes(const PathView& v, int nq) { return rho_work(v, nq).total; }
 
 cudaError_t launch_rhoq32(const PathView& v, const double* d_q, int nq, float2* d_rho,
-                          void* d_work, cudaStream_t s, double maxR2) {
+                          void* d_work, cudaStream_t s, double maxR2, const IsfOperand* split) {
     if (nq <= 0) return cudaSuccess;
-    float4* uf = static_cast<float4*>(d_work);
-    int4* ui = reinterpret_cast<int4*>(uf + (size_t)v.M * v.Ne);
-    int* cnt = nullptr;
-    if (maxR2 > 0.0) {
-        cnt = reinterpret_cast<int*>(ui + (size_t)v.M * v.Ne);
-        k_rho_positions_masked<<<v.M, kMaskBlock, 0, s>>>(v, maxR2, uf, ui, cnt);
-    } else {
-        const size_t nb = (size_t)v.M * v.Ne;
-        const int blocks = (int)std::min<size_t>((nb + 255) / 256, 152 * 16);
-        k_rho_positions<<<blocks, 256, 0, s>>>(v, uf, ui);
-    }
-    dim3 grid((nq + kRhoBlock - 1) / kRhoBlock, v.M);
     size_t smem = (size_t)v.Ne * (sizeof(float4) + sizeof(int4));
     if (smem > 200 * 1024) return cudaErrorInvalidValue;   // one slice must fit in shared memory
     {
-        const cudaError_t ae = set_smem_limit(k_rhoq32, 200 * 1024);
+        const cudaError_t ae = split ? set_smem_limit(k_rhoq32<true>, 200 * 1024) : set_smem_limit(k_rhoq32<false>, 200 * 1024);
         if (ae != cudaSuccess) return ae;
     }
-    // the wave-vector table sits in the unused half of the rho region, which
-    // is sized for FP64 values (16 B per (q, slice)); M is even, so it starts
-    // 16-byte aligned
-    float4* qf = reinterpret_cast<float4*>(d_rho + (size_t)nq * v.M);
-    int4* qi = reinterpret_cast<int4*>(qf + nq);
-    k_rho_qsetup<<<(nq + 255) / 256, 256, 0, s>>>(v, d_q, nq, qf, qi);
-    k_rhoq32<<<grid, kRhoBlock, smem, s>>>(v, uf, ui, cnt, qf, qi, nq, d_rho);
+    const RhoWork w = rho_work(v, nq);
+    char* base = static_cast<char*>(d_work);
+    float4* uf = reinterpret_cast<float4*>(base);
+    int4* ui = reinterpret_cast<int4*>(base + w.ui);
+    float4* qf = reinterpret_cast<float4*>(base + w.qf);
+    int4* qi = reinterpret_cast<int4*>(base + w.qi);
+    int* cnt = nullptr;
+    size_t nb = (size_t)v.M * v.Ne;
+    if (maxR2 > 0.0) {
+        cnt = reinterpret_cast<int*>(base + w.cnt);
+        k_rho_positions_masked<<<v.M, kMaskBlock, 0, s>>>(v, maxR2, uf, ui, cnt);
+        nb = 0;
+    }
+    const int qblocks = (nq + 255) / 256;
+    const int blocks = qblocks + (int)std::min<size_t>((nb + 255) / 256, 152 * 16);
+    k_rho_setup<<<blocks, 256, 0, s>>>(v, d_q, nq, qblocks, nb, uf, ui, qf, qi, split ? split->err : nullptr);
+    const int rows = split ? split->qpad : nq;
+    dim3 grid((rows + kRhoBlock - 1) / kRhoBlock, v.M);
+    if (split) k_rhoq32<true><<<grid, kRhoBlock, smem, s>>>(v, uf, ui, cnt, qf, qi, nq, nullptr, *split);
+    else k_rhoq32<false><<<grid, kRhoBlock, smem, s>>>(v, uf, ui, cnt, qf, qi, nq, d_rho, IsfOperand{});
     return cudaGetLastError();
 }
 

@@ -60,7 +60,7 @@ def test_slice_sums_keep_their_order(pgb, n):
     assert abs(e[3] - vint) <= 1e-14 * (scale[0] + abs(tail))
 
 
-@pytest.mark.parametrize("n,m,nq", [(3, 2, 1), (5, 30, 17), (40, 62, 130), (9, 64, 9), (20, 66, 33), (6, 250, 70),
+@pytest.mark.parametrize("n,m,nq", [(3, 2, 1), (5, 30, 17), (40, 62, 130), (9, 64, 9), (20, 67, 33), (6, 250, 70),
                                     (2, 1030, 3), (2, 15400, 2)])
 def test_correlation(pgb, n, m, nq):
     cfg, L = _path(pgb, n, m, n + m)
