@@ -75,11 +75,13 @@ __global__ void k_update_beads(double* pos, float4* pos32, int Ne, const int2* b
     pos32[(size_t)b.x * Ne + b.y] = make_float4((float)p[3*i], (float)p[3*i+1], (float)p[3*i+2], 0.f);
 }
 
-// full bead records (position, links, active flag) into the device path
+// full bead records (position, links, active flag) into the device path, and
+// numBeadsAtSlice
 struct BeadRec { int s, p, ns, np, ps, pp, on, pad; double x, y, z; };
 __global__ void k_set_beads(double* pos, float4* pos32, int2* nxt, int2* prv, uint8_t* on, int Ne,
-                            const BeadRec* r, int k) {
+                            const BeadRec* r, int k, const int* counts, int* nbs, int M) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int t = i; t < M; t += gridDim.x * blockDim.x) nbs[t] = counts[t];
     if (i >= k) return;
     const BeadRec b = r[i];
     double* X = pos + (size_t)b.s * 3 * Ne;
@@ -113,6 +115,11 @@ using namespace pgb;
 namespace {
 
 thread_local std::string g_last_error;
+
+// lists up to this many beads are read and answered in host memory
+constexpr int kDirectBeads = 2048;
+static_assert((size_t)kDirectBeads * (sizeof(int2) + 3 * sizeof(double)) <= kRingBytes / 2 &&
+              (size_t)kDirectBeads * sizeof(double) <= kResultBytes, "room for a direct list");
 
 int check_ctx(pgb_ctx* c) { return c ? PGB_OK : PGB_EINVAL; }
 
@@ -167,23 +174,58 @@ TermsWanted want_virial(const Ctx& c) {
 int compute_terms(Ctx& c, std::vector<double>& h, TermsWanted want) {
     int rc = need_path(c); if (rc) return rc;
     PathView v = c.view();
-    size_t bytes = (size_t)8 * c.M * sizeof(double);
-    rc = c.ensure_scratch(c.p.precision == PGB_MIXED ? slice_terms32_work(v) : slice_terms64_work(v)); if (rc) return rc;
-    double* d = static_cast<double*>(c.d_scratch);
+    const size_t bytes = (size_t)8 * c.M * sizeof(double);
+    const bool direct = bytes <= kResultBytes;             // the kernel writes host memory
+    const size_t work = ((c.p.precision == PGB_MIXED ? slice_terms32_work(v) : slice_terms64_work(v)) + 255) & ~(size_t)255;
+    rc = c.ensure_scratch(work + (direct ? 0 : bytes)); if (rc) return rc;
+    double* d = reinterpret_cast<double*>(direct ? c.stage.result() : static_cast<char*>(c.d_scratch) + work);
     int window = c.p.virial_window > 0 ? c.p.virial_window : 5;
     cudaError_t e = (c.p.precision == PGB_MIXED)
-        ? launch_slice_terms32(v, c.az, want.window ? window : 0, want.even, want.odd, c.d_arrived, d, c.stream)
-        : launch_slice_terms64(v, want.window ? window : 0, want.even, want.odd, c.d_arrived, d, c.stream);
+        ? launch_slice_terms32(v, c.az, want.window ? window : 0, want.even, want.odd, c.d_arrived, c.d_scratch, d, c.stream)
+        : launch_slice_terms64(v, want.window ? window : 0, want.even, want.odd, c.d_arrived, c.d_scratch, d, c.stream);
     if (e != cudaSuccess) return c.cuda_fail(e, "slice terms launch");
-    h.assign((size_t)8 * c.M, 0.0);
-    PGB_CUDA(&c, cudaMemcpyAsync(h.data(), d, bytes, cudaMemcpyDeviceToHost, c.stream));
+    h.resize((size_t)8 * c.M);
+    if (!direct) PGB_CUDA(&c, cudaMemcpyAsync(h.data(), d, bytes, cudaMemcpyDeviceToHost, c.stream));
     PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
+    if (direct) std::memcpy(h.data(), d, bytes);
     return PGB_OK;
 }
 
 }  // namespace
 
 void pgb::set_global_error(const std::string& msg) { g_last_error = msg; }
+
+namespace {
+std::mutex g_pinned_mutex;
+std::vector<void*> g_pinned_free;
+}  // namespace
+
+void* pgb::pinned_acquire() {
+    for (;;) {
+        void* p = nullptr;
+        {
+            std::lock_guard<std::mutex> lk(g_pinned_mutex);
+            if (!g_pinned_free.empty()) { p = g_pinned_free.back(); g_pinned_free.pop_back(); }
+        }
+        if (!p) {
+            if (cudaMallocHost(&p, kStageBytes) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+            return p;
+        }
+        // a block from before a device reset is no longer pinned
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeHost) return p;
+        cudaGetLastError();
+    }
+}
+
+void pgb::pinned_release(void* block) {
+    if (!block) return;
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mutex);
+        if (g_pinned_free.size() < (size_t)kPinnedKept) { g_pinned_free.push_back(block); return; }
+    }
+    cudaFreeHost(block);
+}
 
 cudaError_t pgb::set_carveout(const void* func, int percent) {
     static std::mutex mu;
@@ -290,6 +332,10 @@ int pgb_create(const pgb_params* p, pgb_ctx** out) {
             if ((e = cudaMalloc(&c.d_trial_count, (2 * nb + 1) * sizeof(int))) != cudaSuccess) break;
         if ((e = cudaMalloc(&c.d_arrived, c.M * sizeof(unsigned))) != cudaSuccess) break;
         if ((e = cudaMemsetAsync(c.d_arrived, 0, c.M * sizeof(unsigned), c.stream)) != cudaSuccess) break;
+        if ((e = cudaMalloc(&c.d_hist, 64 * sizeof(unsigned long long))) != cudaSuccess) break;
+        if ((e = cudaMemsetAsync(c.d_hist, 0, 64 * sizeof(unsigned long long), c.stream)) != cudaSuccess) break;
+        c.stage.block = static_cast<char*>(pinned_acquire());
+        if (!c.stage.block) { e = cudaErrorMemoryAllocation; break; }
         if (p->precision == PGB_FP64 && (p->gradvfactor[0] > kEPS || p->gradvfactor[1] > kEPS))
             if ((e = cudaMalloc(&c.d_force64, nb * 3 * sizeof(double))) != cudaSuccess) break;
     } while (0);
@@ -327,6 +373,8 @@ int pgb_destroy(pgb_ctx* h) {
     if (c.d_force32) cudaFree(c.d_force32);
     if (c.d_force64) cudaFree(c.d_force64);
     if (c.d_arrived) cudaFree(c.d_arrived);
+    if (c.d_hist) cudaFree(c.d_hist);
+    pinned_release(c.stage.block);
     if (c.d_trial_count) cudaFree(c.d_trial_count);
     if (c.h_pinned) cudaFreeHost(c.h_pinned);
     if (c.stream) cudaStreamDestroy(c.stream);
@@ -459,17 +507,24 @@ int pgb_update_beads(pgb_ctx* h, const int32_t* beads, const double* pos, int k)
         if (beads[2*i] < 0 || beads[2*i] >= c.M || beads[2*i+1] < 0 || beads[2*i+1] >= c.Ne)
             return c.fail(PGB_EINVAL, "update_beads: bead out of range");
     size_t bb = (size_t)k * sizeof(int2), pb = (size_t)k * 3 * sizeof(double);
-    rc = c.ensure_scratch(bb + pb + 64); if (rc) return rc;
-    rc = c.ensure_pinned(bb + pb + 64); if (rc) return rc;
-    char* hp = static_cast<char*>(c.h_pinned);
-    std::memcpy(hp, beads, bb);
-    std::memcpy(hp + bb, pos, pb);
-    char* dp = static_cast<char*>(c.d_scratch);
-    PGB_CUDA(&c, cudaMemcpyAsync(dp, hp, bb + pb, cudaMemcpyHostToDevice, c.stream));
+    char* in = c.stage.take(bb + pb, c.stream);              // read by the kernel; no wait
+    const bool direct = in != nullptr;
+    if (!direct) {
+        rc = c.ensure_scratch(bb + pb + 64); if (rc) return rc;
+        rc = c.ensure_pinned(bb + pb + 64); if (rc) return rc;
+        in = static_cast<char*>(c.h_pinned);
+    }
+    std::memcpy(in, beads, bb);
+    std::memcpy(in + bb, pos, pb);
+    const char* dp = in;
+    if (!direct) {
+        PGB_CUDA(&c, cudaMemcpyAsync(c.d_scratch, in, bb + pb, cudaMemcpyHostToDevice, c.stream));
+        dp = static_cast<char*>(c.d_scratch);
+    }
     k_update_beads<<<(k + 127) / 128, 128, 0, c.stream>>>(c.d_pos, c.d_pos32, c.Ne,
         reinterpret_cast<const int2*>(dp), reinterpret_cast<const double*>(dp + bb), k);
     PGB_CUDA(&c, cudaGetLastError());
-    PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
+    if (!direct) PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
     c.force_valid = false;
     return PGB_OK;
 }
@@ -567,14 +622,19 @@ int pgb_bead_actions(pgb_ctx* h, const int32_t* beads, int k, int shift, int mod
         if (beads[2*i] < 0 || beads[2*i] >= c.M || beads[2*i+1] < 0 || beads[2*i+1] >= c.Ne)
             return c.fail(PGB_EINVAL, "bead_actions: bead out of range");
     size_t bb = (size_t)k * sizeof(int2), ob = (size_t)k * sizeof(double);
-    rc = c.ensure_scratch(bb + ob + 64); if (rc) return rc;
-    rc = c.ensure_pinned(bb + ob + 64); if (rc) return rc;
-    char* hp = static_cast<char*>(c.h_pinned);
-    std::memcpy(hp, beads, bb);
+    // few beads: the kernel reads the list and writes the actions in host memory
+    char* in = k <= kDirectBeads ? c.stage.take(bb, c.stream) : nullptr;
+    const bool direct = in != nullptr;
+    if (!direct) {
+        rc = c.ensure_scratch(bb + ob + 64); if (rc) return rc;
+        rc = c.ensure_pinned(bb + ob + 64); if (rc) return rc;
+        in = static_cast<char*>(c.h_pinned);
+    }
+    std::memcpy(in, beads, bb);
     char* dp = static_cast<char*>(c.d_scratch);
-    int2* d_b = reinterpret_cast<int2*>(dp);
-    double* d_o = reinterpret_cast<double*>(dp + ((bb + 15) & ~(size_t)15));
-    PGB_CUDA(&c, cudaMemcpyAsync(dp, hp, bb, cudaMemcpyHostToDevice, c.stream));
+    int2* d_b = reinterpret_cast<int2*>(direct ? in : dp);
+    double* d_o = reinterpret_cast<double*>(direct ? c.stage.result() : dp + ((bb + 15) & ~(size_t)15));
+    if (!direct) PGB_CUDA(&c, cudaMemcpyAsync(dp, in, bb, cudaMemcpyHostToDevice, c.stream));
     PathView v = c.view();
     const float4* fall = slice_forces(c, &rc);
     if (rc) return rc;
@@ -587,8 +647,11 @@ int pgb_bead_actions(pgb_ctx* h, const int32_t* beads, int k, int shift, int mod
         : launch_bead_actions32(v, c.az, d_b, k, shift, mode, c.p.tau, c.p.lambda,
                                 c.p.vfactor, c.p.gradvfactor, nullptr, d_o, c.stream, fall);
     if (e != cudaSuccess) return c.cuda_fail(e, "bead actions launch");
-    double* ho = reinterpret_cast<double*>(hp + ((bb + 15) & ~(size_t)15));
-    PGB_CUDA(&c, cudaMemcpyAsync(ho, d_o, ob, cudaMemcpyDeviceToHost, c.stream));
+    double* ho = d_o;
+    if (!direct) {
+        ho = reinterpret_cast<double*>(in + ((bb + 15) & ~(size_t)15));
+        PGB_CUDA(&c, cudaMemcpyAsync(ho, d_o, ob, cudaMemcpyDeviceToHost, c.stream));
+    }
     PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
     double tot = 0.0;
     for (int i = 0; i < k; ++i) tot += ho[i];
@@ -963,12 +1026,20 @@ int scatter_host(pgb_ctx* h, const double* q, int nq, int what, int mode, double
     size_t off_w = (off_o + ob + 255) & ~(size_t)255;
     rc = c.ensure_scratch(off_w + wb); if (rc) return rc;
     char* base = static_cast<char*>(c.d_scratch);
-    PGB_CUDA(&c, cudaMemcpyAsync(base, q, qb, cudaMemcpyHostToDevice, c.stream));
-    rc = scatter_common(c, reinterpret_cast<double*>(base), nq, what, mode,
-                        reinterpret_cast<double*>(base + off_o), base + off_w);
-    if (rc) return rc;
-    PGB_CUDA(&c, cudaMemcpyAsync(out, base + off_o, ob, cudaMemcpyDeviceToHost, c.stream));
+    // short lists of wave vectors are read, and short results written, in host
+    // memory by the kernels
+    double* d_q = reinterpret_cast<double*>(c.stage.take(qb, c.stream));
+    if (d_q) std::memcpy(d_q, q, qb);
+    else {
+        d_q = reinterpret_cast<double*>(base);
+        PGB_CUDA(&c, cudaMemcpyAsync(d_q, q, qb, cudaMemcpyHostToDevice, c.stream));
+    }
     const bool tc = c.p.precision == PGB_MIXED && what == 1 && mode == 1;
+    const bool direct = ob <= kResultBytes && what != 2;
+    double* d_out = reinterpret_cast<double*>(direct ? c.stage.result() : base + off_o);
+    rc = scatter_common(c, d_q, nq, what, mode, d_out, base + off_w);
+    if (rc) return rc;
+    if (!direct) PGB_CUDA(&c, cudaMemcpyAsync(out, d_out, ob, cudaMemcpyDeviceToHost, c.stream));
     int tc_err = 0;
     if (tc) {
         // the tensor-core pipeline's error word: a bounded wait ran out
@@ -977,6 +1048,7 @@ int scatter_host(pgb_ctx* h, const double* q, int nq, int what, int mode, double
                                      cudaMemcpyDeviceToHost, c.stream));
     }
     PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
+    if (direct) std::memcpy(out, d_out, ob);
     if (tc_err)
         return c.fail(PGB_ETIMEOUT, "F(q,tau): a tensor-core pipeline wait ran out (a staged copy or "
                                     "the MMAs did not complete within the wait limit)");
@@ -1152,18 +1224,28 @@ int pgb_trial_actions(pgb_ctx* h, const int32_t* beads, const double* pos, int k
     size_t bb = ((size_t)k * sizeof(int2) + 255) & ~(size_t)255;
     size_t pb = ((size_t)k * 3 * sizeof(double) + 255) & ~(size_t)255;
     size_t ob = ((size_t)k * 2 * sizeof(double) + 255) & ~(size_t)255;
+    char* in = k <= kDirectBeads ? c.stage.take(bb + pb, c.stream) : nullptr;
+    const bool direct = in != nullptr;
     rc = c.ensure_scratch(bb + pb + ob + (size_t)k * sizeof(double)); if (rc) return rc;
     char* d = static_cast<char*>(c.d_scratch);
-    PGB_CUDA(&c, cudaMemcpyAsync(d, beads, (size_t)k * sizeof(int2), cudaMemcpyHostToDevice, c.stream));
-    PGB_CUDA(&c, cudaMemcpyAsync(d + bb, pos, (size_t)k * 3 * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+    if (direct) {
+        std::memcpy(in, beads, (size_t)k * sizeof(int2));
+        std::memcpy(in + bb, pos, (size_t)k * 3 * sizeof(double));
+    } else {
+        PGB_CUDA(&c, cudaMemcpyAsync(d, beads, (size_t)k * sizeof(int2), cudaMemcpyHostToDevice, c.stream));
+        PGB_CUDA(&c, cudaMemcpyAsync(d + bb, pos, (size_t)k * 3 * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+        in = d;
+    }
     double* d_new = reinterpret_cast<double*>(d + bb + pb);
     double* d_old = d_new + k;
-    double* d_del = reinterpret_cast<double*>(d + bb + pb + ob);
-    rc = trial_launch(c, reinterpret_cast<int2*>(d), reinterpret_cast<double*>(d + bb), k, shift, mode,
+    double* d_del = reinterpret_cast<double*>(direct ? c.stage.result() : d + bb + pb + ob);
+    rc = trial_launch(c, reinterpret_cast<int2*>(in), reinterpret_cast<double*>(in + bb), k, shift, mode,
                       d_new, d_old, d_del);
     if (rc) return rc;
-    PGB_CUDA(&c, cudaMemcpyAsync(out_delta, d_del, (size_t)k * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    if (!direct)
+        PGB_CUDA(&c, cudaMemcpyAsync(out_delta, d_del, (size_t)k * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
+    if (direct) std::memcpy(out_delta, d_del, (size_t)k * sizeof(double));
     return PGB_OK;
 }
 
@@ -1189,11 +1271,8 @@ int pgb_pair_correlation(pgb_ctx* h, int slice, double* out50) {
     Ctx& c = h->c;
     int rc = need_path(c); if (rc) return rc;
     if (slice >= c.M) return c.fail(PGB_EINVAL, "pair_correlation: slice out of range");
-    rc = c.ensure_scratch(64 * sizeof(unsigned long long)); if (rc) return rc;
-    auto* d_hist = static_cast<unsigned long long*>(c.d_scratch);
-    PGB_CUDA(&c, launch_sep_hist(c.view(), slice, d_hist, c.stream));
-    unsigned long long hist[50];
-    PGB_CUDA(&c, cudaMemcpyAsync(hist, d_hist, sizeof(hist), cudaMemcpyDeviceToHost, c.stream));
+    auto* hist = reinterpret_cast<unsigned long long*>(c.stage.result());
+    PGB_CUDA(&c, launch_sep_hist(c.view(), slice, c.d_arrived, c.d_hist, hist, c.stream));
     PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
     // PairCorrelationEstimator: constructor norm (estimator.cpp:3187-3223) and
     // accumulate (estimator.cpp:3238-3246), 3D periodic box
@@ -1218,10 +1297,8 @@ int pgb_superfluid(pgb_ctx* h, double* out26) {
     int rc = need_path(c); if (rc) return rc;
     rc = c.ensure_scratch(winding_work_bytes()); if (rc) return rc;
     double* d_work = static_cast<double*>(c.d_scratch);
-    double* d_out = d_work + (winding_work_bytes() / sizeof(double) - 5);
-    PGB_CUDA(&c, launch_winding(c.view(), c.d_arrived, d_work, d_out, c.stream));
-    double s5[5];
-    PGB_CUDA(&c, cudaMemcpyAsync(s5, d_out, sizeof(s5), cudaMemcpyDeviceToHost, c.stream));
+    double* s5 = reinterpret_cast<double*>(c.stage.result());
+    PGB_CUDA(&c, launch_winding(c.view(), c.d_arrived, d_work, s5, c.stream));
     PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
     // SuperfluidFractionEstimator::accumulate, estimator.cpp:2000-2074
     double W[3] = {s5[0], s5[1], s5[2]};
@@ -1249,11 +1326,11 @@ int pgb_permutation_cycles(pgb_ctx* h, double* out40) {
     const int nw = c.h_nbs.empty() ? 0 : c.h_nbs[0];
     for (int i = 0; i < 40; ++i) out40[i] = 0.0;
     if (nw == 0) return PGB_OK;
-    rc = c.ensure_scratch(cycles_work_ints(c.view(), nw) * sizeof(int)); if (rc) return rc;
-    int* d_len = static_cast<int*>(c.d_scratch);
-    PGB_CUDA(&c, launch_cycles(c.view(), nw, c.d_arrived, d_len, c.stream));
-    std::vector<int> len(nw);
-    PGB_CUDA(&c, cudaMemcpyAsync(len.data(), d_len, nw * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    rc = c.ensure_scratch(cycles_work_ints(c.view()) * sizeof(int)); if (rc) return rc;
+    static_assert(8192 * sizeof(int) <= kResultBytes, "room for one slice's cycle lengths");
+    int* len = reinterpret_cast<int*>(c.stage.result());
+    PGB_CUDA(&c, launch_cycles(c.view(), nw, c.d_arrived, reinterpret_cast<int*>(c.d_hist + 63),
+                               static_cast<int*>(c.d_scratch), len, c.stream));
     PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
     // PermutationCycleEstimator::accumulate, estimator.cpp:2735-2781
     const int N = c.numBeadsOn / c.M;
@@ -1270,28 +1347,36 @@ int pgb_permutation_cycles(pgb_ctx* h, double* out40) {
 
 namespace pgb {
 int upload_beads(Ctx& c, const int* lin, int k, const double* pos_aos) {
-    if (k > 0) {
-        const size_t rb = (size_t)k * sizeof(BeadRec);
-        int rc = c.ensure_scratch(rb + 64); if (rc) return rc;
-        rc = c.ensure_pinned(rb + 64); if (rc) return rc;
-        BeadRec* hr = static_cast<BeadRec*>(c.h_pinned);
-        for (int i = 0; i < k; ++i) {
-            const size_t j = (size_t)lin[i];
-            BeadRec r;
-            r.s = (int)(j / c.Ne); r.p = (int)(j % c.Ne);
-            r.ns = c.h_next[2*j]; r.np = c.h_next[2*j+1];
-            r.ps = c.h_prev[2*j]; r.pp = c.h_prev[2*j+1];
-            r.on = c.h_on[j]; r.pad = 0;
-            r.x = pos_aos[3*j]; r.y = pos_aos[3*j+1]; r.z = pos_aos[3*j+2];
-            hr[i] = r;
-        }
-        PGB_CUDA(&c, cudaMemcpyAsync(c.d_scratch, hr, rb, cudaMemcpyHostToDevice, c.stream));
-        k_set_beads<<<(k + 127) / 128, 128, 0, c.stream>>>(c.d_pos, c.d_pos32, c.d_next, c.d_prev, c.d_on,
-                                                           c.Ne, static_cast<const BeadRec*>(c.d_scratch), k);
-        PGB_CUDA(&c, cudaGetLastError());
+    const size_t rb = (size_t)k * sizeof(BeadRec), nb = c.M * sizeof(int);
+    char* in = c.stage.take(rb + nb, c.stream);              // read by the kernel; no wait
+    const bool direct = in != nullptr;
+    if (!direct) {
+        int rc = c.ensure_scratch(rb + nb); if (rc) return rc;
+        rc = c.ensure_pinned(rb + nb); if (rc) return rc;
+        in = static_cast<char*>(c.h_pinned);
     }
-    PGB_CUDA(&c, cudaMemcpyAsync(c.d_nbs, c.h_nbs.data(), c.M * sizeof(int), cudaMemcpyHostToDevice, c.stream));
-    PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
+    BeadRec* hr = reinterpret_cast<BeadRec*>(in);
+    for (int i = 0; i < k; ++i) {
+        const size_t j = (size_t)lin[i];
+        BeadRec r;
+        r.s = (int)(j / c.Ne); r.p = (int)(j % c.Ne);
+        r.ns = c.h_next[2*j]; r.np = c.h_next[2*j+1];
+        r.ps = c.h_prev[2*j]; r.pp = c.h_prev[2*j+1];
+        r.on = c.h_on[j]; r.pad = 0;
+        r.x = pos_aos[3*j]; r.y = pos_aos[3*j+1]; r.z = pos_aos[3*j+2];
+        hr[i] = r;
+    }
+    std::memcpy(in + rb, c.h_nbs.data(), nb);
+    const char* d = in;
+    if (!direct) {
+        PGB_CUDA(&c, cudaMemcpyAsync(c.d_scratch, in, rb + nb, cudaMemcpyHostToDevice, c.stream));
+        d = static_cast<char*>(c.d_scratch);
+    }
+    k_set_beads<<<std::max(1, (k + 127) / 128), 128, 0, c.stream>>>(
+        c.d_pos, c.d_pos32, c.d_next, c.d_prev, c.d_on, c.Ne, reinterpret_cast<const BeadRec*>(d), k,
+        reinterpret_cast<const int*>(d + rb), c.d_nbs, c.M);
+    PGB_CUDA(&c, cudaGetLastError());
+    if (!direct) PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
     c.force_valid = false;
     return PGB_OK;
 }

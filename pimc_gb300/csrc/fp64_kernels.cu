@@ -881,15 +881,15 @@ k_slice_terms64(PathView v, double invdr, int window, int even, int odd, unsigne
 
 static int slice_blocks(int Ne) { return (Ne + kSliceRows - 1) / kSliceRows; }
 
-size_t slice_terms64_work(const PathView& v) { return (size_t)8 * v.M * (1 + slice_blocks(v.Ne)) * sizeof(double); }
+size_t slice_terms64_work(const PathView& v) { return (size_t)8 * v.M * slice_blocks(v.Ne) * sizeof(double); }
 
 cudaError_t launch_slice_terms64(const PathView& v, int window, int even, int odd, unsigned* d_arrived,
-                                 double* d_terms, cudaStream_t s) {
+                                 void* d_work, double* d_terms, cudaStream_t s) {
     const size_t smem = (size_t)v.Ne * 3 * sizeof(double);
     const cudaError_t ae = set_smem_limit(k_slice_terms64, 200 * 1024);
     if (ae != cudaSuccess) return ae;
     k_slice_terms64<<<dim3(v.M, slice_blocks(v.Ne)), kPairBlock, smem, s>>>(
-        v, 1.0 / v.dr, window, even, odd, d_arrived, d_terms + (size_t)8 * v.M, d_terms);
+        v, 1.0 / v.dr, window, even, odd, d_arrived, static_cast<double*>(d_work), d_terms);
     return cudaGetLastError();
 }
 

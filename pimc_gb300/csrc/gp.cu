@@ -400,6 +400,7 @@ struct pgb_gp {
     cudaStream_t stream = nullptr;
     double4* d_train64 = nullptr;
     float4* d_train32 = nullptr;
+    Staging stage;
     // per-call scratch: positions, values, fold, cut flags (grown on demand)
     void* d_buf = nullptr;
     size_t buf_bytes = 0;
@@ -540,6 +541,10 @@ int pgb_gp_create(const pgb_gp_params* p, const double* training, int n, pgb_gp*
         g.reach[d] = most[d] * g.perInv[d];
     }
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) {
+        h->stage.block = static_cast<char*>(pinned_acquire());
+        if (!h->stage.block) e = cudaErrorMemoryAllocation;
+    }
     if (e == cudaSuccess) e = cudaMalloc(&h->d_train64, t64.size() * sizeof(double4));
     if (e == cudaSuccess) e = cudaMalloc(&h->d_train32, t32.size() * sizeof(float4));
     if (e == cudaSuccess) e = cudaMemcpy(h->d_train64, t64.data(), t64.size() * sizeof(double4), cudaMemcpyHostToDevice);
@@ -558,6 +563,7 @@ int pgb_gp_destroy(pgb_gp* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     cudaFree(h->d_train64); cudaFree(h->d_train32); cudaFree(h->d_buf); cudaFree(h->d_part);
     cudaFree(h->d_arrived);
+    pinned_release(h->stage.block);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return PGB_OK;
@@ -573,10 +579,25 @@ int pgb_gp_eval_device_async(pgb_gp* h, const double* d_pos, double* d_values, i
     return PGB_OK;
 }
 
+// A call's positions as the kernels read them and values as they write them:
+// both in the handle's host block when they fit there, else nullptr.
+static double* gp_direct(pgb_gp* h, const double* pos, size_t pb, size_t vb) {
+    char* in = vb <= kResultBytes ? h->stage.take(pb, h->stream) : nullptr;
+    if (in) std::memcpy(in, pos, pb);
+    return reinterpret_cast<double*>(in);
+}
+
 int pgb_gp_eval(pgb_gp* h, const double* pos, double* values, int count) {
     if (!h || count < 0 || (count > 0 && (!pos || !values))) return PGB_EINVAL;
     if (count == 0) return PGB_OK;
     const size_t pb = (size_t)count * 3 * sizeof(double), vb = (size_t)count * sizeof(double);
+    if (double* in = gp_direct(h, pos, pb, vb)) {
+        cudaError_t e = launch_gp(h, in, count, reinterpret_cast<double*>(h->stage.result()));
+        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+        if (e != cudaSuccess) return h->cfail(e, "GP eval");
+        std::memcpy(values, h->stage.result(), vb);
+        return PGB_OK;
+    }
     int rc = ensure_buf(h, al256(pb) + vb); if (rc) return rc;
     char* base = static_cast<char*>(h->d_buf);
     double* d_pos = reinterpret_cast<double*>(base);
@@ -607,7 +628,10 @@ int pgb_gp_benzene_v(pgb_gp* h, const double* pos, double* values, int count) {
     double* d_val = reinterpret_cast<double*>(base + o_val);
     unsigned char* d_cut = reinterpret_cast<unsigned char*>(base + o_cut);
     const int blocks = (count + 255) / 256;
-    cudaError_t e = cudaMemcpyAsync(d_pos, pos, pb, cudaMemcpyHostToDevice, h->stream);
+    double* in = gp_direct(h, pos, pb, vb);
+    cudaError_t e = cudaSuccess;
+    if (in) { d_pos = in; d_val = reinterpret_cast<double*>(h->stage.result()); }
+    else e = cudaMemcpyAsync(d_pos, pos, pb, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
         k_benzene_fold<<<blocks, 256, 0, h->stream>>>(d_pos, count, d_fold, d_cut);
         e = cudaGetLastError();
@@ -617,8 +641,9 @@ int pgb_gp_benzene_v(pgb_gp* h, const double* pos, double* values, int count) {
         k_benzene_combine<<<blocks, 256, 0, h->stream>>>(b, d_fold, d_cut, d_gp, count, d_val);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(values, d_val, vb, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess && !in) e = cudaMemcpyAsync(values, d_val, vb, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e == cudaSuccess && in) std::memcpy(values, d_val, vb);
     if (e != cudaSuccess) return h->cfail(e, "GP benzene");
     return PGB_OK;
 }

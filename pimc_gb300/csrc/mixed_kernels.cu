@@ -960,20 +960,17 @@ k_slice_terms32(PathView v, AzizF az, BoxF B, int window, int even, int odd, uns
 
 static int slice_blocks32(int Ne) { return (Ne + kSliceRows32 - 1) / kSliceRows32; }
 
-size_t slice_terms32_work(const PathView& v) {
-    return (size_t)8 * v.M * sizeof(double) + (size_t)9 * v.M * v.Ne * sizeof(float);
-}
+size_t slice_terms32_work(const PathView& v) { return (size_t)9 * v.M * v.Ne * sizeof(float); }
 
 cudaError_t launch_slice_terms32(const PathView& v, AzizParams a, int window, int even, int odd, unsigned* d_arrived,
-                                 double* d_terms, cudaStream_t s) {
+                                 void* d_work, double* d_terms, cudaStream_t s) {
     size_t smem = (size_t)v.Ne * sizeof(float4);
     {
         const cudaError_t ae = set_smem_limit(k_slice_terms32, 200 * 1024);
         if (ae != cudaSuccess) return ae;
     }
     k_slice_terms32<<<dim3(v.M, slice_blocks32(v.Ne)), kSliceRows32, smem, s>>>(
-        v, make_aziz_f(a), box_f(v), window, even, odd, d_arrived,
-        reinterpret_cast<float*>(d_terms + (size_t)8 * v.M), d_terms);
+        v, make_aziz_f(a), box_f(v), window, even, odd, d_arrived, static_cast<float*>(d_work), d_terms);
     return cudaGetLastError();
 }
 

@@ -12,6 +12,18 @@ namespace pgb {
 constexpr int kPcfBins = 50;                 // NPCFSEP, include/common.h:85
 constexpr int kEstBlock = 256;
 
+// The last CTA of a grid to arrive; the others' global writes are visible to
+// it.  The counter returns to 0 for the next call.
+__device__ __forceinline__ bool last_to_arrive(unsigned* counter, unsigned blocks) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(counter, blocks - 1) == blocks - 1;
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
 // Separation histogram of the pairs b1 < b2 of slices [t0, t1) with
 // ActionBase::updateSepHist's binning (action.cpp:216-224):
 // nR = int(|r_b2 - r_b1| / dSep).  One CTA per slice.  The slice is staged
@@ -49,7 +61,8 @@ __device__ __forceinline__ int sep_bin64(const PathView& v, int t, int b1, int b
 }
 
 __global__ void __launch_bounds__(kSepBlock)
-k_sep_hist(PathView v, SepF f, int t0, double dSep, unsigned long long* __restrict__ hist) {
+k_sep_hist(PathView v, SepF f, int t0, double dSep, unsigned* __restrict__ arrived,
+           unsigned long long* __restrict__ hist, unsigned long long* __restrict__ out) {
     extern __shared__ float4 sp[];                       // [n] slice positions, FP32
     __shared__ int2 near_pair[kSepNear];
     __shared__ int s_near;
@@ -100,11 +113,12 @@ k_sep_hist(PathView v, SepF f, int t0, double dSep, unsigned long long* __restri
         c = __reduce_add_sync(0xffffffffu, c);
         if (lane == 0 && c) atomicAdd(&hist[b], (unsigned long long)c);
     }
+    // the last slice hands the counts over and leaves zeros for the next call
+    if (last_to_arrive(arrived, gridDim.x) && threadIdx.x < kPcfBins) out[threadIdx.x] = atomicExch(&hist[threadIdx.x], 0ull);
 }
 
-cudaError_t launch_sep_hist(const PathView& v, int slice, unsigned long long* d_hist, cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(d_hist, 0, kPcfBins * sizeof(unsigned long long), s);
-    if (e != cudaSuccess) return e;
+cudaError_t launch_sep_hist(const PathView& v, int slice, unsigned* d_arrived, unsigned long long* d_hist,
+                            unsigned long long* out, cudaStream_t s) {
     const double dSep = 0.5 * sqrt(3.0) * v.side[2] / (1.0 * kPcfBins);   // action.cpp:192
     const int t0 = slice >= 0 ? slice : 0, nt = slice >= 0 ? 1 : v.M;
     const size_t pos = (size_t)v.Ne * sizeof(float4), column = kPcfBins * sizeof(unsigned);
@@ -119,20 +133,8 @@ cudaError_t launch_sep_hist(const PathView& v, int slice, unsigned long long* d_
     for (int d = 0; d < 3; ++d) { f.side[d] = (float)v.side[d]; f.inv[d] = (float)v.sideInv[d]; }
     f.step = (float)((1 << kSepBits) / dSep);
     f.far = (float)(127.0 * dSep);
-    k_sep_hist<<<nt, threads, smem, s>>>(v, f, t0, dSep, d_hist);
+    k_sep_hist<<<nt, threads, smem, s>>>(v, f, t0, dSep, d_arrived, d_hist, out);
     return cudaGetLastError();
-}
-
-// The last CTA of a grid to arrive; the others' global writes are visible to
-// it.  The counter returns to 0 for the next call.
-__device__ __forceinline__ bool last_to_arrive(unsigned* counter, unsigned blocks) {
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = atomicInc(counter, blocks - 1) == blocks - 1;
-    __syncthreads();
-    if (last) __threadfence();
-    return last;
 }
 
 // Winding and area sums of SuperfluidFractionEstimator::accumulate
@@ -226,7 +228,10 @@ k_cycles(PathView v, int nseg, unsigned* __restrict__ arrived, int* __restrict__
     }
     if (!last_to_arrive(arrived, gridDim.x)) return;
     const int nw = v.nbs[0];
-    if (__ldcg(odd)) {
+    const bool skips = __ldcg(odd) != 0;
+    __syncthreads();
+    if (skips) {
+        if (tid == 0) *odd = 0;                              // zero for the next call
         for (int n = tid; n < nw; n += kEstBlock) {
             const long long limit = (long long)v.M * Ne;
             int2 b = make_int2(0, n);
@@ -263,17 +268,14 @@ k_cycles(PathView v, int nseg, unsigned* __restrict__ arrived, int* __restrict__
 
 static int cycle_segments(const PathView& v) { return (v.M + kSegment - 1) / kSegment; }
 
-size_t cycles_work_ints(const PathView& v, int nw) { return 1 + (size_t)nw + (size_t)cycle_segments(v) * v.Ne; }
+size_t cycles_work_ints(const PathView& v) { return (size_t)cycle_segments(v) * v.Ne; }
 
-// d_work: cycles_work_ints ints, the first nw the lengths
-cudaError_t launch_cycles(const PathView& v, int nw, unsigned* d_arrived, int* d_work, cudaStream_t s) {
+cudaError_t launch_cycles(const PathView& v, int nw, unsigned* d_arrived, int* d_odd, int* d_work, int* len,
+                          cudaStream_t s) {
     if (nw <= 0) return cudaSuccess;
-    int* odd = d_work + nw;
-    cudaError_t e = cudaMemsetAsync(odd, 0, sizeof(int), s);
-    if (e != cudaSuccess) return e;
     const int nseg = cycle_segments(v);
-    k_cycles<<<nseg * ((v.Ne + kEstBlock - 1) / kEstBlock), kEstBlock, nw * sizeof(int), s>>>(v, nseg, d_arrived, odd,
-                                                                                            odd + 1, d_work);
+    k_cycles<<<nseg * ((v.Ne + kEstBlock - 1) / kEstBlock), kEstBlock, nw * sizeof(int), s>>>(v, nseg, d_arrived, d_odd,
+                                                                                            d_work, len);
     return cudaGetLastError();
 }
 

@@ -36,6 +36,36 @@ cudaError_t set_carveout(const void* func, int percent);
 template <class F>
 cudaError_t set_carveout(F* func, int percent) { return set_carveout(reinterpret_cast<const void*>(func), percent); }
 
+// Host memory that kernels read and write directly: a call's small inputs and
+// results go through it without copies of their own (a copy each way takes a
+// launch-to-result round trip from 9.7 to 16.7 us on a GB300, whose C2C link
+// serves such accesses at memory speed).  A block of kStageBytes holds a ring
+// for inputs and room for one call's results.  Blocks are pinned once and kept
+// for the next handle, at most kPinnedKept of them: pinning one takes 100 us.
+constexpr size_t kRingBytes = 256 * 1024, kResultBytes = 256 * 1024, kStageBytes = kRingBytes + kResultBytes;
+constexpr int kPinnedKept = 8;
+void* pinned_acquire();          // a block, or nullptr
+void pinned_release(void* block);
+
+struct Staging {
+    char* block = nullptr;
+    size_t at = 0;
+    char* result() const { return block + kRingBytes; }
+    // Room for `bytes` of input until the stream is waited for; nullptr when it
+    // is too large (copy instead).  Waits for the stream where the ring wraps.
+    char* take(size_t bytes, cudaStream_t s) {
+        bytes = (bytes + 255) & ~(size_t)255;
+        if (!block || bytes > kRingBytes / 2) return nullptr;
+        if (at + bytes > kRingBytes) {
+            if (cudaStreamSynchronize(s) != cudaSuccess) return nullptr;   // the caller's next call reports it
+            at = 0;
+        }
+        char* p = block + at;
+        at += bytes;
+        return p;
+    }
+};
+
 // Read-only view of one path handed to kernels by value.
 struct PathView {
     int M, Ne;
@@ -79,6 +109,8 @@ struct Ctx {
     int worm[8] = {-1,-1,-1,-1,-1,-1,-1,-1};
     int numBeadsOn = 0;
     bool loaded = false;
+    Staging stage;
+    unsigned long long* d_hist = nullptr;   // g(r) counts and the cycles' flag, zero between calls
     // scratch (grown on demand)
     void* d_scratch = nullptr; size_t scratch_bytes = 0;
     void* d_tc_tables = nullptr;   // split-BF16 DFT and cosine matrices of this M (built once)
@@ -110,7 +142,7 @@ struct Ctx {
 
 // Write the listed beads (linear index s*Ne + p) from the host mirrors
 // (h_next, h_prev, h_on; positions from pos_aos [M][Ne][3]) and numBeadsAtSlice
-// to the device; synchronous.
+// to the device, before any later work on the stream.
 int upload_beads(Ctx& c, const int* lin, int k, const double* pos_aos);
 
 #define PGB_CUDA(ctx, call)                                              \
@@ -144,11 +176,11 @@ bool launch_trial_actions64(const PathView& v, const int2* d_beads, int k, int s
 // What a slice's terms are asked for: nothing of its pairs, their potential,
 // with forces (g2, r1, d1), with the T matrix (r2, d2)
 enum { kSliceNone = -1, kSliceV = 0, kSliceF = 1, kSliceT = 2 };
-// d_terms: slice_terms64_work(v) bytes, the first [8][M] the result; d_arrived:
-// M counters, zero between calls; window <= 0: no r1, r2, d1, d2, xch
+// d_terms: the result [8][M]; d_work: slice_terms64_work(v) bytes; d_arrived: M
+// counters, zero between calls; window <= 0: no r1, r2, d1, d2, xch
 size_t slice_terms64_work(const PathView& v);
 cudaError_t launch_slice_terms64(const PathView& v, int window, int even, int odd, unsigned* d_arrived,
-                                 double* d_terms, cudaStream_t s);
+                                 void* d_work, double* d_terms, cudaStream_t s);
 // maxR2 > 0: only beads with x^2 + y^2 < maxR2 (cylinder estimators)
 cudaError_t launch_rhoq64(const PathView& v, const double* d_q, int nq,
                           double* d_rho /* [q][M][2] */, cudaStream_t s, double maxR2 = 0.0);
@@ -178,7 +210,7 @@ cudaError_t launch_slice_forces32(const PathView& v, AzizParams az, float4* d_fo
 // as launch_slice_terms64, with slice_terms32_work(v) bytes
 size_t slice_terms32_work(const PathView& v);
 cudaError_t launch_slice_terms32(const PathView& v, AzizParams az, int window, int even, int odd, unsigned* d_arrived,
-                                 double* d_terms, cudaStream_t s);
+                                 void* d_work, double* d_terms, cudaStream_t s);
 cudaError_t launch_pos32_from64(const PathView& v, float4* d_pos32,
                                 cudaStream_t s);
 // scatter.cu
@@ -196,13 +228,17 @@ cudaError_t launch_ssf_from_rho64(const double* d_rho, int nq, int M,
 cudaError_t launch_isf_direct32(const float2* d_rho, int nq, int M, double norm,
                                 double* d_out, cudaStream_t s);
 // path_estimators.cu (g(r), winding, permutation cycles; FP64, -fmad=false)
-cudaError_t launch_sep_hist(const PathView& v, int slice, unsigned long long* d_hist, cudaStream_t s);
+// d_hist: 50 counts, zero between calls; the result goes to out
+cudaError_t launch_sep_hist(const PathView& v, int slice, unsigned* d_arrived, unsigned long long* d_hist,
+                            unsigned long long* out, cudaStream_t s);
 size_t winding_work_bytes();
 // d_arrived: one counter, zero between calls
 cudaError_t launch_winding(const PathView& v, unsigned* d_arrived, double* d_work, double* d_out5, cudaStream_t s);
-// d_work: cycles_work_ints ints, the first nw the cycle lengths
-size_t cycles_work_ints(const PathView& v, int nw);
-cudaError_t launch_cycles(const PathView& v, int nw, unsigned* d_arrived, int* d_work, cudaStream_t s);
+// d_odd: a flag, zero between calls; d_work: cycles_work_ints ints; len: the nw
+// cycle lengths
+size_t cycles_work_ints(const PathView& v);
+cudaError_t launch_cycles(const PathView& v, int nw, unsigned* d_arrived, int* d_odd, int* d_work, int* len,
+                          cudaStream_t s);
 // slice-0 beads with x^2 + y^2 < maxR2 (one int)
 cudaError_t launch_count_inside(const PathView& v, double maxR2, int* d_out, cudaStream_t s);
 // isf_tc.cu (tcgen05 split-BF16 DFT correlation)
