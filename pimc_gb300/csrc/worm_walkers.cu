@@ -204,6 +204,7 @@ struct WormWalker {
         used |= used >> 1; used |= used >> 2; used |= used >> 4; used |= used >> 8; used |= used >> 16;
         uint32_t i;
         int guard = 0;
+#pragma unroll 1
         do { i = u32() & used; } while (i > n && ++guard < 1000);
         return i > n ? n : i;
     }
@@ -215,6 +216,7 @@ struct WormWalker {
     __device__ __noinline__ float randNormZ() {
         float x, y, r;
         int guard = 0;
+#pragma unroll 1
         do {
             x = 2.0f * rand() - 1.0f;
             y = 2.0f * rand() - 1.0f;
@@ -252,6 +254,7 @@ struct WormWalker {
         };
         int have = 0;
         long long base = 0, used = 0;
+#pragma unroll 1
         for (int round = 0; have < cnt && round < 64; ++round, base += 32) {
             const long long a = base + ln;
             const float x = 2.0f * ((float)word(2 * a) * 2.3283064365386963e-10f) - 1.0f;
@@ -266,6 +269,7 @@ struct WormWalker {
             have += __popc(mask);
         }
         if (have < cnt) {                           // never in practice: 2048 attempts
+#pragma unroll 1
             for (int i = have + ln; i < cnt; i += 32) out[i] = 0.0f;
             used = 2 * base;
         }
@@ -378,7 +382,7 @@ struct WormWalker {
     // The fields a pair sum reads, copied once per call into registers: the
     // walker itself lives in local memory around the helpers that are not
     // inlined, and reading it there per pair would cost a load each time.
-    // The out-of-line pair loops (teamShare, teamBeadShares, energyShare)
+    // The out-of-line pair loops (teamShare, energyShare)
     // take it by value, so it arrives in their registers; by reference it
     // would sit in the caller's local memory and every bead would reload it.
     struct PairCtx {
@@ -435,20 +439,27 @@ struct WormWalker {
         const float r2 = ok ? fmaf(dx, dx, fmaf(dy, dy, dz * dz)) : 1.0f;
         k.add(f * aziz_v32_sel(r2, c.az));
     }
+    // Two partners a lane at a time in one rolled loop, the next two loading
+    // meanwhile: the pair terms appear twice in the code for each Plain.
+    // Written out for 128 partners, with a second loop beyond, a walker of 64
+    // beads a slice or fewer summed as many absent partners as present ones,
+    // and a walker's warps wait for instructions more than for anything else:
+    // with this loop, one copy of it for range and per-bead actions, and the
+    // loops of the moves not unrolled the kernel's code is 285 KB instead of
+    // 363 and 1024 walkers take 52.5 ms for four steps instead of 64.8.
     template <bool Plain>
     __device__ static void pairsOf(const PairCtx& c, const BeadLoad& L, int s1, KahanF& k) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) pairTerm<Plain>(c, L.b, s1, 32 * u + c.lane, L.n, L.rb, L.r[u], k);
         const float4* row = c.pos + (size_t)L.b.t * c.Ne;
-        for (int j0 = 128; j0 < L.n; j0 += 128) {
-            float4 r[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int j = j0 + 32 * u + c.lane;
-                r[u] = j < L.n ? row[j] : L.rb;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) pairTerm<Plain>(c, L.b, s1, j0 + 32 * u + c.lane, L.n, L.rb, r[u], k);
+        float4 r0 = L.r[0], r1 = L.r[1], q0 = L.r[2], q1 = L.r[3];
+#pragma unroll 1
+        for (int j = c.lane;;) {
+            pairTerm<Plain>(c, L.b, s1, j, L.n, L.rb, r0, k);
+            pairTerm<Plain>(c, L.b, s1, j + 32, L.n, L.rb, r1, k);
+            j += 64;
+            if (j - c.lane >= L.n) break;
+            r0 = q0; r1 = q1;
+            q0 = j + 64 < L.n ? row[j + 64] : L.rb;
+            q1 = j + 96 < L.n ? row[j + 96] : L.rb;
         }
     }
     // tau-less pair terms of a loaded bead with its active same-slice
@@ -460,25 +471,32 @@ struct WormWalker {
         else pairsOf<false>(c, L, s1, k);
     }
     // One warp's share of a team's range action: the beads chain[c0 + wk],
-    // chain[c0 + wk + T], ..., each with all its partners as the single-warp
-    // form sums them (the next bead of the share loading meanwhile).  The
-    // four warps walk four beads at a time, so a range costs about a quarter
-    // of the dependent load chain of one warp walking it.  Returns the
-    // warp's (double-float) sum; ok false for a locator outside the walker's
-    // arrays.
+    // chain[c0 + wk + T], ..., each with all its partners (the next bead of
+    // the share loading meanwhile).  The four warps walk four beads at a
+    // time, so a range costs about a quarter of the dependent load chain of
+    // one warp walking it.  Returns the warp's (double-float) sum; ok false
+    // for a locator outside the walker's arrays.  With `part` set each bead
+    // is reduced on its own and lane 0 writes it to part[i] (the per-bead
+    // actions of a worm move).
     __device__ __noinline__ static float2 teamShare(const PairCtx c, const int* ch, int c0, int cnt, int wk, int T,
-                                                    bool& ok) {
+                                                    bool& ok, float2* part) {
         KahanF k;
         if (wk < cnt) {
             BeadLoad cur, nx;
             ok &= loadBead(c, ch[c0 + wk], cur);
+#pragma unroll 1
             for (int i = wk; i < cnt; i += T) {
                 if (i + T < cnt) ok &= loadBead(c, ch[c0 + i + T], nx);
                 if (cur.b.p < cur.n) pairsLoaded(c, cur, k);
+                if (part) {
+                    const float2 r = warp_ff(k);
+                    if (c.lane == 0) part[i] = r;
+                    k = KahanF();
+                }
                 cur = nx;
             }
         }
-        return warp_ff(k);
+        return part ? make_float2(0.f, 0.f) : warp_ff(k);
     }
     // warp 0 of a team: post a job, take its own share, collect the others'
     __device__ void teamPost(int op, int a, int b) {
@@ -493,6 +511,7 @@ struct WormWalker {
         team_sync(bar, 32 * team);
         double s = 0.0;
         int bad = 0;
+#pragma unroll 1
         for (int q = 0; q < team; ++q) { s += (double)job->hi[q] + (double)job->lo[q]; bad |= job->bad[q]; }
         if (bad) err = WERR_LINK;
         return s;
@@ -507,32 +526,15 @@ struct WormWalker {
         if (team > 1 && cnt >= kTeamMinBeads) {
             teamPost(1, c0, cnt);
             bool ok = true;
-            const float2 mine = teamShare(pairCtx(), chain, c0, cnt, 0, team, ok);
+            const float2 mine = teamShare(pairCtx(), chain, c0, cnt, 0, team, ok, nullptr);
             return m.tau * teamCollect(mine, ok);
         }
         // one warp: the team form with a team of one (one copy of the pair
         // loop in the kernel's code)
         bool ok = true;
-        const float2 r = teamShare(pairCtx(), chain, c0, cnt, 0, 1, ok);
+        const float2 r = teamShare(pairCtx(), chain, c0, cnt, 0, 1, ok, nullptr);
         if (!ok) err = WERR_LINK;
         return m.tau * ((double)r.x + (double)r.y);
-    }
-    // One warp's share of a team's per-bead actions: the beads of its
-    // teamShare share, each reduced on its own and written to part[i] by
-    // lane 0
-    __device__ __noinline__ static void teamBeadShares(const PairCtx c, const int* ch, int c0, int cnt, int wk,
-                                                       int T, bool& ok, float2* part) {
-        if (wk >= cnt) return;
-        BeadLoad cur, nx;
-        ok &= loadBead(c, ch[c0 + wk], cur);
-        for (int i = wk; i < cnt; i += T) {
-            if (i + T < cnt) ok &= loadBead(c, ch[c0 + i + T], nx);
-            KahanF k;
-            if (cur.b.p < cur.n) pairsLoaded(c, cur, k);
-            const float2 r = warp_ff(k);
-            if (c.lane == 0) part[i] = r;
-            cur = nx;
-        }
     }
     // The bare potential action of each bead chain[c0 .. c0 + cnt - 1]
     // (barePotentialAction, action.cpp:628-645, primitive) with the walker's
@@ -544,12 +546,14 @@ struct WormWalker {
         if (team > 1 && cnt >= kTeamMinBeads && cnt <= kRunCap) {
             teamPost(3, c0, cnt);
             bool ok = true;
-            teamBeadShares(pairCtx(), chain, c0, cnt, 0, team, ok, tpart);
+            teamShare(pairCtx(), chain, c0, cnt, 0, team, ok, tpart);
             if (lane == 0) job->bad[0] = ok ? 0 : 1;
             team_sync(bar, 32 * team);
             int bad = 0;
+#pragma unroll 1
             for (int q = 0; q < team; ++q) bad |= job->bad[q];
             if (bad) err = WERR_LINK;
+#pragma unroll 1
             for (int i = lane; i < cnt; i += 32) out[i] = m.tau * ((double)tpart[i].x + (double)tpart[i].y);
             __syncwarp();
             return;
@@ -558,9 +562,10 @@ struct WormWalker {
         // float) sum written over its own output slot and widened there
         bool ok = true;
         float2* part = reinterpret_cast<float2*>(out);
-        teamBeadShares(pairCtx(), chain, c0, cnt, 0, 1, ok, part);
+        teamShare(pairCtx(), chain, c0, cnt, 0, 1, ok, part);
         if (!ok) err = WERR_LINK;
         __syncwarp();
+#pragma unroll 1
         for (int i = lane; i < cnt; i += 32) {
             const float2 r = part[i];
             out[i] = m.tau * ((double)r.x + (double)r.y);
@@ -638,6 +643,7 @@ struct WormWalker {
     __device__ __noinline__ bool appendRun(WB from, int cnt, int dir, const float4* q, int c0) {
         if (!valid(from) || cnt < 1 || cnt >= m.M) { err = WERR_LINK; return false; }
         bool full = false;
+#pragma unroll 1
         for (int k = lane; k < cnt; k += 32) {
             int t = from.t + dir * (k + 1);
             t = ((t % m.M) + m.M) % m.M;
@@ -648,6 +654,7 @@ struct WormWalker {
         if (lane == 0) chain[c0] = pack(from);
         if (__any_sync(0xffffffffu, full)) { err = WERR_FULL; return false; }
         __syncwarp();
+#pragma unroll 1
         for (int k = lane; k < cnt; k += 32) {
             const WB b = unpack(chain[c0 + 1 + k]);
             const WB before = unpack(chain[c0 + k]);
@@ -672,6 +679,7 @@ struct WormWalker {
     // no other bead; they drop the slice counts and the run's links, and
     // unlink `from`
     __device__ void dropRun(int cnt, int dir, int c0) {
+#pragma unroll 1
         for (int k = lane; k < cnt; k += 32) {
             const WB b = unpack(chain[c0 + 1 + k]);
             nbs[b.t] = b.p;
@@ -696,6 +704,7 @@ struct WormWalker {
         normals(3 * cnt, znorm);
         const float sg = (float)m.sqrt2LambdaTau;
         float ux = r0.x, uy = r0.y, uz = r0.z;
+#pragma unroll 1
         for (int base = 0; base < cnt; base += 32) {
             const int k = base + lane;
             float dx = 0.f, dy = 0.f, dz = 0.f;
@@ -737,6 +746,7 @@ struct WormWalker {
         const int cap = m.mbar + 1;
         const LinkWalk lw = links();
         bool bad = false;
+#pragma unroll 1
         do {
             ++length;
             b = lw.next(b, bad);
@@ -816,6 +826,7 @@ struct WormWalker {
         const float sg0 = (float)m.sqrt2LambdaTau;
         const float Ex = e.x + Lb * wind.x, Ey = e.y + Lb * wind.y, Ez = e.z + Lb * wind.z;
         float ux = start.x, uy = start.y, uz = start.z;
+#pragma unroll 1
         for (int base = 0; base < cnt; base += 32) {
             const int k = base + lane;
             float A = 1.0f, bx = 0.0f, by = 0.0f, bz = 0.0f;
@@ -852,16 +863,19 @@ struct WormWalker {
     // towards e (through qbuf), written lane-parallel
     __device__ void stageChain(int cnt, float4 start, float4 e, int L, int3& wind) {
         stagePositions(cnt, start, e, L, wind, qbuf);
+#pragma unroll 1
         for (int i = lane; i < cnt; i += 32) pos[at(chain[i + 1])] = qbuf[i];
         __syncwarp();
     }
     // save / restore chain[1 .. cnt] positions, lane-parallel
     __device__ void saveChain(int cnt, float4* orig) {
+#pragma unroll 1
         for (int i = lane; i < cnt; i += 32) orig[i] = pos[at(chain[i + 1])];
         __syncwarp();
     }
     __device__ void restoreChain(int cnt, const float4* orig) {
         __syncwarp();
+#pragma unroll 1
         for (int i = lane; i < cnt; i += 32) pos[at(chain[i + 1])] = orig[i];
         __syncwarp();
     }
@@ -893,6 +907,7 @@ struct WormWalker {
         bool closed = false;
         const LinkWalk lw = links();
         bool bad = false;
+#pragma unroll 1
         for (;;) {
             const WB pb = lw.prev(b, bad);
             if (bad) { err = WERR_LINK; return 0; }
@@ -909,6 +924,7 @@ struct WormWalker {
             wl = back + 1;
             if (lane == 0) chain[c0] = pack(first);
         } else {
+#pragma unroll 1
             for (WB s = b;;) {
                 if (wl >= m.M) return 0;
                 if (lane == 0) chain[wl] = pack(s);
@@ -931,6 +947,7 @@ struct WormWalker {
         return wl;
     }
     __device__ void shiftChain(int c0, int cnt, float sx, float sy, float sz) {
+#pragma unroll 1
         for (int i = lane; i < cnt; i += 32) {
             const size_t q = at(chain[c0 + i]);
             const float4 r = pos[q];
@@ -952,6 +969,7 @@ struct WormWalker {
         const LinkWalk lw = links();
         const int* cnts = nbs;
         bool bad = false;
+#pragma unroll 1
         for (int k = 0; k < L; ++k) {
             if (b.p >= cnts[b.t]) return 0;
             const WB nb_ = lw.next(b, bad);
@@ -989,6 +1007,7 @@ struct WormWalker {
     // exp(-dA + dA_previous level) and a rejection restores every bead moved
     // so far.  Returns the beads proposed, as the oracle counts them.
     __device__ void gatherStride(int first, int stride, int cnt) {
+#pragma unroll 1
         for (int i = lane; i < cnt; i += 32) chain[kListOff + i] = chain[first + stride * i];
         __syncwarp();
     }
@@ -1007,6 +1026,7 @@ struct WormWalker {
         const LinkWalk lw = links();
         const int* cnts = nbs;
         bool bad = false;
+#pragma unroll 1
         for (int k = 0; k <= numActive; ++k) {
             if (b.p >= cnts[b.t]) return 0;
             const WB nx = lw.next(b, bad);
@@ -1027,6 +1047,7 @@ struct WormWalker {
         int zoff = 0;
         double oldDelta = 0.0;
         int moved = 0;
+#pragma unroll 1
         for (int level = numLevels; level > 0; --level) {
             const int s = 1 << (level - 1);
             const int cnt = 1 << (numLevels - level);  // offsets s (2i + 1), i < cnt
@@ -1035,6 +1056,7 @@ struct WormWalker {
             const float sg = sgBase * sqrtf((float)s);
             const float* z = znorm + 3 * zoff;
             zoff += cnt;
+#pragma unroll 1
             for (int i = lane; i < cnt; i += 32) {
                 const int j = s * (2 * i + 1);
                 const float4 pp = pos[at(chain[j - s])], pn = pos[at(chain[j + s])];
@@ -1056,9 +1078,11 @@ struct WormWalker {
                 const int pc = (numActive - 1) / 2;
                 gatherStride(2, 2, pc);
                 newA += chainAction(kListOff, pc);
+#pragma unroll 1
                 for (int i = lane; i < pc; i += 32) pos[at(chain[2 * (i + 1)])] = orig[2 * i + 1];
                 __syncwarp();
                 oldA += chainAction(kListOff, pc);
+#pragma unroll 1
                 for (int i = lane; i < pc; i += 32) pos[at(chain[2 * (i + 1)])] = newp[2 * i + 1];
                 __syncwarp();
             }
@@ -1068,6 +1092,7 @@ struct WormWalker {
             } else {
                 // undoMove (move.cpp:1694-1707): every bead moved so far, the
                 // offsets that are multiples of s
+#pragma unroll 1
                 for (int j = lane + 1; j <= numActive; j += 32)
                     if (j % s == 0) pos[at(chain[j])] = orig[j - 1];
                 __syncwarp();
@@ -1100,6 +1125,7 @@ struct WormWalker {
         const LinkWalk lw = links();
         const int cap = m.mbar + 1;
         bool bad = false;
+#pragma unroll 1
         for (int g = 0; g <= cap; ++g) {
             if (isXW(x)) { err = WERR_LINK; break; }
             if (lane == 0) chain[cnt] = pack(x);
@@ -1128,6 +1154,7 @@ struct WormWalker {
     // accepted
     __device__ bool removalTests(int cnt, double actionShift, double corr) {
         int ev = 0, chunk = firstChunk();
+#pragma unroll 1
         for (int k = 0; k < cnt; ++k) {
             actsUpTo(k, cnt, ev, chunk);
             acc->bead_updates++;
@@ -1145,6 +1172,7 @@ struct WormWalker {
     __device__ bool insertionTests(int cnt, double actionShift, double corr, WB* endRef, WB end) {
         int ev = 0, chunk = firstChunk();
         const int total = endRef ? cnt : cnt + 1;
+#pragma unroll 1
         for (int k = 0; k <= cnt; ++k) {
             double u;
             if (k == cnt && endRef) {
@@ -1191,6 +1219,7 @@ struct WormWalker {
         if (removalTests(cnt, actionShift, corrRange(hb, tb))) {
             acc->accepted[WM_OPEN]++;
             WB b = next(hb);
+#pragma unroll 1
             for (int g = 0; g <= m.M && !eqW(b, tb) && !isXW(b); ++g) b = delBeadGetNext(b);
             wormUpdate(hb, tb);
             diag = 0;
@@ -1284,6 +1313,7 @@ struct WormWalker {
         if (removalTests(cnt, actionShift, corrRange(tail, head))) {
             acc->accepted[WM_REMOVE]++;
             WB b = head;
+#pragma unroll 1
             for (int g = 0; g <= m.M * m.Ne && !isXW(b); ++g) b = delBeadGetPrev(b);
             wormReset(); diag = 1;
             return 1;
@@ -1336,6 +1366,7 @@ struct WormWalker {
         if (removalTests(cnt, actionShift, corrRange(tail, tb))) {
             acc->accepted[WM_AT]++;
             WB b = prev(tb);
+#pragma unroll 1
             for (int g = 0; g <= m.M * m.Ne && !isXW(b); ++g) b = delBeadGetPrev(b);
             wormUpdate(head, tb);
             diag = 0;
@@ -1362,6 +1393,7 @@ struct WormWalker {
         if (removalTests(cnt, actionShift, corrRange(sp1, head))) {
             acc->accepted[WM_RH]++;
             WB b = next(hb);
+#pragma unroll 1
             for (int g = 0; g <= m.M * m.Ne && !isXW(b); ++g) b = delBeadGetNext(b);
             wormUpdate(hb, tail);
             diag = 0;
@@ -1426,10 +1458,11 @@ struct WormWalker {
         float acc[32];
 #pragma unroll
         for (int w = 0; w < 32; ++w) acc[w] = 0.0f;
-        for (int n0 = 0; n0 < nL; n0 += 128) {
-            float4 pf[4];
+#pragma unroll 1
+        for (int n0 = 0; n0 < nL; n0 += 64) {
+            float4 pf[2];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < 2; ++u) {
                 const int n = n0 + 32 * u + ln;
                 pf[u] = n < nL ? row[n] : pb;
             }
@@ -1437,7 +1470,7 @@ struct WormWalker {
             // 0, +1, -1 of the winding vector) give the 27 sector weights as
             // products, 9 exponentials a bead instead of 27
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < 2; ++u) {
                 const bool ok = n0 + 32 * u + ln < nL;
                 const float dx = pf[u].x - pb.x, dy = pf[u].y - pb.y, dz = pf[u].z - pb.z;
                 float ex[3], ey[3], ez[3];
@@ -1483,6 +1516,7 @@ struct WormWalker {
             const int3 wv = winding(ws);
             float carry = before;
             int found = nL - 1;
+#pragma unroll 1
             for (int base = 0; base < nL; base += 32) {
                 const int n = base + ln;
                 float v = n < nL ? rho0Shifted(row[n], pb, wv, sign, g3, nden, L) : 0.0f;
@@ -1512,6 +1546,7 @@ struct WormWalker {
         WB b = pivot;
         const LinkWalk lw = links();
         bool bad = false;
+#pragma unroll 1
         for (int k = 0; k < swapLength; k++) {
             if (eqW(b, tail) || isXW(b)) { if (bad) err = WERR_LINK; return -1; }
             if (lane == 0) chain[swapLength - k] = pack(b);
@@ -1566,6 +1601,7 @@ struct WormWalker {
         WB b = pivot;
         const LinkWalk lw = links();
         bool bad = false;
+#pragma unroll 1
         for (int k = 0; k < swapLength; k++) {
             if (eqW(b, head) || isXW(b)) { if (bad) err = WERR_LINK; return -1; }
             if (lane == 0) chain[k] = pack(b);
@@ -1626,6 +1662,7 @@ struct WormWalker {
             if (lane == 0) { job->hi[0] = p.x; job->lo[0] = p.y; job->khi[0] = k.x; job->klo[0] = k.y; }
             team_sync(bar, 32 * team);
             double pot = 0.0, kin = 0.0;
+#pragma unroll 1
             for (int q = 0; q < team; ++q) {
                 pot += (double)job->hi[q] + (double)job->lo[q];
                 kin += (double)job->khi[q] + (double)job->klo[q];
@@ -1641,10 +1678,12 @@ struct WormWalker {
     __device__ __noinline__ static void energyShare(const PairCtx c, const int* nx_, int t0, int t1, int step,
                                                     float2& pot_out, float2& kin_out) {
         KahanF pot, kin;
+#pragma unroll 1
         for (int t = t0; t < t1; t += step) {
             const int n = c.nbs[t];
             const int tn = t + 1 == c.M ? 0 : t + 1;
             const float4* row = c.pos + (size_t)t * c.Ne;
+#pragma unroll 1
             for (int i = c.lane; i < n; i += 32) {
                 const int pn = nx_[(size_t)i * c.M + t];
                 if (pn >= 0 && pn < c.Ne) {
@@ -1655,17 +1694,19 @@ struct WormWalker {
                     kin.add(fmaf(vx, vx, fmaf(vy, vy, vz * vz)));
                 }
             }
+#pragma unroll 1
             for (int i = 0; i + 1 < n; ++i) {
                 const float4 ri = row[i];
-                for (int j0 = i + 1; j0 < n; j0 += 128) {
-                    float4 r[4];
+#pragma unroll 1
+                for (int j0 = i + 1; j0 < n; j0 += 64) {
+                    float4 r[2];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
+                    for (int u = 0; u < 2; ++u) {
                         const int j = j0 + 32 * u + c.lane;
                         r[u] = j < n ? row[j] : ri;
                     }
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
+                    for (int u = 0; u < 2; ++u) {
                         const bool ok = j0 + 32 * u + c.lane < n;
                         const float dx = min_image32(ri.x - r[u].x, c.L, c.Linv);
                         const float dy = min_image32(ri.y - r[u].y, c.L, c.Linv);
@@ -1745,12 +1786,14 @@ __device__ __noinline__ void run_walker(int w, int team, int bar, TeamJob* job, 
     double* cumD = s_cum;
     double* cumO = s_cum + WM_N;
     if (ww.lane == 0 && diag_only) {
+#pragma unroll 1
         for (int i = 0; i < WM_N; ++i) cumD[i] = cumO[i] = 1.0 + 1e-7;
         cumD[WM_COM] = cumO[WM_COM] = 0.05;
     } else if (ww.lane == 0) {
         const double prob[WM_N] = {0.01, 0.19, 0.4, 0.15, 0.4, 0.15, 0.075, 0.075, 0.075, 0.075, 0.1, 0.1};
         const int onDiag[WM_N] = {1, 1, 1, 0, 1, 0, 0, 0, 0, 0, 0, 0};
         double cd = 0.0, co = 0.0;
+#pragma unroll 1
         for (int i = 0; i < WM_N; ++i) {
             if (onDiag[i]) cd += prob[i];
             cumD[i] = cd;
@@ -1801,6 +1844,7 @@ __device__ __noinline__ void run_walker(int w, int team, int bar, TeamJob* job, 
                 const double x = ww.rand();
                 const double* cum = ww.diag ? cumD : cumO;
                 int index = WM_N - 1;
+#pragma unroll 1
                 for (int i = 0; i < WM_N; ++i) if (cum[i] >= x) { index = i; break; }
                 bool acc = false;
                 int moved = 0;
@@ -1893,11 +1937,11 @@ __device__ __noinline__ void team_helper(int w, int wk, int T, int bar, const WW
         const WormWalker::PairCtx c = ww.pairCtx();
         if (op == 1) {
             bool ok = true;
-            const float2 r = WormWalker::teamShare(c, chain, job->a, job->b, wk, T, ok);
+            const float2 r = WormWalker::teamShare(c, chain, job->a, job->b, wk, T, ok, nullptr);
             if (ww.lane == 0) { job->hi[wk] = r.x; job->lo[wk] = r.y; job->bad[wk] = ok ? 0 : 1; }
         } else if (op == 3) {
             bool ok = true;
-            WormWalker::teamBeadShares(c, chain, job->a, job->b, wk, T, ok, tpart);
+            WormWalker::teamShare(c, chain, job->a, job->b, wk, T, ok, tpart);
             if (ww.lane == 0) job->bad[wk] = ok ? 0 : 1;
         } else {
             float2 p, k;
