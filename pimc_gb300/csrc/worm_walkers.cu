@@ -14,31 +14,38 @@
 // action in FP32 pair sums reduced in double-float, so they agree with it
 // statistically.
 //
-// Execution model: a small walker is one warp; a walker of N0 >= 32 is a
-// team of two or four warps (kTeamMinN, kTeam4MinN).  The move logic runs
-// redundantly and uniformly in all 32 lanes of the walker's first warp
-// (every lane draws the same random numbers and makes the same decisions);
-// scalar state (worm locators, gap, length, counters) lives in registers,
-// identical in every lane; array writes (positions, links, numBeadsAtSlice)
-// are made by lane 0, or lane-parallel for independent beads, and published
-// with __syncwarp; a team's other warps take their share of every range
-// action, per-bead action and energy sample.  Links store the partner
-// particle only: next(t, p) is on slice t + 1 and prev on t - 1.
+// Execution model: a walker is a team of two, four or eight warps
+// (kTeamMinN, kTeam4MinN).  The move logic runs redundantly and uniformly in
+// all 32 lanes of the team's first warp (every lane draws the same random
+// numbers and makes the same decisions); scalar state (worm locators, gap,
+// length, counters) is identical in every lane; array writes (positions,
+// links, numBeadsAtSlice) are made by lane 0, or lane-parallel for
+// independent beads, and published with __syncwarp; the other warps take
+// their share of every range action, per-bead action and energy sample.
+// Links store the partner particle only: next(t, p) is on slice t + 1 and
+// prev on t - 1.
 //
 // Latency, not throughput, bounds a walker: a move is a chain of dependent
-// link loads, pair sums and warp reductions.  So (1) a move walks its range
-// once and caches the beads in shared memory (chain[]), and the actions,
-// saves, restores and centre-of-mass shifts index that cache; (2) the pair
-// terms of a lane have no branches (absent partners add zero), so its four
-// partner terms schedule together, and a team splits a range by beads, so
-// several beads' load chains are in flight; (3) position chains (staging
-// bridges, free-particle walks) are scans over the lanes, and a worm move's
-// run of new beads is placed at once and evaluated in doubling chunks; (4)
-// the heavy helpers are not inlined: one copy of each serves all twelve
-// moves, which keeps the kernel's code small for the instruction caches;
-// (5) the largest walkers are launched first; (6) a move's normal deviates
-// come from the lanes together (normals()), from the same words as serial
-// draws.
+// link loads, pair sums and warp reductions, run by few warps.  So (1) a
+// move collects its range once in shared memory (chain[]), a stretch of up to
+// 32 beads that keep their particle index at a time (segment()), and the
+// actions, saves, restores and shifts index that cache; (2) the pair terms
+// of a lane have no branches (absent partners add zero), two a lane are in
+// flight, and a team splits a range by beads; (3) position chains (staging
+// bridges, free-particle walks) are scans over the lanes; a worm move's run
+// of new beads is placed at once, evaluated in doubling chunks, tested
+// (testsOf()) and taken out again (dropBeads()) by the lanes together; (4)
+// the heavy helpers are not inlined and loops are not unrolled: a walker's
+// warps wait for instructions more than for anything else; (5) the largest
+// walkers are launched first; (6) a move's normal deviates come from the
+// lanes together (normals()), from the same words as serial draws; (7) FP64
+// instructions are few: each holds a quarter of an SM for 64 clocks, so
+// constants are rounded once on the host and sums widened by lanes.
+// Walking, testing and removing bead by bead with the FP64 logarithms and
+// quotients in the moves 1024 walkers took 52.5 ms for four steps, the
+// largest of them alone 44.0; so, 40.1 and 32.3; with eight warps a CTA
+// instead of four and shares added by lanes, 37.2 and 29.3 (a walker of 24
+// beads a slice 12.6 -> 10.2).
 //
 // Differences from the reference, all documented where they occur:
 //  * the swap pivot is drawn from the pivot slice's beads in index order
@@ -72,7 +79,20 @@ struct WWMeta {
     float L, Linv;
     double tau, lambda, mu, C, volume, tailV0, sqrt2LambdaTau, sqrtLambdaTau, comDelta;
     uint2 key;
+    // what the moves need of the above, rounded as they would round it: an
+    // FP64 product costs the walker's chain 64 clocks, a quotient about 700
+    float sg2, sg1, comStep, swapDen;   // sqrt2LambdaTau, sqrtLambdaTau, comDelta, 4 lambda Mbar tau
+    double lambda4, costScale;          // 4 lambda, 0.25 / (lambda tau)
 };
+
+static void meta_constants(WWMeta& m) {
+    m.sg2 = (float)m.sqrt2LambdaTau;
+    m.sg1 = (float)m.sqrtLambdaTau;
+    m.comStep = (float)m.comDelta;
+    m.swapDen = (float)(4.0 * m.lambda * m.mbar * m.tau);
+    m.lambda4 = 4.0 * m.lambda;
+    m.costScale = 0.25 / (m.lambda * m.tau);
+}
 
 struct WWState {
     int head[2], tail[2], sp1[2], sp2[2];
@@ -98,22 +118,23 @@ enum { WM_COM = 0, WM_DIAG, WM_OPEN, WM_CLOSE, WM_INSERT, WM_REMOVE, WM_AH, WM_R
        WM_SH, WM_ST, WM_N };
 enum { WERR_FULL = 1, WERR_LINK = 2, WERR_LOOP = 3 };
 
-// A CTA holds kCtaWarps warps: kCtaWarps small walkers of one warp each, two
-// walkers of kTeamMinN <= N0 < kTeam4MinN served by teams of two warps, or
-// one walker of N0 >= kTeam4MinN served by a team of all four.  In a team,
-// its first warp runs the move logic as a single-warp walker does, and every
-// pair sum (a move's range or bead action) and every energy sample is split
-// over the team's warps: the first warp posts the job in shared memory, the
-// team meets at its own named barrier, each warp sums its share of the beads
-// (or slices), and after a second barrier the first warp adds the shares in
-// warp order.  A large walker's chain of dependent moves stays on one warp;
-// its pair work, most of its instructions, runs on the team.
-constexpr int kCtaWarps = 4;
+// A CTA holds kCtaWarps warps, shared by one walker of N0 >= kTeam4MinN, two
+// of kTeamMinN <= N0 < kTeam4MinN or four smaller ones, each served by a team
+// of as many warps as that leaves.  A team's first warp runs the move logic,
+// and every pair sum (a move's range or bead action) and every energy sample
+// is split over the team's warps: the first warp posts the job in shared
+// memory, the team meets at its own named barrier, each warp sums its share
+// of the beads (or slices), and after a second barrier the first warp adds
+// the shares.  A walker's chain of dependent moves stays on one warp; its
+// pair work, most of its instructions, runs on the team.  Two CTAs share an
+// SM (64 KB of shared memory, the rest is L1: the paths stream through it).
+constexpr int kCtaWarps = 8;
+constexpr int kCtaWalkers = 4;       // at most, with as many sets of move buffers
 constexpr int kTeamMinN = 32;
-constexpr int kTeam4MinN = 64;
+constexpr int kTeam4MinN = 64;      // a CTA of its own from here
 constexpr int kTeamMinBeads = 4;     // shorter range actions of a team walker stay on its warp 0
 constexpr int kRunCap = 128;         // per-bead shares a team warp keeps (a worm move's run <= Mbar + 1)
-constexpr int kOrigCap = 72;         // saved positions per move (Mbar - 1 <= 63)
+constexpr int kOrigCap = 66;         // a move's beads (Mbar + 1 <= 65)
 constexpr int kMaxWind = 27;         // (2 maxWind + 1)^3 with maxWind = 1
 constexpr int kChainCap = 1024;      // beads of one move's range cached per walker (M < 1024)
 // A bisection's per-level bead lists are gathered into chain[kListOff ..]: the
@@ -129,11 +150,13 @@ struct TeamJob {
     float khi[kCtaWarps], klo[kCtaWarps];    // each warp's kinetic share (energy)
     int bad[kCtaWarps];                      // a warp met a locator outside the arrays
 };
-// named barrier `id` (1 + the team's place in its CTA: 1 or 2) over the
-// team's threads; constant ids, so the kernel reserves three barriers
+// named barrier `id` (1 + the team's place in its CTA) over the team's
+// threads; constant ids, so the kernel reserves five barriers
 __device__ __forceinline__ void team_sync(int id, int nthreads) {
     if (id == 1) asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
-    else asm volatile("bar.sync 2, %0;" ::"r"(nthreads) : "memory");
+    else if (id == 2) asm volatile("bar.sync 2, %0;" ::"r"(nthreads) : "memory");
+    else if (id == 3) asm volatile("bar.sync 3, %0;" ::"r"(nthreads) : "memory");
+    else asm volatile("bar.sync 4, %0;" ::"r"(nthreads) : "memory");
 }
 
 // Aziz V with the reference's hard-core branch (potential.cpp:1821-1843):
@@ -176,6 +199,7 @@ struct WormWalker {
     float2* tpart = nullptr;         // shared: a team's per-bead sums, kRunCap at most
     float4* qbuf = nullptr;          // shared: a move's new bead positions, kOrigCap at most
     double* acts = nullptr;          // shared: a move's per-bead actions (aliases znorm)
+    double* stepShift = nullptr;     // shared: tau mu l / l of the steps l = 2, 4, .. Mbar, as the moves round it
     // uniform scalar state
     WB head, tail, sp1, sp2;
     int gap, length, diag, numBeadsOn;
@@ -189,8 +213,11 @@ struct WormWalker {
 
     // ---- random numbers (MTRand's conversions on Philox words) ----
     // the next draw block (one copy of the Philox rounds for every call site)
-    __device__ __noinline__ void refill() {
-        buf = philox4x32(make_uint4((uint32_t)ctr, (uint32_t)(ctr >> 32), 0x574F524Du, 0u), m.key);
+    __device__ __noinline__ uint4 block(unsigned long long c) const {
+        return philox4x32(make_uint4((uint32_t)c, (uint32_t)(c >> 32), 0x574F524Du, 0u), m.key);
+    }
+    __device__ void refill() {
+        buf = block(ctr);
         ++ctr;
         bidx = 0;
     }
@@ -228,60 +255,65 @@ struct WormWalker {
     }
     __device__ float randNorm(float mean, float sd) { return mean + randNormZ() * sd; }
     // the next cnt deviates that cnt calls of randNormZ() would return, made
-    // by the lanes together from the same words: lane l tests attempt
-    // a = base + l on words 2a and 2a + 1, the accepted attempts in order
-    // give the deviates, and the stream then moves past the last attempt
-    // used, exactly where the serial draws would leave it
-    // (the stream position is read into registers once: the walker's own
-    // copy lives in local memory)
+    // by the lanes together from the same words: a lane makes one block of the
+    // stream a round and tests the two attempts that end in it (with an odd
+    // number of words left in the current block each block's first attempt
+    // begins with the last word of the one before); the accepted attempts in
+    // order give the deviates, and the stream then stands after the last
+    // attempt used, exactly where the serial draws would leave it.  One
+    // block serves two attempts: 93 deviates take two rounds of one block a
+    // lane, where an attempt a lane took four rounds of two.
     __device__ __noinline__ void normals(int cnt, float* out) {
-        const int rem = 4 - bidx;
-        const int bi = bidx;
-        const uint4 bf = buf;
+        const int rem = 4 - bidx, odd = rem & 1;
         const unsigned long long c0 = ctr;
-        const uint2 key = m.key;
         const int ln = lane;
-        auto word = [&](long long i) -> uint32_t {
-            if (i < rem) {
-                const int q = bi + (int)i;
-                return q == 0 ? bf.x : q == 1 ? bf.y : q == 2 ? bf.z : bf.w;
-            }
-            const long long j = i - rem;
-            const unsigned long long c = c0 + (unsigned long long)(j >> 2);
-            const uint4 w = philox4x32(make_uint4((uint32_t)c, (uint32_t)(c >> 32), 0x574F524Du, 0u), key);
-            const int q = (int)(j & 3);
-            return q == 0 ? w.x : q == 1 ? w.y : q == 2 ? w.z : w.w;
-        };
+        const unsigned below = (1u << ln) - 1u;
+        uint4 w = buf;
+        uint32_t carry = 0;                         // the last word of the round before's last block
         int have = 0;
-        long long base = 0, used = 0;
 #pragma unroll 1
-        for (int round = 0; have < cnt && round < 64; ++round, base += 32) {
-            const long long a = base + ln;
-            const float x = 2.0f * ((float)word(2 * a) * 2.3283064365386963e-10f) - 1.0f;
-            const float y = 2.0f * ((float)word(2 * a + 1) * 2.3283064365386963e-10f) - 1.0f;
-            const float r = __fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y));
-            const bool ok = !(r >= 1.0f || r == 0.0f);
-            const unsigned mask = __ballot_sync(0xffffffffu, ok);
-            const int rank = __popc(mask & ((1u << ln) - 1u));
-            if (ok && have + rank < cnt) out[have + rank] = x * sqrtf(-2.0f * logf(r) / r);
-            const unsigned last = __ballot_sync(0xffffffffu, ok && rank == cnt - have - 1);
-            if (last) used = 2 * (base + __ffs(last));
-            have += __popc(mask);
+        for (int round = 0; have < cnt && round < 33; ++round) {
+            // lane 0 of the first round has the current block
+            const int blk = 32 * round + ln - 1;
+            if (blk >= 0) w = block(c0 + (unsigned)blk);
+            uint32_t before = __shfl_up_sync(0xffffffffu, w.w, 1);
+            if (ln == 0) before = carry;
+            carry = __shfl_sync(0xffffffffu, w.w, 31);
+            const uint32_t wa[2] = {odd ? before : w.x, odd ? w.y : w.z};
+            const uint32_t wb[2] = {odd ? w.x : w.y, odd ? w.z : w.w};
+            float x[2], r[2];
+            bool ok[2];
+            unsigned mask[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                x[u] = 2.0f * ((float)wa[u] * 2.3283064365386963e-10f) - 1.0f;
+                const float y = 2.0f * ((float)wb[u] * 2.3283064365386963e-10f) - 1.0f;
+                r[u] = __fadd_rn(__fmul_rn(x[u], x[u]), __fmul_rn(y, y));
+                // of the current block only the words still unused
+                const bool there = blk >= 0 || (u == 0 ? rem == 4 : rem >= 2);
+                ok[u] = there && !(r[u] >= 1.0f || r[u] == 0.0f);
+                mask[u] = __ballot_sync(0xffffffffu, ok[u]);
+            }
+            int rank = have + __popc(mask[0] & below) + __popc(mask[1] & below);
+            unsigned last[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (ok[u] && rank < cnt) out[rank] = x[u] * sqrtf(-2.0f * logf(r[u]) / r[u]);
+                last[u] = __ballot_sync(0xffffffffu, ok[u] && rank == cnt - 1);
+                rank += ok[u];
+            }
+            have += __popc(mask[0]) + __popc(mask[1]);
+            const unsigned any = last[0] | last[1];
+            const int src = any ? __ffs(any) - 1 : 31;
+            if (any || round == 32) {
+                buf = make_uint4(__shfl_sync(0xffffffffu, w.x, src), __shfl_sync(0xffffffffu, w.y, src),
+                                 __shfl_sync(0xffffffffu, w.z, src), __shfl_sync(0xffffffffu, w.w, src));
+                ctr = c0 + (unsigned)(32 * round + src);
+                bidx = !any ? 4 : (last[0] ? 2 : 4) - odd;
+            }
         }
-        if (have < cnt) {                           // never in practice: 2048 attempts
-#pragma unroll 1
+        if (have < cnt)                             // never in practice: 2048 attempts
             for (int i = have + ln; i < cnt; i += 32) out[i] = 0.0f;
-            used = 2 * base;
-        }
-        if (used <= rem) {
-            bidx += (int)used;
-        } else {
-            const long long wb = used - rem, nb = (wb + 3) >> 2;
-            const unsigned long long c = c0 + (unsigned long long)(nb - 1);
-            buf = philox4x32(make_uint4((uint32_t)c, (uint32_t)(c >> 32), 0x574F524Du, 0u), key);
-            ctr = c + 1;
-            bidx = (int)(wb - 4 * (nb - 1));
-        }
         __syncwarp();
     }
 
@@ -308,33 +340,34 @@ struct WormWalker {
         if (p >= m.Ne) { err = WERR_LINK; return {-1, -1}; }
         return {b.t == 0 ? m.M - 1 : b.t - 1, p};
     }
-    // The link arrays and extents in registers for the walks along worldlines
-    // (next/prev with the same checks, a bad locator or link reported in
-    // `bad`): a walk reads one link a step and stores each bead to the move
-    // cache, after which the walker's own copy of these fields would be read
-    // again from local memory.
-    struct LinkWalk {
-        const int* nx;
-        const int* pv;
-        int M, Ne;
-        __device__ WB next(WB b, bool& bad) const {
-            if (b.t < 0 || b.t >= M || b.p < 0 || b.p >= Ne) { bad = true; return {-1, -1}; }
-            const int p = nx[(size_t)b.p * M + b.t];
-            if (p < 0) return {-1, -1};
-            if (p >= Ne) { bad = true; return {-1, -1}; }
-            return {b.t + 1 == M ? 0 : b.t + 1, p};
-        }
-        __device__ WB prev(WB b, bool& bad) const {
-            if (b.t < 0 || b.t >= M || b.p < 0 || b.p >= Ne) { bad = true; return {-1, -1}; }
-            const int p = pv[(size_t)b.p * M + b.t];
-            if (p < 0) return {-1, -1};
-            if (p >= Ne) { bad = true; return {-1, -1}; }
-            return {b.t == 0 ? M - 1 : b.t - 1, p};
-        }
-    };
-    __device__ LinkWalk links() const { return LinkWalk{nxt, prv, m.M, m.Ne}; }
-    __device__ WB nextN(WB b, int n) { for (int i = 0; i < n && !isXW(b); ++i) b = next(b); return b; }
-    __device__ WB prevN(WB b, int n) { for (int i = 0; i < n && !isXW(b); ++i) b = prev(b); return b; }
+    // The beads from x along the links of direction dir, as far as they keep
+    // x's particle index, at most `want` of them: lane i has the i-th, (t, p).
+    // A worldline keeps its index over almost every link (99 % of them on the
+    // 1024-walker workload), and links are particle-major, so a segment is
+    // one load a lane where a walk bead by bead is a chain of loads.  Returns
+    // their number c (at most 32 and M) and, in `on`, the bead after them;
+    // a bad locator or link ends the walk with `bad` set.
+    struct Segment { int c; WB mine, on; bool bad; };
+    __device__ __noinline__ Segment segment(WB x, int dir, int want) const {
+        const int M = m.M, Ne = m.Ne;
+        Segment s{0, x, WB{-1, -1}, false};
+        if (x.t < 0 || x.t >= M || x.p < 0 || x.p >= Ne) { s.bad = true; return s; }
+        const int lim = min(min(want, 32), M);
+        int t = x.t + dir * lane;
+        if (t >= M) t -= M;
+        else if (t < 0) t += M;
+        const int v = lane < lim ? (dir > 0 ? nxt : prv)[(size_t)x.p * M + t] : -1;
+        const int turn = __ffs(__ballot_sync(0xffffffffu, v != x.p)) - 1;    // the first link to another index
+        s.c = turn >= 0 && turn < lim ? turn + 1 : lim;
+        s.mine.t = t;
+        const int p = __shfl_sync(0xffffffffu, v, s.c - 1);
+        int tn = x.t + dir * s.c;
+        if (tn >= M) tn -= M;
+        else if (tn < 0) tn += M;
+        if (p >= Ne) s.bad = true;
+        else if (p >= 0) s.on = WB{tn, p};
+        return s;
+    }
     // every access checks its bead: a bad locator sets the error word and
     // touches no memory
     __device__ float4 P(WB b) {
@@ -509,12 +542,19 @@ struct WormWalker {
     __device__ double teamCollect(float2 mine, bool ok) {
         if (lane == 0) { job->hi[0] = mine.x; job->lo[0] = mine.y; job->bad[0] = ok ? 0 : 1; }
         team_sync(bar, 32 * team);
-        double s = 0.0;
-        int bad = 0;
-#pragma unroll 1
-        for (int q = 0; q < team; ++q) { s += (double)job->hi[q] + (double)job->lo[q]; bad |= job->bad[q]; }
-        if (bad) err = WERR_LINK;
-        return s;
+        const bool in = lane < team;
+        if (__any_sync(0xffffffffu, in && job->bad[lane])) err = WERR_LINK;
+        return sumShares(in ? job->hi[lane] : 0.f, in ? job->lo[lane] : 0.f);
+    }
+    // the sum of the first kCtaWarps lanes' (double-float) shares in every
+    // lane.  An FP64 instruction occupies a quarter of an SM for 64 clocks
+    // whatever its lanes do, so the shares are widened and added by lanes:
+    // six instructions, where adding eight shares one after another took 32.
+    __device__ static double sumShares(float hi, float lo) {
+        double s = (double)hi + (double)lo;
+#pragma unroll
+        for (int o = 1; o < kCtaWarps; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        return __shfl_sync(0xffffffffu, s, 0);
     }
     // potentialAction over chain[c0 .. c0 + cnt - 1]: the lanes keep one
     // running sum over the whole range and reduce once (a team: each warp
@@ -549,10 +589,7 @@ struct WormWalker {
             teamShare(pairCtx(), chain, c0, cnt, 0, team, ok, tpart);
             if (lane == 0) job->bad[0] = ok ? 0 : 1;
             team_sync(bar, 32 * team);
-            int bad = 0;
-#pragma unroll 1
-            for (int q = 0; q < team; ++q) bad |= job->bad[q];
-            if (bad) err = WERR_LINK;
+            if (__any_sync(0xffffffffu, lane < team && job->bad[lane])) err = WERR_LINK;
 #pragma unroll 1
             for (int i = lane; i < cnt; i += 32) out[i] = m.tau * ((double)tpart[i].x + (double)tpart[i].y);
             __syncwarp();
@@ -582,8 +619,8 @@ struct WormWalker {
         __syncwarp();
         return chainAction(kChainCap - 1, 1);
     }
-    // the primitive action has no gradient correction (gradVFactor = 0)
-    __device__ double corrRange(WB, WB) { return 0.0; }
+    // (the primitive action has no gradient correction, gradVFactor = 0, so
+    // the worm moves' correction over the run is zero)
 
     // ---- Path bookkeeping (path.cpp:205-420) ----
     __device__ __noinline__ WB addBead(int slice, float x, float y, float z) {
@@ -702,7 +739,7 @@ struct WormWalker {
     // wraps every step) gives, up to rounding.
     __device__ __noinline__ void freeWalk(float4 r0, int cnt) {
         normals(3 * cnt, znorm);
-        const float sg = (float)m.sqrt2LambdaTau;
+        const float sg = m.sg2;
         float ux = r0.x, uy = r0.y, uz = r0.z;
 #pragma unroll 1
         for (int base = 0; base < cnt; base += 32) {
@@ -723,35 +760,105 @@ struct WormWalker {
         }
         __syncwarp();
     }
-    __device__ WB delBeadGetNext(WB b) { WB n = next(b); delBead(b); return n; }
-    __device__ WB delBeadGetPrev(WB b) { WB p = prev(b); delBead(b); return p; }
+    // The cnt beads chain[c0 .. c0 + cnt - 1] of one worldline, taken in link
+    // order (dir = +1) or against it, leave the path: what cnt calls of
+    // delBead leave, made one lane a bead.  Their slices are distinct (cnt <
+    // M or a whole open worm of at most Mbar + 1 <= M beads), so on each the
+    // slice's last bead takes the place of the one that leaves, whatever the
+    // order.  All of the old state is read into the move's buffers first;
+    // then each moved bead's links are written with both ends under their new
+    // names, and where a link joins two moved beads both write the same.
+    __device__ __noinline__ void dropBeads(int c0, int cnt, int dir) {
+        int* on = reinterpret_cast<int*>(znorm);        // the last bead's next and prev, and its place
+        int* op = on + kOrigCap;
+        int* ol = op + kOrigCap;
+        const int M = m.M, Ne = m.Ne;
+        bool bad = cnt < 1 || cnt > kOrigCap || cnt > M;
+#pragma unroll 1
+        for (int k = lane; k < cnt && !bad; k += 32) {
+            const WB b = unpack(chain[c0 + k]);
+            const int l = nbs[b.t] - 1;
+            if (l < b.p || l >= Ne) { bad = true; break; }
+            const WB last{b.t, l};
+            ol[k] = l;
+            on[k] = nxt[lk(last)];
+            op[k] = prv[lk(last)];
+            qbuf[k] = pos[li(last)];
+        }
+        if (__any_sync(0xffffffffu, bad)) { err = WERR_LINK; return; }
+        const WB first = unpack(chain[c0 + (dir > 0 ? 0 : cnt - 1)]), end = unpack(chain[c0 + (dir > 0 ? cnt - 1 : 0)]);
+        const int before = prv[lk(first)], after = nxt[lk(end)];    // the run's neighbours, -1 none
+        __syncwarp();
+        // index r on run place k's slice after the removal
+        auto moved = [&](int k, int r) {
+            if (k < 0 || k >= cnt) return r;
+            const int p = chain[c0 + k] & 4095;
+            return r == ol[k] && p < r ? p : r;
+        };
+#pragma unroll 1
+        for (int k = lane; k < cnt; k += 32) {
+            const WB b = unpack(chain[c0 + k]);
+            const int l = ol[k];
+            if (b.p < l) {
+                const int tn = b.t + 1 == M ? 0 : b.t + 1, tp = b.t == 0 ? M - 1 : b.t - 1;
+                const int n = moved(k + dir, on[k]), p = moved(k - dir, op[k]);
+                pos[li(b)] = qbuf[k];
+                nxt[lk(b)] = n;
+                prv[lk(b)] = p;
+                if (n >= 0 && n < Ne) prv[lk(WB{tn, n})] = b.p;
+                if (p >= 0 && p < Ne) nxt[lk(WB{tp, p})] = b.p;
+            }
+            nxt[lk(WB{b.t, l})] = -1;
+            prv[lk(WB{b.t, l})] = -1;
+            nbs[b.t] = l;
+        }
+        if (lane == 0) {
+            if (before >= 0 && before < Ne) nxt[lk(WB{first.t == 0 ? M - 1 : first.t - 1, before})] = -1;
+            if (after >= 0 && after < Ne) prv[lk(WB{end.t + 1 == M ? 0 : end.t + 1, after})] = -1;
+        }
+        auto follow = [&](WB& s) {
+            if (isXW(s)) return;
+            int k = s.t - first.t;
+            if (k < 0) k += M;
+            if (k < cnt) s.p = moved(dir > 0 ? k : cnt - 1 - k, s.p);
+        };
+        follow(head); follow(tail); follow(sp1); follow(sp2);
+        numBeadsOn -= cnt;
+        __syncwarp();
+    }
 
     // ---- Worm (worm.cpp:52-101, worm.h:68-81) ----
     __device__ void wormReset() {
         gap = -1; length = 0; sep[0] = sep[1] = sep[2] = 0.f;
         head = tail = sp1 = sp2 = WB{-1, -1};
     }
-    __device__ __noinline__ void wormUpdate(WB nh, WB nt) {
+    __device__ __noinline__ void wormUpdate(WB nh, WB nt, int known) {
         head = nh; tail = nt;
         gap = nt.t - nh.t;
         if (gap < 0) gap += m.M;
         // Worm::update (worm.cpp:52-101) counts the worm's beads by walking it
         // from tail to head.  The moves only compare that length with Mbar
         // (remove needs length <= Mbar; advance tail and recede head need it
-        // above their step, which is at most Mbar), so the walk stops after
-        // Mbar + 1 links and a longer worm counts as Mbar + 1: the same
-        // decisions without chasing up to N M dependent links.
-        WB b = nt;
-        length = 0;
+        // above their step, which is at most Mbar), so a worm longer than Mbar
+        // counts as Mbar + 1, and the walk stops after that many links.  A
+        // move that lengthens the worm, or shortens one not longer than Mbar,
+        // gives the new length (known > 0) and nothing is walked.
         const int cap = m.mbar + 1;
-        const LinkWalk lw = links();
-        bool bad = false;
+        if (known > 0) {
+            length = min(known, cap);
+        } else {
+            length = 0;
 #pragma unroll 1
-        do {
-            ++length;
-            b = lw.next(b, bad);
-            if (isXW(b)) { err = WERR_LOOP; break; }
-        } while (!eqW(b, nh) && length < cap);
+            for (WB b = nt; length < cap;) {
+                const Segment s = segment(b, +1, cap - length);
+                const unsigned hit = __ballot_sync(0xffffffffu, lane > 0 && lane < s.c && eqW(s.mine, nh));
+                if (hit) { length += __ffs(hit) - 1; break; }
+                length += s.c;
+                b = s.on;
+                if (isXW(b)) { err = WERR_LOOP; break; }
+                if (eqW(b, nh)) break;
+            }
+        }
         const float4 rt = P(nt), rh = P(nh);
         sep[0] = putInBC(rt.x - rh.x);
         sep[1] = putInBC(rt.y - rh.y);
@@ -759,9 +866,13 @@ struct WormWalker {
         setNext(nh, {-1, -1}); setPrev(nt, {-1, -1});
         sp1 = sp2 = WB{-1, -1};
     }
+    // the length of a worm shortened by n links (0: only a walk can tell)
+    __device__ int shortened(int n) const { return length <= m.mbar ? length - n : 0; }
     __device__ bool tooCostly(double sx, double sy, double sz, int g) const {
+        // x / g > 4 as x > 4 g: the next double above 4 g is more than
+        // half an ulp of 4 above it when divided by g, so they agree
         if (g == 0) return true;
-        return ((sx * sx + sy * sy + sz * sz) * (0.25 / (m.lambda * m.tau)) / (1.0 * g)) > 4.0;
+        return (sx * sx + sy * sy + sz * sz) * m.costScale > 4.0 * g;
     }
     __device__ double ensembleWeight(int d) const {
         if (m.window >= 0) {
@@ -788,7 +899,7 @@ struct WormWalker {
         // cumulative weights in sector order
         const float4 pe = P(eb), ps = P(sb);
         const float Lb = m.L;
-        const float den = (float)(4.0 * m.lambda * L * m.tau);
+        const float den = (float)(m.lambda4 * L * m.tau);
         const float g = rsqrtf(3.14159265358979f * den);
         const float g3 = g * g * g;
         const int ln = lane;
@@ -823,7 +934,7 @@ struct WormWalker {
     __device__ __noinline__ void stagePositions(int cnt, float4 start, float4 e, int L, int3& wind, float4* out) {
         normals(3 * cnt, znorm);
         const float Lb = m.L;
-        const float sg0 = (float)m.sqrt2LambdaTau;
+        const float sg0 = m.sg2;
         const float Ex = e.x + Lb * wind.x, Ey = e.y + Lb * wind.y, Ez = e.z + Lb * wind.z;
         float ux = start.x, uy = start.y, uz = start.z;
 #pragma unroll 1
@@ -881,7 +992,7 @@ struct WormWalker {
     }
     __device__ __noinline__ void freePos(WB nbd, float& x, float& y, float& z) {
         const float4 p = P(nbd);
-        const float sg = (float)m.sqrt2LambdaTau;
+        const float sg = m.sg2;
         x = putInBC(randNorm(p.x, sg));
         y = putInBC(randNorm(p.y, sg));
         z = putInBC(randNorm(p.z, sg));
@@ -890,6 +1001,34 @@ struct WormWalker {
     __device__ bool metro(double dA) { return rand() < expf(-(float)dA); }
     __device__ int randLen() { return 2 * (1 + (int)randInt((uint32_t)(m.mbar / 2 - 1))); }
     __device__ int trueN() const { return numBeadsOn / m.M; }
+
+    // the beads from `a` along n links of direction dir into chain[c0 + step k],
+    // k = 0 .. n; false where the worldline ends before (err set for a broken
+    // link)
+    __device__ __noinline__ bool collectRun(WB a, int n, int dir, int c0, int step) {
+        int k = 0;
+#pragma unroll 1
+        for (WB x = a; k <= n;) {
+            if (isXW(x)) return false;
+            const Segment s = segment(x, dir, n + 1 - k);
+            if (lane < s.c) chain[c0 + step * (k + lane)] = pack(s.mine);
+            k += s.c;
+            if (s.bad && k <= n) { err = WERR_LINK; return false; }
+            x = s.on;
+        }
+        __syncwarp();
+        return true;
+    }
+    // whether chain[0 .. n - 1] are all beads below their slices' counts
+    __device__ bool activeRun(int n) const {
+        bool off = false;
+#pragma unroll 1
+        for (int k = lane; k < n; k += 32) {
+            const WB b = unpack(chain[k]);
+            off |= b.p >= nbs[b.t];
+        }
+        return !__any_sync(0xffffffffu, off);
+    }
 
     // ---- diagonal moves ----
     // CenterOfMassMove (move.cpp:1124-1262).  The worldline through a
@@ -902,43 +1041,40 @@ struct WormWalker {
         accepted = false;
         if (numBeadsOn == 0 || nb(0) == 0) return 0;
         const WB first{0, (int)randInt((uint32_t)(nb(0) - 1))};
-        WB b = first;
-        int back = 0;
+        int wl = 0, c0;
         bool closed = false;
-        const LinkWalk lw = links();
-        bool bad = false;
+        WB b = first, start = first;
 #pragma unroll 1
         for (;;) {
-            const WB pb = lw.prev(b, bad);
-            if (bad) { err = WERR_LINK; return 0; }
-            if (isXW(pb)) break;
-            if (eqW(pb, first)) { closed = true; break; }
-            if (back + 1 >= m.M) return 0;
-            ++back;
-            b = pb;
-            if (lane == 0) chain[m.M - back] = pack(b);
+            const Segment s = segment(b, -1, m.M - wl);
+            if (lane < s.c && wl + lane > 0) chain[m.M - wl - lane] = pack(s.mine);
+            wl += s.c;
+            if (s.bad) { err = WERR_LINK; return 0; }
+            start = WB{__shfl_sync(0xffffffffu, s.mine.t, s.c - 1), b.p};
+            b = s.on;
+            if (isXW(b)) break;
+            if (eqW(b, first)) { closed = true; break; }
+            if (wl >= m.M) return 0;
         }
-        int c0 = 0, wl = 0;
+        c0 = m.M - wl;
         if (closed) {
-            c0 = m.M - back - 1;
-            wl = back + 1;
             if (lane == 0) chain[c0] = pack(first);
         } else {
+            c0 = wl = 0;
 #pragma unroll 1
-            for (WB s = b;;) {
+            for (b = start; !isXW(b);) {
                 if (wl >= m.M) return 0;
-                if (lane == 0) chain[wl] = pack(s);
-                ++wl;
-                const WB ns = lw.next(s, bad);
-                if (bad) { err = WERR_LINK; return 0; }
-                if (isXW(ns)) break;
-                s = ns;
+                const Segment s = segment(b, +1, m.M - wl);
+                if (lane < s.c) chain[wl + lane] = pack(s.mine);
+                wl += s.c;
+                if (s.bad) { err = WERR_LINK; return 0; }
+                b = s.on;
             }
         }
         __syncwarp();
         acc->attempted[WM_COM]++;
         float sh[3];
-        for (int i = 0; i < 3; ++i) sh[i] = (float)m.comDelta * (-0.5f + rand());
+        for (int i = 0; i < 3; ++i) sh[i] = m.comStep * (-0.5f + rand());
         const double oldA = chainAction(c0, wl);
         shiftChain(c0, wl, sh[0], sh[1], sh[2]);
         const double newA = chainAction(c0, wl);
@@ -965,22 +1101,8 @@ struct WormWalker {
         if (nb(sb.t) == 0) return 0;
         sb.p = (int)randInt((uint32_t)(nb(sb.t) - 1));
         const int L = 2 + (int)randInt((uint32_t)(m.mbar - 2));
-        WB b = sb;
-        const LinkWalk lw = links();
-        const int* cnts = nbs;
-        bool bad = false;
-#pragma unroll 1
-        for (int k = 0; k < L; ++k) {
-            if (b.p >= cnts[b.t]) return 0;
-            const WB nb_ = lw.next(b, bad);
-            if (bad) { err = WERR_LINK; return 0; }
-            if (isXW(nb_)) return 0;
-            if (lane == 0) chain[k] = pack(b);
-            b = nb_;
-        }
-        if (lane == 0) chain[L] = pack(b);
-        __syncwarp();
-        const WB eb = b;
+        if (!collectRun(sb, L, +1, 0, 1) || !activeRun(L)) return 0;
+        const WB eb = unpack(chain[L]);
         acc->attempted[WM_DIAG]++;
         double tot;
         int3 wind = sampleWinding(sb, eb, L, tot);
@@ -1022,24 +1144,10 @@ struct WormWalker {
         if (nb(sb.t) == 0) return 0;
         sb.p = (int)randInt((uint32_t)(nb(sb.t) - 1));
         if (numActive > kOrigCap) { err = WERR_LOOP; return 0; }
-        WB b = sb;
-        const LinkWalk lw = links();
-        const int* cnts = nbs;
-        bool bad = false;
-#pragma unroll 1
-        for (int k = 0; k <= numActive; ++k) {
-            if (b.p >= cnts[b.t]) return 0;
-            const WB nx = lw.next(b, bad);
-            if (bad) { err = WERR_LINK; return 0; }
-            if (isXW(nx)) return 0;
-            if (lane == 0) chain[k] = pack(b);
-            b = nx;
-        }
-        if (lane == 0) chain[numActive + 1] = pack(b);
-        __syncwarp();
+        if (!collectRun(sb, numActive + 1, +1, 0, 1) || !activeRun(numActive + 1)) return 0;
         acc->attempted[WM_DIAG]++;
         saveChain(numActive, orig);                     // orig[j - 1]: bead at offset j
-        const float sgBase = (float)m.sqrtLambdaTau;
+        const float sgBase = m.sg1;
         // the normal deviates of every level at once, level by level in the
         // reference's order (a level rejected early leaves the later levels'
         // deviates unused: independent draws, the same distribution)
@@ -1116,78 +1224,79 @@ struct WormWalker {
     // all drawn before its uniform ones: a different order of independent
     // draws, the same distribution.
 
-    // the beads from `a` along next (dir > 0) or prev links to `b` inclusive,
-    // into chain[0 ..]; returns their number (b not reached: the walk's end,
-    // with err set for a broken link)
-    __device__ int collectRun(WB a, WB b, int dir) {
-        int cnt = 0;
-        WB x = a;
-        const LinkWalk lw = links();
-        const int cap = m.mbar + 1;
-        bool bad = false;
-#pragma unroll 1
-        for (int g = 0; g <= cap; ++g) {
-            if (isXW(x)) { err = WERR_LINK; break; }
-            if (lane == 0) chain[cnt] = pack(x);
-            ++cnt;
-            if (eqW(x, b)) break;
-            x = dir > 0 ? lw.next(x, bad) : lw.prev(x, bad);
-        }
-        __syncwarp();
-        return cnt;
-    }
-    // acts[k] for chain[k], evaluated a chunk at a time once the tests reach
-    // it: the first chunk one bead (kTeamMinBeads for a team), each next one
+    // A run's actions are evaluated a chunk at a time once the tests reach it:
+    // the first chunk one bead (kTeamMinBeads for a team), each next one
     // twice as long, so that a run rejected at its first beads costs about
     // what the sequential form costs and a long accepted run is evaluated in
     // a few batches
-    __device__ void actsUpTo(int k, int total, int& ev, int& chunk) {
-        if (k < ev) return;
-        const int n = min(chunk, total - ev);
-        beadActions(ev, n, acts + ev);
-        ev += n;
-        chunk = min(2 * chunk, kRunCap);
-    }
     __device__ int firstChunk() const { return team > 1 ? kTeamMinBeads : 1; }
-    // removal-type test over the beads chain[0 .. cnt - 1]: -(U_k - f_k
-    // shift), f = 1/2 at both ends and 1 between; true when every bead is
-    // accepted
-    __device__ bool removalTests(int cnt, double actionShift, double corr) {
-        int ev = 0, chunk = firstChunk();
+    // the Metropolis tests of beads from .. to - 1 of a run whose last bead
+    // is `last`: rand() < exp(sign (U_k - f_k shift)), sign = -1 for an
+    // insertion and 1 for a removal, f = 1/2 at both ends and 1 between, made
+    // by the lanes together from the words that the tests one
+    // after another would draw.  The stream moves past the first failing
+    // test, or past them all.
+    __device__ __noinline__ bool testsOf(int from, int to, int last, float sign, double actionShift) {
+        const int ln = lane;
+        int used = 0, ln_used = 0;
+        bool pass = true;
+        uint4 w = buf;
 #pragma unroll 1
-        for (int k = 0; k < cnt; ++k) {
-            actsUpTo(k, cnt, ev, chunk);
-            acc->bead_updates++;
-            double dA = -(acts[k] - ((k == 0 || k == cnt - 1) ? 0.5 : 1.0) * actionShift);
-            if (k == cnt - 1) dA -= corr;
-            if (!metro(dA)) return false;
+        for (int base = from; base < to && pass; base += 32) {
+            const int k = base + ln;
+            const int i = k - from - (4 - bidx);          // the word's place after the current block
+            w = i < 0 ? buf : block(ctr + (unsigned)(i >> 2));
+            const int q = (i < 0 ? 4 + i : i) & 3;
+            const uint32_t word = q == 0 ? w.x : q == 1 ? w.y : q == 2 ? w.z : w.w;
+            const float u = (float)(acts[min(k, to - 1)] - ((k == 0 || k == last) ? 0.5 : 1.0) * actionShift);
+            const bool ok = (float)word * 2.3283064365386963e-10f < expf(sign * u);
+            const unsigned fail = __ballot_sync(0xffffffffu, k < to && !ok);
+            ln_used = fail ? __ffs(fail) - 1 : min(to - base, 32) - 1;
+            used = base - from + ln_used + 1;
+            pass = fail == 0;
+        }
+        acc->bead_updates += used;
+        // the block of the last word used becomes the current one
+        const int over = used - (4 - bidx);
+        if (over <= 0) {
+            bidx += used;
+        } else {
+            buf = make_uint4(__shfl_sync(0xffffffffu, w.x, ln_used), __shfl_sync(0xffffffffu, w.y, ln_used),
+                             __shfl_sync(0xffffffffu, w.z, ln_used), __shfl_sync(0xffffffffu, w.w, ln_used));
+            ctr += (unsigned)((over + 3) >> 2);
+            bidx = over - 4 * ((over - 1) >> 2);
+        }
+        return pass;
+    }
+    // the tests of beads 0 .. total - 1, each chunk's actions evaluated when
+    // the tests reach it
+    __device__ __noinline__ bool runTests(int total, int last, float sign, double actionShift) {
+        int chunk = firstChunk();
+#pragma unroll 1
+        for (int ev = 0; ev < total;) {
+            const int n = min(chunk, total - ev);
+            beadActions(ev, n, acts + ev);
+            if (!testsOf(ev, ev + n, last, sign, actionShift)) return false;
+            ev += n;
+            chunk = min(2 * chunk, kRunCap);
         }
         return true;
     }
-    // insertion-type test over the beads chain[0 .. cnt]: U_k - f_k shift,
-    // f = 1/2 at both ends and 1 between.  With `endRef` set, the last bead
-    // `end` becomes that worm end (*endRef = end) before its action is taken,
-    // as the reference sets the new head or tail before its test; chain[cnt]
-    // is then not read.
-    __device__ bool insertionTests(int cnt, double actionShift, double corr, WB* endRef, WB end) {
-        int ev = 0, chunk = firstChunk();
-        const int total = endRef ? cnt : cnt + 1;
-#pragma unroll 1
-        for (int k = 0; k <= cnt; ++k) {
-            double u;
-            if (k == cnt && endRef) {
-                *endRef = end;
-                u = bare(end);
-            } else {
-                actsUpTo(k, total, ev, chunk);
-                u = acts[k];
-            }
-            acc->bead_updates++;
-            double dA = u - ((k == 0 || k == cnt) ? 0.5 : 1.0) * actionShift;
-            if (k == cnt) dA += corr;
-            if (!metro(dA)) return false;
-        }
-        return true;
+    // removal-type test over the beads chain[0 .. cnt - 1]: -(U_k - f_k
+    // shift); true when every bead is accepted
+    __device__ bool removalTests(int cnt, double actionShift) { return runTests(cnt, cnt - 1, 1.0f, actionShift); }
+    // insertion-type test over the beads chain[0 .. cnt]: U_k - f_k shift.
+    // With `endRef` set, the last bead `end` becomes that worm end (*endRef =
+    // end) before its action is taken, as the reference sets the new head or
+    // tail before its test; chain[cnt] is then not read.
+    __device__ bool insertionTests(int cnt, double actionShift, WB* endRef, WB end) {
+        if (!runTests(endRef ? cnt : cnt + 1, cnt, -1.0f, actionShift)) return false;
+        if (!endRef) return true;
+        *endRef = end;
+        const double u = bare(end);
+        if (lane == 0) acts[cnt] = u;
+        __syncwarp();
+        return testsOf(cnt, cnt + 1, cnt, -1.0f, actionShift);
     }
 
     __device__ int open() {
@@ -1197,8 +1306,10 @@ struct WormWalker {
         hb.t = 2 * (int)randInt((uint32_t)(m.M / 2 - 1));
         if (nb(hb.t) == 0) return -1;
         hb.p = (int)randInt((uint32_t)(nb(hb.t) - 1));
-        tb = nextN(hb, gapLength);
-        if (isXW(tb)) return -1;
+        // hb, the gap's beads and tb
+        const int cnt = gapLength + 1;
+        if (!collectRun(hb, gapLength, +1, 0, 1)) return -1;
+        tb = unpack(chain[gapLength]);
         double totalrho0;
         const int3 wind = sampleWinding(hb, tb, gapLength, totalrho0);
         const float4 pt = P(tb), ph = P(hb);
@@ -1213,15 +1324,11 @@ struct WormWalker {
         acc->attempted[WM_OPEN]++;
         sp1 = hb; sp2 = tb;
         const double actionShift = (-log(norm) + muShift) / gapLength;
-        // hb, the gap's beads and tb: removed but the ends
-        const int cnt = collectRun(hb, tb, +1);
-        if (err) return -2;
-        if (removalTests(cnt, actionShift, corrRange(hb, tb))) {
+        // removed but the ends
+        if (removalTests(cnt, actionShift)) {
             acc->accepted[WM_OPEN]++;
-            WB b = next(hb);
-#pragma unroll 1
-            for (int g = 0; g <= m.M && !eqW(b, tb) && !isXW(b); ++g) b = delBeadGetNext(b);
-            wormUpdate(hb, tb);
+            dropBeads(1, cnt - 2, +1);
+            wormUpdate(hb, tb, 0);
             diag = 0;
             return 1;
         }
@@ -1261,7 +1368,7 @@ struct WormWalker {
         if (lane == 0) chain[g0] = pack(tail);
         __syncwarp();
         // head, the new beads and the tail
-        if (insertionTests(g0, actionShift, corrRange(head, tail), nullptr, tail)) {
+        if (insertionTests(g0, actionShift, nullptr, tail)) {
             acc->accepted[WM_CLOSE]++; wormReset(); diag = 1; return 1;
         }
         closeUndo(nnew);
@@ -1292,8 +1399,8 @@ struct WormWalker {
         if (!appendRun(tb, wl, +1, qbuf, 0)) return -2;
         const WB hb = unpack(chain[wl]);
         // tb, the intermediate beads and the head (sp1 = hb before its test)
-        if (insertionTests(wl, actionShift, corrRange(tb, hb), &sp1, hb)) {
-            acc->accepted[WM_INSERT]++; wormUpdate(hb, tb); diag = 0; return 1;
+        if (insertionTests(wl, actionShift, &sp1, hb)) {
+            acc->accepted[WM_INSERT]++; wormUpdate(hb, tb, wl); diag = 0; return 1;
         }
         insertUndo(tb, wl);
         return 0;
@@ -1308,13 +1415,11 @@ struct WormWalker {
         if (norm < 2.220446049250313e-16) return 0;
         const double actionShift = (-log(norm) + muShift) / length;
         // the worm from the head back to the tail
-        const int cnt = collectRun(head, tail, -1);
-        if (err) return -2;
-        if (removalTests(cnt, actionShift, corrRange(tail, head))) {
+        const int cnt = length + 1;
+        if (!collectRun(head, length, -1, 0, 1) || !eqW(unpack(chain[length]), tail)) { err = WERR_LINK; return -2; }
+        if (removalTests(cnt, actionShift)) {
             acc->accepted[WM_REMOVE]++;
-            WB b = head;
-#pragma unroll 1
-            for (int g = 0; g <= m.M * m.Ne && !isXW(b); ++g) b = delBeadGetPrev(b);
+            dropBeads(0, cnt, -1);
             wormReset(); diag = 1;
             return 1;
         }
@@ -1331,19 +1436,17 @@ struct WormWalker {
         if (numBeadsOn == 0) return -1;
         const int al = randLen();
         acc->attempted[WM_AH]++;
-        const double muShift = al * m.tau * m.mu;
-        double norm = 1.0;
-        norm *= ensembleWeight(al);
+        // log(norm) is 0 or, outside the window, -infinity
+        const double actionShift = ensembleWeight(al) > 0.0 ? stepShift[al / 2 - 1] : -INFINITY;
         sp1 = head; head = WB{-1, -1};
-        const double actionShift = (log(norm) + muShift) / al;
         // the old head and al new beads, the last the new head
         freeWalk(P(sp1), al);
         if (!appendRun(sp1, al, +1, qbuf, 0)) return -2;
         const WB hb = unpack(chain[al]);
         // the old head, the intermediate beads and the new head, set before
         // its test (potentialAction(head): primitive)
-        if (insertionTests(al, actionShift, corrRange(sp1, hb), &head, hb)) {
-            acc->accepted[WM_AH]++; wormUpdate(hb, tail); diag = 0; return 1;
+        if (insertionTests(al, actionShift, &head, hb)) {
+            acc->accepted[WM_AH]++; wormUpdate(hb, tail, length + al); diag = 0; return 1;
         }
         ahUndo(al);
         return 0;
@@ -1352,23 +1455,17 @@ struct WormWalker {
         if (numBeadsOn == 0) return -1;
         const int al = randLen();
         if (!(al < length)) return -1;
-        const WB tb = nextN(tail, al);
-        if (isXW(tb)) return -1;
-        const double muShift = al * m.tau * m.mu;
-        double norm = 1.0;
-        norm *= ensembleWeight(-al);
+        // the tail and the beads up to tb: removed but tb
+        const int cnt = al + 1;
+        if (!collectRun(tail, al, +1, 0, 1)) return -1;
+        const WB tb = unpack(chain[al]);
+        const double actionShift = ensembleWeight(-al) > 0.0 ? stepShift[al / 2 - 1] : INFINITY;
         acc->attempted[WM_AT]++;
         sp1 = tb;
-        const double actionShift = (-log(norm) + muShift) / al;
-        // the tail and the beads up to tb: removed but tb
-        const int cnt = collectRun(tail, tb, +1);
-        if (err) return -2;
-        if (removalTests(cnt, actionShift, corrRange(tail, tb))) {
+        if (removalTests(cnt, actionShift)) {
             acc->accepted[WM_AT]++;
-            WB b = prev(tb);
-#pragma unroll 1
-            for (int g = 0; g <= m.M * m.Ne && !isXW(b); ++g) b = delBeadGetPrev(b);
-            wormUpdate(head, tb);
+            dropBeads(0, al, +1);
+            wormUpdate(head, tb, shortened(al));
             diag = 0;
             return 1;
         }
@@ -1379,23 +1476,17 @@ struct WormWalker {
         if (numBeadsOn == 0) return -1;
         const int rl = randLen();
         if (!(rl < length)) return -1;
-        const WB hb = prevN(head, rl);
-        if (isXW(hb)) return -1;
-        const double muShift = rl * m.tau * m.mu;
-        double norm = 1.0;
-        norm *= ensembleWeight(-rl);
+        // the head and the beads back to hb: removed but hb
+        const int cnt = rl + 1;
+        if (!collectRun(head, rl, -1, 0, 1)) return -1;
+        const WB hb = unpack(chain[rl]);
+        const double actionShift = ensembleWeight(-rl) > 0.0 ? stepShift[rl / 2 - 1] : INFINITY;
         acc->attempted[WM_RH]++;
         sp1 = hb;
-        const double actionShift = (-log(norm) + muShift) / rl;
-        // the head and the beads back to hb: removed but hb
-        const int cnt = collectRun(head, hb, -1);
-        if (err) return -2;
-        if (removalTests(cnt, actionShift, corrRange(sp1, head))) {
+        if (removalTests(cnt, actionShift)) {
             acc->accepted[WM_RH]++;
-            WB b = next(hb);
-#pragma unroll 1
-            for (int g = 0; g <= m.M * m.Ne && !isXW(b); ++g) b = delBeadGetNext(b);
-            wormUpdate(hb, tail);
+            dropBeads(0, rl, -1);
+            wormUpdate(hb, tail, shortened(rl));
             diag = 0;
             return 1;
         }
@@ -1412,19 +1503,17 @@ struct WormWalker {
         if (numBeadsOn == 0) return -1;
         const int rl = randLen();
         acc->attempted[WM_RT]++;
-        const double muShift = rl * m.tau * m.mu;
-        double norm = 1.0;
-        norm *= ensembleWeight(rl);
+        // log(norm) is 0 or, outside the window, -infinity
+        const double actionShift = ensembleWeight(rl) > 0.0 ? stepShift[rl / 2 - 1] : -INFINITY;
         sp1 = tail; tail = WB{-1, -1};
-        const double actionShift = (log(norm) + muShift) / rl;
         // the old tail and rl new beads before it, the last the new tail
         freeWalk(P(sp1), rl);
         if (!appendRun(sp1, rl, -1, qbuf, 0)) return -2;
         const WB tb = unpack(chain[rl]);
         // the old tail, the intermediate beads and the new tail, set before
         // its test
-        if (insertionTests(rl, actionShift, corrRange(tb, sp1), &tail, tb)) {
-            acc->accepted[WM_RT]++; wormUpdate(head, tb); diag = 0; return 1;
+        if (insertionTests(rl, actionShift, &tail, tb)) {
+            acc->accepted[WM_RT]++; wormUpdate(head, tb, length + rl); diag = 0; return 1;
         }
         rtUndo(rl);
         return 0;
@@ -1443,11 +1532,11 @@ struct WormWalker {
                     az_ = (pf.z - pb.z) + (float)(sign * wv.z) * L;
         return g3 * expf(ax * ax * nden) * expf(ay * ay * nden) * expf(az_ * az_ * nden);
     }
-    __device__ __noinline__ double towerNorm(WB b, int pivotSlice, int sign, float x, WB& pivot, int3& wind) {
+    __device__ __noinline__ float towerNorm(WB b, int pivotSlice, int sign, float x, WB& pivot, int3& wind) {
         const int nL = nb(pivotSlice);
         const float4 pb = P(b);
         const float4* row = pos + (size_t)pivotSlice * m.Ne;
-        const float den = (float)(4.0 * m.lambda * m.mbar * m.tau);
+        const float den = m.swapDen;
         const float g = rsqrtf(3.14159265358979f * den);
         const float g3 = g * g * g;
         const float L = m.L;
@@ -1458,33 +1547,28 @@ struct WormWalker {
         float acc[32];
 #pragma unroll
         for (int w = 0; w < 32; ++w) acc[w] = 0.0f;
+        // (a rolled loop over 32 beads: nine exponentials and 27 sums of a
+        // bead keep the lane busy, and one copy of them is in the code)
+        float4 pf = row[min(ln, max(nL - 1, 0))];
 #pragma unroll 1
-        for (int n0 = 0; n0 < nL; n0 += 64) {
-            float4 pf[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int n = n0 + 32 * u + ln;
-                pf[u] = n < nL ? row[n] : pb;
-            }
+        for (int n0 = 0; n0 < nL; n0 += 32) {
+            const bool ok = n0 + ln < nL;
             // rho0 factorises over the axes: three shifts per axis (component
             // 0, +1, -1 of the winding vector) give the 27 sector weights as
             // products, 9 exponentials a bead instead of 27
+            const float dx = pf.x - pb.x, dy = pf.y - pb.y, dz = pf.z - pb.z;
+            pf = row[min(n0 + 32 + ln, nL - 1)];
+            float ex[3], ey[3], ez[3];
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const bool ok = n0 + 32 * u + ln < nL;
-                const float dx = pf[u].x - pb.x, dy = pf[u].y - pb.y, dz = pf[u].z - pb.z;
-                float ex[3], ey[3], ez[3];
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const float sh = (float)(sign * (k == 2 ? -1 : k)) * L;
-                    const float ax = dx + sh, ay = dy + sh, az_ = dz + sh;
-                    ex[k] = ok ? g3 * expf(ax * ax * nden) : 0.0f;
-                    ey[k] = expf(ay * ay * nden);
-                    ez[k] = expf(az_ * az_ * nden);
-                }
-#pragma unroll
-                for (int w = 0; w < kMaxWind; ++w) acc[w] = fmaf(ex[(w / 9) % 3] * ey[(w / 3) % 3], ez[w % 3], acc[w]);
+            for (int k = 0; k < 3; ++k) {
+                const float sh = (float)(sign * (k == 2 ? -1 : k)) * L;
+                const float ax = dx + sh, ay = dy + sh, az_ = dz + sh;
+                ex[k] = ok ? g3 * expf(ax * ax * nden) : 0.0f;
+                ey[k] = expf(ay * ay * nden);
+                ez[k] = expf(az_ * az_ * nden);
             }
+#pragma unroll
+            for (int w = 0; w < kMaxWind; ++w) acc[w] = fmaf(ex[(w / 9) % 3] * ey[(w / 3) % 3], ez[w % 3], acc[w]);
         }
         // sector totals over the lanes by recursive halving: at each step a
         // lane keeps the half of its slots that its partner lane does not,
@@ -1531,7 +1615,7 @@ struct WormWalker {
             pivot = WB{pivotSlice, found};
             wind = wv;
         }
-        return (double)sum;
+        return sum;
     }
     // SwapHeadMove (move.cpp:3388-3622): chain[0 .. Mbar] runs from the swap
     // bead to the pivot; after relinking chain[0] is the old head
@@ -1542,25 +1626,17 @@ struct WormWalker {
         if (pivotSlice >= m.M) pivotSlice -= m.M;
         if (nb(pivotSlice) == 0) return -1;
         WB pivot; int3 wind;
-        const double SigmaHead = towerNorm(head, pivotSlice, 1, rand(), pivot, wind);
-        WB b = pivot;
-        const LinkWalk lw = links();
-        bool bad = false;
+        const float SigmaHead = towerNorm(head, pivotSlice, 1, rand(), pivot, wind);
+        if (!collectRun(pivot, swapLength, -1, swapLength, -1)) return -1;
+        bool met = false;                           // the other worm end is on the way
 #pragma unroll 1
-        for (int k = 0; k < swapLength; k++) {
-            if (eqW(b, tail) || isXW(b)) { if (bad) err = WERR_LINK; return -1; }
-            if (lane == 0) chain[swapLength - k] = pack(b);
-            b = lw.prev(b, bad);
-        }
-        if (bad) err = WERR_LINK;
-        const WB swp = b;
-        if (isXW(swp) || eqW(tail, swp)) return -1;
-        if (lane == 0) chain[0] = pack(swp);
-        __syncwarp();
+        for (int k = lane; k <= swapLength; k += 32) met |= chain[k] == pack(tail);
+        if (__any_sync(0xffffffffu, met)) return -1;
+        const WB swp = unpack(chain[0]);
         acc->attempted[WM_SH]++;
         WB dummy; int3 dw;
-        const double SigmaSwap = towerNorm(swp, pivotSlice, 1, -1.0f, dummy, dw);
-        const float PNorm = (float)fmin(SigmaHead / SigmaSwap, 1.0);
+        const float SigmaSwap = towerNorm(swp, pivotSlice, 1, -1.0f, dummy, dw);
+        const float PNorm = fminf(SigmaHead / SigmaSwap, 1.0f);
         if (rand() < PNorm) {
             const int nm = swapLength - 1;
             sp1 = swp; sp2 = pivot;
@@ -1576,7 +1652,7 @@ struct WormWalker {
             stageChain(nm, P(sp1), P(pivot), swapLength, wind);
             acc->bead_updates += nm;
             const double newA = chainAction(0, swapLength + 1);
-            if (metro(newA - oldA)) { acc->accepted[WM_SH]++; wormUpdate(swp, tail); return 1; }
+            if (metro(newA - oldA)) { acc->accepted[WM_SH]++; wormUpdate(swp, tail, 0); return 1; }
             head = sp1;
             setNext(head, {-1, -1});
             setNext(swp, nextSwap);
@@ -1597,25 +1673,17 @@ struct WormWalker {
         if (pivotSlice < 0) pivotSlice += m.M;
         if (nb(pivotSlice) == 0) return -1;
         WB pivot; int3 wind;
-        const double SigmaTail = towerNorm(tail, pivotSlice, -1, rand(), pivot, wind);
-        WB b = pivot;
-        const LinkWalk lw = links();
-        bool bad = false;
+        const float SigmaTail = towerNorm(tail, pivotSlice, -1, rand(), pivot, wind);
+        if (!collectRun(pivot, swapLength, +1, 0, 1)) return -1;
+        bool met = false;                           // the other worm end is on the way
 #pragma unroll 1
-        for (int k = 0; k < swapLength; k++) {
-            if (eqW(b, head) || isXW(b)) { if (bad) err = WERR_LINK; return -1; }
-            if (lane == 0) chain[k] = pack(b);
-            b = lw.next(b, bad);
-        }
-        if (bad) err = WERR_LINK;
-        const WB swp = b;
-        if (isXW(swp) || eqW(head, swp)) return -1;
-        if (lane == 0) chain[swapLength] = pack(swp);
-        __syncwarp();
+        for (int k = lane; k <= swapLength; k += 32) met |= chain[k] == pack(head);
+        if (__any_sync(0xffffffffu, met)) return -1;
+        const WB swp = unpack(chain[swapLength]);
         acc->attempted[WM_ST]++;
         WB dummy; int3 dw;
-        const double SigmaSwap = towerNorm(swp, pivotSlice, 1, -1.0f, dummy, dw);
-        const float PNorm = (float)fmin(SigmaTail / SigmaSwap, 1.0);
+        const float SigmaSwap = towerNorm(swp, pivotSlice, 1, -1.0f, dummy, dw);
+        const float PNorm = fminf(SigmaTail / SigmaSwap, 1.0f);
         if (rand() < PNorm) {
             const int nm = swapLength - 1;
             sp1 = swp; sp2 = pivot;
@@ -1632,7 +1700,7 @@ struct WormWalker {
             stageChain(nm, P(pivot), P(s1), swapLength, wind);
             acc->bead_updates += nm;
             const double newA = chainAction(0, swapLength + 1);
-            if (metro(newA - oldA)) { acc->accepted[WM_ST]++; wormUpdate(head, swp); return 1; }
+            if (metro(newA - oldA)) { acc->accepted[WM_ST]++; wormUpdate(head, swp, 0); return 1; }
             tail = s1;
             setPrev(tail, {-1, -1});
             setPrev(swp, prevSwap);
@@ -1654,19 +1722,19 @@ struct WormWalker {
     // link to the next slice
     // (a team: warp wk sums the slices t0 + wk, t0 + wk + T, ..., and warp 0
     // adds the warps' sums in warp order)
+    // (half of a team's warps: eight slices at a time leave no more work, and
+    // the FP32 sums of a slice keep the order they had)
+    __device__ static int energyWarps(int team) { return (team + 1) / 2; }
     __device__ __noinline__ double2 energySums(int t0, int t1) {
         if (team > 1) {
             teamPost(2, t0, t1);
             float2 p, k;
-            energyShare(pairCtx(), nxt, t0, t1, team, p, k);
+            energyShare(pairCtx(), nxt, t0, t1, energyWarps(team), p, k);
             if (lane == 0) { job->hi[0] = p.x; job->lo[0] = p.y; job->khi[0] = k.x; job->klo[0] = k.y; }
             team_sync(bar, 32 * team);
-            double pot = 0.0, kin = 0.0;
-#pragma unroll 1
-            for (int q = 0; q < team; ++q) {
-                pot += (double)job->hi[q] + (double)job->lo[q];
-                kin += (double)job->khi[q] + (double)job->klo[q];
-            }
+            const bool in = lane < energyWarps(team);
+            const double pot = sumShares(in ? job->hi[lane] : 0.f, in ? job->lo[lane] : 0.f);
+            const double kin = sumShares(in ? job->khi[lane] : 0.f, in ? job->klo[lane] : 0.f);
             return make_double2(pot, kin);
         }
         float2 p, k;
@@ -1783,12 +1851,20 @@ __device__ __noinline__ void run_walker(int w, int team, int bar, TeamJob* job, 
     ww.acc = &local;
     // cumulative probabilities over the default move list (pimc.cpp:120-152),
     // one copy per warp in shared memory
-    double* cumD = s_cum;
-    double* cumO = s_cum + WM_N;
+    // (rounded down to FP32: x <= c for an FP32 deviate x exactly when x is
+    // not above the rounded c)
+    float* cumD = reinterpret_cast<float*>(s_cum + 32);
+    float* cumO = cumD + WM_N;
+    ww.stepShift = s_cum;
+    {
+        const int l = 2 * (ww.lane + 1);
+        const double shift = l * ww.m.tau * ww.m.mu;
+        ww.stepShift[ww.lane] = shift / l;
+    }
     if (ww.lane == 0 && diag_only) {
 #pragma unroll 1
-        for (int i = 0; i < WM_N; ++i) cumD[i] = cumO[i] = 1.0 + 1e-7;
-        cumD[WM_COM] = cumO[WM_COM] = 0.05;
+        for (int i = 0; i < WM_N; ++i) cumD[i] = cumO[i] = 1.0f;
+        cumD[WM_COM] = cumO[WM_COM] = __double2float_rd(0.05);
     } else if (ww.lane == 0) {
         const double prob[WM_N] = {0.01, 0.19, 0.4, 0.15, 0.4, 0.15, 0.075, 0.075, 0.075, 0.075, 0.1, 0.1};
         const int onDiag[WM_N] = {1, 1, 1, 0, 1, 0, 0, 0, 0, 0, 0, 0};
@@ -1796,12 +1872,11 @@ __device__ __noinline__ void run_walker(int w, int team, int bar, TeamJob* job, 
 #pragma unroll 1
         for (int i = 0; i < WM_N; ++i) {
             if (onDiag[i]) cd += prob[i];
-            cumD[i] = cd;
+            cumD[i] = __double2float_rd(cd);
             if (!onDiag[i] || i < 2) co += prob[i];
-            cumO[i] = co;
+            cumO[i] = __double2float_rd(co);
         }
-        cumD[WM_N - 1] = 1.0 + 1e-7;
-        cumO[WM_N - 1] = 1.0 + 1e-7;
+        cumD[WM_N - 1] = cumO[WM_N - 1] = 1.0f;        // 1 + 1e-7
     }
     __syncwarp();
     float4* orig = s_orig;
@@ -1841,11 +1916,10 @@ __device__ __noinline__ void run_walker(int w, int team, int bar, TeamJob* job, 
             int u = u0;
             for (; u < ww.m.num_updates && !ww.err; ++u) {
                 if (out_of_time()) { stopped = true; break; }
-                const double x = ww.rand();
-                const double* cum = ww.diag ? cumD : cumO;
-                int index = WM_N - 1;
-#pragma unroll 1
-                for (int i = 0; i < WM_N; ++i) if (cum[i] >= x) { index = i; break; }
+                const float x = ww.rand();
+                const float* cum = ww.diag ? cumD : cumO;
+                const unsigned at = __ballot_sync(0xffffffffu, ww.lane < WM_N && cum[min(ww.lane, WM_N - 1)] >= x);
+                const int index = at ? __ffs(at) - 1 : WM_N - 1;
                 bool acc = false;
                 int moved = 0;
                 switch (index) {
@@ -1943,20 +2017,19 @@ __device__ __noinline__ void team_helper(int w, int wk, int T, int bar, const WW
             bool ok = true;
             WormWalker::teamShare(c, chain, job->a, job->b, wk, T, ok, tpart);
             if (ww.lane == 0) job->bad[wk] = ok ? 0 : 1;
-        } else {
+        } else if (wk < WormWalker::energyWarps(T)) {
             float2 p, k;
-            WormWalker::energyShare(c, ww.nxt, job->a + wk, job->b, T, p, k);
+            WormWalker::energyShare(c, ww.nxt, job->a + wk, job->b, WormWalker::energyWarps(T), p, k);
             if (ww.lane == 0) { job->hi[wk] = p.x; job->lo[wk] = p.y; job->khi[wk] = k.x; job->klo[wk] = k.y; }
         }
         team_sync(bar, 32 * T);
     }
 }
 
-// plan[4 b .. 4 b + 3] lists the walkers of CTA b: up to four small walkers
-// (-1 for an empty place); or one large walker and kPlanTeam in the second
-// place, served by the CTA's four warps as a team; or two walkers in the
-// first and third places (the third -1 when there is one) and kPlanPair in
-// the second, each served by a team of two warps
+// plan[4 b .. 4 b + 3] lists the walkers of CTA b: one and kPlanTeam in the
+// second place, served by all its warps; or two in the first and third places
+// (the third -1 when there is one) and kPlanPair in the second; or up to four
+// (-1 for an empty place)
 constexpr int kPlanTeam = -2;
 constexpr int kPlanPair = -3;
 
@@ -1966,41 +2039,30 @@ k_worm_walkers(const WWMeta* __restrict__ meta, float4* __restrict__ pos, int* _
                WWState* __restrict__ states, pgb_worm_walker_stats* __restrict__ stats,
                AzizF az, int sweeps, const int* __restrict__ plan, const int* __restrict__ limit,
                unsigned long long budget_ns, int diag_only) {
-    __shared__ float4 s_orig[kCtaWarps][kOrigCap];
-    __shared__ float4 s_newp[kCtaWarps][kOrigCap];
-    __shared__ int s_chain[kCtaWarps][kChainCap];
-    __shared__ double s_scr[kCtaWarps][3 * kOrigCap / 2];
-    __shared__ double s_cum[kCtaWarps][2 * WM_N];
-    __shared__ TeamJob s_job[2];
+    __shared__ float4 s_orig[kCtaWalkers][kOrigCap];
+    __shared__ float4 s_newp[kCtaWalkers][kOrigCap];
+    __shared__ int s_chain[kCtaWalkers][kChainCap];
+    __shared__ double s_scr[kCtaWalkers][3 * kOrigCap / 2];
+    __shared__ double s_cum[kCtaWalkers][32 + WM_N];
+    __shared__ TeamJob s_job[kCtaWalkers];
     const int warp = threadIdx.x >> 5;
-    const int* pl = plan + kCtaWarps * blockIdx.x;
-    if (pl[1] == kPlanTeam || pl[1] == kPlanPair) {
-        const int T = pl[1] == kPlanTeam ? kCtaWarps : 2;
-        const int g = warp / T;                 // the team's place in the CTA
-        const int first = g * T;                // its first warp
-        const int w = pl[2 * g];
-        if (w < 0) return;                      // an empty pair place: no barrier is used
-        const int bar = 1 + g;
-        // a team uses its first warp's buffers; its second warp's chain cache
-        // holds the team's per-bead shares
-        float2* tpart = reinterpret_cast<float2*>(s_chain[first + 1]);
-        if (warp == first) {
-            run_walker(w, T, bar, &s_job[g], meta, pos, nxt, prv, nbs, nbs_off, states, stats, az, sweeps, limit,
-                       budget_ns, diag_only, s_orig[first], s_newp[first], s_chain[first], s_scr[first],
-                       s_cum[first], tpart);
-            // every path out of run_walker ends here: release the helpers
-            if ((threadIdx.x & 31) == 0) s_job[g].op = 0;
-            team_sync(bar, 32 * T);
-        } else {
-            team_helper(w, warp - first, T, bar, meta, pos, nxt, nbs, nbs_off, az, s_chain[first], &s_job[g],
-                        tpart);
-        }
-        return;
+    const int* pl = plan + kCtaWalkers * blockIdx.x;
+    const int T = pl[1] == kPlanTeam ? kCtaWarps : pl[1] == kPlanPair ? kCtaWarps / 2 : kCtaWarps / kCtaWalkers;
+    const int g = warp / T;                     // the team's place in the CTA
+    const int w = pl[T == kCtaWarps / 2 ? 2 * g : g];
+    if (w < 0) return;                          // an empty place: no barrier is used
+    const int first = g * T, bar = 1 + g;
+    // worm moves' runs stay below kListOff, where bisections keep their lists
+    float2* tpart = reinterpret_cast<float2*>(s_chain[g] + kListOff);
+    if (warp == first) {
+        run_walker(w, T, bar, &s_job[g], meta, pos, nxt, prv, nbs, nbs_off, states, stats, az, sweeps, limit,
+                   budget_ns, diag_only, s_orig[g], s_newp[g], s_chain[g], s_scr[g], s_cum[g], tpart);
+        // every path out of run_walker ends here: release the helpers
+        if ((threadIdx.x & 31) == 0) s_job[g].op = 0;
+        team_sync(bar, 32 * T);
+    } else {
+        team_helper(w, warp - first, T, bar, meta, pos, nxt, nbs, nbs_off, az, s_chain[g], &s_job[g], tpart);
     }
-    const int w = pl[warp];
-    if (w < 0) return;
-    run_walker(w, 1, 1, nullptr, meta, pos, nxt, prv, nbs, nbs_off, states, stats, az, sweeps, limit, budget_ns,
-               diag_only, s_orig[warp], s_newp[warp], s_chain[warp], s_scr[warp], s_cum[warp], nullptr);
 }
 
 // an admitted job's seeded closed worldlines: particle i's centre uniform in
@@ -2091,11 +2153,12 @@ __global__ void k_normals_check(uint2 key, int skip, int count, float* serial, f
 using namespace pgb;
 
 // The CTAs of a launch over walkers listed largest first: a walker of
-// N0 >= kTeam4MinN gets a CTA of its own, served by a team of four warps;
-// walkers of kTeamMinN <= N0 < kTeam4MinN share CTAs two to one, each served
-// by a team of two; the others share CTAs four to one; each kind in the
+// N0 >= kTeam4MinN gets a CTA of its own, walkers of kTeamMinN <= N0 <
+// kTeam4MinN share CTAs two to one, the others four to one; each kind in the
 // same order.  A walker's schedule depends only on its own N0, so its chain
-// does not depend on which walkers run beside it.
+// does not depend on which walkers run beside it.  (The CTAs of all kinds
+// sorted by their walkers' moves a step took the same 37 ms: the largest
+// walker, 29 ms alone on an SM, bounds the launch.)
 static int build_plan(const std::vector<int>& order, const std::vector<WWMeta>& meta, std::vector<int>& plan) {
     plan.clear();
     std::vector<int> small;
@@ -2108,9 +2171,9 @@ static int build_plan(const std::vector<int>& order, const std::vector<WWMeta>& 
         } else small.push_back(w);
     }
     if (pending >= 0) plan.insert(plan.end(), {pending, kPlanPair, -1, -1});
-    for (size_t i = 0; i < small.size(); i += kCtaWarps)
-        for (int k = 0; k < kCtaWarps; ++k) plan.push_back(i + k < small.size() ? small[i + k] : -1);
-    return (int)(plan.size() / kCtaWarps);
+    for (size_t i = 0; i < small.size(); i += kCtaWalkers)
+        for (int k = 0; k < kCtaWalkers; ++k) plan.push_back(i + k < small.size() ? small[i + k] : -1);
+    return (int)(plan.size() / kCtaWalkers);
 }
 
 // bisection levels b of ConstantParameters::initConstants
@@ -2218,6 +2281,7 @@ int pgb_worm_walkers_create(const pgb_worm_walkers_params* p, pgb_worm_walkers**
         m.comDelta = 0.04 * 2.0 * std::sqrt(M_PI * p->lambda / T);
         const uint64_t s = p->seed * 0x9E3779B97F4A7C15ull + (uint64_t)w * 0xBF58476D1CE4E5B9ull + 0x94D049BB133111EBull;
         m.key = make_uint2((uint32_t)s, (uint32_t)(s >> 32));
+        meta_constants(m);
         h->meta.push_back(m);
         h->nbs_off.push_back(soff);
         off += (long long)M * ne;
@@ -2233,7 +2297,7 @@ int pgb_worm_walkers_create(const pgb_worm_walkers_params* p, pgb_worm_walkers**
     if (e == cudaSuccess) e = cudaMalloc(&h->d_nbs_off, h->W * sizeof(long long));
     if (e == cudaSuccess) e = cudaMalloc(&h->d_state, h->W * sizeof(WWState));
     if (e == cudaSuccess) e = cudaMalloc(&h->d_stats, h->W * sizeof(pgb_worm_walker_stats));
-    if (e == cudaSuccess) e = cudaMalloc(&h->d_plan, (size_t)kCtaWarps * h->W * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&h->d_plan, (size_t)kCtaWalkers * h->W * sizeof(int));
     if (e == cudaSuccess) {
         // the sweep lasts as long as the largest walker needs: start the
         // largest first so that they spread over the SMs
@@ -2303,9 +2367,9 @@ int pgb_worm_walkers_load(pgb_worm_walkers* h, int w, const double* pos) {
 // The walkers' state lives in local memory around the helpers that are not
 // inlined, and a large walker's positions (up to a megabyte) and links stream
 // through L1, so the kernel trades shared memory for L1: a carveout of 25 %
-// (two 30 KB CTAs an SM) measured fastest on the 1024-walker workload (27 ms
-// a step against 31 ms at 50 %, 35 ms at the smallest that fits one CTA,
-// 45 ms at 100 %).
+// (two 30 KB CTAs an SM) measured fastest on the 1024-walker workload (53.9
+// ms for four steps, when a CTA had four warps, against 66.7 at 58 %, 75.1 at
+// 100 % and 75.2 at the smallest that fits one CTA).
 constexpr int kWWCarveoutPercent = 25;
 static cudaError_t ww_prefer_l1() { return set_carveout(k_worm_walkers, kWWCarveoutPercent); }
 
@@ -2651,7 +2715,7 @@ int pgb_worm_server_create(const pgb_server_params* p, pgb_worm_server** out) {
         if ((e = cudaMalloc(&s->d_state, s->max_slots * sizeof(WWState))) != cudaSuccess) break;
         if ((e = cudaMalloc(&s->d_stats, s->max_slots * sizeof(pgb_worm_walker_stats))) != cudaSuccess) break;
         if ((e = cudaMalloc(&s->d_nbs_off, s->max_slots * sizeof(long long))) != cudaSuccess) break;
-        if ((e = cudaMalloc(&s->d_plan, (size_t)kCtaWarps * s->max_slots * sizeof(int))) != cudaSuccess) break;
+        if ((e = cudaMalloc(&s->d_plan, (size_t)kCtaWalkers * s->max_slots * sizeof(int))) != cudaSuccess) break;
         if ((e = cudaMalloc(&s->d_limit, s->max_slots * sizeof(int))) != cudaSuccess) break;
     } while (0);
     if (e != cudaSuccess) {
@@ -2736,6 +2800,7 @@ int pgb_worm_server_step(pgb_worm_server* s, int* n_active, int* n_queued) {
         m.comDelta = 0.04 * 2.0 * std::sqrt(M_PI * s->p.lambda / T);
         const uint64_t sd = job.spec.seed * 0x9E3779B97F4A7C15ull + 0x94D049BB133111EBull;
         m.key = make_uint2((uint32_t)sd, (uint32_t)(sd >> 32));
+        meta_constants(m);
         s->h_meta[k] = m;
         s->h_nbs_off[k] = so;
         // the job's seeded worldlines are made on the device; its constants,
