@@ -36,8 +36,8 @@
 // of new beads is placed at once, evaluated in doubling chunks, tested
 // (testsOf()) and taken out again (dropBeads()) by the lanes together; (4)
 // the heavy helpers are not inlined and loops are not unrolled: a walker's
-// warps wait for instructions more than for anything else; (5) the largest
-// walkers are launched first; (6) a move's normal deviates come from the
+// warps wait for instructions more than for anything else; (5) CTAs start in
+// the order of their walkers' moves a step; (6) a move's normal deviates come from the
 // lanes together (normals()), from the same words as serial draws; (7) FP64
 // instructions are few: each holds a quarter of an SM for 64 clocks, so
 // constants are rounded once on the host and sums widened by lanes.
@@ -2152,28 +2152,44 @@ __global__ void k_normals_check(uint2 key, int skip, int count, float* serial, f
 // --------------------------------------------------------------------------
 using namespace pgb;
 
-// The CTAs of a launch over walkers listed largest first: a walker of
-// N0 >= kTeam4MinN gets a CTA of its own, walkers of kTeamMinN <= N0 <
-// kTeam4MinN share CTAs two to one, the others four to one; each kind in the
-// same order.  A walker's schedule depends only on its own N0, so its chain
-// does not depend on which walkers run beside it.  (The CTAs of all kinds
-// sorted by their walkers' moves a step took the same 37 ms: the largest
-// walker, 29 ms alone on an SM, bounds the launch.)
+// The CTAs of a launch: a walker of N0 >= kTeam4MinN gets a CTA of its own,
+// walkers of kTeamMinN <= N0 < kTeam4MinN share CTAs two to one and the
+// others four to one, each kind largest first, and the CTAs start in the
+// order of their longest member's moves a step: a move takes 10 to 18 us
+// whatever the walker's size, so that number orders the CTAs by their time.
+// (All teams before all pairs before all fours ended with small walkers that
+// make 250 moves a step: 40.8 ms for four steps of the 1024-walker workload,
+// 37.6 in this order.)  A walker's schedule depends only on its own N0, so
+// its chain does not depend on which walkers run beside it.
 static int build_plan(const std::vector<int>& order, const std::vector<WWMeta>& meta, std::vector<int>& plan) {
-    plan.clear();
+    struct Cta { int w[kCtaWalkers]; int moves; };
+    std::vector<Cta> ctas;
     std::vector<int> small;
     int pending = -1;                           // a pair walker waiting for its partner
     for (int w : order) {
-        if (meta[w].N0 >= kTeam4MinN) plan.insert(plan.end(), {w, kPlanTeam, -1, -1});
+        const int nu = meta[w].num_updates;
+        if (meta[w].N0 >= kTeam4MinN) ctas.push_back({{w, kPlanTeam, -1, -1}, nu});
         else if (meta[w].N0 >= kTeamMinN) {
             if (pending < 0) pending = w;
-            else { plan.insert(plan.end(), {pending, kPlanPair, w, -1}); pending = -1; }
+            else {
+                ctas.push_back({{pending, kPlanPair, w, -1}, std::max(nu, meta[pending].num_updates)});
+                pending = -1;
+            }
         } else small.push_back(w);
     }
-    if (pending >= 0) plan.insert(plan.end(), {pending, kPlanPair, -1, -1});
-    for (size_t i = 0; i < small.size(); i += kCtaWalkers)
-        for (int k = 0; k < kCtaWalkers; ++k) plan.push_back(i + k < small.size() ? small[i + k] : -1);
-    return (int)(plan.size() / kCtaWalkers);
+    if (pending >= 0) ctas.push_back({{pending, kPlanPair, -1, -1}, meta[pending].num_updates});
+    for (size_t i = 0; i < small.size(); i += kCtaWalkers) {
+        Cta c{{-1, -1, -1, -1}, 0};
+        for (size_t k = 0; k < kCtaWalkers && i + k < small.size(); ++k) {
+            c.w[k] = small[i + k];
+            c.moves = std::max(c.moves, meta[c.w[k]].num_updates);
+        }
+        ctas.push_back(c);
+    }
+    std::stable_sort(ctas.begin(), ctas.end(), [](const Cta& a, const Cta& b) { return a.moves > b.moves; });
+    plan.clear();
+    for (const Cta& c : ctas) plan.insert(plan.end(), c.w, c.w + kCtaWalkers);
+    return (int)ctas.size();
 }
 
 // bisection levels b of ConstantParameters::initConstants
