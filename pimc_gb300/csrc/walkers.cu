@@ -296,18 +296,20 @@ __device__ __forceinline__ bool metropolis(double dV, double tau, uint32_t hi, u
 struct MetroDraw {
     double x;
     float lx;
+    int some;                        // x > 0
 };
 
 __device__ __forceinline__ MetroDraw metropolis_draw(uint32_t hi, uint32_t lo) {
     MetroDraw d;
     d.x = u01d(hi, lo);
-    d.lx = (d.x > 0.0) ? __logf((float)d.x) : 0.f;
+    d.some = d.x > 0.0;
+    d.lx = d.some ? __logf((float)d.x) : 0.f;
     return d;
 }
 
 __device__ __forceinline__ bool metropolis_ff(float hi, float lo, double tau, float tauf,
                                               const MetroDraw& d) {
-    if (d.x > 0.0) {
+    if (d.some) {
         const float diff = -(tauf * (hi + lo)) - d.lx;
         if (diff > 1e-3f) return true;
         if (diff < -1e-3f) return false;
@@ -1196,17 +1198,31 @@ k_walkers_tma(const WalkerMeta* __restrict__ meta, const int4* __restrict__ team
 // ---------------------------------------------------------------------------
 // Pipelined TMA schedule.  Teams of up to CTA/32 warps; each team owns two
 // shared-memory buffers of Mbar + 1 slab rows and two sets of bridge
-// increments.  Move descriptions come from the counter-based generator, so
-// the next staging move is known before the current one is decided: its rows
-// (both fixed ends and the moved slices) are copied into the other buffer and
-// its Gaussian increments drawn while the current move sums its pairs.  If
-// the current move is accepted and shares beads with the prefetched rows, the
-// deciding warp's write-back also patches the prefetched copy (after its copy
-// has landed), so every move reads the configuration its predecessor left.
-// A staging move costs two team barriers: one after the bridge, one before
-// the decision; warp 0 alone decides, writes back and patches while the other
-// warps wait at the next move's first barrier.  Centre-of-mass moves and
-// energy samples stream the slab through the two buffers in Mbar-row chunks.
+// increments.  Everything a move needs that does not depend on the decision
+// before it is made ahead, and by other warps than the one that decides:
+// move descriptions come from the counter-based generator, so the next
+// staging move is known before the current one is decided, and its rows (both
+// fixed ends and the moved slices) are copied into the other buffer while the
+// current move sums its pairs.  When the pairs are summed, warps 0 and 5 take
+// the decision; if the move is accepted, warp 5 writes it back and warp 0
+// patches the prefetched copy where it shares beads with the move (after the
+// copy has landed), so every move reads the configuration its predecessor
+// left; meanwhile warp 1 builds the next move's bridge (warp 0 after its
+// patch where the current move may have moved that bridge's ends), and warps
+// 2, 3 and 4 make the increments of the move after, the next acceptance draw
+// and the next description but two (a small team's last warp takes the parts
+// of the warps it lacks).  A staging move costs two team barriers: one after
+// the decision and the bridge, one before the decision.  Centre-of-mass moves
+// and energy samples stream the slab through the two buffers in Mbar-row
+// chunks.
+//
+// A chain's time is its moves' latency.  With warp 0 waiting for the rows,
+// building the bridge and making the draws itself, a staging move of the
+// largest walker of the 1024-walker mix (N = 127, M = 244, 16 warps) took
+// 6,300 clocks: wait 490, bridge 580, draws 1,730, pairs 2,090, decision
+// 1,190; now pairs 2,490, sums 240, decision and bridge 1,300.  Ten steps of
+// that walker alone 38.9 -> 34.5 ms, of the mix 47.3 -> 42.1 (schedule 6016;
+// 6008: 49.3 -> 43.0).
 // ---------------------------------------------------------------------------
 struct MoveDesc {
     int com, i, s0, len, nmove;
@@ -1239,6 +1255,70 @@ __device__ __forceinline__ void stage_increments(float4* inc, const WalkerMeta& 
     }
 }
 
+// one warp waits (bounded) for a copy of rows to land; false with the team's
+// and the walker's error set when it does not
+__device__ __forceinline__ bool rows_landed(uint64_t* bar, uint32_t parity, int lane, int* fail, int* err) {
+    long long n = 0;
+    bool landed = true;
+    while (!mbar_try_wait(bar, parity))
+        if (++n > kWaitLimit) { landed = false; break; }
+    landed = __all_sync(0xffffffffu, landed);
+    if (!landed && lane == 0) { atomicExch(fail, 1); atomicExch(err, 1); }
+    return landed;
+}
+
+// the nw warps' (hi, lo) sums added as ff_butterfly() would with zeros in the
+// other lanes; the total in lane 0
+__device__ __forceinline__ float2 team_ff(const float2* ffr, int lane, int nw) {
+    const float2 v = lane < nw ? ffr[lane] : make_float2(0.f, 0.f);
+    float hi = v.x, lo = v.y;
+    for (int o = nw >> 1; o > 0; o >>= 1) {
+        const float h2 = __shfl_xor_sync(0xffffffffu, hi, o);
+        const float l2 = __shfl_xor_sync(0xffffffffu, lo, o);
+        const float sum = hi + h2;
+        const float bp = sum - hi;
+        const float err = (hi - (sum - bp)) + (h2 - bp);
+        hi = sum;
+        lo = (lo + l2) + err;
+    }
+    return make_float2(hi, lo);
+}
+
+// One warp builds the Brownian bridge of a staging move from its copied rows
+// and its increments:
+// W_j = sum_{i<=j} sigma z_i, x_j = x0 + (j/len)(xe - x0) + W_j - (j/len) W_len
+__device__ __forceinline__ void stage_bridge(float4* sn, const float4* buf, const float4* inc, const MoveDesc& D,
+                                             int N, const WalkerMeta& m, int lane) {
+    const int len = D.len;
+    const float4 x0 = buf[D.i], xe = buf[(size_t)len * N + D.i];
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 i1 = (lane < len) ? inc[lane] : zero;
+    const float4 i2 = (lane + 32 < len) ? inc[lane + 32] : zero;
+    const float W1x = warp_scan_incl(i1.x, lane), W1y = warp_scan_incl(i1.y, lane), W1z = warp_scan_incl(i1.z, lane);
+    const float W2x = warp_scan_incl(i2.x, lane) + __shfl_sync(0xffffffffu, W1x, 31);
+    const float W2y = warp_scan_incl(i2.y, lane) + __shfl_sync(0xffffffffu, W1y, 31);
+    const float W2z = warp_scan_incl(i2.z, lane) + __shfl_sync(0xffffffffu, W1z, 31);
+    const int src = (len <= 32) ? len - 1 : len - 33;
+    const float Lx = __shfl_sync(0xffffffffu, len <= 32 ? W1x : W2x, src);
+    const float Ly = __shfl_sync(0xffffffffu, len <= 32 ? W1y : W2y, src);
+    const float Lz = __shfl_sync(0xffffffffu, len <= 32 ? W1z : W2z, src);
+    const float dx = min_image32(xe.x - x0.x, m.L, m.Linv);
+    const float dy = min_image32(xe.y - x0.y, m.L, m.Linv);
+    const float dz = min_image32(xe.z - x0.z, m.L, m.Linv);
+    const float il = 1.0f / (float)len;
+    #pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int k = lane + 32 * h;
+        if (k < D.nmove) {
+            const float f = (float)(k + 1) * il;
+            const float Wx = h ? W2x : W1x, Wy = h ? W2y : W1y, Wz = h ? W2z : W1z;
+            sn[k] = make_float4(put_inside(x0.x + fmaf(f, dx - Lx, Wx), m.L, m.Linv),
+                                put_inside(x0.y + fmaf(f, dy - Ly, Wy), m.L, m.Linv),
+                                put_inside(x0.z + fmaf(f, dz - Lz, Wz), m.L, m.Linv), 0.f);
+        }
+    }
+}
+
 template <int CTA, int MINB>
 __global__ void __launch_bounds__(CTA, MINB)
 k_walkers_pipe(const WalkerMeta* __restrict__ meta, const int4* __restrict__ teams,
@@ -1254,8 +1334,9 @@ k_walkers_pipe(const WalkerMeta* __restrict__ meta, const int4* __restrict__ tea
     __shared__ int s_fail[NW];
     __shared__ __align__(8) uint64_t s_bar[NW][2];
     // move descriptors: one warp draws them and the team reads them, a ring
-    // of three per team (move u + 2 is written while u + 1 is being read)
-    __shared__ MoveDesc s_mv[NW][3];
+    // of four per team (move u + 3 is written while u + 1 and u + 2 are read)
+    __shared__ MoveDesc s_mv[NW][4];
+    __shared__ MetroDraw s_md[NW][2];             // acceptance draws of moves u, u + 1
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int4 tm = make_int4(-1, 0, 0, 0);
     for (int k = 0; k < NW; ++k) {
@@ -1280,7 +1361,9 @@ k_walkers_pipe(const WalkerMeta* __restrict__ meta, const int4* __restrict__ tea
     auto Isel = [&](int x) { return x ? I1 : I0; };
     double* red = s_red[slot];
     float2* ffr = s_ff[slot];
-    float4* sn = s_new[slot];
+    // new positions of moves u and u + 1 (a one-warp team builds a bridge only
+    // when the move before is done with its own)
+    auto snsel = [&](int u) { return s_new[slot + (nw > 1 ? u & 1 : 0)]; };
     int* fail = &s_fail[slot];
     if (tt == 0) { mbar_init(bar0, 1); mbar_init(bar1, 1); *fail = 0; }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1296,6 +1379,7 @@ k_walkers_pipe(const WalkerMeta* __restrict__ meta, const int4* __restrict__ tea
     const int kb0 = (T >= N) ? tt / N : 0;
     const int jstep = (T >= N) ? N : T;
     int cur = 0;
+    const float tauf = (float)tau;
     // bounded wait for a copy this team issued and will not read (error path)
     auto drain = [&](int b) {
         long long n = 0;
@@ -1306,107 +1390,40 @@ k_walkers_pipe(const WalkerMeta* __restrict__ meta, const int4* __restrict__ tea
     for (int sw = 0; sw < min(sweeps, m.max_sweeps); ++sw) {
         const unsigned long long gs = sweep0 + sw;
         const uint32_t g0 = (uint32_t)gs, g1 = (uint32_t)(gs >> 32);
-        bool have = false;                        // rows of the current move already in Bsel(cur)
-        // warp 0 alone runs the generator for the move descriptors; the other
-        // warps read them from shared memory once a barrier has ordered them
-        MoveDesc D, Dn;
-        if (wi == 0) {
-            D = draw_move(0, g0, g1, m, p_com, var_updates);
-            Dn = (m.num_updates > 1) ? draw_move(1, g0, g1, m, p_com, var_updates) : D;
-            if (lane == 0) { s_mv[slot][0] = D; s_mv[slot][1] = Dn; }
-        }
+        // descriptors 0 .. 2, the increments of moves 0 and 1
+        if (wi == 0 && lane < min(3, m.num_updates)) s_mv[slot][lane] = draw_move(lane, g0, g1, m, p_com, var_updates);
         team_sync(slot, T);
-        if (wi != 0) { D = s_mv[slot][0]; Dn = s_mv[slot][1]; }
-        // the bridge increments of a staging move depend on the draws alone:
-        // those of move u + 1 are made while move u sums its pairs
+        MoveDesc D = s_mv[slot][0], Dn = D;
         if (!D.com) stage_increments(Isel(0), m, 0, g0, g1, D.len, tt, T);
-        team_sync(slot, T);
-        for (int u = 0; u < m.num_updates; ++u) {
-            const bool last = (u + 1 == m.num_updates);
-            const bool has_nn = (u + 2 < m.num_updates);
-            if (!D.com) {
-                bool pre = !last && !Dn.com;             // exact in warp 0, which issues the copies
-                const int i = D.i, s0 = D.s0, len = D.len, nmove = D.nmove;
-                // rows s0 .. s0 + len: the two fixed ends and the moved slices
-                if (tt == 0) {
-                    if (!have) issue_rows(Bsel(cur), P, N, M, s0, len + 1, barsel(cur));
-                    if (pre) issue_rows(Bsel(cur ^ 1), P, N, M, Dn.s0, Dn.len + 1, barsel(cur ^ 1));
-                }
+        for (int u = -1; u < m.num_updates; ++u) {
+            // D is move u (none at u = -1) and Dn move u + 1
+            const int v = u + 1;
+            const bool more = v < m.num_updates;
+            bool pre = false;                         // move v's rows are on their way into Bsel(cur ^ 1)
+            bool bound = true;                        // its bridge has to wait for the decision on move u
+            if (u >= 0 && !D.com) {
+                const int i = D.i, s0 = D.s0, nmove = D.nmove;
                 const float4* buf = Bsel(cur);
-                if (wi == 0) {
-                    // one warp waits for the rows and builds the Brownian bridge
-                    // W_j = sum_{i<=j} sigma z_i, x_j = x0 + (j/len)(xe - x0) + W_j - (j/len) W_len
-                    long long nwait = 0;
-                    bool landed = true;
-                    while (!mbar_try_wait(barsel(cur), phsel(cur)))
-                        if (++nwait > kWaitLimit) { landed = false; break; }
-                    landed = __all_sync(0xffffffffu, landed);
-                    if (!landed) {
-                        if (lane == 0) { atomicExch(fail, 1); atomicExch(err + w, 1); }
-                    } else {
-                        const float4 x0 = buf[i], xe = buf[(size_t)len * N + i];
-                        const float4* inc = Isel(u & 1);
-                        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-                        const float4 i1 = (lane < len) ? inc[lane] : zero;
-                        const float4 i2 = (lane + 32 < len) ? inc[lane + 32] : zero;
-                        const float W1x = warp_scan_incl(i1.x, lane), W1y = warp_scan_incl(i1.y, lane),
-                                    W1z = warp_scan_incl(i1.z, lane);
-                        const float W2x = warp_scan_incl(i2.x, lane) + __shfl_sync(0xffffffffu, W1x, 31);
-                        const float W2y = warp_scan_incl(i2.y, lane) + __shfl_sync(0xffffffffu, W1y, 31);
-                        const float W2z = warp_scan_incl(i2.z, lane) + __shfl_sync(0xffffffffu, W1z, 31);
-                        const int src = (len <= 32) ? len - 1 : len - 33;
-                        const float Lx = __shfl_sync(0xffffffffu, len <= 32 ? W1x : W2x, src);
-                        const float Ly = __shfl_sync(0xffffffffu, len <= 32 ? W1y : W2y, src);
-                        const float Lz = __shfl_sync(0xffffffffu, len <= 32 ? W1z : W2z, src);
-                        const float dx = min_image32(xe.x - x0.x, m.L, m.Linv);
-                        const float dy = min_image32(xe.y - x0.y, m.L, m.Linv);
-                        const float dz = min_image32(xe.z - x0.z, m.L, m.Linv);
-                        const float il = 1.0f / (float)len;
-                        #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const int k = lane + 32 * h;
-                            if (k < nmove) {
-                                const float f = (float)(k + 1) * il;
-                                const float Wx = h ? W2x : W1x, Wy = h ? W2y : W1y, Wz = h ? W2z : W1z;
-                                sn[k] = make_float4(put_inside(x0.x + fmaf(f, dx - Lx, Wx), m.L, m.Linv),
-                                                    put_inside(x0.y + fmaf(f, dy - Ly, Wy), m.L, m.Linv),
-                                                    put_inside(x0.z + fmaf(f, dz - Lz, Wz), m.L, m.Linv), 0.f);
-                            }
-                        }
-                    }
-                }
-                phflip(cur);
-                team_sync(slot, T);
-                // move u + 1 was written by warp 0 during move u - 1 (or at the
-                // start of the sweep); the barrier above orders it
-                if (wi != 0) Dn = s_mv[slot][(u + 1) % 3];
-                pre = !last && !Dn.com;
-                if (*(volatile int*)fail) {
-                    if (tt == 0 && pre) drain(cur ^ 1);
-                    return;
-                }
-                // while the pairs are summed: the next move's increments, the
-                // move after it (drawn by the team's last warp, which waits at
-                // the barriers rather than leading the critical path), and this
-                // move's acceptance draw
-                if (pre) stage_increments(Isel((u + 1) & 1), m, u + 1, g0, g1, Dn.len, tt, T);
-                MoveDesc Dnn = Dn;
-                if (wi == nw - 1 && has_nn) {
-                    Dnn = draw_move(u + 2, g0, g1, m, p_com, var_updates);
-                    if (lane == 0) s_mv[slot][(u + 2) % 3] = Dnn;
-                }
-                MetroDraw md{0.0, 0.f};
-                if (tt == 0) {
-                    const uint4 ra = wrand(m.key, (uint32_t)u, g0, g1, 0xFFFFu);
-                    md = metropolis_draw(ra.x, ra.y);
+                const float4* sn = snsel(u);
+                pre = more && !Dn.com;
+                if (pre) {
+                    // rows s0 .. s0 + len: the two fixed ends and the moved slices
+                    if (wi == nw - 1 && lane == 0)
+                        issue_rows(Bsel(cur ^ 1), P, N, M, Dn.s0, Dn.len + 1, barsel(cur ^ 1));
+                    auto moves = [&](int t) {
+                        int q = t - s0; if (q < 0) q += M;
+                        return q >= 1 && q <= nmove;
+                    };
+                    int se = Dn.s0 + Dn.len; if (se >= M) se -= M;
+                    bound = Dn.i == i && (moves(Dn.s0) || moves(se));
                 }
                 KahanF acc;
                 for (int j = j0; j < N; j += jstep) {
                     if (j == i) continue;
                     #pragma unroll 4
                     for (int k = kb0; k < nmove; k += G) {
-                        const float4 pj = buf[(size_t)(k + 1) * N + j];
-                        const float4 a = sn[k], b = buf[(size_t)(k + 1) * N + i];
+                        const float4* row = buf + (k + 1) * N;
+                        const float4 pj = row[j], a = sn[k], b = row[i];
                         const float ax = min_image32(a.x - pj.x, m.L, m.Linv);
                         const float ay = min_image32(a.y - pj.y, m.L, m.Linv);
                         const float az_ = min_image32(a.z - pj.z, m.L, m.Linv);
@@ -1420,58 +1437,40 @@ k_walkers_pipe(const WalkerMeta* __restrict__ meta, const int4* __restrict__ tea
                 const float2 part = warp_ff(acc);
                 if (lane == 0) ffr[wi] = part;
                 team_sync(slot, T);
-                if (wi == 0) {
-                    // the decision, the write-back and the patch belong to one warp;
-                    // the others go on to the next move's barrier
-                    if (has_nn && nw > 1) Dnn = s_mv[slot][(u + 2) % 3];
-                    const float2 v = ff_butterfly(lane < nw ? ffr[lane].x : 0.f, lane < nw ? ffr[lane].y : 0.f);
+                // two warps take the same decision: warp 0 patches the
+                // prefetched rows, the other (warp 0 too in a small team)
+                // writes back
+                const int wb = nw > 5 ? 5 : 0;
+                if (wi == 0 || wi == wb) {
+                    const float2 x = team_ff(ffr, lane, nw);
                     int ok = 0;
-                    if (lane == 0) {
-                        ok = metropolis_ff(v.x, v.y, tau, (float)tau, md) ? 1 : 0;
-                        att1 += 1; acc1 += ok; nbu += nmove;
-                    }
+                    if (lane == 0) ok = metropolis_ff(x.x, x.y, tau, tauf, s_md[slot][u & 1]) ? 1 : 0;
                     ok = __shfl_sync(0xffffffffu, ok, 0);
-                    if (ok) {
+                    if (ok && wi == wb) {
                         for (int k = lane; k < nmove; k += 32) {
                             int sl = s0 + 1 + k; if (sl >= M) sl -= M;
                             P[(size_t)sl * N + i] = sn[k];
                         }
                         fence_proxy_async_global();
-                        if (pre) {
-                            // the prefetched rows must have landed before they are patched
-                            long long n = 0;
-                            bool landed = true;
-                            while (!mbar_try_wait(barsel(cur ^ 1), phsel(cur ^ 1)))
-                                if (++n > kWaitLimit) { landed = false; break; }
-                            landed = __all_sync(0xffffffffu, landed);
-                            if (!landed) {
-                                if (lane == 0) { atomicExch(fail, 1); atomicExch(err + w, 1); }
-                            } else {
-                                float4* nb = Bsel(cur ^ 1);
-                                for (int k = lane; k < nmove; k += 32) {
-                                    int sl = s0 + 1 + k; if (sl >= M) sl -= M;
-                                    int q = sl - Dn.s0; if (q < 0) q += M;
-                                    if (q <= Dn.len) nb[(size_t)q * N + i] = sn[k];
-                                }
-                                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                            }
-                        }
                     }
+                    if (ok && wi == 0 && pre && rows_landed(barsel(cur ^ 1), phsel(cur ^ 1), lane, fail, err + w)) {
+                        // (the prefetched rows must have landed before they are patched)
+                        float4* nb = Bsel(cur ^ 1);
+                        for (int k = lane; k < nmove; k += 32) {
+                            int sl = s0 + 1 + k; if (sl >= M) sl -= M;
+                            int q = sl - Dn.s0; if (q < 0) q += M;
+                            if (q <= Dn.len) nb[(size_t)q * N + i] = sn[k];
+                        }
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    }
+                    if (tt == 0) { att1 += 1; acc1 += ok; nbu += nmove; }
                     __syncwarp();
                 }
-                if (pre) { cur ^= 1; have = true; } else { have = false; }
-                D = Dn;
-                Dn = Dnn;
-            } else {
+            } else if (u >= 0) {
                 const int i = D.i;
                 const float sx = D.sx, sy = D.sy;
                 const uint4 r1 = wrand(m.key, (uint32_t)u, g0, g1, 0xFFFEu);
                 const float sz = m.com_delta * (u01f(r1.x) - 0.5f);
-                MoveDesc Dnn = Dn;
-                if (wi == nw - 1 && has_nn) {
-                    Dnn = draw_move(u + 2, g0, g1, m, p_com, var_updates);
-                    if (lane == 0) s_mv[slot][(u + 2) % 3] = Dnn;
-                }
                 KahanF acc;
                 int b = cur;
                 if (tt == 0) issue_rows(Bsel(b), P, N, M, 0, min(C, M), barsel(b));
@@ -1507,17 +1506,11 @@ k_walkers_pipe(const WalkerMeta* __restrict__ meta, const int4* __restrict__ tea
                 if (lane == 0) ffr[wi] = part;
                 team_sync(slot, T);
                 if (wi == 0) {
-                    const float2 v = ff_butterfly(lane < nw ? ffr[lane].x : 0.f, lane < nw ? ffr[lane].y : 0.f);
-                    if (lane == 0) s_acc[slot] = metropolis((double)v.x + (double)v.y, tau, r1.y, r1.z) ? 1 : 0;
+                    const float2 x = team_ff(ffr, lane, nw);
+                    if (lane == 0) s_acc[slot] = metropolis((double)x.x + (double)x.y, tau, r1.y, r1.z) ? 1 : 0;
                 }
                 team_sync(slot, T);
                 const int ok = s_acc[slot];
-                // move u + 1 (written during move u - 1 or at the sweep start)
-                // and its bridge increments, before this move's last barrier;
-                // warp 0 also takes move u + 2
-                if (wi != 0) Dn = s_mv[slot][(u + 1) % 3];
-                if (wi == 0 && has_nn && nw > 1) Dnn = s_mv[slot][(u + 2) % 3];
-                if (!last && !Dn.com) stage_increments(Isel((u + 1) & 1), m, u + 1, g0, g1, Dn.len, tt, T);
                 if (ok) {
                     for (int t2 = tt; t2 < M; t2 += T) {
                         float4 pi = P[(size_t)t2 * N + i];
@@ -1530,10 +1523,40 @@ k_walkers_pipe(const WalkerMeta* __restrict__ meta, const int4* __restrict__ tea
                 }
                 team_sync(slot, T);
                 att0 += 1; acc0 += ok; nbu += M;
-                have = false;
-                D = Dn;
-                Dn = Dnn;
+            } else {
+                team_sync(slot, T);                   // the first move's increments
             }
+            // move v made ready.  Its increments were made one window earlier.
+            const int nb = pre ? cur ^ 1 : cur;
+            const bool staged = more && !Dn.com;
+            if (staged) {
+                if (!pre && tt == 0) issue_rows(Bsel(nb), P, N, M, Dn.s0, Dn.len + 1, barsel(nb));
+                if (wi == (bound || nw == 1 ? 0 : 1) &&
+                    rows_landed(barsel(nb), phsel(nb), lane, fail, err + w))
+                    stage_bridge(snsel(v), Bsel(nb), Isel(v & 1), Dn, N, m, lane);
+            }
+            if (v + 1 < m.num_updates && wi == (nw > 2 ? 2 : nw - 1)) {
+                const MoveDesc Dv = s_mv[slot][(v + 1) & 3];
+                if (!Dv.com) stage_increments(Isel((v + 1) & 1), m, v + 1, g0, g1, Dv.len, lane, 32);
+            }
+            if (staged && wi == (nw > 3 ? 3 : nw - 1) && lane == 0) {
+                const uint4 ra = wrand(m.key, (uint32_t)v, g0, g1, 0xFFFFu);
+                s_md[slot][v & 1] = metropolis_draw(ra.x, ra.y);
+            }
+            if (v + 2 < m.num_updates && v + 2 > 2 && wi == (nw > 4 ? 4 : nw - 1) && lane == 0)
+                s_mv[slot][(v + 2) & 3] = draw_move(v + 2, g0, g1, m, p_com, var_updates);
+            team_sync(slot, T);
+            if (staged) {
+                if (*(volatile int*)fail) {
+                    // one more bounded wait for the copy before the team leaves
+                    if (tt == 0) drain(nb);
+                    return;
+                }
+                phflip(nb);
+                cur = nb;
+            }
+            D = Dn;
+            Dn = s_mv[slot][(v + 1) & 3];
         }
         if (measure > 0 && ((gs + 1) % (unsigned long long)measure) == 0) {
             KahanF pot, kin;
@@ -1718,7 +1741,7 @@ k_walkers_group(const WalkerMeta* __restrict__ meta, const int4* __restrict__ te
                 float2* const ffr = s_ff[slot + sg * qw];
                 uint64_t* const bar = &s_bar[slot][active ? sg : 0];
                 auto gsync = [&]() { if (gsize == 1) team_sync(slot, T); else sub_sync(slot, sg, HT); };
-                MetroDraw md{0.0, 0.f};
+                MetroDraw md{0.0, 0.f, 0};
                 if (active) {
                     // rows s0 .. s0 + len, increments and the acceptance draw
                     if (ht == 0) issue_rows(buf, P, N, M, s0, len + 1, bar);
