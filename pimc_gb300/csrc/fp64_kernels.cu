@@ -906,23 +906,35 @@ cudaError_t launch_slice_terms64(const PathView& v, int window, int even, int od
 // where sincos and the phase take about seventy, and the FP64 pipe (16 clocks
 // of an SM a warp instruction) is the bound.  A list that enumerates a grid
 // symmetric about 0 has -q at the mirrored place; its density is the complex
-// conjugate and is written, not summed.  Thread i takes vectors i and
-// nq - 1 - i.  Other vectors (shells) take the sine and cosine of q . r.
-// 64 beads, 124 slices, 389 vectors with |q| < 2 in mirrored order: 219 -> 52 us;
-// 128 beads, 250 slices, 300 lattice vectors in no order: 623 -> 230 us (ncu,
-// cold).  Relative error against 113-bit phases, before and now: 4e-16 and
+// conjugate and is written, not summed.  Other vectors (shells) take the sine
+// and cosine of q . r.
+//
+// A cluster of CTAs shares a slice's beads, each with all the vectors and a
+// table of its own beads' powers, and adds the parts through distributed
+// shared memory: slices are too few and too long to even out over the SMs
+// (250 on 152: two on some, one on others), and a table built by every CTA
+// that takes some of the vectors is built twice.
+// 64 beads, 124 slices, 389 vectors with |q| < 2 in mirrored order: 219 us with
+// a sine a term, 57 with a CTA a slice and 128 pairs of vectors, 44 now; 128
+// beads, 250 slices, 300 lattice vectors in no order: 623, 229, 187 (ncu,
+// cold).  Relative error against 113-bit phases, sines and now: 4e-16 and
 // 7e-16, 6e-16 and 5e-16, at 500 beads 2.4e-15 and 2.0e-15; of F(q,tau) 2e-16
 // both.
 // ---------------------------------------------------------------------------
-constexpr int kRhoThreads = 128;                 // one warp a sub-partition
+constexpr int kRhoThreads = 512;                 // vectors a CTA at most
+constexpr int kRhoLeast = 128;                   // threads at least: few vectors share the beads out
 constexpr int kRhoPowers = 64;                   // largest |n_d| of the table form
-constexpr int kRhoSmem = 96 * 1024;              // two CTAs an SM
+constexpr int kRhoSmem = 48 * 1024;              // four CTAs an SM
+constexpr int kRhoCluster = 4;
+constexpr int kRhoBeads = 16;                    // a CTA has at least
+
+// 2 pi / L and L / 2 pi
+struct Lattice { double step[3], turn[3]; };
 
 // n_d when q_d is 2 pi n_d / L_d to rounding, else kRhoPowers + 1
-__device__ __forceinline__ int lattice_index(double q, double L) {
-    const double kTwoPi = 6.283185307179586476925;
-    const double n = rint(q * L / kTwoPi);
-    const bool ok = fabs(n) <= (double)kRhoPowers && fabs(q - n * (kTwoPi / L)) <= 1.0e-15 * fabs(q);
+__device__ __forceinline__ int lattice_index(double q, double step, double turn) {
+    const double n = rint(q * turn);
+    const bool ok = fabs(n) <= (double)kRhoPowers && fabs(q - n * step) <= 1.0e-15 * fabs(q);
     return ok ? (int)n : kRhoPowers + 1;
 }
 
@@ -933,121 +945,110 @@ __device__ __forceinline__ double2 power_of(const double2* E, int n) {
     return e;
 }
 
+// blockDim.x = wide * parts; thread slot + wide * part has vector slot of the
+// CTA's vectors and every parts-th of its beads
 __global__ void __launch_bounds__(kRhoThreads)
-k_rhoq64(PathView v, const double* __restrict__ q, int nq, double maxR2, double* __restrict__ rho) {
+k_rhoq64(PathView v, const double* __restrict__ q, int nq, Lattice lat, double maxR2, int wide, int csize,
+         double* __restrict__ rho) {
     extern __shared__ double2 E[];               // [bead][dimension][power]
     __shared__ int s_max;
-    __shared__ double2 half[2][kRhoThreads];
-    const int t = blockIdx.x, tid = threadIdx.x, n = v.nbs[t];
-    // few vectors: several parts of the beads a vector
-    const int slots = (nq + 1) / 2, first = blockIdx.y * kRhoThreads, mine = min(kRhoThreads, slots - first);
-    const int wide = mine > 64 ? 128 : mine > 32 ? 64 : 32, parts = kRhoThreads / wide;
-    const int sl = tid & (wide - 1), part = tid / wide;
-    const int iq = first + sl, jq = nq - 1 - iq;
-    const bool live = sl < mine;
+    const int t = blockIdx.x / csize, rank = blockIdx.x - t * csize, tid = threadIdx.x, T = blockDim.x;
+    const int parts = T / wide, part = tid / wide, n = v.nbs[t];
+    const int b0 = (int)((long long)n * rank / csize), b1 = (int)((long long)n * (rank + 1) / csize);
+    const int i = blockIdx.y * wide + tid - part * wide, j = nq - 1 - i;
     const double* X = v.pos + (size_t)t * 3 * v.Ne;
-    int ka[3] = {0, 0, 0}, kb[3] = {0, 0, 0};
-    bool mirrored = true, second = false;
+    bool live = i < nq, mirrored = live;
+    int k[3] = {0, 0, 0};
     if (tid == 0) s_max = 0;
     __syncthreads();
     if (live) {
-        second = jq != iq;
+        double a[3];
+        #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            const double a = q[3 * iq + d], b = q[3 * jq + d];
-            mirrored = mirrored && a == -b;
-            ka[d] = lattice_index(a, v.side[d]);
-            kb[d] = lattice_index(b, v.side[d]);
+            a[d] = q[3 * i + d];
+            mirrored = mirrored && a[d] == -q[3 * j + d];
         }
+        live = i <= j || !mirrored;              // the other half of a mirrored pair writes both
+        #pragma unroll
+        for (int d = 0; d < 3; ++d)
+            if (live) k[d] = lattice_index(a[d], lat.step[d], lat.turn[d]);
     }
-    auto top = [](const int* k) { return max(abs(k[0]), max(abs(k[1]), abs(k[2]))); };
-    const bool latA = live && top(ka) <= kRhoPowers;
-    const bool sumB = live && second && !mirrored, latB = sumB && top(kb) <= kRhoPowers;
-    const int most = max(latA ? top(ka) : -1, latB ? top(kb) : -1);
-    if (most >= 0) atomicMax(&s_max, most + 1);
+    const int most = max(abs(k[0]), max(abs(k[1]), abs(k[2])));
+    const bool powers = live && most <= kRhoPowers;
+    const int warp_most = __reduce_max_sync(0xffffffffu, powers ? most + 1 : 0);
+    if ((tid & 31) == 0 && warp_most) atomicMax(&s_max, warp_most);
     __syncthreads();
-    double2 A = make_double2(0.0, 0.0), B = A;
+    double2 S = make_double2(0.0, 0.0);
     const int np = s_max;                        // powers 0 .. np - 1; 0: no lattice vector here
     if (np > 0) {
         const int chunk = max(parts, kRhoSmem / (3 * np * (int)sizeof(double2)));
-        const bool any = __any_sync(0xffffffffu, latA), two = __any_sync(0xffffffffu, latB);
-        for (int j0 = 0; j0 < n; j0 += chunk) {
-            const int nj = min(chunk, n - j0);
+        for (int j0 = b0; j0 < b1; j0 += chunk) {
+            const int nj = min(chunk, b1 - j0);
             __syncthreads();
-            for (int x = tid; x < 3 * nj; x += kRhoThreads) {
-                const int d = x / nj, j = x - d * nj;
-                const double r = X[d * v.Ne + j0 + j];
-                double2* e = E + (size_t)(3 * j + d) * np;
+            for (int x = tid; x < 3 * nj; x += T) {
+                const int d = x / nj, p = x - d * nj;
+                const double r = X[d * v.Ne + j0 + p];
+                double2* e = E + (size_t)(3 * p + d) * np;
                 double sn, cs;
                 sincospi(2.0 * (r * v.sideInv[d]), &sn, &cs);
                 // cylinder restriction: beads outside x^2 + y^2 < maxR^2 count 0
-                const double rx = X[j0 + j], ry = X[v.Ne + j0 + j];
+                const double rx = X[j0 + p], ry = X[v.Ne + j0 + p];
                 const double one = (d == 0 && maxR2 > 0.0 && !(rx * rx + ry * ry < maxR2)) ? 0.0 : 1.0;
                 e[0] = make_double2(one, 0.0);
                 if (np > 1) e[1] = make_double2(one * cs, one * sn);
-                for (int k = 2; k < np; ++k) {
-                    const double2 a = e[k >> 1], b = e[k - (k >> 1)];
-                    e[k] = make_double2(__fma_rn(a.x, b.x, -(a.y * b.y)), __fma_rn(a.x, b.y, a.y * b.x));
+                for (int h = 2; h < np; ++h) {
+                    const double2 a = e[h >> 1], b = e[h - (h >> 1)];
+                    e[h] = make_double2(__fma_rn(a.x, b.x, -(a.y * b.y)), __fma_rn(a.x, b.y, a.y * b.x));
                 }
             }
             __syncthreads();
-            if (any && two) {
-                for (int j = part; j < nj; j += parts) {
-                    const double2* e = E + (size_t)3 * j * np;
-                    if (latA) {
-                        const double2 x = power_of(e, ka[0]), y = power_of(e + np, ka[1]), z = power_of(e + 2 * np, ka[2]);
-                        const double cr = __fma_rn(y.x, z.x, -(y.y * z.y)), ci = __fma_rn(y.x, z.y, y.y * z.x);
-                        A.x = __fma_rn(x.x, cr, __fma_rn(-x.y, ci, A.x));
-                        A.y = __fma_rn(x.x, ci, __fma_rn(x.y, cr, A.y));
-                    }
-                    if (latB) {
-                        const double2 x = power_of(e, kb[0]), y = power_of(e + np, kb[1]), z = power_of(e + 2 * np, kb[2]);
-                        const double cr = __fma_rn(y.x, z.x, -(y.y * z.y)), ci = __fma_rn(y.x, z.y, y.y * z.x);
-                        B.x = __fma_rn(x.x, cr, __fma_rn(-x.y, ci, B.x));
-                        B.y = __fma_rn(x.x, ci, __fma_rn(x.y, cr, B.y));
-                    }
+            if (powers)
+                for (int p = part; p < nj; p += parts) {
+                    const double2* e = E + (size_t)3 * p * np;
+                    const double2 x = power_of(e, k[0]), y = power_of(e + np, k[1]), z = power_of(e + 2 * np, k[2]);
+                    const double cr = __fma_rn(y.x, z.x, -(y.y * z.y)), ci = __fma_rn(y.x, z.y, y.y * z.x);
+                    S.x = __fma_rn(x.x, cr, __fma_rn(-x.y, ci, S.x));
+                    S.y = __fma_rn(x.x, ci, __fma_rn(x.y, cr, S.y));
                 }
-            } else if (any || two) {
-                const bool lat = any ? latA : latB;
-                const int k0 = any ? ka[0] : kb[0], k1 = any ? ka[1] : kb[1], k2 = any ? ka[2] : kb[2];
-                double2 S = make_double2(0.0, 0.0);
-                if (lat)
-                    for (int j = part; j < nj; j += parts) {
-                        const double2* e = E + (size_t)3 * j * np;
-                        const double2 x = power_of(e, k0), y = power_of(e + np, k1), z = power_of(e + 2 * np, k2);
-                        const double cr = __fma_rn(y.x, z.x, -(y.y * z.y)), ci = __fma_rn(y.x, z.y, y.y * z.x);
-                        S.x = __fma_rn(x.x, cr, __fma_rn(-x.y, ci, S.x));
-                        S.y = __fma_rn(x.x, ci, __fma_rn(x.y, cr, S.y));
-                    }
-                if (any) { A.x += S.x; A.y += S.y; } else { B.x += S.x; B.y += S.y; }
-            }
         }
     }
-    auto direct = [&](int i, double2& S) {
+    if (live && !powers) {
         const double qx = q[3 * i], qy = q[3 * i + 1], qz = q[3 * i + 2];
-        for (int j = part; j < n; j += parts) {
-            if (maxR2 > 0.0 && !(X[j] * X[j] + X[v.Ne + j] * X[v.Ne + j] < maxR2)) continue;
+        for (int p = b0 + part; p < b1; p += parts) {
+            if (maxR2 > 0.0 && !(X[p] * X[p] + X[v.Ne + p] * X[v.Ne + p] < maxR2)) continue;
             double ph = 0.0;
-            ph += qx * X[j]; ph += qy * X[v.Ne + j]; ph += qz * X[2 * v.Ne + j];
+            ph += qx * X[p]; ph += qy * X[v.Ne + p]; ph += qz * X[2 * v.Ne + p];
             double sn, cs;
             sincos(ph, &sn, &cs);
             S.x += cs; S.y += sn;
         }
-    };
-    if (live && !latA) direct(iq, A);
-    if (sumB && !latB) direct(jq, B);
-    if (parts > 1) {                             // uniform over the CTA
-        half[0][tid] = A; half[1][tid] = B;
-        __syncthreads();
-        if (part) return;
-        for (int k = 1; k < parts; ++k) {
-            const double2 a = half[0][tid + k * wide], b = half[1][tid + k * wide];
-            A.x += a.x; A.y += a.y; B.x += b.x; B.y += b.y;
-        }
     }
-    if (!live) return;
     double2* R = reinterpret_cast<double2*>(rho);
-    R[(size_t)iq * v.M + t] = A;
-    if (second) R[(size_t)jq * v.M + t] = mirrored ? make_double2(A.x, -A.y) : B;
+    auto write = [&](double2 A) {
+        R[(size_t)i * v.M + t] = A;
+        if (mirrored && i < j) R[(size_t)j * v.M + t] = make_double2(A.x, -A.y);
+    };
+    if (parts * csize == 1) {
+        if (live) write(S);
+        return;
+    }
+    // the parts, then the CTAs, added in order; the CTAs take turns at the vectors
+    __syncthreads();
+    E[tid] = S;
+    if (csize > 1) cg::this_cluster().sync();
+    else __syncthreads();
+    if (live && part == 0 && (tid / 32) % csize == rank) {
+        S = make_double2(0.0, 0.0);
+        for (int r = 0; r < csize; ++r) {
+            const double2* Er = csize > 1 ? cg::this_cluster().map_shared_rank(E, r) : E;
+            for (int h = 0; h < parts; ++h) {
+                const double2 a = Er[tid + h * wide];
+                S.x += a.x; S.y += a.y;
+            }
+        }
+        write(S);
+    }
+    if (csize > 1) cg::this_cluster().sync();    // no CTA leaves while another reads its part
 }
 
 cudaError_t launch_rhoq64(const PathView& v, const double* d_q, int nq, double* d_rho,
@@ -1055,9 +1056,30 @@ cudaError_t launch_rhoq64(const PathView& v, const double* d_q, int nq, double* 
     if (nq < 1) return cudaSuccess;
     const cudaError_t ae = set_smem_limit(k_rhoq64, kRhoSmem);
     if (ae != cudaSuccess) return ae;
-    const int slots = (nq + 1) / 2;
-    k_rhoq64<<<dim3(v.M, (slots + kRhoThreads - 1) / kRhoThreads), kRhoThreads, kRhoSmem, s>>>(v, d_q, nq, maxR2, d_rho);
-    return cudaGetLastError();
+    const int sets = (nq + kRhoThreads - 1) / kRhoThreads, each = (nq + sets - 1) / sets;
+    const int wide = (each + 31) / 32 * 32, parts = std::max(1, kRhoLeast / wide);
+    // rounds of the SMs, in units of a whole slice: a cluster costs two
+    // barriers and a table each, so it has to gain (124 slices of 64 beads, one
+    // round either way: 357 us a sample with one CTA a slice, 367 with two,
+    // 390 with four; 250 of 128: 464 with two, 439 with four)
+    auto rounds = [&](int c) { return (double)(((long long)v.M * sets * c + 151) / 152) / c; };
+    int c = 1;
+    for (int d = 2; d <= kRhoCluster && d * kRhoBeads <= v.Ne; d *= 2)
+        if (rounds(d) < 0.95 * rounds(c)) c = d;
+    Lattice lat;
+    const double kTwoPi = 6.283185307179586476925;
+    for (int d = 0; d < 3; ++d) { lat.step[d] = kTwoPi / v.side[d]; lat.turn[d] = v.side[d] / kTwoPi; }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)v.M * c, (unsigned)sets);
+    cfg.blockDim = dim3(wide * parts);
+    cfg.dynamicSmemBytes = kRhoSmem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = c; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = c > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_rhoq64, v, d_q, nq, lat, maxR2, wide, c, d_rho);
 }
 
 // F(q,tau) = norm * sum_t Re(rho_t conj(rho_{t+tau})), tau in [0, M/2].  One
