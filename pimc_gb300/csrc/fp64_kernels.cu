@@ -1,8 +1,10 @@
 // fp64_kernels.cu -- the FP64 "plain form" kernels.
 //
 // Compiled with -fmad=false: every multiply and add rounds once, in the order
-// the reference writes it, so each pair term equals the oracle's bit for bit
-// and totals differ only through summation order (parallel reductions).
+// it is written, and fused operations are spelt out.  The tables, the direct
+// pair form and the path arithmetic keep the reference's order; the fast pair
+// form (pair64.cuh) rounds differently in the last bit or two, and totals
+// differ through that and through summation order (parallel reductions).
 #include <cooperative_groups.h>
 
 #include "pair64.cuh"
@@ -181,8 +183,9 @@ __device__ __forceinline__ bool worm_on_slice(const PathView& v, int s) {
 // Bound: the FP64 pipe, about 27 instructions a pair, 16 clocks of an SM a
 // warp instruction.  31 beads of a 64-particle GSF path (a bisection's range):
 // 173 us with one thread a member and every ordered pair in the direct form,
-// 15.6 us here; as trials 2 x 173 and 21.6 us.  kBoth evaluates the trial and the current position of the
-// bead over one pass of the members' pairs, and writes the difference.
+// 15.6 us here; as trials 2 x 173 and 21.6 us.  kBoth evaluates the trial and
+// the current position of the bead over one pass of the members' pairs, and
+// writes the difference.
 // ---------------------------------------------------------------------------
 constexpr int kMaxCluster = 8;
 
@@ -475,9 +478,12 @@ k_bead_warp64(PathView v, double invdr, const int2* __restrict__ beads, int k, B
     }
 }
 
-// From kManyBeads on the warp form is the faster: below, it leaves warps idle
-// (a GSF call also needs the forces of all slices first).
-constexpr int kManyBeads = 1216;                 // two beads a sub-partition of 152 SMs
+// From here on the warp form is the faster; below, it leaves warps idle, and a
+// GSF call needs the forces of all slices first.  Whole calls, clusters against
+// warps: primitive, 64 beads a slice, 1824 beads 45 and 46 us, 2432 63 and 54
+// (128 beads a slice: 50 and 59, 63 and 68, 4864 105 and 79); GSF, 608 beads 89
+// and 83 us, 912 98 and 84 (269 and 290, 280 and 292, 1216 349 and 292).
+constexpr int kManyBeads = 2048, kManyGradient = 912;
 
 template <bool kBoth>
 static cudaError_t bead_pairs64(const PathView& v, const int2* d_beads, int k, const BeadSpec& a, bool corr,
@@ -625,7 +631,7 @@ static bool has_corr(int shift, int mode, const double gf[2]) {
 static bool bead_warp64(const PathView& v, const int2* d_beads, int k, const BeadSpec& a, bool corr,
                         const double* d_over, double* d_force, double* d_out, cudaStream_t s, cudaError_t* e) {
     const size_t fsmem = (size_t)v.Ne * (3 * sizeof(double) + 3 * sizeof(float));
-    if (k < kManyBeads || (corr && (!d_force || fsmem > 200 * 1024))) return false;
+    if (k < (corr ? kManyGradient : kManyBeads) || (corr && (!d_force || fsmem > 200 * 1024))) return false;
     if (corr) {
         if ((*e = set_smem_limit(k_slice_forces64, 200 * 1024)) != cudaSuccess) return true;
         k_slice_forces64<<<dim3(v.M, (v.Ne + kForceRows - 1) / kForceRows), kPairBlock, fsmem, s>>>(

@@ -161,7 +161,7 @@ cudaError_t launch_potential_batch64(const PathView& v, const double* d_sep,
                                      cudaStream_t s);
 // `whole`: the cutoff takes in every separation, so a bead's list is its whole
 // slice; d_force: room for the FP64 slice forces [M][3][Ne], needed from
-// kManyBeads beads on with a gradient term
+// kManyGradient beads on with a gradient term
 cudaError_t launch_bead_actions64(const PathView& v, const int2* d_beads, int k,
                                   int shift, int mode, double tau, double lambda,
                                   const double vf[2], const double gf[2],

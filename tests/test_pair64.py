@@ -12,7 +12,8 @@ from helpers import make_pair, rel_err
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [(9, 8, 3), (33, 6, 31), (64, 6, 40), (65, 4, 160), (257, 4, 5), (40, 4, 1215), (40, 4, 1216), (70, 4, 2000)]
+SIZES = [(9, 8, 3), (33, 6, 31), (64, 6, 40), (65, 4, 160), (257, 4, 5), (40, 4, 911), (40, 4, 912), (40, 4, 1216),
+         (70, 4, 2047), (70, 4, 2048)]
 
 
 def _setup(pgb, oracle_lib, n, m, rc, worm, shift_box=0.0):
