@@ -565,7 +565,7 @@ def run_isf(args, pgb):
                         "note": "2 special-function ops (sin, cos) per phase evaluation, Q M N of "
                                 "them, over the S(q) call time (rho_q + an O(Q M) reduction); peak "
                                 "= nominal %d/clk/SM x SMs x median SM clock" % SFU_PER_SM_CLK},
-           "roofline_correlation": {"bound": "tensor", "kernel": "k_gemm_split_bf16 + split/prep kernels",
+           "roofline_correlation": {"bound": "tensor", "kernel": "k_gemm_split_bf16",
                                     "achieved": corr_flops / t_corr / 1e12, "peak": bf16,
                                     "unit": "TFLOP/s", "frac": corr_flops / t_corr / 1e12 / bf16,
                                     "note": "algorithmic 2 M^2 2Q FLOP of the correlation over "
@@ -703,7 +703,7 @@ def run_pair(args, pgb):
     err["note"] = ("trial-move action differences dU of 256 of the trials and the full-path action "
                    "against the FP64 oracle")
     mx = res["mixed"]
-    roof = pair_roofline(mx.pop("_pv"), mx.pop("_pvg"), mx.pop("_t"), "k_bead_actions32_full",
+    roof = pair_roofline(mx.pop("_pv"), mx.pop("_pvg"), mx.pop("_t"), "k_trials32",
                          measured_fp32_peak(), clocks.get("sm_mhz"))
     for r in res.values():
         for key in ("_pv", "_pvg", "_t"):
