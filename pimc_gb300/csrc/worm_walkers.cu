@@ -37,10 +37,10 @@
 // (testsOf()) and taken out again (dropBeads()) by the lanes together; (4)
 // the heavy helpers are not inlined and loops are not unrolled: a walker's
 // warps wait for instructions more than for anything else; (5) CTAs start in
-// the order of their walkers' moves a step; (6) a move's normal deviates come from the
-// lanes together (normals()), from the same words as serial draws; (7) FP64
-// instructions are few: each holds a quarter of an SM for 64 clocks, so
-// constants are rounded once on the host and sums widened by lanes.
+// the order of their walkers' moves a step; (6) a move's normal deviates come
+// from the lanes together (normals()), from the same words as serial draws;
+// (7) FP64 instructions are few: each holds a quarter of an SM for 64 clocks,
+// so constants are rounded once on the host and sums widened by lanes.
 // Walking, testing and removing bead by bead with the FP64 logarithms and
 // quotients in the moves 1024 walkers took 52.5 ms for four steps, the
 // largest of them alone 44.0; so, 40.1 and 32.3; with eight warps a CTA
@@ -159,15 +159,9 @@ __device__ __forceinline__ void team_sync(int id, int nthreads) {
     else asm volatile("bar.sync 4, %0;" ::"r"(nthreads) : "memory");
 }
 
-// Aziz V with the reference's hard-core branch (potential.cpp:1821-1843):
-// below x = 0.01 the attractive part is dropped
-__device__ __forceinline__ float aziz_v32_core(float r2, const AzizF& a) {
-    const float x = sqrtf(r2) * a.rminv;
-    if (x < 0.01f) return a.eps * a.A * __expf(x * fmaf(a.beta, x, -a.alpha));
-    return aziz_v32(r2, a);
-}
-// the same without branches, so that the pair terms of a lane schedule
-// together: below x = 0.01 the attractive terms are selected away
+// Aziz V with the reference's hard-core branch (potential.cpp:1821-1843:
+// below x = 0.01 the attractive part is dropped), without branches, so that
+// the pair terms of a lane schedule together
 __device__ __forceinline__ float aziz_v32_sel(float r2, const AzizF& a) {
     const float rinv = rsqrtf(r2);
     const float x = r2 * rinv * a.rminv;
@@ -239,7 +233,7 @@ struct WormWalker {
     // FP64 transcendentals are slow on this GPU
     __device__ float rand() { return (float)u32() * 2.3283064365386963e-10f; }
     __device__ float randExc() { return (float)(u32() >> 8) * 5.9604644775390625e-08f; }
-    // polar-method deviate z; randNorm(mean, sd) is mean + z * sd
+    // polar-method deviate
     __device__ __noinline__ float randNormZ() {
         float x, y, r;
         int guard = 0;
@@ -253,7 +247,6 @@ struct WormWalker {
         if (r >= 1.0f || r == 0.0f) return 0.0f;
         return x * sqrtf(-2.0f * logf(r) / r);
     }
-    __device__ float randNorm(float mean, float sd) { return mean + randNormZ() * sd; }
     // the next cnt deviates that cnt calls of randNormZ() would return, made
     // by the lanes together from the same words: a lane makes one block of the
     // stream a round and tests the two attempts that end in it (with an odd
@@ -633,20 +626,6 @@ struct WormWalker {
         setP(last, x, y, z);
         return last;
     }
-    __device__ WB addNextBead(WB pb, float x, float y, float z) {
-        const int slice = pb.t + 1 == m.M ? 0 : pb.t + 1;
-        WB b = addBead(slice, x, y, z);
-        if (err) return b;
-        setNext(pb, b); setPrev(b, pb);
-        return b;
-    }
-    __device__ WB addPrevBead(WB nb_, float x, float y, float z) {
-        const int slice = nb_.t == 0 ? m.M - 1 : nb_.t - 1;
-        WB b = addBead(slice, x, y, z);
-        if (err) return b;
-        setPrev(nb_, b); setNext(b, nb_);
-        return b;
-    }
     __device__ __noinline__ void delBead(WB b) {
         if (!valid(b)) { err = WERR_LINK; return; }
         const int k = nb(b.t) - 1;
@@ -989,13 +968,6 @@ struct WormWalker {
 #pragma unroll 1
         for (int i = lane; i < cnt; i += 32) pos[at(chain[i + 1])] = orig[i];
         __syncwarp();
-    }
-    __device__ __noinline__ void freePos(WB nbd, float& x, float& y, float& z) {
-        const float4 p = P(nbd);
-        const float sg = m.sg2;
-        x = putInBC(randNorm(p.x, sg));
-        y = putInBC(randNorm(p.y, sg));
-        z = putInBC(randNorm(p.z, sg));
     }
     // a NaN difference rejects
     __device__ bool metro(double dA) { return rand() < expf(-(float)dA); }
