@@ -234,23 +234,34 @@ __device__ __forceinline__ float pair_factor32(int st1, int st2) {
     return 0.5f;
 }
 
+// What a bead's sums are multiplied by, vf t and gf t^3 lambda for t = shift
+// tau, even and odd slices: products made once on the host in the order the
+// action takes them (a kernel's one lane would wait 64 clocks for each).
+struct Scales32 { double bare[2], cor[2], gf[2]; };
+
+static Scales32 scales32(int shift, double tau, double lambda, const double vf[2], const double gf[2]) {
+    const double t = (double)shift * tau;
+    Scales32 a;
+    for (int o = 0; o < 2; ++o) { a.bare[o] = vf[o] * t; a.cor[o] = gf[o] * t * t * t * lambda; a.gf[o] = gf[o]; }
+    return a;
+}
+
 // A bead's action from its FP64 sums; the roundings are spelt out so that the
 // two kernels that assemble actions give the same bits.
-__device__ __forceinline__ double assemble32(int mode, bool need_c, double vf, double gf, double t, double lambda,
-                                             double V, double T, double fx, double fy, double fz) {
-    const double bareU = __dmul_rn(__dmul_rn(vf, t), V);
+__device__ __forceinline__ double assemble32(int mode, bool need_c, double bare, double cor, double V, double T,
+                                             double fx, double fy, double fz) {
+    const double bareU = __dmul_rn(bare, V);
     double corU = 0.0;
     if (need_c) {
         const double f2 = __fma_rn(fx, fx, __fma_rn(fy, fy, __dmul_rn(fz, fz)));
-        corU = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(gf, t), t), t), lambda), __dadd_rn(T, f2));
+        corU = __dmul_rn(cor, __dadd_rn(T, f2));
     }
     return (mode == PGB_ACTION_BARE) ? bareU : (mode == PGB_ACTION_CORR) ? corU : __dadd_rn(bareU, corU);
 }
 
 __global__ void __launch_bounds__(kWarpBeadBlock)
 k_bead_actions32_full(PathView v, AzizF az, const int2* __restrict__ beads, int k, int shift,
-                      int mode, double tau, double lambda, double vf0, double vf1, double gf0,
-                      double gf1, const double* __restrict__ over, const float4* __restrict__ fall,
+                      int mode, const Scales32 sc, const double* __restrict__ over, const float4* __restrict__ fall,
                       int delta, double* __restrict__ out) {
     // per bead of the block: Vn Vo Tn To Fnx Fny Fnz Fox Foy Foz as (hi, lo)
     __shared__ float2 s_part[kBeadsPerBlock][10];
@@ -270,7 +281,7 @@ k_bead_actions32_full(PathView v, AzizF az, const int2* __restrict__ beads, int 
             continue;
         }
         const int eo = s % 2;
-        const double gf = eo ? gf1 : gf0;
+        const double gf = eo ? sc.gf[1] : sc.gf[0];
         const bool need_v = (mode != PGB_ACTION_CORR);
         const bool need_c = (mode == PGB_ACTION_CORR) ? (gf > kEPS)
                           : (mode == PGB_ACTION_FULL) ? (shift == 1 && gf > kEPS) : false;
@@ -349,15 +360,15 @@ k_bead_actions32_full(PathView v, AzizF az, const int2* __restrict__ beads, int 
             if (s_state[lane]) {
                 const int s = beads[b].x;
                 const int eo = s % 2;
-                const double vf = eo ? vf1 : vf0, gf = eo ? gf1 : gf0;
-                const double t = (double)shift * tau;
+                const double bare = eo ? sc.bare[1] : sc.bare[0], cor = eo ? sc.cor[1] : sc.cor[0];
+                const double gf = eo ? sc.gf[1] : sc.gf[0];
                 const bool need_v = (mode != PGB_ACTION_CORR);
                 const bool need_c = (mode == PGB_ACTION_CORR) ? (gf > kEPS)
                                   : (mode == PGB_ACTION_FULL) ? (shift == 1 && gf > kEPS) : false;
                 const float2* q = s_part[lane];
                 auto dd = [](float2 x) { return (double)x.x + (double)x.y; };
                 auto action = [&](double V, double T, double fx, double fy, double fz) {
-                    return assemble32(mode, need_c, vf, gf, t, lambda, V, T, fx, fy, fz);
+                    return assemble32(mode, need_c, bare, cor, V, T, fx, fy, fz);
                 };
                 res = action(need_v ? dd(q[0]) : 0.0, dd(q[2]), dd(q[4]), dd(q[5]), dd(q[6]));
                 if (both)
@@ -375,7 +386,7 @@ cudaError_t launch_bead_actions32_full(const PathView& v, AzizParams a, const in
                                        cudaStream_t s) {
     if (k <= 0) return cudaSuccess;
     k_bead_actions32_full<<<(k + kBeadsPerBlock - 1) / kBeadsPerBlock, kWarpBeadBlock, 0, s>>>(
-        v, make_aziz_f(a), d_beads, k, shift, mode, tau, lambda, vf[0], vf[1], gf[0], gf[1],
+        v, make_aziz_f(a), d_beads, k, shift, mode, scales32(shift, tau, lambda, vf, gf),
         d_over, d_force, delta, d_out);
     return cudaGetLastError();
 }
@@ -570,8 +581,8 @@ __device__ __forceinline__ void trial_group(const float4* __restrict__ trial, in
 
 __global__ void __launch_bounds__(kTrialWarps * 32, 5)
 k_trials32(PathView v, AzizF az, BoxF B, const int* __restrict__ count, const int* __restrict__ offset,
-           const float4* __restrict__ sorted, const float4* __restrict__ fall, int shift, int mode, double tau,
-           double lambda, double vf0, double vf1, double gf0, double gf1, double* __restrict__ out) {
+           const float4* __restrict__ sorted, const float4* __restrict__ fall, int shift, int mode,
+           const Scales32 sc, double* __restrict__ out) {
     extern __shared__ float4 sp[];
     __shared__ TrialBuffer buffers[kTrialWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, Ne = v.Ne;
@@ -579,7 +590,7 @@ k_trials32(PathView v, AzizF az, BoxF B, const int* __restrict__ count, const in
     TrialBuffer& buf = buffers[warp];
     const bool need_v = (mode != PGB_ACTION_CORR);
     auto corr = [&](int s) {
-        const double gf = s % 2 ? gf1 : gf0;
+        const double gf = s % 2 ? sc.gf[1] : sc.gf[0];
         return (mode == PGB_ACTION_CORR) ? (gf > kEPS) : (mode == PGB_ACTION_FULL) ? (shift == 1 && gf > kEPS) : false;
     };
     const bool even_c = corr(0), odd_c = corr(1);
@@ -587,12 +598,11 @@ k_trials32(PathView v, AzizF az, BoxF B, const int* __restrict__ count, const in
     auto flush = [&]() {
         if (lane < used) {
             const int s = buf.slice[lane];
-            const double vf = s % 2 ? vf1 : vf0, gf = s % 2 ? gf1 : gf0;
-            const double t = (double)shift * tau;
+            const double bare = s % 2 ? sc.bare[1] : sc.bare[0], cor = s % 2 ? sc.cor[1] : sc.cor[0];
             const bool need_c = s % 2 ? odd_c : even_c;
             auto dd = [&](int q) { const float2 x = buf.part[q][lane]; return (double)x.x + (double)x.y; };
             auto action = [&](double V, double T, double fx, double fy, double fz) {
-                return assemble32(mode, need_c, vf, gf, t, lambda, V, T, fx, fy, fz);
+                return assemble32(mode, need_c, bare, cor, V, T, fx, fy, fz);
             };
             double res;
             if (need_c) {
@@ -694,7 +704,7 @@ cudaError_t launch_trials32(const PathView& v, AzizParams a, const int2* d_beads
     const size_t each = std::max<size_t>(1, std::min<size_t>(2, nb / (152 * 16)));
     const int grid = (int)((nb + kTrialWarps * each - 1) / (kTrialWarps * each));
     k_trials32<<<grid, kTrialWarps * 32, smem, s>>>(v, make_aziz_f(a), B, d_count, offset, d_sorted, d_force, shift, mode,
-                                                    tau, lambda, vf[0], vf[1], gf[0], gf[1], d_out);
+                                                    scales32(shift, tau, lambda, vf, gf), d_out);
     return cudaGetLastError();
 }
 
