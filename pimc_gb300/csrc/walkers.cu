@@ -1222,7 +1222,7 @@ k_walkers_tma(const WalkerMeta* __restrict__ meta, const int4* __restrict__ team
 // 6,300 clocks: wait 490, bridge 580, draws 1,730, pairs 2,090, decision
 // 1,190; now pairs 2,490, sums 240, decision and bridge 1,300.  Ten steps of
 // that walker alone 38.9 -> 34.5 ms, of the mix 47.3 -> 42.1 (schedule 6016;
-// 6008: 49.3 -> 43.0).
+// 6008: 49.3 -> 43.0), 41.3 with the pair loop of now.
 // ---------------------------------------------------------------------------
 struct MoveDesc {
     int com, i, s0, len, nmove;
@@ -1420,7 +1420,8 @@ k_walkers_pipe(const WalkerMeta* __restrict__ meta, const int4* __restrict__ tea
                 KahanF acc;
                 for (int j = j0; j < N; j += jstep) {
                     if (j == i) continue;
-                    #pragma unroll 4
+                    // (unrolled by four: 42.1 ms for the mix, 41.3 by two)
+                    #pragma unroll 2
                     for (int k = kb0; k < nmove; k += G) {
                         const float4* row = buf + (k + 1) * N;
                         const float4 pj = row[j], a = sn[k], b = row[i];
