@@ -306,7 +306,11 @@ int pgb_walkers_stats(pgb_walkers* w, pgb_walker_stats* per_walker);
 int pgb_walkers_reset_stats(pgb_walkers* w);
 /* launches of walker kernels issued so far */
 long long pgb_walkers_launch_count(pgb_walkers* w);
-/* schedule chosen by the autotuner (or set): 64/128/256 = one CTA of that
+/* schedule chosen by the autotuner (or set).  The results of a run follow from
+ * its schedule: 3002/3003 make another chain than the rest, and the last bits
+ * of the energies depend on the team sizes.  The autotuner takes the results
+ * of the fastest schedule outside 5000..6016 and runs the fastest one that
+ * gives them; name a schedule to fix them.  64/128/256 = one CTA of that
  * size per walker; 1004/1008/1016 (2004/2008/2016) = walkers packed as thread
  * teams of 1-8 warps into 256-thread CTAs sized for 4/8/16 pair evaluations
  * per thread per move, 3 (2) CTAs per SM; 3003 (3002) = one warp per
