@@ -916,10 +916,11 @@ cudaError_t launch_slice_terms64(const PathView& v, int window, int even, int od
 // and cosine of q . r.
 //
 // A cluster of CTAs shares a slice's beads, each with all the vectors and a
-// table of its own beads' powers, and adds the parts through distributed
-// shared memory: slices are too few and too long to even out over the SMs
-// (250 on 152: two on some, one on others), and a table built by every CTA
-// that takes some of the vectors is built twice.
+// table of its own beads, and adds the parts through distributed shared
+// memory: slices are too few and too long to even out over the SMs (250 on
+// 152: two on some, one on others), and a table built by every CTA that takes
+// some of the vectors is built twice.
+//
 // 64 beads, 124 slices, 389 vectors with |q| < 2 in mirrored order: 219 us with
 // a sine a term, 57 with a CTA a slice and 128 pairs of vectors, 44 now; 128
 // beads, 250 slices, 300 lattice vectors in no order: 623, 229, 187 (ncu,
@@ -931,8 +932,15 @@ constexpr int kRhoThreads = 512;                 // vectors a CTA at most
 constexpr int kRhoLeast = 128;                   // threads at least: few vectors share the beads out
 constexpr int kRhoPowers = 64;                   // largest |n_d| of the table form
 constexpr int kRhoSmem = 48 * 1024;              // four CTAs an SM
-constexpr int kRhoCluster = 4;
-constexpr int kRhoBeads = 16;                    // a CTA has at least
+constexpr int kRhoCluster = 8;
+constexpr int kRhoBeads = 3;                     // a CTA has at least
+// Fewer vectors than kRhoFew, or fewer slices than kRhoShort, take a warp a
+// vector and slice: a CTA a slice and cluster rank leaves the GPU empty there.
+// S(q) in this form and the other, us: 65 beads, 250 slices, 1 vector 17 and 34,
+// 16 40 and 40, 24 48 and 50, 32 62 and 55; 64 beads, 124 slices, 16 19 and 22,
+// 24 25 and 25, 32 30 and 29.  S(q) and F(q,tau) of 24 beads, 16 slices, 400
+// vectors 60 and 74 (lattice), 60 and 209 (others).
+constexpr int kRhoFew = 24, kRhoShort = 32;
 
 // 2 pi / L and L / 2 pi
 struct Lattice { double step[3], turn[3]; };
@@ -944,31 +952,84 @@ __device__ __forceinline__ int lattice_index(double q, double step, double turn)
     return ok ? (int)n : kRhoPowers + 1;
 }
 
-// exp(2 pi i n u) from the table of powers, the conjugate for n < 0
+// exp(i q_d r_d) from the table, the conjugate for n < 0
 __device__ __forceinline__ double2 power_of(const double2* E, int n) {
     double2 e = E[n < 0 ? -n : n];
     e.y = __hiloint2double(__double2hiint(e.y) ^ (n & 0x80000000), __double2loint(e.y));
     return e;
 }
 
-// blockDim.x = wide * parts; thread slot + wide * part has vector slot of the
-// CTA's vectors and every parts-th of its beads
+// (cos x, sin x): x less the nearest quarter turn in two parts (Cody and
+// Waite's reduction), Taylor's series of the rest (|r| <= pi/4: the terms left
+// out are below 5e-17 of the sine, 2e-18 of the cosine), the quarter turns by
+// swap and signs.  21 FP64 instructions; sincos() takes about thirty.
+static __device__ __noinline__ double2 far_sines(double x) {
+    double sn, cs;
+    sincos(x, &sn, &cs);
+    return make_double2(cs, sn);
+}
+__device__ __forceinline__ double2 sines64(double x) {
+    if ((__double2hiint(x) & 0x7fffffff) >= 0x4197D784) return far_sines(x);     // 1e8 and up, NaN
+    const double magic = 6755399441055744.0;                         // 1.5 2^52
+    const double t = __fma_rn(x, 0.63661977236758134308, magic), f = t - magic;      // 2 / pi
+    const int k = __double2loint(t);
+    // pi / 2 rounded, and what is left of it
+    const double r = __fma_rn(f, -6.12323399573676588614e-17, __fma_rn(f, -1.57079632679489661923, x)), y = r * r;
+    double s = -1.0 / 1307674368000.0, c = 1.0 / 20922789888000.0;   // 1 / 15!, 1 / 16!
+    s = __fma_rn(s, y, 1.0 / 6227020800.0); c = __fma_rn(c, y, -1.0 / 87178291200.0);
+    s = __fma_rn(s, y, -1.0 / 39916800.0); c = __fma_rn(c, y, 1.0 / 479001600.0);
+    s = __fma_rn(s, y, 1.0 / 362880.0); c = __fma_rn(c, y, -1.0 / 3628800.0);
+    s = __fma_rn(s, y, -1.0 / 5040.0); c = __fma_rn(c, y, 1.0 / 40320.0);
+    s = __fma_rn(s, y, 1.0 / 120.0); c = __fma_rn(c, y, -1.0 / 720.0);
+    s = __fma_rn(s, y, -1.0 / 6.0); c = __fma_rn(c, y, 1.0 / 24.0);
+    s = __fma_rn(r * y, s, r); c = __fma_rn(c, y, -0.5);
+    c = __fma_rn(c, y, 1.0);
+    const double a = k & 1 ? s : c, b = k & 1 ? c : s;
+    return make_double2(__hiloint2double(__double2hiint(a) ^ ((k + 1) & 2) << 30, __double2loint(a)),
+                        __hiloint2double(__double2hiint(b) ^ (k & 2) << 30, __double2loint(b)));
+}
+
+// Few vectors: one warp per (q, t), a sine and a cosine a bead.
+__global__ void __launch_bounds__(256)
+k_rhoq64_few(PathView v, const double* __restrict__ q, int nq, double maxR2, double* __restrict__ rho) {
+    const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (gw >= (long long)nq * v.M) return;
+    const int iq = (int)(gw / v.M), t = (int)(gw - (long long)iq * v.M), n = v.nbs[t];
+    const double qx = q[3 * iq], qy = q[3 * iq + 1], qz = q[3 * iq + 2];
+    const double* X = v.pos + (size_t)t * 3 * v.Ne;
+    double re = 0.0, im = 0.0;
+    for (int j = lane; j < n; j += 32) {
+        // cylinder restriction: only beads with x^2 + y^2 < maxR^2
+        if (maxR2 > 0.0 && !(X[j] * X[j] + X[v.Ne + j] * X[v.Ne + j] < maxR2)) continue;
+        double ph = 0.0;
+        ph += qx * X[j]; ph += qy * X[v.Ne + j]; ph += qz * X[2 * v.Ne + j];
+        double sn, cs;
+        sincos(ph, &sn, &cs);
+        re += cs; im += sn;
+    }
+    re = warp_sum(re); im = warp_sum(im);
+    if (lane == 0) reinterpret_cast<double2*>(rho)[gw] = make_double2(re, im);
+}
+
+// Thread slot + wide * part, part < parts, has vector slot of the CTA's vectors
+// and every parts-th of its beads.
 __global__ void __launch_bounds__(kRhoThreads)
-k_rhoq64(PathView v, const double* __restrict__ q, int nq, Lattice lat, double maxR2, int wide, int csize,
+k_rhoq64(PathView v, const double* __restrict__ q, int nq, Lattice lat, double maxR2, int wide, int parts, int csize,
          double* __restrict__ rho) {
     extern __shared__ double2 E[];               // [bead][dimension][power]
     __shared__ int s_max;
     const int t = blockIdx.x / csize, rank = blockIdx.x - t * csize, tid = threadIdx.x, T = blockDim.x;
-    const int parts = T / wide, part = tid / wide, n = v.nbs[t];
+    const int part = tid / wide, n = v.nbs[t];
     const int b0 = (int)((long long)n * rank / csize), b1 = (int)((long long)n * (rank + 1) / csize);
     const int i = blockIdx.y * wide + tid - part * wide, j = nq - 1 - i;
     const double* X = v.pos + (size_t)t * 3 * v.Ne;
-    bool live = i < nq, mirrored = live;
+    bool live = part < parts && i < nq, mirrored = live;
     int k[3] = {0, 0, 0};
     if (tid == 0) s_max = 0;
     __syncthreads();
+    double a[3] = {0.0, 0.0, 0.0};
     if (live) {
-        double a[3];
         #pragma unroll
         for (int d = 0; d < 3; ++d) {
             a[d] = q[3 * i + d];
@@ -1022,11 +1083,8 @@ k_rhoq64(PathView v, const double* __restrict__ q, int nq, Lattice lat, double m
         const double qx = q[3 * i], qy = q[3 * i + 1], qz = q[3 * i + 2];
         for (int p = b0 + part; p < b1; p += parts) {
             if (maxR2 > 0.0 && !(X[p] * X[p] + X[v.Ne + p] * X[v.Ne + p] < maxR2)) continue;
-            double ph = 0.0;
-            ph += qx * X[p]; ph += qy * X[v.Ne + p]; ph += qz * X[2 * v.Ne + p];
-            double sn, cs;
-            sincos(ph, &sn, &cs);
-            S.x += cs; S.y += sn;
+            const double2 e = sines64(__fma_rn(qx, X[p], __fma_rn(qy, X[v.Ne + p], qz * X[2 * v.Ne + p])));
+            S.x += e.x; S.y += e.y;
         }
     }
     double2* R = reinterpret_cast<double2*>(rho);
@@ -1060,24 +1118,32 @@ k_rhoq64(PathView v, const double* __restrict__ q, int nq, Lattice lat, double m
 cudaError_t launch_rhoq64(const PathView& v, const double* d_q, int nq, double* d_rho,
                           cudaStream_t s, double maxR2) {
     if (nq < 1) return cudaSuccess;
+    if (nq < kRhoFew || v.M < kRhoShort) {
+        k_rhoq64_few<<<(int)(((long long)nq * v.M + 7) / 8), 256, 0, s>>>(v, d_q, nq, maxR2, d_rho);
+        return cudaGetLastError();
+    }
     const cudaError_t ae = set_smem_limit(k_rhoq64, kRhoSmem);
     if (ae != cudaSuccess) return ae;
     const int sets = (nq + kRhoThreads - 1) / kRhoThreads, each = (nq + sets - 1) / sets;
-    const int wide = (each + 31) / 32 * 32, parts = std::max(1, kRhoLeast / wide);
+    const int wide = each, parts = std::max(1, kRhoLeast / wide);
     // rounds of the SMs, in units of a whole slice: a cluster costs two
     // barriers and a table each, so it has to gain (124 slices of 64 beads, one
     // round either way: 357 us a sample with one CTA a slice, 367 with two,
     // 390 with four; 250 of 128: 464 with two, 439 with four)
     auto rounds = [&](int c) { return (double)(((long long)v.M * sets * c + 151) / 152) / c; };
     int c = 1;
-    for (int d = 2; d <= kRhoCluster && d * kRhoBeads <= v.Ne; d *= 2)
+    // (a cluster of eight pays for short paths and many vectors: 160 beads, 80
+    // slices, 400 vectors off the lattice 1.37 of the sines' time with four, 1.18
+    // with eight, 17 lattice vectors 0.71 and 1.01)
+    const int most = v.M < 84 && nq >= 128 ? kRhoCluster : 4;
+    for (int d = 2; d <= most && d * kRhoBeads <= v.Ne; d *= 2)
         if (rounds(d) < 0.95 * rounds(c)) c = d;
     Lattice lat;
     const double kTwoPi = 6.283185307179586476925;
     for (int d = 0; d < 3; ++d) { lat.step[d] = kTwoPi / v.side[d]; lat.turn[d] = v.side[d] / kTwoPi; }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)v.M * c, (unsigned)sets);
-    cfg.blockDim = dim3(wide * parts);
+    cfg.blockDim = dim3((wide * parts + 31) / 32 * 32);
     cfg.dynamicSmemBytes = kRhoSmem;
     cfg.stream = s;
     cudaLaunchAttribute at{};
@@ -1085,7 +1151,7 @@ cudaError_t launch_rhoq64(const PathView& v, const double* d_q, int nq, double* 
     at.val.clusterDim.x = c; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
     cfg.attrs = &at;
     cfg.numAttrs = c > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k_rhoq64, v, d_q, nq, lat, maxR2, wide, c, d_rho);
+    return cudaLaunchKernelEx(&cfg, k_rhoq64, v, d_q, nq, lat, maxR2, wide, parts, c, d_rho);
 }
 
 // F(q,tau) = norm * sum_t Re(rho_t conj(rho_{t+tau})), tau in [0, M/2].  One
