@@ -904,16 +904,18 @@ cudaError_t launch_slice_terms64(const PathView& v, int window, int even, int od
 // raw bead coordinates).
 //
 // A lattice vector q = 2 pi n / L (every vector of the reference's lattice
-// lists) needs no sine per bead: exp(i q . r) is the product of
-// exp(2 pi i n_d r_d / L_d) over the dimensions, and a CTA keeps those powers
-// of its slice's beads in shared memory, n_d = 0 .. the largest |n_d| of its
-// vectors, each power the product of the two half powers (log2 n roundings).
-// One thread sums one vector over the beads: eight FP64 multiply-adds a bead
-// where sincos and the phase take about seventy, and the FP64 pipe (16 clocks
-// of an SM a warp instruction) is the bound.  A list that enumerates a grid
-// symmetric about 0 has -q at the mirrored place; its density is the complex
-// conjugate and is written, not summed.  Other vectors (shells) take the sine
-// and cosine of q . r.
+// lists) needs no sine per bead: exp(i q . r) is the product of the
+// exp(i q_d r_d), and a CTA keeps these of its slice's beads in shared memory
+// for every |q_d| that its vectors have, at the place |n_d|.  (Each is a sine
+// and a cosine of its own.  Made by products from exp(2 pi i r_d / L_d) they
+// were cheaper, but the roundings of 1 / L and of q_d itself then shift all
+// phases alike, which F(q,tau) does not average out.)  One thread sums one
+// vector over the beads: eight FP64 multiply-adds a bead where the phase and
+// its sines take 26, and the FP64 pipe (16 clocks of an SM a warp instruction)
+// is the bound.  A list that enumerates a grid symmetric about 0 has -q at the
+// mirrored place; its density is the complex conjugate and is written, not
+// summed.  Other vectors (shells), and lattice vectors that are too few for
+// their table, take the sines.
 //
 // A cluster of CTAs shares a slice's beads, each with all the vectors and a
 // table of its own beads, and adds the parts through distributed shared
@@ -921,12 +923,14 @@ cudaError_t launch_slice_terms64(const PathView& v, int window, int even, int od
 // 152: two on some, one on others), and a table built by every CTA that takes
 // some of the vectors is built twice.
 //
-// 64 beads, 124 slices, 389 vectors with |q| < 2 in mirrored order: 219 us with
-// a sine a term, 57 with a CTA a slice and 128 pairs of vectors, 44 now; 128
-// beads, 250 slices, 300 lattice vectors in no order: 623, 229, 187 (ncu,
-// cold).  Relative error against 113-bit phases, sines and now: 4e-16 and
-// 7e-16, 6e-16 and 5e-16, at 500 beads 2.4e-15 and 2.0e-15; of F(q,tau) 2e-16
-// both.
+// S(q) calls, a warp a vector and slice with sincos, and here: 64 beads, 124
+// slices, 400 lattice vectors 232 and 83 us, 400 others 232 and 220; 160 beads,
+// 250 slices, 200: 525 and 228, 525 and 513; 17 beads, 1000 slices, 96: 255 and
+// 62, 255 and 117.  Error of the densities relative to extended precision,
+// sincos and here: 40 beads, 62 slices 1.1e-15 and 6.8e-16, 64 beads, |q| < 2
+// 4.2e-16 and 3.6e-16, 160 beads 1.6e-15 and 1.0e-15, shells of 100 beads 4.8e-16
+// and 4.1e-16; of F(q,tau) 3.7e-16 and 2.7e-16, 2.2e-16 and 2.5e-16, 4.1e-16 and
+// 3.1e-16, 2.3e-16 and 1.8e-16.
 // ---------------------------------------------------------------------------
 constexpr int kRhoThreads = 512;                 // vectors a CTA at most
 constexpr int kRhoLeast = 128;                   // threads at least: few vectors share the beads out
@@ -941,6 +945,8 @@ constexpr int kRhoBeads = 3;                     // a CTA has at least
 // 24 25 and 25, 32 30 and 29.  S(q) and F(q,tau) of 24 beads, 16 slices, 400
 // vectors 60 and 74 (lattice), 60 and 209 (others).
 constexpr int kRhoFew = 24, kRhoShort = 32;
+// FP64 instructions that a table saves a vector and bead, and that it takes an entry
+constexpr int kRhoSaved = 18, kRhoEntry = 24;
 
 // 2 pi / L and L / 2 pi
 struct Lattice { double step[3], turn[3]; };
@@ -1019,6 +1025,7 @@ k_rhoq64(PathView v, const double* __restrict__ q, int nq, Lattice lat, double m
          double* __restrict__ rho) {
     extern __shared__ double2 E[];               // [bead][dimension][power]
     __shared__ int s_max;
+    __shared__ unsigned long long comp[3][kRhoPowers + 1];   // the |q_d| that a table entry stands for
     const int t = blockIdx.x / csize, rank = blockIdx.x - t * csize, tid = threadIdx.x, T = blockDim.x;
     const int part = tid / wide, n = v.nbs[t];
     const int b0 = (int)((long long)n * rank / csize), b1 = (int)((long long)n * (rank + 1) / csize);
@@ -1027,6 +1034,7 @@ k_rhoq64(PathView v, const double* __restrict__ q, int nq, Lattice lat, double m
     bool live = part < parts && i < nq, mirrored = live;
     int k[3] = {0, 0, 0};
     if (tid == 0) s_max = 0;
+    for (int x = tid; x < 3 * (kRhoPowers + 1); x += T) comp[0][x] = ~0ull;
     __syncthreads();
     double a[3] = {0.0, 0.0, 0.0};
     if (live) {
@@ -1041,32 +1049,37 @@ k_rhoq64(PathView v, const double* __restrict__ q, int nq, Lattice lat, double m
             if (live) k[d] = lattice_index(a[d], lat.step[d], lat.turn[d]);
     }
     const int most = max(abs(k[0]), max(abs(k[1]), abs(k[2])));
-    const bool powers = live && most <= kRhoPowers;
+    bool powers = live && most <= kRhoPowers;
+    // components of one index that differ in the last places: the smallest has the entry
+    auto bits = [&](int d) { return (unsigned long long)__double_as_longlong(fabs(a[d])); };
+    if (powers)
+        for (int d = 0; d < 3; ++d) atomicMin(&comp[d][abs(k[d])], bits(d));
+    __syncthreads();
+    if (powers)
+        for (int d = 0; d < 3; ++d) powers = powers && comp[d][abs(k[d])] == bits(d);
+    const int nv = __syncthreads_count(powers && part == 0);
     const int warp_most = __reduce_max_sync(0xffffffffu, powers ? most + 1 : 0);
     if ((tid & 31) == 0 && warp_most) atomicMax(&s_max, warp_most);
     __syncthreads();
     double2 S = make_double2(0.0, 0.0);
-    const int np = s_max;                        // powers 0 .. np - 1; 0: no lattice vector here
+    int np = s_max;                              // entries 0 .. np - 1; 0: no lattice vector here
+    if (nv * kRhoSaved < 3 * kRhoEntry * (np - 1)) { powers = false; np = 0; }
     if (np > 0) {
         const int chunk = max(parts, kRhoSmem / (3 * np * (int)sizeof(double2)));
         for (int j0 = b0; j0 < b1; j0 += chunk) {
             const int nj = min(chunk, b1 - j0);
             __syncthreads();
-            for (int x = tid; x < 3 * nj; x += T) {
-                const int d = x / nj, p = x - d * nj;
-                const double r = X[d * v.Ne + j0 + p];
-                double2* e = E + (size_t)(3 * p + d) * np;
-                double sn, cs;
-                sincospi(2.0 * (r * v.sideInv[d]), &sn, &cs);
+            for (int x = tid; x < 3 * nj * np; x += T) {
+                const int h = x / (3 * nj), dp = x - h * (3 * nj), d = dp / nj, p = dp - d * nj;
+                double2 e = make_double2(1.0, 0.0);
+                const unsigned long long m = comp[d][h];
+                if (h > 0) e = sines64(m == ~0ull ? 0.0 : __longlong_as_double((long long)m) * X[d * v.Ne + j0 + p]);
                 // cylinder restriction: beads outside x^2 + y^2 < maxR^2 count 0
-                const double rx = X[j0 + p], ry = X[v.Ne + j0 + p];
-                const double one = (d == 0 && maxR2 > 0.0 && !(rx * rx + ry * ry < maxR2)) ? 0.0 : 1.0;
-                e[0] = make_double2(one, 0.0);
-                if (np > 1) e[1] = make_double2(one * cs, one * sn);
-                for (int h = 2; h < np; ++h) {
-                    const double2 a = e[h >> 1], b = e[h - (h >> 1)];
-                    e[h] = make_double2(__fma_rn(a.x, b.x, -(a.y * b.y)), __fma_rn(a.x, b.y, a.y * b.x));
+                if (d == 0 && maxR2 > 0.0) {
+                    const double rx = X[j0 + p], ry = X[v.Ne + j0 + p];
+                    if (!(rx * rx + ry * ry < maxR2)) e = make_double2(0.0, 0.0);
                 }
+                E[(size_t)(3 * p + d) * np + h] = e;
             }
             __syncthreads();
             if (powers)
