@@ -1168,10 +1168,12 @@ cudaError_t launch_rhoq64(const PathView& v, const double* d_q, int nq, double* 
 }
 
 // F(q,tau) = norm * sum_t Re(rho_t conj(rho_{t+tau})), tau in [0, M/2].  One
-// CTA a wave vector, its densities in shared memory with the first half
-// repeated behind them (no wrap in the loop), one thread a tau: two FP64
-// multiply-adds a term, the FP64 pipe the bound.  300 vectors, M = 250:
-// 79 us with one thread an output from L1, 35 us here.
+// CTA a wave vector and kIsfThreads tau, the vector's densities in shared
+// memory with the first half repeated behind them (no wrap in the loop), one
+// thread a tau: two FP64 multiply-adds a term, even and odd slices in sums of
+// their own, the FP64 pipe the bound.  300 vectors, M = 250: 79 us with one
+// thread an output from L1, 35 us here; one vector, M = 1000, whole calls: 340 us,
+// 378 with all tau in one CTA, 109 here.
 constexpr int kIsfThreads = 128;
 
 __global__ void __launch_bounds__(kIsfThreads)
@@ -1181,16 +1183,20 @@ k_isf_direct64(const double* __restrict__ rho, int M, double norm, double* __res
     const double2* r = reinterpret_cast<const double2*>(rho) + (size_t)blockIdx.x * M;
     for (int t = threadIdx.x; t < M + nt; t += kIsfThreads) E[t] = r[t < M ? t : t - M];
     __syncthreads();
-    for (int tau = threadIdx.x; tau < nt; tau += kIsfThreads) {
-        double re = 0.0, im = 0.0;
-        #pragma unroll 4
-        for (int t = 0; t < M; ++t) {
-            const double2 a = E[t], b = E[t + tau];
-            re = __fma_rn(a.x, b.x, re);
-            im = __fma_rn(a.y, b.y, im);
+    const int tau = blockIdx.y * kIsfThreads + threadIdx.x;
+    if (tau >= nt) return;
+    double sum[2] = {0.0, 0.0};
+    int t = 0;
+    #pragma unroll 2
+    for (; t + 1 < M; t += 2) {
+        #pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const double2 a = E[t + u], b = E[t + u + tau];
+            sum[u] = __fma_rn(a.x, b.x, __fma_rn(a.y, b.y, sum[u]));
         }
-        out[(size_t)blockIdx.x * nt + tau] = (re + im) * norm;
     }
+    if (t < M) sum[0] = __fma_rn(E[t].x, E[t + tau].x, __fma_rn(E[t].y, E[t + tau].y, sum[0]));
+    out[(size_t)blockIdx.x * nt + tau] = (sum[0] + sum[1]) * norm;
 }
 
 // the same straight from memory, for slices whose densities do not fit
@@ -1216,7 +1222,8 @@ cudaError_t launch_isf_direct64(const double* d_rho, int nq, int M, double norm,
     if (smem <= 200 * 1024) {
         const cudaError_t ae = set_smem_limit(k_isf_direct64, 200 * 1024);
         if (ae != cudaSuccess) return ae;
-        k_isf_direct64<<<nq, kIsfThreads, smem, s>>>(d_rho, M, norm, d_out);
+        const dim3 grid(nq, (M / 2 + kIsfThreads) / kIsfThreads);        // M / 2 + 1 tau
+        k_isf_direct64<<<grid, kIsfThreads, smem, s>>>(d_rho, M, norm, d_out);
         return cudaGetLastError();
     }
     long long n = (long long)nq * (M / 2 + 1);
