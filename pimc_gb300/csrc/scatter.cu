@@ -189,10 +189,14 @@ cudaError_t launch_rhoq32(const PathView& v, const double* d_q, int nq, float2* 
     return cudaGetLastError();
 }
 
-// S(q) = norm sum_t |rho_q(t)|^2, one warp a wave vector: four FP64
-// instructions a density, the FP64 pipe the bound, and one reduction a vector
-// instead of eight.  2048 vectors, M = 512: 26 -> 13 us.
-constexpr int kSsfBlock = 128;
+// S(q) = norm sum_t |rho_q(t)|^2: four FP64 instructions a density, the FP64
+// pipe the bound, so one warp a wave vector and one reduction a vector instead
+// of eight (2048 vectors, M = 512: 26 -> 13 us); but a CTA a vector for fewer
+// than kSsfFew, where a warp's own chain is the time.  S(q) in the first form
+// and the second, us: M = 1000, 1 vector 19.1 and 15.0, 150 23.1 and 18.1, 300
+// 26.2 and 22.2, 608 28.1 and 28.1, 1579 47 and 55; M = 124, 150 17.1 and 15.0,
+// 300 17.9 both, 608 20.2 and 22.1.
+constexpr int kSsfBlock = 128, kSsfFew = 300;
 
 __global__ void __launch_bounds__(kSsfBlock)
 k_ssf_from_rho32(const float2* __restrict__ rho, int nq, int M, double norm, double* __restrict__ out) {
@@ -210,11 +214,25 @@ k_ssf_from_rho32(const float2* __restrict__ rho, int nq, int M, double norm, dou
     if (lane == 0) out[iq] = s * norm;
 }
 
+__global__ void __launch_bounds__(256)
+k_ssf_from_rho32_few(const float2* __restrict__ rho, int M, double norm, double* __restrict__ out) {
+    __shared__ double red[8];
+    double acc = 0.0;
+    for (int t = threadIdx.x; t < M; t += 256) {
+        const float2 r = rho[(size_t)blockIdx.x * M + t];
+        const double x = r.x, y = r.y;
+        acc = __fma_rn(x, x, __fma_rn(y, y, acc));
+    }
+    const double s = block_sum(acc, red);
+    if (threadIdx.x == 0) out[blockIdx.x] = s * norm;
+}
+
 cudaError_t launch_ssf_from_rho32(const float2* d_rho, int nq, int M, double norm,
                                   double* d_out, cudaStream_t s) {
     if (nq <= 0) return cudaSuccess;
     constexpr int each = kSsfBlock / 32;
-    k_ssf_from_rho32<<<(nq + each - 1) / each, kSsfBlock, 0, s>>>(d_rho, nq, M, norm, d_out);
+    if (nq < kSsfFew) k_ssf_from_rho32_few<<<nq, 256, 0, s>>>(d_rho, M, norm, d_out);
+    else k_ssf_from_rho32<<<(nq + each - 1) / each, kSsfBlock, 0, s>>>(d_rho, nq, M, norm, d_out);
     return cudaGetLastError();
 }
 
@@ -226,7 +244,8 @@ cudaError_t launch_ssf_from_rho32(const float2* d_rho, int nq, int M, double nor
 // repeated beyond M for the window, with one entry of padding in eight, so
 // that the threads' windows, eight entries apart, fall into different banks.
 // 1579 vectors, M = 250: 36 us with one vector a CTA, a modulo a step and the
-// windows in four banks, 25 us here.
+// windows in four banks, 25 us here; 341 vectors, M = 4, whole calls 50 us, 83
+// with 128 vectors a CTA copied one after another, 35 here.
 constexpr int kTauPerThread = 8;
 constexpr int kIsfBlock = 128;
 
@@ -240,9 +259,10 @@ k_isf_direct32(const float2* __restrict__ rho, int nq, int M, int each, int per,
     extern __shared__ float2 sr[];
     const int nt = M / 2 + 1, row = isf_row(M), ext = M + nt + 2 * kTauPerThread;
     const int q0 = blockIdx.x * each, qn = min(each, nq - q0);
-    for (int q = 0; q < qn; ++q)
-        for (int t = threadIdx.x; t < ext; t += kIsfBlock)
-            sr[q * row + isf_pad(t)] = rho[(size_t)(q0 + q) * M + t % M];
+    for (int x = threadIdx.x; x < qn * ext; x += kIsfBlock) {
+        const int q = x / ext, t = x - q * ext;
+        sr[q * row + isf_pad(t)] = rho[(size_t)(q0 + q) * M + t % M];
+    }
     __syncthreads();
     for (int w = threadIdx.x; w < qn * per; w += kIsfBlock) {
         const int q = w / per, tau0 = (w - q * per) * kTauPerThread;
@@ -319,7 +339,9 @@ cudaError_t launch_isf_direct32(const float2* d_rho, int nq, int M, double norm,
     const int per = (M / 2 + 1 + kTauPerThread - 1) / kTauPerThread;
     const size_t row = (size_t)isf_row(M) * sizeof(float2);
     if (row <= 200 * 1024) {
-        const int each = std::max<int>(1, std::min<size_t>(std::max(1, kIsfBlock / per), 200 * 1024 / row));
+        // no more vectors a CTA than leave every SM one
+        const int most = std::min(std::max(1, kIsfBlock / per), (nq + 151) / 152);
+        const int each = std::max<int>(1, std::min<size_t>(most, 200 * 1024 / row));
         const cudaError_t ae = set_smem_limit(k_isf_direct32, 200 * 1024);
         if (ae != cudaSuccess) return ae;
         k_isf_direct32<<<(nq + each - 1) / each, kIsfBlock, each * row, s>>>(d_rho, nq, M, each, per, norm, d_out);
