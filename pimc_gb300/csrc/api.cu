@@ -292,6 +292,14 @@ int pgb_create(const pgb_params* p, pgb_ctx** out) {
         g_last_error = "precision must be PGB_FP64 or PGB_MIXED"; return PGB_EINVAL;
     }
     if (p->num_ptcl_ext > 8192) { g_last_error = "num_ptcl_ext > 8192 not supported"; return PGB_EINVAL; }
+    {
+        // the kernels index the table's 10^-6 rm steps up to half the box's
+        // diagonal with 31 bits, a grid's stride of them ahead
+        const double d2 = p->side[0] * p->side[0] + p->side[1] * p->side[1] + p->side[2] * p->side[2];
+        if (!(0.5 * std::sqrt(d2) / (1.0E-6 * aziz_params(p->aziz_year).rm) < 2147483648.0 - 1048576.0)) {
+            g_last_error = "box too large for the potential's table (2^31 steps of 1e-6 rm)"; return PGB_EINVAL;
+        }
+    }
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
         g_last_error = "no CUDA device available"; return PGB_ECUDA;
