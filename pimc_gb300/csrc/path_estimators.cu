@@ -35,8 +35,11 @@ __device__ __forceinline__ bool last_to_arrive(unsigned* counter, unsigned block
 // and its image by twice that each, so |r| is off by at most sqrt(3) 3 2^-24 L,
 // 1.8e-5 of a bin; the sum of squares, the reciprocal root and 1/dSep add
 // 2e-5 at 50 bins, the step of the quotient 8e-6: together less than half of
-// the edge, kSepEdge steps.  The FP64 recomputation
-// runs for 2e-4 of the pairs; its sixty dependent FP64 instructions take a
+// the edge, kSepEdge steps.  In a box that is no cube the first part grows with
+// the longer sides over the third, which the bins are made of, and the edge
+// with it; a slice with a bead beyond a side's length from the origin takes the
+// FP64 form throughout.  The FP64 recomputation
+// runs for 2e-4 of the pairs in a cube; its sixty dependent FP64 instructions take a
 // warp about 5 us (the FP64 pipe takes 64 clocks of a sub-partition for a warp
 // instruction), so these pairs are listed and done together at the end, one a
 // thread.  A shared-memory atomic takes about a clock a lane even without
@@ -47,13 +50,13 @@ __device__ __forceinline__ bool last_to_arrive(unsigned* counter, unsigned block
 // floor, compare and IEEE root in floating point (64 instructions), 27 us
 // here.
 constexpr int kSepBits = 16;                 // 127 bins of 2^16 steps fill the mantissa
-constexpr int kSepEdge = 7;                  // 1.07e-4 of a bin
+constexpr int kSepEdge = 7;                  // 1.07e-4 of a bin, in a cube
 constexpr int kSepBlock = 512;               // 256 where a slice leaves no room for sixteen histograms
 constexpr int kSepNear = 512;
 
 // FP32 constants made on the host: a division or conversion in FP64 by every
 // warp of every CTA takes longer than the pairs of a small slice
-struct SepF { float side[3], inv[3], step, far; };
+struct SepF { float side[3], inv[3], step, far; int edge; };
 
 __device__ __forceinline__ int sep_bin64(const PathView& v, int t, int b1, int b2, double dSep) {
     const double3 d = sep64(v, t, b2, b1);
@@ -73,8 +76,13 @@ k_sep_hist(PathView v, SepF f, int t0, double dSep, unsigned* __restrict__ arriv
     for (int b = threadIdx.x; b < warps * 32 * kPcfBins; b += threads) counts[b] = 0u;
     const int t = t0 + blockIdx.x;
     const int n = v.nbs[t];
-    for (int j = threadIdx.x; j < n; j += threads) sp[j] = v.pos32[(size_t)t * v.Ne + j];
-    __syncthreads();
+    bool out_of_box = false;
+    for (int j = threadIdx.x; j < n; j += threads) {
+        const float4 r = v.pos32[(size_t)t * v.Ne + j];
+        sp[j] = r;
+        out_of_box |= fabsf(r.x) > f.side[0] || fabsf(r.y) > f.side[1] || fabsf(r.z) > f.side[2];
+    }
+    const int edge = __syncthreads_or(out_of_box) ? 1 << (kSepBits - 1) : f.edge;
     const float Lx = f.side[0], Ly = f.side[1], Lz = f.side[2], Lix = f.inv[0], Liy = f.inv[1], Liz = f.inv[2];
     const float step = f.step, far = f.far;
     for (int b1 = warp; b1 < n - 1; b1 += warps) {
@@ -90,7 +98,7 @@ k_sep_hist(PathView v, SepF f, int t0, double dSep, unsigned* __restrict__ arriv
             asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ri) : "f"(fmaxf(rr, 1.0e-30f)));
             // x with kSepBits fraction bits in the mantissa of 2^23 + x 2^kSepBits
             const int i = __float_as_int(fmaf(fminf(rr * ri, far), step, 8388608.0f));
-            if (((i + kSepEdge) & ((1 << kSepBits) - 1)) < 2 * kSepEdge) {
+            if (((i + edge) & ((1 << kSepBits) - 1)) < 2 * edge) {
                 const int at = atomicAdd(&s_near, 1);
                 if (at < kSepNear) { near_pair[at] = make_int2(b1, b2); continue; }
                 const int nR = sep_bin64(v, t, b1, b2, dSep);
@@ -133,6 +141,9 @@ cudaError_t launch_sep_hist(const PathView& v, int slice, unsigned* d_arrived, u
     for (int d = 0; d < 3; ++d) { f.side[d] = (float)v.side[d]; f.inv[d] = (float)v.sideInv[d]; }
     f.step = (float)((1 << kSepBits) / dSep);
     f.far = (float)(127.0 * dSep);
+    // 1.18 steps of 2^-16 a unit of |L| / (sqrt(3) L_z), and 1.83; more than twice that
+    const double longer = sqrt((v.side[0] * v.side[0] + v.side[1] * v.side[1] + v.side[2] * v.side[2]) / 3.0) / v.side[2];
+    f.edge = std::max(kSepEdge, (int)std::min<double>(1 << (kSepBits - 1), ceil(2.72 * longer + 4.2)));
     k_sep_hist<<<nt, threads, smem, s>>>(v, f, t0, dSep, d_arrived, d_hist, out);
     return cudaGetLastError();
 }
