@@ -130,7 +130,10 @@ cudaError_t launch_sep_hist(const PathView& v, int slice, unsigned* d_arrived, u
     const double dSep = 0.5 * sqrt(3.0) * v.side[2] / (1.0 * kPcfBins);   // action.cpp:192
     const int t0 = slice >= 0 ? slice : 0, nt = slice >= 0 ? 1 : v.M;
     const size_t pos = (size_t)v.Ne * sizeof(float4), column = kPcfBins * sizeof(unsigned);
-    const int threads = pos + kSepBlock * column <= 200 * 1024 ? kSepBlock : 256;
+    // small slices, more than two CTAs an SM: clearing and adding sixteen
+    // histograms is the time (17 beads, 1000 slices: 34 us a call, 31 with eight)
+    const bool small = v.Ne <= 32 && nt > 2 * 152;
+    const int threads = !small && pos + kSepBlock * column <= 200 * 1024 ? kSepBlock : 256;
     const size_t smem = pos + threads * column;
     if (smem > 200 * 1024) return cudaErrorInvalidValue;   // one slice in shared memory
     {

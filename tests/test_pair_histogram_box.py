@@ -43,3 +43,13 @@ def test_counts(pgb, ratio, spread):
     a = pgb.Action(side, m, n, 0.004, 6.0596)
     a.load(cfg)
     assert np.array_equal(a.pair_correlation(-1), _histogram(cfg["pos"], side))
+
+
+@pytest.mark.parametrize("n,m", [(32, 305), (33, 305), (2, 304)])
+def test_counts_of_many_small_slices(pgb, n, m):
+    side = np.array([9.0, 9.0, 9.0])
+    cfg = pgb.worldlines.seeded_worldlines(n, m, 9.0, 6.0596, 0.004, 1)
+    cfg["pos"] = np.random.default_rng(n).uniform(-4.5, 4.5, (m, n, 3))
+    a = pgb.Action(side, m, n, 0.004, 6.0596)
+    a.load(cfg)
+    assert np.array_equal(a.pair_correlation(-1), _histogram(cfg["pos"], side))
