@@ -845,13 +845,29 @@ struct SliceRow32 {
     }
 };
 
+// 8 values a lane summed over the warp by recursive halving, in warp_sum's own
+// tree (9 FP64 adds instead of 40): lane l returns the sum of value l / 4
+__device__ __forceinline__ double warp_sum8(double (&x)[8], int lane) {
+    #pragma unroll
+    for (int h = 4, o = 16; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = lane & o;
+        #pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const double give = up ? x[i] : x[i + h];
+            x[i] = (up ? x[i + h] : x[i]) + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    x[0] += __shfl_xor_sync(0xffffffffu, x[0], 2);
+    return x[0] + __shfl_xor_sync(0xffffffffu, x[0], 1);
+}
+
 // work: [M][9][Ne] floats, the beads' terms 1..7 and the columns' potential as
 // Kahan pairs in 0 and 8
 __global__ void __launch_bounds__(kSliceRows32)
 k_slice_terms32(PathView v, AzizF az, BoxF B, int window, int even, int odd, unsigned* __restrict__ arrived,
                 float* __restrict__ work, double* __restrict__ terms) {
     extern __shared__ float4 sp[];
-    __shared__ double sums[8][kSliceRows32 / 32];
+    __shared__ double sums[8][kSliceColumns32 / 32];
     __shared__ bool last;
     const int s = blockIdx.x, Ne = v.Ne, n = v.nbs[s], nblk = gridDim.y, tid = threadIdx.x;
     const int level = s % 2 ? odd : even, b1 = blockIdx.y * kSliceRows32 + tid;
@@ -948,24 +964,26 @@ k_slice_terms32(PathView v, AzizF az, BoxF B, int window, int even, int odd, uns
         if (!last) return;
         __threadfence();
     }
-    // the columns' sums, in double-float over the warp, FP64 from there on
-    #pragma unroll 1
-    for (int q = 0; q < 8; ++q) {
-        float2 t = make_float2(0.f, 0.f);
-        for (int c = tid; c < kSliceColumns32; c += kSliceRows32) {
+    // the columns' sums widened to FP64 and added over the warps' 32 columns,
+    // then the four groups of columns in order
+    const int lane = tid & 31;
+    for (int g = tid >> 5; g < kSliceColumns32 / 32; g += kSliceRows32 / 32) {
+        const int c = 32 * g + lane;
+        double x[8];
+        #pragma unroll
+        for (int q = 0; q < 8; ++q) {
             KahanF k;
             if (q == 0) {
                 if (c < n) { k.s = __ldcg(W + c); k.c = __ldcg(W + (size_t)8 * Ne + c); }
             } else
                 for (int b = c; b < n; b += kSliceColumns32) k.add(__ldcg(W + (size_t)q * Ne + b));
-            const float2 u = warp_ff(k);
-            const float sum = t.x + u.x, bp = sum - t.x;
-            t = make_float2(sum, (t.y + u.y) + ((t.x - (sum - bp)) + (u.x - bp)));
+            x[q] = k.value();
         }
-        if ((tid & 31) == 0) sums[q][tid >> 5] = (double)t.x + (double)t.y;
+        const double t = warp_sum8(x, lane);
+        if ((lane & 3) == 0) sums[lane >> 2][g] = t;
     }
     __syncthreads();
-    if (tid < 8) terms[(size_t)tid * v.M + s] = sums[tid][0] + sums[tid][1];
+    if (tid < 8) terms[(size_t)tid * v.M + s] = sums[tid][0] + sums[tid][1] + sums[tid][2] + sums[tid][3];
 }
 
 static int slice_blocks32(int Ne) { return (Ne + kSliceRows32 - 1) / kSliceRows32; }
