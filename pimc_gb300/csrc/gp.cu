@@ -239,7 +239,7 @@ struct GpF { float ps[3], si[3], il[3]; };
 template <int NU2>
 __global__ void __launch_bounds__(kGpThreads32)
 k_gp32(GpDev g, GpF f, const float4* __restrict__ train, const float4* __restrict__ points, int count,
-       int chunk, unsigned* __restrict__ arrived, float2* __restrict__ part, double* __restrict__ out) {
+       int chunk, float2* __restrict__ part, double* __restrict__ out) {
     __shared__ float4 tile[kGpTile];
     const int kb = blockIdx.y * chunk, ke = min(g.n, kb + chunk);
     int i[2];
@@ -288,20 +288,27 @@ k_gp32(GpDev g, GpF f, const float4* __restrict__ train, const float4* __restric
         if (split) part[(size_t)blockIdx.y * count + i[p]] = make_float2(hi[p], lo[p]);
         else out[i[p]] = gp_value(g, (double)hi[p] + (double)lo[p]);
     }
-    if (!split || !gp_last(arrived)) return;
-    #pragma unroll
-    for (int p = 0; p < 2; ++p) {
-        if (i[p] >= count) continue;
-        // leading parts by TwoSum, the trailing parts with their errors
-        float h = 0.f, l = 0.f;
-        #pragma unroll 8
-        for (int s = 0; s < gridDim.y; ++s) {
-            const float2 x = __ldcg(part + (size_t)s * count + i[p]);
-            two_sum_acc(h, l, x.x);
-            l += x.y;
+}
+
+// The chunks' parts added in FP64, kGpLanes threads a point.  (Four FP64
+// instructions a part: the last CTA of a block of points to arrive would take
+// 19 us for 256 points and 76 chunks.)
+constexpr int kGpLanes = 4;
+
+__global__ void __launch_bounds__(128)
+k_gp32_sums(GpDev g, const float2* __restrict__ part, int nsplit, int count, double* __restrict__ out) {
+    const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) / kGpLanes), lane = threadIdx.x % kGpLanes;
+    double acc = 0.0;
+    if (i < count) {
+        #pragma unroll 4
+        for (int s = lane; s < nsplit; s += kGpLanes) {
+            const float2 x = part[(size_t)s * count + i];
+            acc += (double)x.x + (double)x.y;
         }
-        out[i[p]] = gp_value(g, (double)h + (double)l);
     }
+    #pragma unroll
+    for (int o = 1; o < kGpLanes; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (i < count && lane == 0) out[i] = gp_value(g, acc);
 }
 
 // --------------------------------------------------------------------------
@@ -451,7 +458,7 @@ cudaError_t launch_gp(pgb_gp* h, const double* d_pos, int count, double* d_out) 
         if (e != cudaSuccess) { h->d_part = nullptr; return e; }
         h->part_bytes = need;
     }
-    if (nsplit > 1 && bx > h->arrived_blocks) {
+    if (h->p.precision != PGB_MIXED && nsplit > 1 && bx > h->arrived_blocks) {
         if (h->d_arrived) { cudaStreamSynchronize(h->stream); cudaFree(h->d_arrived); h->d_arrived = nullptr; h->arrived_blocks = 0; }
         const int blocks = std::max(bx, 4 * 152);        // more blocks than that take one chunk
         cudaError_t e = cudaMalloc(&h->d_arrived, blocks * sizeof(unsigned));
@@ -468,8 +475,12 @@ cudaError_t launch_gp(pgb_gp* h, const double* d_pos, int count, double* d_out) 
             for (int d = 0; d < 3; ++d) { f.ps[d] = (float)g.pside[d]; f.si[d] = (float)g.sideInv[d]; f.il[d] = (float)g.invell[d]; }
             float4* r = reinterpret_cast<float4*>(base);
             k_gp_points<float4><<<(count + 127) / 128, 128, 0, h->stream>>>(g, d_pos, count, r);
-            k32<<<grid, kGpThreads32, 0, h->stream>>>(g, f, h->d_train32, r, count, chunk, h->d_arrived,
-                                                      reinterpret_cast<float2*>(base + points), d_out);
+            float2* part = reinterpret_cast<float2*>(base + points);
+            k32<<<grid, kGpThreads32, 0, h->stream>>>(g, f, h->d_train32, r, count, chunk, part, d_out);
+            if (nsplit > 1) {
+                const int each = 128 / kGpLanes;
+                k_gp32_sums<<<(count + each - 1) / each, 128, 0, h->stream>>>(g, part, nsplit, count, d_out);
+            }
         } else {
             double4* r = reinterpret_cast<double4*>(base);
             k_gp_points<double4><<<(count + 127) / 128, 128, 0, h->stream>>>(g, d_pos, count, r);
