@@ -590,7 +590,10 @@ typedef struct {
     double sigma2;
     double side[3];
     int    periodic[3];
-    int    precision;          /* PGB_FP64: the CPU form up to an ulp of sqrt and exp;
+    int    precision;          /* PGB_FP64: the CPU form with a root within half an ulp, an
+                                  exponential within 1.01 ulp and, unless a call has so many
+                                  points that they fill the device (155 thousand), the
+                                  training points' sum in chunks of 8 rows or more;
                                   PGB_MIXED: FP32 kernel values, compensated sum */
 } pgb_gp_params;
 int pgb_gp_create(const pgb_gp_params* p, const double* training /* [n][4] */, int n,
@@ -601,6 +604,9 @@ void* pgb_gp_stream(pgb_gp* gp);
 /* GaussianProcessPotential::GP(const dVec*, double*, int), positions AoS */
 int pgb_gp_eval(pgb_gp* gp, const double* pos, double* values, int count);
 int pgb_gp_eval_device_async(pgb_gp* gp, const double* d_pos, double* d_values, int count);
+/* Self-check of the FP64 form's functions: out[i] of x[i] on the device, what =
+ * 0 sqrt(x), 1 x / 3, 2 exp(-x), 3 1 / sqrt(x) */
+int pgb_gp_math_check(const double* x, int n, int what, double* out);
 /* GPHeBenzenePotential::V(const dVec*, double*, int) (src/potential.cpp:
  * 5610-5681): symmetry fold, hard core 10000 K, GP, long-range switch */
 int pgb_gp_benzene_v(pgb_gp* gp, const double* pos, double* values, int count);

@@ -195,6 +195,7 @@ _SIGS = {
     "pgb_gp_stream": (C.c_void_p, [_VP]),
     "pgb_gp_eval": (C.c_int, [_VP, _DP, _DP, C.c_int]),
     "pgb_gp_eval_device_async": (C.c_int, [_VP, _VP, _VP, C.c_int]),
+    "pgb_gp_math_check": (C.c_int, [_DP, C.c_int, C.c_int, _DP]),
     "pgb_gp_benzene_v": (C.c_int, [_VP, _DP, _DP, C.c_int]),
     "pgb_plain_set_rng": (C.c_int, [_VP, C.POINTER(C.c_uint32)]),
     "pgb_walkers_get_all_positions": (C.c_int, [_VP, _DP]),

@@ -23,7 +23,7 @@
 // GPHeBenzenePotential::V (src/potential.cpp:5610-5681): points are folded
 // into the 30-degree wedge of the ring's symmetry on the device, passed
 // through the GP, then switched to the long-range form beyond the core.
-#include "pgb_device.cuh"
+#include "pair64.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -57,23 +57,23 @@ __device__ __forceinline__ double third(double x) {
     return __fma_rn(__fma_rn(-3.0, q, x), k, q);
 }
 
-// sqrt(d) for 2^-960 <= d < 2^960 from the hardware's 20-bit reciprocal root,
-// Householder's third-order step and one residual correction: within an ulp
-// of the correctly rounded root, 9 FP64 instructions
+// sqrt(d) for 2^-960 <= d < 2^960: r = d / sqrt(d) and one step of Newton's
+// iteration for the root, r + (d - r^2) / 2 r, with the reciprocal root in the
+// place of 1 / r and the residual exact (P. W. Markstein, IBM J. Res. Dev. 34,
+// 1990).  Half an ulp and 2^-100: correctly rounded but for near ties; 9 FP64
+// instructions
 __device__ __forceinline__ double root64(double d) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-    const double e = __fma_rn(-(d * y), y, 1.0);
-    y = __fma_rn(y * e, __fma_rn(0.375, e, 0.5), y);
-    const double r = d * y;
+    const double y = inv_root64(d), r = d * y;
     return __fma_rn(__fma_rn(-r, r, d), 0.5 * y, r);
 }
 
 // exp(-x), x >= 0, by Tang's table method (ACM TOMS 15, 1989): with
 // n = round(-64 x / ln 2), exp(-x) = 2^(n/64) exp(-x - n ln 2 / 64), the first
 // factor from the 64 tabulated 2^(j/64), the second, whose argument is below
-// ln 2 / 128, from five Taylor terms (relative remainder 4e-17).  Ten FP64
-// instructions where exp() takes about forty; below one ulp in all.
+// ln 2 / 128, from six Taylor terms (relative remainder 3e-20).  Eleven FP64
+// instructions where exp() takes about forty.  Half an ulp of the table, half
+// an ulp of the last rounding and a hundredth for the argument and the series:
+// within 1.01 ulp, and from 700 on (and for NaN) exp() itself.
 constexpr int kExpTable = 64;
 __device__ __forceinline__ double exp_neg64(double x, const double* T) {
     if ((unsigned)__double2hiint(x) >= 0x4085E000u) return exp(-x);     // 700 and up, NaN
@@ -81,14 +81,23 @@ __device__ __forceinline__ double exp_neg64(double x, const double* T) {
     const double t = __fma_rn(x, -92.332482616893657, magic);         // 64 / ln 2
     const int n = __double2loint(t);
     const double f = t - magic;
-    // ln 2 / 64 in two parts; f times the first is exact
+    // ln 2 / 64 in two parts, those of fdlibm's exp (Sun Microsystems, 1993) a
+    // 64th; f times the first is exact
     double r = __fma_rn(f, -6.93147180369123816490e-01 / 64.0, -x);
     r = __fma_rn(f, -1.90821492927058770002e-10 / 64.0, r);
-    const double q = __fma_rn(r, __fma_rn(r, __fma_rn(r, 1.0 / 120.0, 1.0 / 24.0), 1.0 / 6.0), 0.5);
+    const double q = __fma_rn(r, __fma_rn(r, __fma_rn(r, __fma_rn(r, 1.0 / 720.0, 1.0 / 120.0), 1.0 / 24.0), 1.0 / 6.0), 0.5);
     const double p = __fma_rn(r * r, q, r);
     const double s = T[n & (kExpTable - 1)];
     const double y = __fma_rn(s, p, s);
     return __hiloint2double(__double2hiint(y) + ((n >> 6) << 20), __double2loint(y));
+}
+
+// the three functions and the reciprocal root by themselves, for their test
+__global__ void k_gp_math(const double* __restrict__ x, int n, int what, const double* __restrict__ table,
+                          double* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    out[i] = what == 0 ? root64(x[i]) : what == 1 ? third(x[i]) : what == 2 ? exp_neg64(x[i], table) : inv_root64(x[i]);
 }
 
 template <int NU2>
@@ -619,6 +628,24 @@ int pgb_gp_eval(pgb_gp* h, const double* pos, double* values, int count) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return h->cfail(e, "GP eval");
     return PGB_OK;
+}
+
+int pgb_gp_math_check(const double* x, int n, int what, double* out) {
+    if (n <= 0 || !x || !out || what < 0 || what > 3) return PGB_EINVAL;
+    double t[kExpTable];
+    for (int j = 0; j < kExpTable; ++j) t[j] = std::exp2(j / 64.0);
+    double* d = nullptr;
+    const size_t nb = (size_t)n * sizeof(double);
+    cudaError_t e = cudaMalloc(&d, 2 * nb + sizeof(t));
+    if (e == cudaSuccess) e = cudaMemcpy(d, x, nb, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d + 2 * (size_t)n, t, sizeof(t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        k_gp_math<<<(n + 255) / 256, 256>>>(d, n, what, d + 2 * (size_t)n, d + n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, d + n, nb, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? PGB_OK : PGB_ECUDA;
 }
 
 int pgb_gp_benzene_v(pgb_gp* h, const double* pos, double* values, int count) {

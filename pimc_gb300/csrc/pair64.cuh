@@ -15,7 +15,7 @@ namespace pgb {
 //     same FP64 value as min_image's.
 //   * 1/r is the hardware's 20-bit reciprocal root refined by one step of
 //     Householder's third-order iteration, y (1 + e/2 + 3 e^2/8) with
-//     e = 1 - r^2 y^2; the error left is 5 e^3 / 16 < 2^-54.
+//     e = 1 - r^2 y^2; the series leaves 5 e^3 / 16 < 2^-54.
 //   * The table index int(r / dr) is read off the bits of r (1/dr) + 1.5 2^32,
 //     whose last place is 2^-20.
 // A pair whose FP32 fraction lies within kImageEdge of an image boundary, or
@@ -32,6 +32,15 @@ struct Pair64 {
 // A box fraction (FP32 position times FP32 1/L) is within 3 2^-24 for |u| <= 1,
 // the difference of two within 4.2e-7: below the edge.
 constexpr float kImageEdge = 1.0e-6f;
+
+// 1 / sqrt(d), 2^-960 <= d < 2^960, within 2^-52 of it: half an ulp of e, the
+// last rounding, and the series' remainder
+__device__ __forceinline__ double inv_root64(double d) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = __fma_rn(-(d * y), y, 1.0);
+    return __fma_rn(y * e, __fma_rn(0.375, e, 0.5), y);
+}
 
 // x / L for the image screen; NaN outside the range where its error bound holds
 __device__ __forceinline__ float box_fraction(float x, float Linv) {
@@ -71,10 +80,7 @@ __device__ __forceinline__ Pair64 pair64(const PathView& v, double invdr, double
     p.dy = image64(y, uy, v.side[1], ok);
     p.dz = image64(z, uz, v.side[2], ok);
     p.r2 = dot3(make_double3(p.dx, p.dy, p.dz), make_double3(p.dx, p.dy, p.dz));
-    double y0;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(p.r2));
-    const double e = __fma_rn(-(p.r2 * y0), y0, 1.0);
-    p.y = __fma_rn(y0 * e, __fma_rn(0.375, e, 0.5), y0);
+    p.y = inv_root64(p.r2);
     const double t = __fma_rn(p.r2 * p.y, invdr, 6442450944.0);      // 1.5 2^32
     const long long b = __double_as_longlong(t);
     const unsigned frac = (unsigned)b & 0xFFFFFu;
