@@ -507,33 +507,10 @@ int pgb_load_positions_device_async(pgb_ctx* h, const double* d_pos) {
 }
 
 int pgb_update_beads(pgb_ctx* h, const int32_t* beads, const double* pos, int k) {
-    if (check_ctx(h) || k < 0 || (k > 0 && (!beads || !pos))) return PGB_EINVAL;
+    if (check_ctx(h)) return PGB_EINVAL;
     Ctx& c = h->c;
-    int rc = need_path(c); if (rc) return rc;
-    if (k == 0) return PGB_OK;
-    for (int i = 0; i < k; ++i)
-        if (beads[2*i] < 0 || beads[2*i] >= c.M || beads[2*i+1] < 0 || beads[2*i+1] >= c.Ne)
-            return c.fail(PGB_EINVAL, "update_beads: bead out of range");
-    size_t bb = (size_t)k * sizeof(int2), pb = (size_t)k * 3 * sizeof(double);
-    char* in = c.stage.take(bb + pb, c.stream);              // read by the kernel; no wait
-    const bool direct = in != nullptr;
-    if (!direct) {
-        rc = c.ensure_scratch(bb + pb + 64); if (rc) return rc;
-        rc = c.ensure_pinned(bb + pb + 64); if (rc) return rc;
-        in = static_cast<char*>(c.h_pinned);
-    }
-    std::memcpy(in, beads, bb);
-    std::memcpy(in + bb, pos, pb);
-    const char* dp = in;
-    if (!direct) {
-        PGB_CUDA(&c, cudaMemcpyAsync(c.d_scratch, in, bb + pb, cudaMemcpyHostToDevice, c.stream));
-        dp = static_cast<char*>(c.d_scratch);
-    }
-    k_update_beads<<<(k + 127) / 128, 128, 0, c.stream>>>(c.d_pos, c.d_pos32, c.Ne,
-        reinterpret_cast<const int2*>(dp), reinterpret_cast<const double*>(dp + bb), k);
-    PGB_CUDA(&c, cudaGetLastError());
-    if (!direct) PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
-    c.force_valid = false;
+    int rc = queue_update_beads(c, beads, pos, k); if (rc) return rc;
+    PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
     return PGB_OK;
 }
 
@@ -575,7 +552,10 @@ int pgb_set_beads(pgb_ctx* h, const int32_t* beads, const double* pos, const int
     c.h_nbs = nbs2;
     c.numBeadsOn = total;
     c.lk_valid = false;
-    return upload_beads(c, lin.data(), k, aos.data());
+    rc = upload_beads(c, lin.data(), k, aos.data());
+    if (rc) return rc;
+    PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
+    return PGB_OK;
 }
 
 int pgb_set_worm(pgb_ctx* h, const int32_t* worm8) {
@@ -1354,9 +1334,39 @@ int pgb_permutation_cycles(pgb_ctx* h, double* out40) {
 }  // extern "C"
 
 namespace pgb {
+int queue_update_beads(Ctx& c, const int32_t* beads, const double* pos, int k) {
+    if (k < 0 || (k > 0 && (!beads || !pos))) return PGB_EINVAL;
+    int rc = need_path(c); if (rc) return rc;
+    if (k == 0) return PGB_OK;
+    for (int i = 0; i < k; ++i)
+        if (beads[2*i] < 0 || beads[2*i] >= c.M || beads[2*i+1] < 0 || beads[2*i+1] >= c.Ne)
+            return c.fail(PGB_EINVAL, "update_beads: bead out of range");
+    size_t bb = (size_t)k * sizeof(int2), pb = (size_t)k * 3 * sizeof(double);
+    char* in = c.stage.take(bb + pb, c.stream);              // read by the kernel
+    const bool direct = in != nullptr;
+    if (!direct) {
+        rc = c.ensure_scratch(bb + pb + 64); if (rc) return rc;
+        rc = c.ensure_pinned(bb + pb + 64); if (rc) return rc;
+        in = static_cast<char*>(c.h_pinned);
+    }
+    std::memcpy(in, beads, bb);
+    std::memcpy(in + bb, pos, pb);
+    const char* dp = in;
+    if (!direct) {
+        PGB_CUDA(&c, cudaMemcpyAsync(c.d_scratch, in, bb + pb, cudaMemcpyHostToDevice, c.stream));
+        dp = static_cast<char*>(c.d_scratch);
+    }
+    k_update_beads<<<(k + 127) / 128, 128, 0, c.stream>>>(c.d_pos, c.d_pos32, c.Ne,
+        reinterpret_cast<const int2*>(dp), reinterpret_cast<const double*>(dp + bb), k);
+    PGB_CUDA(&c, cudaGetLastError());
+    if (!direct) PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
+    c.force_valid = false;
+    return PGB_OK;
+}
+
 int upload_beads(Ctx& c, const int* lin, int k, const double* pos_aos) {
     const size_t rb = (size_t)k * sizeof(BeadRec), nb = c.M * sizeof(int);
-    char* in = c.stage.take(rb + nb, c.stream);              // read by the kernel; no wait
+    char* in = c.stage.take(rb + nb, c.stream);              // read by the kernel
     const bool direct = in != nullptr;
     if (!direct) {
         int rc = c.ensure_scratch(rb + nb); if (rc) return rc;

@@ -144,6 +144,9 @@ struct Ctx {
 // (h_next, h_prev, h_on; positions from pos_aos [M][Ne][3]) and numBeadsAtSlice
 // to the device, before any later work on the stream.
 int upload_beads(Ctx& c, const int* lin, int k, const double* pos_aos);
+// pgb_update_beads without its wait: new positions of the listed beads before
+// any later work on the stream, the host arrays reusable at once
+int queue_update_beads(Ctx& c, const int32_t* beads, const double* pos, int k);
 
 #define PGB_CUDA(ctx, call)                                              \
     do {                                                                 \

@@ -117,7 +117,7 @@ struct Plain {
             bl.push_back(beads[i][0]); bl.push_back(beads[i][1]);
             for (int d = 0; d < 3; ++d) { pl.push_back(p[i][d]); pos[((size_t)beads[i][0] * c.Ne + beads[i][1]) * 3 + d] = p[i][d]; }
         }
-        err = pgb_update_beads(reinterpret_cast<pgb_ctx*>(&c), bl.data(), pl.data(), (int)beads.size());
+        err = pgb::queue_update_beads(c, bl.data(), pl.data(), (int)beads.size());
     }
     double action_list(const std::vector<Bead>& beads) {
         flush();
@@ -1112,6 +1112,7 @@ int pgb_plain_run(pgb_ctx* h, const pgb_move_params* mp, int nsteps, int32_t* tr
             energies[step] = e[8];
         }
     }
+    PGB_CUDA(&c, cudaStreamSynchronize(c.stream));           // the last move's positions
     if (trace_len) *trace_len = ntr;
     if (stats) *stats = pl.st;
     return PGB_OK;
@@ -1209,6 +1210,7 @@ extern "C" int pgb_plain_worm_run(pgb_ctx* h, const pgb_worm_params* wp, int nst
     }
     pl.flush();
     if (pl.err) return pl.err;
+    PGB_CUDA(&c, cudaStreamSynchronize(c.stream));
     pl.wst.diagonal = c.w_diag ? 1 : 0;
     if (trace_len) *trace_len = ntr;
     if (stats) *stats = pl.wst;
