@@ -722,7 +722,7 @@ __device__ __forceinline__ double3 link64(const PathView& v, double3 a, float3 u
 
 // The sum over g < window of the displacement from a bead to its g-th
 // neighbour along `link`, the displacement to the window-th one and the first
-// step; an open end stops the walk.
+// step.  An open end stops the walk, and stands for the neighbours behind it.
 struct ChainSums { double3 sum, reach, step; };
 __device__ __forceinline__ ChainSums chain64(const PathView& v, const int2* __restrict__ link, int s, int p, int window) {
     ChainSums c{};
@@ -731,8 +731,8 @@ __device__ __forceinline__ ChainSums chain64(const PathView& v, const int2* __re
     float3 u = fraction64(v, at);
     for (int g = 0; g < window; ++g) {
         c.sum.x += c.reach.x; c.sum.y += c.reach.y; c.sum.z += c.reach.z;
-        at = link[(size_t)at.x * v.Ne + at.y];
-        if (at.x < 0) break;
+        if (at.x >= 0) at = link[(size_t)at.x * v.Ne + at.y];
+        if (at.x < 0) continue;
         const double3 q = pos64(v, at);
         const float3 w = fraction64(v, at);
         const double3 d = link64(v, q, w, r, u);

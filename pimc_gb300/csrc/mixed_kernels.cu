@@ -909,7 +909,7 @@ k_slice_terms32(PathView v, AzizF az, BoxF B, int window, int even, int odd, uns
                         if (cn.x >= 0) cn = v.next[(size_t)cn.x * Ne + cn.y];
                         if (cp.x >= 0) cp = v.prev[(size_t)cp.x * Ne + cp.y];
                     }
-                    // an open end stops the walk
+                    // an open end stops the walk, and stands for the neighbours behind it
                     const float4 qn = cn.x >= 0 ? v.pos32[(size_t)cn.x * Ne + cn.y] : pn;
                     const float4 qp = cp.x >= 0 ? v.pos32[(size_t)cp.x * Ne + cp.y] : pp;
                     mx += min_image32(qn.x - pn.x, B.L0, B.I0); my += min_image32(qn.y - pn.y, B.L1, B.I1);
