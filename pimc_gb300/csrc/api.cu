@@ -337,7 +337,7 @@ int pgb_create(const pgb_params* p, pgb_ctx** out) {
         if ((e = cudaMalloc(&c.d_on, nb)) != cudaSuccess) break;
         if ((e = cudaMalloc(&c.d_nbs, c.M * sizeof(int))) != cudaSuccess) break;
         if (p->precision == PGB_MIXED)
-            if ((e = cudaMalloc(&c.d_trial_count, (2 * nb + 1) * sizeof(int))) != cudaSuccess) break;
+            if ((e = cudaMalloc(&c.d_trial_count, (2 * nb + 2) * sizeof(int))) != cudaSuccess) break;
         if ((e = cudaMalloc(&c.d_arrived, c.M * sizeof(unsigned))) != cudaSuccess) break;
         if ((e = cudaMemsetAsync(c.d_arrived, 0, c.M * sizeof(unsigned), c.stream)) != cudaSuccess) break;
         if ((e = cudaMalloc(&c.d_hist, 64 * sizeof(unsigned long long))) != cudaSuccess) break;

@@ -396,9 +396,8 @@ cudaError_t launch_bead_actions32_full(const PathView& v, AzizParams a, const in
 // action and, for the gradient term, every partner's force less the bead's
 // own term: the same for all trials of the bead.  The trials are sorted by
 // bead on the device (count, offsets, scatter: the sorted record is the FP32
-// position and the trial's index), a warp takes a bead, evaluates its current
-// position once, keeps the partners (and those forces) in shared memory and
-// then makes the trials four at a time, so four independent chains of pair
+// position and the trial's index), a warp takes a bead and a run of its trials, evaluates its current position once, keeps the partners (and
+// those forces) in shared memory and then makes the trials four at a time, so four independent chains of pair
 // arithmetic are in flight.  The sums of a group are reduced together by
 // recursive halving, in the butterfly's own tree, so every sum has the bits
 // k_bead_actions32_full gives it; the FP64 assembly runs one trial a lane.
@@ -409,8 +408,18 @@ cudaError_t launch_bead_actions32_full(const PathView& v, AzizParams a, const in
 // and the reductions are not inlined (1.01 -> 0.87 ms).  10^6 trials, N = 256,
 // M = 250, GSF: 2.75 ms with both positions evaluated for every trial, 0.87 ms
 // here.
+//
+// A run is as long as two average beads' trials and 16 more, so that evenly
+// spread trials stay whole.  A second launch makes the trials of a bead
+// beyond its first run, which go to the warps by their place: of a run's length
+// of consecutive sorted trials at most one starts another run, and it belongs
+// to the bead of the first of them.  With all trials of a bead on one warp, 10^6
+// trials of one slice's 256 beads took 4.6 ms, of one worldline's 250 beads 7.9
+// ms, 10^5 trials of one bead of 64 particles 51 ms; 1.2, 0.95 and 0.18 ms here
+// (unsorted 2.7, 2.6 and 0.15).
 // ---------------------------------------------------------------------------
 constexpr int kTrialWarps = 4;
+constexpr int kTrialRun = 32;                    // trials in a run at least, and their step
 // Sorting pays from about three trials a bead on (N = 256, gradient: 2 a bead
 // 306 against 374 us, 4 a bead 398 against 719; N = 400: 2 a bead 227 against
 // 220, 4 a bead 282 against 395) once its three small launches, 12 us, are
@@ -434,13 +443,16 @@ __global__ void k_trial_count(PathView v, const int2* __restrict__ beads, int k,
 }
 
 // a slice's beads get consecutive places; the slices any order
+// (cursor[0] ends as the number of trials; cursor[1] tells that a bead has more
+// than a run)
 __global__ void __launch_bounds__(256)
-k_trial_offsets(PathView v, const int* __restrict__ count, int* __restrict__ cursor, int* __restrict__ offset) {
+k_trial_offsets(PathView v, const int* __restrict__ count, int run, int* __restrict__ cursor, int* __restrict__ offset) {
     __shared__ int wsum[8], s_base;
     const int s = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int b0 = 0; b0 < v.Ne; b0 += 256) {
         const int b = b0 + threadIdx.x;
         const int c = b < v.Ne ? count[(size_t)s * v.Ne + b] : 0;
+        if (c > run) cursor[1] = 1;
         int x = c;
         #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -579,10 +591,12 @@ __device__ __forceinline__ void trial_group(const float4* __restrict__ trial, in
     __syncwarp();
 }
 
+// the beads' first runs, or (kRuns) the others
+template <bool kRuns>
 __global__ void __launch_bounds__(kTrialWarps * 32, 5)
-k_trials32(PathView v, AzizF az, BoxF B, const int* __restrict__ count, const int* __restrict__ offset,
-           const float4* __restrict__ sorted, const float4* __restrict__ fall, int shift, int mode,
-           const Scales32 sc, double* __restrict__ out) {
+k_trials32(PathView v, AzizF az, BoxF B, const int2* __restrict__ beads, const int* __restrict__ count,
+           const int* __restrict__ cursor, const int* __restrict__ offset, const float4* __restrict__ sorted,
+           const float4* __restrict__ fall, int run, int shift, int mode, const Scales32 sc, double* __restrict__ out) {
     extern __shared__ float4 sp[];
     __shared__ TrialBuffer buffers[kTrialWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, Ne = v.Ne;
@@ -617,17 +631,32 @@ k_trials32(PathView v, AzizF az, BoxF B, const int* __restrict__ count, const in
         used = 0;
         __syncwarp();
     };
-    const size_t beads = (size_t)v.M * Ne;
-    for (size_t b = (size_t)blockIdx.x * kTrialWarps + warp; b < beads; b += (size_t)gridDim.x * kTrialWarps) {
-        // the even slices' beads, then the odd ones': an SM's warps run the
-        // same loops, whose code does not fit the instruction cache together
-        const int line = (int)(b / Ne), p = (int)(b - (size_t)line * Ne), evens = (v.M + 1) / 2;
-        const int s = line < evens ? 2 * line : 2 * (line - evens) + 1;
-        const size_t at = (size_t)s * Ne + p;
-        const int n = count[at];
-        if (n == 0) continue;
+    if (kRuns && !cursor[1]) return;
+    const size_t items = kRuns ? ((size_t)cursor[0] + run - 1) / run : (size_t)v.M * Ne;
+    for (size_t b = (size_t)blockIdx.x * kTrialWarps + warp; b < items; b += (size_t)gridDim.x * kTrialWarps) {
+        int s, p, n, first;
+        if (kRuns) {
+            const int place = (int)(b * run);
+            const int2 bead = beads[__float_as_int(sorted[place].w)];
+            s = bead.x; p = bead.y;
+            const size_t at = (size_t)s * Ne + p;
+            const int o = offset[at];
+            first = o + (place - o + run - 1) / run * run;
+            n = min(o + count[at] - first, run);
+            if (first == o || n <= 0) continue;
+        } else {
+            // the even slices' beads, then the odd ones': an SM's warps run the
+            // same loops, whose code does not fit the instruction cache together
+            const int line = (int)(b / Ne), evens = (v.M + 1) / 2;
+            p = (int)(b - (size_t)line * Ne);
+            s = line < evens ? 2 * line : 2 * (line - evens) + 1;
+            const size_t at = (size_t)s * Ne + p;
+            n = min(count[at], run);
+            if (n == 0) continue;
+            first = offset[at];
+        }
         const bool need_c = s % 2 ? odd_c : even_c;
-        const float4* trial = sorted + offset[at];
+        const float4* trial = sorted + first;
         // the current position, and the partners for the trials
         const float4* R = v.pos32 + (size_t)s * Ne;
         const float4* Fs = fall + (size_t)s * Ne;
@@ -690,21 +719,27 @@ cudaError_t launch_trials32(const PathView& v, AzizParams a, const int2* d_beads
                             double lambda, const double vf[2], const double gf[2], const double* d_pos,
                             const float4* d_force, int* d_count, float4* d_sorted, double* d_out, cudaStream_t s) {
     const size_t nb = (size_t)v.M * v.Ne, smem = (size_t)v.Ne * 2 * kTrialWarps * sizeof(float4);
-    int *offset = d_count + nb + 1, *cursor = d_count + nb;
-    cudaError_t e = set_smem_limit(k_trials32, 160 * 1024);
+    int *offset = d_count + nb + 2, *cursor = d_count + nb;
+    cudaError_t e = set_smem_limit(k_trials32<false>, 160 * 1024);
+    if (e == cudaSuccess) e = set_smem_limit(k_trials32<true>, 160 * 1024);
     if (e != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(d_count, 0, (nb + 1) * sizeof(int), s)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(d_count, 0, (nb + 2) * sizeof(int), s)) != cudaSuccess) return e;
     const int blocks = (k + 255) / 256;
     k_trial_count<<<blocks, 256, 0, s>>>(v, d_beads, k, d_count, d_out);
-    k_trial_offsets<<<v.M, 256, 0, s>>>(v, d_count, cursor, offset);
+    const int run = std::max<int>(kTrialRun, (int)((2.0 * k / nb + 47.0) / 32.0) * 32);
+    k_trial_offsets<<<v.M, 256, 0, s>>>(v, d_count, run, cursor, offset);
     k_trial_scatter<<<blocks, 256, 0, s>>>(v, d_beads, d_pos, k, offset, d_sorted, d_out);
     const BoxF B = box_f(v);
     // two beads a warp: the assembly's lanes half full, the CTAs short enough
     // to even out (eight beads a warp 1.05 ms, two 1.01)
     const size_t each = std::max<size_t>(1, std::min<size_t>(2, nb / (152 * 16)));
     const int grid = (int)((nb + kTrialWarps * each - 1) / (kTrialWarps * each));
-    k_trials32<<<grid, kTrialWarps * 32, smem, s>>>(v, make_aziz_f(a), B, d_count, offset, d_sorted, d_force, shift, mode,
-                                                    scales32(shift, tau, lambda, vf, gf), d_out);
+    const AzizF az = make_aziz_f(a);
+    const Scales32 sc = scales32(shift, tau, lambda, vf, gf);
+    k_trials32<false><<<grid, kTrialWarps * 32, smem, s>>>(v, az, B, d_beads, d_count, cursor, offset, d_sorted, d_force, run,
+                                                           shift, mode, sc, d_out);
+    k_trials32<true><<<std::min(152 * 5, (k / run + kTrialWarps) / kTrialWarps), kTrialWarps * 32, smem, s>>>(
+        v, az, B, d_beads, d_count, cursor, offset, d_sorted, d_force, run, shift, mode, sc, d_out);
     return cudaGetLastError();
 }
 

@@ -203,7 +203,7 @@ cudaError_t launch_bead_actions32_full(const PathView& v, AzizParams az, const i
                                        const float4* d_force, int delta, double* d_out,
                                        cudaStream_t s);
 // trials sorted by bead, for whole lists and enough trials a bead
-// (trials32_sorted): d_count 2 M Ne + 1 ints, d_sorted k records
+// (trials32_sorted): d_count 2 M Ne + 2 ints, d_sorted k records
 bool trials32_sorted(const PathView& v, int k);
 cudaError_t launch_trials32(const PathView& v, AzizParams a, const int2* d_beads, int k, int shift, int mode, double tau,
                             double lambda, const double vf[2], const double gf[2], const double* d_pos,
