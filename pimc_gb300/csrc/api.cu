@@ -939,10 +939,12 @@ int pgb_qvectors(const char* type, const char* input, const double side[3], doub
 // ---------------------------------------------------------------------------
 namespace {
 
-// work layout: rho_q (room for FP64 values), then for the FP32 path the slices
-// as box fractions, then the tensor-core scratch
-size_t rho_region(const Ctx& c, int nq) {
-    return ((size_t)nq * c.M * 2 * sizeof(double) + 255) & ~(size_t)255;
+// work layout: rho_q (none where the tensor-core form splits it as it is made),
+// then for the FP32 path the slices as box fractions, then the tensor-core scratch
+size_t rho_region(const Ctx& c, int nq, int what, int mode) {
+    const bool fp32 = c.p.precision == PGB_MIXED && what != 2;
+    const size_t each = !fp32 ? 2 * sizeof(double) : what == 1 && mode == 1 ? 0 : sizeof(float2);
+    return ((size_t)nq * c.M * each + 255) & ~(size_t)255;
 }
 size_t posbuf_region(const Ctx& c, int nq) {
     return (c.p.precision == PGB_MIXED) ? ((rhoq32_work_bytes(c.view(), nq) + 255) & ~(size_t)255) : 0;
@@ -968,7 +970,7 @@ int scatter_common(Ctx& c, const double* d_q, int nq, int what, int mode, double
         }
     } else {
         float2* d_rho = static_cast<float2*>(d_work);
-        void* posbuf = static_cast<char*>(d_work) + rho_region(c, nq);
+        void* posbuf = static_cast<char*>(d_work) + rho_region(c, nq, what, mode);
         if (what == 1 && mode == 1) {
             if (!isf_tc_supported(c.M))
                 return c.fail(PGB_EINVAL, "tensor-core F(q,tau) needs M a multiple of 128 and <= 2048");
@@ -978,7 +980,7 @@ int scatter_common(Ctx& c, const double* d_q, int nq, int what, int mode, double
                 e = isf_tc_build_tables(c.M, c.d_tc_tables, c.stream);
                 if (e != cudaSuccess) return c.cuda_fail(e, "F(q,tau) tables");
             }
-            void* tc = static_cast<char*>(d_work) + rho_region(c, nq) + posbuf_region(c, nq);
+            void* tc = static_cast<char*>(d_work) + rho_region(c, nq, what, mode) + posbuf_region(c, nq);
             const IsfOperand split = isf_tc_operand(nq, c.M, tc);
             e = launch_rhoq32(v, d_q, nq, nullptr, posbuf, c.stream, 0.0, &split);
             if (e == cudaSuccess) e = launch_isf_tc(nq, c.M, norm, d_out, tc, c.d_tc_tables, c.stream);
@@ -996,7 +998,7 @@ int scatter_common(Ctx& c, const double* d_q, int nq, int what, int mode, double
 size_t scatter_work_bytes(const Ctx& c, int nq, int what, int mode) {
     size_t extra = (c.p.precision == PGB_MIXED && what == 1 && mode == 1)
                        ? isf_tc_scratch_bytes(nq, c.M) : 0;
-    return rho_region(c, nq) + posbuf_region(c, nq) + extra;
+    return rho_region(c, nq, what, mode) + posbuf_region(c, nq) + extra;
 }
 
 int scatter_host(pgb_ctx* h, const double* q, int nq, int what, int mode, double* out) {
@@ -1031,7 +1033,7 @@ int scatter_host(pgb_ctx* h, const double* q, int nq, int what, int mode, double
     int tc_err = 0;
     if (tc) {
         // the tensor-core pipeline's error word: a bounded wait ran out
-        const char* w = base + off_w + rho_region(c, nq) + posbuf_region(c, nq);
+        const char* w = base + off_w + rho_region(c, nq, what, mode) + posbuf_region(c, nq);
         PGB_CUDA(&c, cudaMemcpyAsync(&tc_err, w + isf_tc_error_offset(nq, c.M), sizeof(int),
                                      cudaMemcpyDeviceToHost, c.stream));
     }

@@ -200,7 +200,7 @@ k_winding(PathView v, unsigned* __restrict__ arrived, double* __restrict__ part,
 
 constexpr int kWindBlocks = 152;
 
-size_t winding_work_bytes() { return (size_t)kWindBlocks * 5 * sizeof(double) + 5 * sizeof(double); }
+size_t winding_work_bytes() { return (size_t)kWindBlocks * 5 * sizeof(double); }
 
 cudaError_t launch_winding(const PathView& v, unsigned* d_arrived, double* d_work, double* d_out5, cudaStream_t s) {
     const size_t nb = (size_t)v.M * v.Ne;
