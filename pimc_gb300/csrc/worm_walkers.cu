@@ -186,7 +186,7 @@ struct WormWalker {
     int* chain;                      // shared: the beads of the current move's range, packed
     float* znorm;                    // shared: a move's normal deviates, 3 (Mbar - 1) at most
     int lane;
-    int team = 1;                    // warps serving this walker (1, 2 or kCtaWarps)
+    int team = 1;                    // warps serving this walker (2, 4 or kCtaWarps; 1 in the check kernel)
     int bar = 1;                     // the team's named barrier
     int wk = 0;                      // this warp's place in the team
     TeamJob* job = nullptr;          // the team's mailbox
@@ -498,9 +498,9 @@ struct WormWalker {
     }
     // One warp's share of a team's range action: the beads chain[c0 + wk],
     // chain[c0 + wk + T], ..., each with all its partners (the next bead of
-    // the share loading meanwhile).  The four warps walk four beads at a
-    // time, so a range costs about a quarter of the dependent load chain of
-    // one warp walking it.  Returns the warp's (double-float) sum; ok false
+    // the share loading meanwhile).  The T warps walk T beads at a time, so a
+    // range costs about a T-th of the dependent load chain of one warp walking
+    // it.  Returns the warp's (double-float) sum; ok false
     // for a locator outside the walker's arrays.  With `part` set each bead
     // is reduced on its own and lane 0 writes it to part[i] (the per-bead
     // actions of a worm move).
@@ -550,13 +550,13 @@ struct WormWalker {
         return __shfl_sync(0xffffffffu, s, 0);
     }
     // potentialAction over chain[c0 .. c0 + cnt - 1]: the lanes keep one
-    // running sum over the whole range and reduce once (a team: each warp
-    // over its share of the partners)
+    // running sum over the whole range and reduce once, each of the team's
+    // warps over its share of the beads
     __device__ __noinline__ double chainAction(int c0, int cnt) {
         // short ranges (a single bead's action in the worm moves) stay on
         // warp 0: the team's two barriers and mailbox cost more than the
         // few pair terms a lane would give away
-        if (team > 1 && cnt >= kTeamMinBeads) {
+        if (cnt >= kTeamMinBeads) {
             teamPost(1, c0, cnt);
             bool ok = true;
             const float2 mine = teamShare(pairCtx(), chain, c0, cnt, 0, team, ok, nullptr);
@@ -576,7 +576,7 @@ struct WormWalker {
     // the reference's order.  A bead's value equals bare() of that bead; the
     // next bead's loads are in flight while a bead's terms are summed.
     __device__ __noinline__ void beadActions(int c0, int cnt, double* out) {
-        if (team > 1 && cnt >= kTeamMinBeads && cnt <= kRunCap) {
+        if (cnt >= kTeamMinBeads) {
             teamPost(3, c0, cnt);
             bool ok = true;
             teamShare(pairCtx(), chain, c0, cnt, 0, team, ok, tpart);
@@ -1197,11 +1197,10 @@ struct WormWalker {
     // draws, the same distribution.
 
     // A run's actions are evaluated a chunk at a time once the tests reach it:
-    // the first chunk one bead (kTeamMinBeads for a team), each next one
-    // twice as long, so that a run rejected at its first beads costs about
-    // what the sequential form costs and a long accepted run is evaluated in
-    // a few batches
-    __device__ int firstChunk() const { return team > 1 ? kTeamMinBeads : 1; }
+    // the first chunk kTeamMinBeads, each next one twice as long, kRunCap at
+    // most, so that a run rejected at its first beads costs about what the
+    // sequential form costs and a long accepted run is evaluated in a few
+    // batches
     // the Metropolis tests of beads from .. to - 1 of a run whose last bead
     // is `last`: rand() < exp(sign (U_k - f_k shift)), sign = -1 for an
     // insertion and 1 for a removal, f = 1/2 at both ends and 1 between, made
@@ -1243,7 +1242,7 @@ struct WormWalker {
     // the tests of beads 0 .. total - 1, each chunk's actions evaluated when
     // the tests reach it
     __device__ __noinline__ bool runTests(int total, int last, float sign, double actionShift) {
-        int chunk = firstChunk();
+        int chunk = kTeamMinBeads;
 #pragma unroll 1
         for (int ev = 0; ev < total;) {
             const int n = min(chunk, total - ev);
@@ -1691,27 +1690,20 @@ struct WormWalker {
     // the sums of the primitive energy over slices [t0, t1): the pair
     // potential of every slice (row i against the partners j > i, four
     // partners a lane at a time without branches) and every bead's squared
-    // link to the next slice
-    // (a team: warp wk sums the slices t0 + wk, t0 + wk + T, ..., and warp 0
-    // adds the warps' sums in warp order)
-    // (half of a team's warps: eight slices at a time leave no more work, and
-    // the FP32 sums of a slice keep the order they had)
+    // link to the next slice.  Half of the team's warps take the slices in
+    // turn (eight slices at a time leave no more work, and the FP32 sums of a
+    // slice keep the order they had); warp 0 adds their sums
     __device__ static int energyWarps(int team) { return (team + 1) / 2; }
     __device__ __noinline__ double2 energySums(int t0, int t1) {
-        if (team > 1) {
-            teamPost(2, t0, t1);
-            float2 p, k;
-            energyShare(pairCtx(), nxt, t0, t1, energyWarps(team), p, k);
-            if (lane == 0) { job->hi[0] = p.x; job->lo[0] = p.y; job->khi[0] = k.x; job->klo[0] = k.y; }
-            team_sync(bar, 32 * team);
-            const bool in = lane < energyWarps(team);
-            const double pot = sumShares(in ? job->hi[lane] : 0.f, in ? job->lo[lane] : 0.f);
-            const double kin = sumShares(in ? job->khi[lane] : 0.f, in ? job->klo[lane] : 0.f);
-            return make_double2(pot, kin);
-        }
+        teamPost(2, t0, t1);
         float2 p, k;
-        energyShare(pairCtx(), nxt, t0, t1, 1, p, k);
-        return make_double2((double)p.x + (double)p.y, (double)k.x + (double)k.y);
+        energyShare(pairCtx(), nxt, t0, t1, energyWarps(team), p, k);
+        if (lane == 0) { job->hi[0] = p.x; job->lo[0] = p.y; job->khi[0] = k.x; job->klo[0] = k.y; }
+        team_sync(bar, 32 * team);
+        const bool in = lane < energyWarps(team);
+        const double pot = sumShares(in ? job->hi[lane] : 0.f, in ? job->lo[lane] : 0.f);
+        const double kin = sumShares(in ? job->khi[lane] : 0.f, in ? job->klo[lane] : 0.f);
+        return make_double2(pot, kin);
     }
     // the energy sums of slices t0, t0 + step, ... below t1 by one warp:
     // (pot, kin) as double-float pairs
@@ -1771,8 +1763,7 @@ struct WormWalker {
 };
 
 
-// One walker's launch: run by the single warp of a small walker, or by warp 0
-// of a team (team > 1, job the team's mailbox).  limit[w] caps the walker's
+// One walker's launch: run by warp 0 of its team (job the team's mailbox).  limit[w] caps the walker's
 // completed sweeps; with budget_ns > 0 a walker stops between two moves (the
 // clock read before each) once that much device time has passed, and the
 // next launch resumes the sweep there.
