@@ -478,12 +478,27 @@ k_bead_warp64(PathView v, double invdr, const int2* __restrict__ beads, int k, B
     }
 }
 
-// From here on the warp form is the faster; below, it leaves warps idle, and a
-// GSF call needs the forces of all slices first.  Whole calls, clusters against
-// warps: primitive, 64 beads a slice, 1824 beads 45 and 46 us, 2432 63 and 54
-// (128 beads a slice: 50 and 59, 63 and 68, 4864 105 and 79); GSF, 608 beads 89
-// and 83 us, 912 98 and 84 (269 and 290, 280 and 292, 1216 349 and 292).
-constexpr int kManyBeads = 2048, kManyGradient = 912;
+// From here on the warp form is the faster; below, it leaves warps idle.  Whole
+// calls, clusters against warps, without a gradient term: 64 beads a slice, 1824
+// beads 45 and 46 us, 2432 63 and 54 (128 beads a slice: 50 and 59, 63 and 68,
+// 4864 105 and 79).  With one the warp form makes the forces of all slices
+// first, M n^2 pairs on few CTAs while M is small, and a cluster n^2 / 2 pairs a
+// bead, which fill the SMs from about 10^5 / n beads on.  GSF, whole calls, n
+// beads a slice, M slices, clusters and warps in us:
+//   n = 16   M = 62: 496 beads 31 and 44; M = 1000: 1000 42 and 56, 3000 79 and 66
+//   n = 64   M = 62: 248 55 and 81, 496 89 and 82; M = 124: 372 72 and 81, 496 88
+//            and 82; M = 500: 1500 139 and 165, 2000 174 and 166; M = 1000: 2000
+//            173 and 166
+//   n = 128  M = 124: 248 145 and 182, 372 206 and 182; M = 250: 1000 283 and 291,
+//            1500 412 and 291; M = 500: 1000 285 and 292, 1500 411 and 292
+//   n = 256  M = 62: 124 269 and 333, 186 503 and 334; M = 250: 250 505 and 549,
+//            500 987 and 551
+constexpr int kManyBeads = 2048;
+static double many_gradient(const PathView& v) {
+    const double n = v.Ne, slices = std::max(v.M * std::min(4.0, 640.0 / n), 2.5e4 / n);
+    return std::min(std::min(2048.0, slices), std::min(1.24e5 / n, 1.8e7 / (n * n)));
+}
+
 
 template <bool kBoth>
 static cudaError_t bead_pairs64(const PathView& v, const int2* d_beads, int k, const BeadSpec& a, bool corr,
@@ -631,7 +646,7 @@ static bool has_corr(int shift, int mode, const double gf[2]) {
 static bool bead_warp64(const PathView& v, const int2* d_beads, int k, const BeadSpec& a, bool corr,
                         const double* d_over, double* d_force, double* d_out, cudaStream_t s, cudaError_t* e) {
     const size_t fsmem = (size_t)v.Ne * (3 * sizeof(double) + 3 * sizeof(float));
-    if (k < (corr ? kManyGradient : kManyBeads) || (corr && (!d_force || fsmem > 200 * 1024))) return false;
+    if (k < (corr ? many_gradient(v) : kManyBeads) || (corr && (!d_force || fsmem > 200 * 1024))) return false;
     if (corr) {
         if ((*e = set_smem_limit(k_slice_forces64, 200 * 1024)) != cudaSuccess) return true;
         k_slice_forces64<<<dim3(v.M, (v.Ne + kForceRows - 1) / kForceRows), kPairBlock, fsmem, s>>>(

@@ -163,8 +163,8 @@ cudaError_t launch_potential_batch64(const PathView& v, const double* d_sep,
                                      double* d_out, int n, int what,
                                      cudaStream_t s);
 // `whole`: the cutoff takes in every separation, so a bead's list is its whole
-// slice; d_force: room for the FP64 slice forces [M][3][Ne], needed from
-// kManyGradient beads on with a gradient term
+// slice; d_force: room for the FP64 slice forces [M][3][Ne], needed by the
+// many-bead form of an action with a gradient term
 cudaError_t launch_bead_actions64(const PathView& v, const int2* d_beads, int k,
                                   int shift, int mode, double tau, double lambda,
                                   const double vf[2], const double gf[2],
