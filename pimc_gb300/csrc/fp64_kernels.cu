@@ -953,12 +953,14 @@ constexpr int kRhoPowers = 64;                   // largest |n_d| of the table f
 constexpr int kRhoSmem = 48 * 1024;              // four CTAs an SM
 constexpr int kRhoCluster = 8;
 constexpr int kRhoBeads = 3;                     // a CTA has at least
-// Fewer vectors than kRhoFew, or fewer slices than kRhoShort, take a warp a
-// vector and slice: a CTA a slice and cluster rank leaves the GPU empty there.
+// Fewer vectors than kRhoFew, or fewer slices than kRhoShort and CTAs (a slice
+// and set of vectors each) than three times that, take a warp a vector and
+// slice: a CTA a slice and cluster rank leaves the GPU empty there.
 // S(q) in this form and the other, us: 65 beads, 250 slices, 1 vector 17 and 34,
 // 16 40 and 40, 24 48 and 50, 32 62 and 55; 64 beads, 124 slices, 16 19 and 22,
 // 24 25 and 25, 32 30 and 29.  S(q) and F(q,tau) of 24 beads, 16 slices, 400
-// vectors 60 and 74 (lattice), 60 and 209 (others).
+// vectors 60 and 74 (lattice), 60 and 209 (others); of 5 beads, 20 slices, 4000
+// lattice vectors 267 and 97.
 constexpr int kRhoFew = 24, kRhoShort = 32;
 // FP64 instructions that a table saves a vector and bead, and that it takes an entry
 constexpr int kRhoSaved = 18, kRhoEntry = 24;
@@ -1146,13 +1148,14 @@ k_rhoq64(PathView v, const double* __restrict__ q, int nq, Lattice lat, double m
 cudaError_t launch_rhoq64(const PathView& v, const double* d_q, int nq, double* d_rho,
                           cudaStream_t s, double maxR2) {
     if (nq < 1) return cudaSuccess;
-    if (nq < kRhoFew || v.M < kRhoShort) {
+    const int sets = (nq + kRhoThreads - 1) / kRhoThreads;
+    if (nq < kRhoFew || (v.M < kRhoShort && v.M * sets < 3 * kRhoShort)) {
         k_rhoq64_few<<<(int)(((long long)nq * v.M + 7) / 8), 256, 0, s>>>(v, d_q, nq, maxR2, d_rho);
         return cudaGetLastError();
     }
     const cudaError_t ae = set_smem_limit(k_rhoq64, kRhoSmem);
     if (ae != cudaSuccess) return ae;
-    const int sets = (nq + kRhoThreads - 1) / kRhoThreads, each = (nq + sets - 1) / sets;
+    const int each = (nq + sets - 1) / sets;
     const int wide = each, parts = std::max(1, kRhoLeast / wide);
     // rounds of the SMs, in units of a whole slice: a cluster costs two
     // barriers and a table each, so it has to gain (124 slices of 64 beads, one

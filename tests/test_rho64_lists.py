@@ -49,3 +49,18 @@ def test_lists(pgb, n, m):
             continue
         z = ((np.cos(ph) * inside).sum(-1) ** 2 + (np.sin(ph) * inside).sum(-1) ** 2).sum(1) / m
         assert np.all(np.abs(a.ssf_cylinder(q, 3.0)[0] - z) <= 3 * n * tol[:, 0, 0]), name
+
+
+@pytest.mark.parametrize("n,m,nq", [(5, 8, 4609), (9, 31, 1200), (24, 24, 1500), (40, 31, 1663)])
+def test_many_vectors_of_short_paths(pgb, n, m, nq):
+    """Both forms of a short path: many vectors on the lattice, a few off it."""
+    L = 2.9 * n ** (1.0 / 3.0)
+    rng = np.random.default_rng(nq)
+    cfg = pgb.worldlines.seeded_worldlines(n, m, L, 6.0596, 0.004, n)
+    a = pgb.Action(L, m, n, 0.004, 6.0596)
+    a.load(cfg)
+    q = (2 * np.pi / L) * rng.integers(-9, 10, (nq, 3))
+    q[::97] = rng.normal(0, 2.0, (len(q[::97]), 3))
+    for part in (q, q[:400]):
+        part = np.ascontiguousarray(part)
+        assert np.all(np.abs(a.rhoq(part) - exact(cfg["pos"], part)[1]) <= bound(cfg["pos"], part))
