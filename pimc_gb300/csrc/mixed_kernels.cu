@@ -405,8 +405,8 @@ cudaError_t launch_bead_actions32_full(const PathView& v, AzizParams a, const in
 // Bound: the issue rate, 47 instructions a pair (79 with the gradient), and
 // instruction fetch: the loops of both parities and the reductions together
 // are larger than the instruction caches, so the even slices' beads go first
-// and the reductions are not inlined (1.01 -> 0.87 ms).  10^6 trials, N = 256,
-// M = 250, GSF: 2.75 ms with both positions evaluated for every trial, 0.87 ms
+// and the reductions are not inlined (1.01 -> 0.87 ms at the time).  10^6 trials, N = 256,
+// M = 250, GSF: 2.75 ms with both positions evaluated for every trial, 0.81 ms
 // here.
 //
 // A run is as long as two average beads' trials and 16 more, so that evenly
@@ -422,7 +422,7 @@ constexpr int kTrialWarps = 4;
 constexpr int kTrialRun = 32;                    // trials in a run at least, and their step
 // Sorting pays from about three trials a bead on (N = 256, gradient: 2 a bead
 // 306 against 374 us, 4 a bead 398 against 719; N = 400: 2 a bead 227 against
-// 220, 4 a bead 282 against 395) once its three small launches, 12 us, are
+// 220, 4 a bead 282 against 395) once its small launches, 12 to 15 us, are
 // less than the pairs saved (N = 64: 4 a bead, 32 k trials 58 against 54 us, 16
 // a bead 92 against 168; N = 16: 8 k trials 34 against 19).
 constexpr double kTrialsPerBead = 3.0;
