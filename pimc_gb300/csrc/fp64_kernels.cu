@@ -499,7 +499,6 @@ static double many_gradient(const PathView& v) {
     return std::min(std::min(2048.0, slices), std::min(1.24e5 / n, 1.8e7 / (n * n)));
 }
 
-
 template <bool kBoth>
 static cudaError_t bead_pairs64(const PathView& v, const int2* d_beads, int k, const BeadSpec& a, bool corr,
                                 const double* d_over, double* d_out, cudaStream_t s) {

@@ -396,18 +396,19 @@ cudaError_t launch_bead_actions32_full(const PathView& v, AzizParams a, const in
 // action and, for the gradient term, every partner's force less the bead's
 // own term: the same for all trials of the bead.  The trials are sorted by
 // bead on the device (count, offsets, scatter: the sorted record is the FP32
-// position and the trial's index), a warp takes a bead and a run of its trials, evaluates its current position once, keeps the partners (and
-// those forces) in shared memory and then makes the trials four at a time, so four independent chains of pair
-// arithmetic are in flight.  The sums of a group are reduced together by
+// position and the trial's index), a warp takes a bead and a run of its
+// trials, evaluates its current position once, keeps the partners (and those
+// forces) in shared memory and then makes the trials four at a time, so four
+// independent chains of pair arithmetic are in flight.  The sums of a group are reduced together by
 // recursive halving, in the butterfly's own tree, so every sum has the bits
 // k_bead_actions32_full gives it; the FP64 assembly runs one trial a lane.
 //
 // Bound: the issue rate, 47 instructions a pair (79 with the gradient), and
 // instruction fetch: the loops of both parities and the reductions together
 // are larger than the instruction caches, so the even slices' beads go first
-// and the reductions are not inlined (1.01 -> 0.87 ms at the time).  10^6 trials, N = 256,
-// M = 250, GSF: 2.75 ms with both positions evaluated for every trial, 0.81 ms
-// here.
+// and the reductions are not inlined (1.01 -> 0.87 ms at the time).  10^6
+// trials, N = 256, M = 250, GSF: 2.75 ms with both positions evaluated for every
+// trial, 0.81 ms here.
 //
 // A run is as long as two average beads' trials and 16 more, so that evenly
 // spread trials stay whole.  A second launch makes the trials of a bead
